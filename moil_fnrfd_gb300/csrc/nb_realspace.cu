@@ -11,8 +11,9 @@
 //   primary vs image: a pair whose minimum-image shift is zero is a primary-box pair
 //                 (e_vdw/e_el); any other shift is one of MOIL's translated images
 //                 (e_vsym/e_lsym).
-// Lists are full (each pair appears under both atoms); every lane owns its own gradient,
-// so nothing is written twice and no atomics are needed.  Energies are halved at the end.
+// Lists are full (each pair appears under both atoms); a water or atom owns its own gradient,
+// so nothing is written twice and no atomics are needed, except where a kernel evaluates each
+// water pair once (k_water_h, k_water_d).  Energies are halved at the end.
 #include "nb_internal.h"
 
 namespace {
@@ -122,13 +123,14 @@ __device__ __forceinline__ void flush(double g[], long long G[], int n)
     }
 }
 
-// water sites of molecule i against its W2 list of non-water atoms: atom semantics per site
-// pair; partial gradients and energies go to g / e4, flushed every CHUNK entries
+// water sites of molecule i against its W2 list of non-water atoms (entries first, first +
+// stride, ...): atom semantics per site pair; partial gradients and energies go to g / e4,
+// flushed every CHUNK entries
 template <typename T, typename Flush>
 __device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const typename vec4<T>::type *pos,
                                                const void *lj_v, const unsigned *__restrict__ sflags,
                                                const int *__restrict__ wl2_off, const int *__restrict__ wl2, int cap2,
-                                               T g[9], T e4[4], int &npair, Flush &flush_all)
+                                               int first, int stride, T g[9], T e4[4], int &npair, Flush &flush_all)
 {
     typedef typename vec4<T>::type T4;
     typedef typename cplx<T>::type T2;
@@ -141,7 +143,7 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const typ
     const T2 lji[3] = {lj[3 * i], lj[3 * i + 1], lj[3 * i + 2]};
     const unsigned fi[3] = {sflags[3 * i], sflags[3 * i + 1], sflags[3 * i + 2]};
     int cnt = 0;
-    for (int k = q0; k < q1; ++k) {
+    for (int k = q0 + first; k < q1; k += stride) {
         nb_prefetch_l1(wl2 + min(k + 32, q1 - 1));
         int s = wl2[k];
         T4 xj = pos[s];
@@ -195,122 +197,155 @@ struct W1Row {
     __device__ int at(int v) const { return base + (int)*addr(v); }
 };
 
-// Plain FP64 path: one water per thread in blocks of WBLOCK64 (the FP64 pipe of this GPU is a
-// small fraction of the FP32 one, so a replica of a few hundred waters needs every
-// multiprocessor it can get: 32-thread blocks spread it over four times more SMs than 128)
-#define WBLOCK64 32
-template <typename T, typename E>
-__global__ void __launch_bounds__(WBLOCK64) k_water(int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
-                                                     const void *pos_v, const void *woff_v, const void *lj_v,
-                                                     const unsigned *__restrict__ sflags,
-                                                     const int2 *__restrict__ wl1_cnt, const void *__restrict__ wl1,
-                                                     int cap_row, const int *__restrict__ wl2_off,
-                                                     const int *__restrict__ wl2, int cap2, long long *__restrict__ grad,
-                                                     double *__restrict__ e_unit)
+// Sum over the W lanes of a subgroup (W a power of two, all lanes of the warp present).
+template <int W> __device__ __forceinline__ long long sub_sum(long long v)
 {
-    __shared__ long long sG[9][WBLOCK64];
-    __shared__ double sE[6][WBLOCK64];
-    const int t = threadIdx.x;
-    int i = blockIdx.x * WBLOCK64 + t;
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, W);
+    return v;
+}
+template <int W> __device__ __forceinline__ int sub_sum(int v)
+{
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, W);
+    return v;
+}
+template <int W> __device__ __forceinline__ double sub_sum(double v)
+{
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, W);
+    return v;
+}
+
+// Plain FP64 path: one warp per water.  Bound: the FP64 pipe (two lanes per clock and SM), about
+// 120 FP64 instructions per site pair, so every molecule pair is evaluated once, by its owner
+// (nb_half_owner on the full rows), and a warp's 32 lanes share one water's pairs: the owned
+// in-cutoff entries are compacted into shared memory (their image-shifted O-O vectors with
+// them), and the lanes take (partner site, entry) items, three site pairs each, so about 50
+// entries fill five rounds of 32 items.  Gradients of both sides go to the int64 site gradient
+// (cleared before the launch) with atomics: integer sums, independent of their order.  erfc(x) is
+// exp(-x^2) erfcx(x), one exponential for the energy and the force.  A whole evaluation: 216
+// waters 3258 -> 226 us, 1,334 waters 3867 -> 485 us (before: one water per thread, full lists).
+#define WARPS64 2
+#define WBUF64 96
+template <typename E>
+__global__ void __launch_bounds__(32 * WARPS64) k_water_d(int nW, const RepDev *__restrict__ reps,
+                                                          const int *__restrict__ site_rep,
+                                                          const double4 *__restrict__ pos,
+                                                          const double4 *__restrict__ woff, const void *lj_v,
+                                                          const unsigned *__restrict__ sflags,
+                                                          const int2 *__restrict__ wl1_cnt,
+                                                          const void *__restrict__ wl1, int cap_row,
+                                                          const int *__restrict__ wl2_off,
+                                                          const int *__restrict__ wl2, int cap2,
+                                                          unsigned long long *__restrict__ grad,
+                                                          double *__restrict__ e_unit)
+{
+    __shared__ double sD[WARPS64][3][WBUF64];
+    __shared__ int sJ[WARPS64][WBUF64];      // partner, negative (~partner) for an image pair
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * WARPS64 + warp;
     if (i >= nW) return;
-    typedef typename vec4<T>::type T4;
-    typedef typename cplx<T>::type T2;
-    const T4 *pos = (const T4 *)pos_v;
-    const T4 *woff = (const T4 *)woff_v;
+    double (*D)[WBUF64] = sD[warp];
+    int *J = sJ[warp];
     const RepDev &R = reps[site_rep[3 * i]];
+    const double4 oi0 = pos[3 * i], oi1 = woff[3 * i + 1], oi2 = woff[3 * i + 2];
+    const double hi[2][3] = {{oi1.x, oi1.y, oi1.z}, {oi2.x, oi2.y, oi2.z}};
+    double g[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) sG[k][t] = 0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) sE[k][t] = 0.0;
-    const T4 oi0 = pos[3 * i];
-    // i-site offsets from O (a = 0 is O itself)
-    const T4 oi1 = woff[3 * i + 1], oi2 = woff[3 * i + 2];
-    const T oi[3][3] = {{(T)0, (T)0, (T)0}, {oi1.x, oi1.y, oi1.z}, {oi2.x, oi2.y, oi2.z}};
-    T g[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) g[k] = 0;
-    T e4[6] = {0, 0, 0, 0, 0, 0};   // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
-    auto flush_all = [&]() {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) { sG[k][t] += nb_fix(g[k]); g[k] = 0; }
-#pragma unroll
-        for (int k = 0; k < 6; ++k) { sE[k][t] += (double)e4[k]; e4[k] = 0; }
-    };
+    for (int k = 0; k < 9; ++k) g[k] = 0.0;
+    double e4[6] = {0, 0, 0, 0, 0, 0};   // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
     int npair = 0;
-    const T iL0 = rep_invL<T>(R, 0), iL1 = rep_invL<T>(R, 1), iL2 = rep_invL<T>(R, 2);
-    const T rmax2 = (T)R.rmax2, rv2 = (T)R.rv2, alpha = Consts<T>::alpha(R), ex2c = (T)R.ex2c, c2a = (T)R.c2a;
-    const T qOO = Consts<T>::qq(R, 0), qOH = Consts<T>::qq(R, 1), qHH = Consts<T>::qq(R, 2);
-    const T w12 = Consts<T>::w12(R), w6 = Consts<T>::w6(R);
+    const double rmax2 = (double)R.rmax2, rv2 = (double)R.rv2, alpha = R.alphad, c2a = (double)R.c2a;
+    const double qOO = R.qqd[0], qOH = R.qqd[1], qHH = R.qqd[2], w12 = R.w12d, w6 = R.w6d;
     const W1Row<E> L1(wl1_cnt, wl1, cap_row, i, R.wat0);
-    int cnt = 0;
-    // software pipeline: the next entry's index and oxygen are loaded one iteration ahead
-    int jn = L1.n > 0 ? L1.at(0) : 0;
-    T4 ojn = pos[3 * jn];
-    for (int k = 0; k < L1.n; ++k) {
-        const int j = jn;
-        const T4 oj = ojn;
-        if (k + 1 < L1.n) {
-            jn = L1.at(k + 1);
-            ojn = pos[3 * jn];
-        }
-        T dx = oi0.x - oj.x, dy = oi0.y - oj.y, dz = oi0.z - oj.z;
-        T nx = nb_rint(dx * iL0), ny = nb_rint(dy * iL1), nz = nb_rint(dz * iL2);
-        dx = nb_shift(R, 0, dx, nx);
-        dy = nb_shift(R, 1, dy, ny);
-        dz = nb_shift(R, 2, dz, nz);
-        T r2oo = dx * dx + dy * dy + dz * dz;
-        if (r2oo <= rmax2) {
-            T4 oj1 = woff[3 * j + 1], oj2 = woff[3 * j + 2];
-            // q[b] = (O_i - O_j - nL) - offset_j[b]; site displacement = offset_i[a] + q[b]
-            const T q[3][3] = {{dx, dy, dz}, {dx - oj1.x, dy - oj1.y, dz - oj1.z}, {dx - oj2.x, dy - oj2.y, dz - oj2.z}};
-            T e_el = 0, e_lj = 0, v_lj = 0;
+    // the buffered entries: items b-major, so a round's lanes share a partner site (almost)
+    auto work_off = [&](int cnt) {
+        __syncwarp();
+        for (int it = lane; it < 3 * cnt; it += 32) {
+            const int b = it >= 2 * cnt ? 2 : (it >= cnt ? 1 : 0), e = it - b * cnt;
+            const int jj = J[e];
+            const bool img = jj < 0;
+            const int j = img ? ~jj : jj;
+            double q[3] = {D[0][e], D[1][e], D[2][e]};
+            if (b) {
+                const double4 oj = woff[3 * (size_t)j + b];
+                q[0] -= oj.x; q[1] -= oj.y; q[2] -= oj.z;
+            }
+            double H[3] = {0.0, 0.0, 0.0}, e_el = 0.0;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    T ddx = a ? oi[a][0] + q[b][0] : q[b][0];
-                    T ddy = a ? oi[a][1] + q[b][1] : q[b][1];
-                    T ddz = a ? oi[a][2] + q[b][2] : q[b][2];
-                    T rr2 = ddx * ddx + ddy * ddy + ddz * ddz;
-                    T rinv = nb_rsqrt(rr2);
-                    T s2 = rinv * rinv;
-                    T x = alpha * rr2 * rinv;
-                    T ex;
-                    T erfcv = nb_erfc_ex(x, rr2 * ex2c, &ex);
-                    const T qq = (a == 0 && b == 0) ? qOO : ((a == 0 || b == 0) ? qOH : qHH);
-                    T e = qq * erfcv * rinv;
-                    T df = -(e + qq * c2a * ex) * s2;
-                    if (a == 0 && b == 0) {
-                        if (rr2 <= rv2) {
-                            T s6 = s2 * s2 * s2, A = w12 * s6 * s6, B = w6 * s6;
-                            T e1 = A - B, df1 = (T)-6 * s2 * (A + e1);
-                            lj_switch_apply<T>(R, rr2, e1, df1);
-                            e_lj += e1;
-                            v_lj -= df1 * rr2;   // watwat_ewald_press.f:146-152
-                            df += df1;
-                        }
-                    }
-                    e_el += e;
-                    g[3 * a] += df * ddx;
-                    g[3 * a + 1] += df * ddy;
-                    g[3 * a + 2] += df * ddz;
+                const double dx = a ? hi[a - 1][0] + q[0] : q[0], dy = a ? hi[a - 1][1] + q[1] : q[1],
+                             dz = a ? hi[a - 1][2] + q[2] : q[2];
+                const double rr2 = dx * dx + dy * dy + dz * dz, rinv = rsqrt(rr2), s2 = rinv * rinv;
+                const double x = alpha * rr2 * rinv, ex = exp(-x * x);
+                const double qq = a == 0 ? (b == 0 ? qOO : qOH) : (b == 0 ? qOH : qHH);
+                const double ee = qq * (ex * erfcx(x)) * rinv;
+                double df = -(ee + qq * c2a * ex) * s2;
+                if (a == 0 && b == 0 && rr2 <= rv2) {
+                    const double s6 = s2 * s2 * s2, A = w12 * s6 * s6, B = w6 * s6;
+                    double e1 = A - B, df1 = -6.0 * s2 * (A + e1);
+                    lj_switch_apply<double>(R, rr2, e1, df1);
+                    e4[img ? 1 : 0] += e1;
+                    e4[img ? 5 : 4] -= df1 * rr2;   // watwat_ewald_press.f:146-152
+                    df += df1;
                 }
+                e_el += ee;
+                g[3 * a] += df * dx; g[3 * a + 1] += df * dy; g[3 * a + 2] += df * dz;
+                H[0] -= df * dx; H[1] -= df * dy; H[2] -= df * dz;
             }
-            const bool img = (nx != (T)0) | (ny != (T)0) | (nz != (T)0);
-            e4[img ? 1 : 0] += e_lj;
             e4[img ? 3 : 2] += e_el;
-            e4[img ? 5 : 4] += v_lj;
-            npair += 9;
-        }
-        if (++cnt == CHUNK) { flush_all(); cnt = 0; }
-    }
-    flush_all();
-    water_vs_atoms<T>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, g, e4, npair, flush_all);
+            unsigned long long *gj = grad + 9 * (size_t)j + 3 * b;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) grad[(size_t)9 * i + k] = sG[k][t];
-    double *eu = e_unit + NB_EU * (size_t)i;
-    eu[0] = sE[0][t]; eu[1] = sE[1][t]; eu[2] = sE[2][t]; eu[3] = sE[3][t]; eu[4] = (double)npair;
-    eu[5] = 0.0; eu[6] = sE[4][t]; eu[7] = sE[5][t];
+            for (int d = 0; d < 3; ++d) atomicAdd(gj + d, (unsigned long long)nb_fix(H[d]));
+        }
+        __syncwarp();
+    };
+    const int il = i - R.wat0;
+    int cnt = 0;
+    for (int k0 = 0; k0 < L1.n; k0 += 32) {
+        const int k = k0 + lane;
+        bool in = false, img = false;
+        double dx = 0.0, dy = 0.0, dz = 0.0;
+        int j = 0;
+        if (k < L1.n) {
+            j = L1.at(k);
+            if (nb_half_owner(il, j - R.wat0) == il) {
+                const double4 oj = pos[3 * (size_t)j];
+                dx = oi0.x - oj.x; dy = oi0.y - oj.y; dz = oi0.z - oj.z;
+                min_image<double>(R, dx, dy, dz, img);
+                in = dx * dx + dy * dy + dz * dz <= rmax2;
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (cnt + __popc(m) > WBUF64) { work_off(cnt); cnt = 0; }
+        if (in) {
+            const int p = cnt + __popc(m & ((1u << lane) - 1u));
+            D[0][p] = dx; D[1][p] = dy; D[2][p] = dz;
+            J[p] = img ? ~j : j;
+        }
+        cnt += __popc(m);
+        npair += in ? 18 : 0;
+    }
+    work_off(cnt);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) e4[k] *= 2.0;   // each pair once; the energy reduction halves
+    // water sites against non-water atoms (W2, full list): a lane's share of the entries
+    auto none = []() {};
+    water_vs_atoms<double>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, lane, 32, g, e4, npair, none);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const long long v = sub_sum<32>(nb_fix(g[k]));
+        if (lane == k) atomicAdd(grad + 9 * (size_t)i + k, (unsigned long long)v);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) e4[k] = sub_sum<32>(e4[k]);
+    npair = sub_sum<32>(npair);
+    if (lane == 0) {
+        double *eu = e_unit + NB_EU * (size_t)i;
+        eu[0] = e4[0]; eu[1] = e4[1]; eu[2] = e4[2]; eu[3] = e4[3]; eu[4] = (double)npair;
+        eu[5] = 0.0; eu[6] = e4[4]; eu[7] = e4[5];
+    }
 }
 
 // FP32 water exclusion corrections (cdie_ewald.f:117-199 for the pairs O-H1, O-H2, H1-H2 of
@@ -565,7 +600,7 @@ __global__ void __launch_bounds__(WBLOCK, 4) k_water_f(int nW, const RepDev *__r
         if (cnt >= CHUNK) { flush_all(); cnt = 0; }
     }
     flush_all();
-    water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, g, e4, npair, flush_all);
+    water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, g, e4, npair, flush_all);
 #pragma unroll
     for (int k = 0; k < 9; ++k) grad[(size_t)9 * i + k] = sG[k][t];
     double *eu = e_unit + NB_EU * (size_t)i;
@@ -823,7 +858,7 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
             if (cnt >= CHUNK) { flush(2.f); cnt = 0; }
         }
         flush(2.f);
-        water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, g, e4, npair, flush1);
+        water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, g, e4, npair, flush1);
 #pragma unroll
         for (int k = 0; k < 4; ++k) eu[k] = (double)sE[k][t].x + (double)sE[k][t].y;
         eu[4] = (double)npair;
@@ -1196,11 +1231,15 @@ void realspace_t(NbCtx *c)
                 (int)c->nW, c->d_reps, c->d_site_rep, (const float4 *)c->d_pos, (const float4 *)c->d_woff,
                 c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2,
                 cap_int(c->cap_wl2), c->d_grad_site, c->d_e_unit, c->water_excl_fast);
-        else
-            (c->row16 ? k_water<T, unsigned short> : k_water<T, int>)<<<(int)((c->nW + WBLOCK64 - 1) / WBLOCK64), WBLOCK64, 0, s>>>((int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_woff,
-                                             c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1,
-                                             c->d_wl2_off, c->d_wl2, cap_int(c->cap_wl2), c->d_grad_site,
-                                             c->d_e_unit);
+        else {
+            // both sides of every pair are added with atomics: the waters' gradient starts at zero
+            cudaMemsetAsync(c->d_grad_site, 0, sizeof(long long) * 9 * (size_t)c->nW, s);
+            (c->row16 ? k_water_d<unsigned short> : k_water_d<int>)<<<(int)((c->nW + WARPS64 - 1) / WARPS64),
+                                                                      32 * WARPS64, 0, s>>>(
+                (int)c->nW, c->d_reps, c->d_site_rep, (const double4 *)c->d_pos, (const double4 *)c->d_woff,
+                c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2,
+                cap_int(c->cap_wl2), (unsigned long long *)c->d_grad_site, c->d_e_unit);
+        }
         c->launches++;
     }
     if (c->timing) cudaEventRecord(c->ev[3], s);
