@@ -44,10 +44,10 @@ F_PAIR = 50            # FP32 operations per in-cutoff site pair (FMA = 2, MUFU 
 LIST_PERIOD = 10
 SKIN = 1.0
 # DRAM bytes per water molecule of one water-kernel launch (ncu dram__bytes_read.sum +
-# dram__bytes_write.sum, 48-replica captures over 74,171 waters): k_water_f (full lists)
+# dram__bytes_write.sum, 48-replica captures over 74,171 waters): full lists (one water per thread)
 # 37.44 MB, k_water_h (half lists, 256-water blocks) 38.48 MB
 WATER_KERNEL_DRAM_BYTES_PER_WATER = {1: 504.9, 2: 518.8}
-WATER_KERNEL_NAME = {1: "k_water_f (full lists)", 2: "k_water_h (half lists)"}
+WATER_KERNEL_NAME = {1: "k_water_s (full lists)", 2: "k_water_h (half lists)"}
 # DRAM bytes per atom of one evaluation's PME kernels (k_pme_bin, k_plane_fwd_f, k_zconv_f,
 # k_plane_inv_f, k_pme_gather_f: 5.37 + 4.55 + 10.86 + 10.82 + 15.00 MB, 48-replica capture over
 # 222,513 atoms, caches flushed before each launch, so an upper bound)

@@ -209,6 +209,13 @@ int alloc_half(NbCtx *c)
     return MOIL_NB_OK;
 }
 
+// The automatic shape takes full lists up to this many waters (of the whole handle): a block
+// of 256 waters per multiprocessor leaves most of the GPU idle below it, while the full-list
+// kernel spreads each water over 8 or 32 lanes.  One evaluation in us, half / full lists:
+// 216 waters 116 / 98, 3,000 154 / 126, 12,000 210 / 177, 19,272 (24 replicas) 167 / 145,
+// 20,000 (one box) 200 / 214, 32,000 248 / 264.
+#define NB_FULL_MAX_WATERS 19500
+
 // Half-list set-up for the current shape: on for FP32 handles whose replicas all have fewer
 // than 65,536 waters (16-bit rows) unless full lists were asked for; blocks of hb waters
 // never straddle replicas.  Capacities start from the full rows and the replica sizes and
@@ -219,6 +226,7 @@ int setup_half(NbCtx *c)
     free_ptr(c->d_hrow); free_ptr(c->d_jset);
     c->hblocks.clear();
     c->whalf = c->precision != MOIL_NB_FP64 && c->row16 && c->nW > 0 && c->want_whalf != MOIL_NB_WATER_FULL;
+    if (c->want_whalf == MOIL_NB_WATER_AUTO && c->nw_handle <= NB_FULL_MAX_WATERS) c->whalf = 0;
     if (!c->whalf) return MOIL_NB_OK;
     int maxw = 0;
     for (int r = 0; r < c->nrep; ++r) {
@@ -514,6 +522,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     c->natom = atom0;
     c->nW = wat0;
     c->nA = oth0;
+    c->nw_handle = std::max(c->nw_handle, c->nW);
     c->row16 = 1;
     for (int r = 0; r < nrep; ++r) c->row16 &= c->rd[r].nwat < 65536;
     c->nsite = 3 * c->nW + c->nA;
@@ -1089,6 +1098,10 @@ int init_groups(moil_nb_ctx *h, int nrep, const moil_replica *reps, int P)
     }
     h->grp_rep0.push_back(nrep);
     h->grp_atom0.push_back(total);
+    int64_t nwat = 0;
+    for (int r = 0; r < nrep; ++r)
+        if (reps[r].topo && reps[r].topo->montype)
+            nwat += std::count(reps[r].topo->montype, reps[r].topo->montype + std::max(reps[r].topo->totmon, 0), (int)MOIL_MON_WATER);
     for (size_t g = 0; g + 1 < h->grp_rep0.size(); ++g) {
         moil_nb_ctx *c = nullptr;
         int rc = moil_nb_create(&c, h->device);
@@ -1099,6 +1112,7 @@ int init_groups(moil_nb_ctx *h, int nrep, const moil_replica *reps, int P)
         c->want_whalf = h->want_whalf;
         c->hb = h->hb;
         c->want_tiled = h->want_tiled;
+        c->nw_handle = nwat;
         {
             // streams for host-buffer evaluations: earlier groups at higher priority finish
             // first, so their gradient copies overlap the later groups' kernels (device-
@@ -1196,6 +1210,7 @@ int moil_nb_init(moil_nb_ctx *h, const moil_nb_params *p, const moil_topology *t
     moil_replica r = {p, t};
     cudaSetDevice(h->device);
     destroy_groups(h);
+    h->nw_handle = 0;
     return init_impl(h, 1, &r);
 }
 
@@ -1212,6 +1227,7 @@ int moil_nb_init_batch(moil_nb_ctx *h, int nrep, const moil_replica *reps)
     }
     if (reps) nb_tune_cached_shape(h, nrep, reps);
     const int P = reps ? choose_groups(h, nrep, natom) : 1;
+    h->nw_handle = 0;
     if (P <= 1) return init_impl(h, nrep, reps);
     if (h->inited) release_device(h);
     h->inited = 0;

@@ -52,6 +52,7 @@ struct NbCtx {
     std::vector<RepDev> rd;
     RepDev *d_reps = nullptr;
     int64_t natom = 0, nW = 0, nA = 0, nsite = 0, nunit = 0;
+    int64_t nw_handle = 0;        // waters of the whole handle: all replica groups together
     float skin = 1.0f, rwat = 1.1f;
     int list_period = 0;
     int water_excl_fast = 0;      // every water's exclusions are exactly O-H1, O-H2, H1-H2

@@ -124,13 +124,13 @@ __device__ __forceinline__ void flush(double g[], long long G[], int n)
 }
 
 // water sites of molecule i against its W2 list of non-water atoms (entries first, first +
-// stride, ...): atom semantics per site pair; partial gradients and energies go to g / e4,
-// flushed every CHUNK entries
+// stride, ...): atom semantics per site pair; partial gradients and energies go to g / e4, which
+// already hold cnt entries, flushed every CHUNK entries and left to the caller after the last
 template <typename T, typename Flush>
 __device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const typename vec4<T>::type *pos,
                                                const void *lj_v, const unsigned *__restrict__ sflags,
                                                const int *__restrict__ wl2_off, const int *__restrict__ wl2, int cap2,
-                                               int first, int stride, T g[9], T e4[4], int &npair, Flush &flush_all)
+                                               int first, int stride, int cnt, T g[9], T e4[4], int &npair, Flush &flush_all)
 {
     typedef typename vec4<T>::type T4;
     typedef typename cplx<T>::type T2;
@@ -142,7 +142,6 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const typ
     const T4 si[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
     const T2 lji[3] = {lj[3 * i], lj[3 * i + 1], lj[3 * i + 2]};
     const unsigned fi[3] = {sflags[3 * i], sflags[3 * i + 1], sflags[3 * i + 2]};
-    int cnt = 0;
     for (int k = q0 + first; k < q1; k += stride) {
         nb_prefetch_l1(wl2 + min(k + 32, q1 - 1));
         int s = wl2[k];
@@ -166,7 +165,6 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const typ
         }
         if (++cnt == CHUNK) { flush_all(); cnt = 0; }
     }
-    flush_all();
 }
 
 // ---------------------------------------------------------------------------------
@@ -332,7 +330,7 @@ __global__ void __launch_bounds__(32 * WARPS64) k_water_d(int nW, const RepDev *
     for (int k = 0; k < 6; ++k) e4[k] *= 2.0;   // each pair once; the energy reduction halves
     // water sites against non-water atoms (W2, full list): a lane's share of the entries
     auto none = []() {};
-    water_vs_atoms<double>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, lane, 32, g, e4, npair, none);
+    water_vs_atoms<double>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, lane, 32, 0, g, e4, npair, none);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const long long v = sub_sum<32>(nb_fix(g[k]));
@@ -404,19 +402,68 @@ __device__ __forceinline__ float water_intra_f(const RepDev &R, float4 h1, float
 }
 
 // ---------------------------------------------------------------------------------
-// FP32 water kernel on the packed two-lane FP32 pipe: list entries are taken two at a
-// time and every quantity of the 9 site pairs is a float2 over (entry k, entry k+1).  A
-// molecule outside the O-O cutoff (or the missing partner of an odd tail) is moved 1e4 Å
-// away, where erfc and exp underflow to exactly zero, so it adds nothing without a branch.
-// Gradients are accumulated per lane as float2 and folded at each flush; W2 (water sites vs
-// non-water atoms) runs the scalar code of k_water.
+// FP32 water kernels on the packed two-lane FP32 pipe.
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-// VIR: also the water-water LJ virial terms (two more accumulators, which the 128-register
-// budget of the plain evaluation does not hold without spilling; off unless requested)
-template <bool VIR, typename E>
-__global__ void __launch_bounds__(WBLOCK, 4) k_water_f(int nW, const RepDev *__restrict__ reps,
+// Real-space Ewald Coulomb of two site pairs (packed) and of one: the energy qq erfc(alpha r)/r
+// and minus its (dE/dr)/r.  erfc(x) = exp(-x^2) t P(A t + B), t = 1 / (1 + P x), x = alpha r, with
+// no clamp to the fitted range x <= 4.5: beyond it the fit extrapolates smoothly (relative
+// error 1e-5 at x = 7, 2e-3 at x = 3500) and exp(-x^2) < 1e-8 makes the term negligible.
+struct WaterK {
+    float palpha, ex2c, c2a;
+};
+__device__ __forceinline__ float2 ewald2(const WaterK &K, float2 rr2, float2 qq, float2 &e)
+{
+    const float2 rinv = f2(nb_rsqrt_approx(rr2.x), nb_rsqrt_approx(rr2.y));
+    const float2 arg = __fmul2_rn(rr2, f2(K.ex2c));
+    const float2 den = __ffma2_rn(f2(K.palpha), __fmul2_rn(rr2, rinv), f2(1.f));
+    const float2 tt = f2(nb_rcp_approx(den.x), nb_rcp_approx(den.y));
+    const float2 u = __ffma2_rn(f2(ERFCX_A), tt, f2(ERFCX_B));
+    const float C[ERFCX_NC] = ERFCX_COEFS;
+    float2 p = f2(C[ERFCX_NC - 1]);
+#pragma unroll
+    for (int m = ERFCX_NC - 2; m >= 0; --m) p = __ffma2_rn(p, u, f2(C[m]));
+    const float2 ex = f2(nb_ex2_approx(-arg.x), nb_ex2_approx(-arg.y));
+    e = __fmul2_rn(__fmul2_rn(qq, __fmul2_rn(ex, __fmul2_rn(tt, p))), rinv);
+    return __fmul2_rn(__ffma2_rn(__fmul2_rn(qq, f2(K.c2a)), ex, e), __fmul2_rn(rinv, rinv));
+}
+__device__ __forceinline__ float ewald1(const WaterK &K, float rr2, float rinv, float qq, float &e)
+{
+    const float tt = nb_rcp_approx(fmaf(K.palpha, rr2 * rinv, 1.f)), u = fmaf(ERFCX_A, tt, ERFCX_B);
+    const float C[ERFCX_NC] = ERFCX_COEFS;
+    float p = C[ERFCX_NC - 1];
+#pragma unroll
+    for (int m = ERFCX_NC - 2; m >= 0; --m) p = fmaf(p, u, C[m]);
+    const float ex = nb_ex2_approx(-rr2 * K.ex2c);
+    e = qq * (ex * (tt * p)) * rinv;
+    return fmaf(qq * K.c2a, ex, e) * (rinv * rinv);
+}
+// hi + lo += v (TwoSum, Knuth: the rounding error of hi + v collects in lo)
+__device__ __forceinline__ void two_add(float2 &a, float v)
+{
+    const float sm = a.x + v, bb = sm - a.x;
+    a = make_float2(sm, a.y + ((a.x - (sm - bb)) + (v - bb)));
+}
+template <int W> __device__ __forceinline__ float2 sub_two_sum(float2 a)
+{
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+        const float hi = __shfl_xor_sync(0xffffffffu, a.x, o, W), lo = __shfl_xor_sync(0xffffffffu, a.y, o, W);
+        two_add(a, hi);
+        a.y += lo;
+    }
+    return a;
+}
+
+// FP32 water kernel over full rows, LPW lanes per water: the lanes take the row's entries in
+// turn (consecutive lanes read consecutive entries) and each owns a partial gradient of its
+// water, summed over the lanes at the end (FP32 butterfly, then fixed point).  Of an entry's nine
+// site pairs eight run packed two by two on the FP32x2 pipe -- (O; H, H) and (H, H; each
+// partner site) -- and the O-O pair with its LJ part runs scalar, so one partner record is
+// live at a time.  VIR: also the water-water LJ virial terms.
+template <int LPW, bool VIR, typename E>
+__global__ void __launch_bounds__(WBLOCK, 5) k_water_s(int nW, const RepDev *__restrict__ reps,
                                                        const int *__restrict__ site_rep, const float4 *__restrict__ pos,
                                                        const float4 *__restrict__ woff, const void *lj_v,
                                                        const unsigned *__restrict__ sflags,
@@ -425,197 +472,162 @@ __global__ void __launch_bounds__(WBLOCK, 4) k_water_f(int nW, const RepDev *__r
                                                        const int *__restrict__ wl2, int cap2, long long *__restrict__ grad,
                                                        double *__restrict__ e_unit, int intra)
 {
-    __shared__ long long sG[9][WBLOCK];
-    __shared__ float2 sE[6][WBLOCK];     // energies as unevaluated sums hi + lo (no FP64 pipe)
-    const int t = threadIdx.x;
-    const int i = blockIdx.x * WBLOCK + t;
-    if (i >= nW) return;
+    constexpr int NE = VIR ? 6 : 4;
+    __shared__ unsigned long long sG[WBLOCK / LPW][9];   // rows longer than CHUNK entries per lane
+    __shared__ float2 sE[NE][WBLOCK];
+    const int t = threadIdx.x, sub = t & (LPW - 1), w = t / LPW;
+    const int iw = blockIdx.x * (WBLOCK / LPW) + w;
+    const bool act = iw < nW;
+    const int i = act ? iw : nW - 1;         // idle lanes of the last block: an empty row, no output
     const RepDev &R = reps[site_rep[3 * i]];
+    for (int k = sub; k < 9; k += LPW) sG[w][k] = 0ull;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) sG[k][t] = 0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) sE[k][t] = make_float2(0.f, 0.f);
-    const float4 oi0 = woff[3 * i];
-    const float4 oi1 = woff[3 * i + 1], oi2 = woff[3 * i + 2];
-    // H offsets of molecule i, duplicated into both lanes
-    const float2 hi[2][3] = {{f2(oi1.x), f2(oi1.y), f2(oi1.z)}, {f2(oi2.x), f2(oi2.y), f2(oi2.z)}};
-    float2 G[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) G[k] = f2(0.f);
+    for (int k = 0; k < NE; ++k) sE[k][t] = make_float2(0.f, 0.f);
+    __syncwarp();
+    const float4 oi0 = woff[3 * i], oi1 = woff[3 * i + 1], oi2 = woff[3 * i + 2];
+    const float2 hx = f2(oi1.x, oi2.x), hy = f2(oi1.y, oi2.y), hz = f2(oi1.z, oi2.z);   // (H1, H2) offsets
+    // minus the gradient: of O as two partials, of (H1, H2)
+    float2 GO[3] = {f2(0.f), f2(0.f), f2(0.f)}, GH[3] = {f2(0.f), f2(0.f), f2(0.f)};
     float g[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) g[k] = 0.f;
-    // LJ prim, LJ img, Coulomb prim, Coulomb img (, LJ virial prim, LJ virial img)
-    constexpr int NE = VIR ? 6 : 4;
-    float e4[NE];
+    float e4[NE];    // LJ prim, LJ img, Coulomb prim, Coulomb img (, LJ virial prim, LJ virial img)
 #pragma unroll
     for (int k = 0; k < NE; ++k) e4[k] = 0.f;
-    // the molecule's own exclusion corrections (every water excludes exactly its three pairs)
-    float ecorr = 0.f;
-    if (intra) {
-        const float qs[3] = {oi0.w, pos[3 * i + 1].w, pos[3 * i + 2].w};
-        ecorr = water_intra_f(R, oi1, oi2, qs, g);
-    }
+    auto fold = [&]() {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            g[d] -= GO[d].x + GO[d].y; g[3 + d] -= GH[d].x; g[6 + d] -= GH[d].y;
+            GO[d] = f2(0.f); GH[d] = f2(0.f);
+        }
+    };
+    auto flush_e = [&]() {
+#pragma unroll
+        for (int k = 0; k < NE; ++k) { two_add(sE[k][t], e4[k]); e4[k] = 0.f; }
+    };
     auto flush_all = [&]() {
+        fold();
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            sG[k][t] += nb_fix(g[k] - (G[k].x + G[k].y));   // G holds minus the gradient
-            g[k] = 0.f;
-            G[k] = f2(0.f);
-        }
-#pragma unroll
-        for (int k = 0; k < NE; ++k) {
-            // TwoSum (Knuth): hi + e4 = s + err exactly; the errors collect in lo
-            const float2 a = sE[k][t];
-            const float sm = a.x + e4[k], bb = sm - a.x, err = (a.x - (sm - bb)) + (e4[k] - bb);
-            sE[k][t] = make_float2(sm, a.y + err);
-            e4[k] = 0.f;
-        }
+        for (int k = 0; k < 9; ++k) { atomicAdd(&sG[w][k], (unsigned long long)nb_fix(g[k])); g[k] = 0.f; }
+        flush_e();
     };
     int npair = 0;
     const float iL0 = R.invL[0], iL1 = R.invL[1], iL2 = R.invL[2];
     const float rmax2 = R.rmax2, rv2 = R.rv2;
-    const float2 palpha = f2(ERFCX_P * R.alpha), ex2c = f2(R.ex2c);
-    const float2 w12 = f2(R.w12), nw6 = f2(-R.w6);
-    const float2 c12 = f2(R.w12c), c6 = f2(R.w6c);
-    const float qqv[3] = {R.qq[0], R.qq[1], R.qq[2]};
-    const float c2a = R.c2a;
+    const WaterK K = {ERFCX_P * R.alpha, R.ex2c, R.c2a};
+    const float qOO = R.qq[0], qOH = R.qq[1], qHH = R.qq[2], w12 = R.w12, w6 = R.w6;
     const W1Row<E> L1(wl1_cnt, wl1, cap_row, i, R.wat0);
-    const int k1 = L1.n;
+    const int n = act ? L1.n : 0;
+    // two iterations ahead the entry, one ahead the partner's oxygen
+    int j1 = sub < n ? L1.at(sub) : i, j2 = sub + LPW < n ? L1.at(sub + LPW) : i;
+    float4 o1 = woff[3 * j1];
     int cnt = 0;
-    // next pair of entries, loaded one iteration ahead
-    int ja = k1 > 0 ? L1.at(0) : 0;
-    int jb = k1 > 1 ? L1.at(1) : ja;
-    float4 oa = woff[3 * ja], ob = woff[3 * jb];
-    for (int k = 0; k < k1; k += 2) {
-        const bool hasb = k + 1 < k1;
-        const int j0 = ja, j1 = jb;
-        const float4 o0 = oa, o1 = ob;
-        // each lane streams its own row (a DRAM stream): pull the line 32 entries ahead
-        nb_prefetch_l1(L1.addr(min(k + 32, k1 - 1)));
-        if (k + 2 < k1) {
-            ja = L1.at(k + 2);
-            jb = k + 3 < k1 ? L1.at(k + 3) : ja;
-            oa = woff[3 * ja];
-            ob = woff[3 * jb];
-        }
-        // O-O minimum image per entry; (x + 1.5*2^23) - 1.5*2^23 rounds x to nearest (|x| < 2^22)
-        float dx0 = oi0.x - o0.x, dy0 = oi0.y - o0.y, dz0 = oi0.z - o0.z;
-        float dx1 = oi0.x - o1.x, dy1 = oi0.y - o1.y, dz1 = oi0.z - o1.z;
-        const float nx0 = fmaf(dx0, iL0, 12582912.f) - 12582912.f, ny0 = fmaf(dy0, iL1, 12582912.f) - 12582912.f, nz0 = fmaf(dz0, iL2, 12582912.f) - 12582912.f;
-        const float nx1 = fmaf(dx1, iL0, 12582912.f) - 12582912.f, ny1 = fmaf(dy1, iL1, 12582912.f) - 12582912.f, nz1 = fmaf(dz1, iL2, 12582912.f) - 12582912.f;
-        dx0 = nb_shift(R, 0, dx0, nx0); dy0 = nb_shift(R, 1, dy0, ny0); dz0 = nb_shift(R, 2, dz0, nz0);
-        dx1 = nb_shift(R, 0, dx1, nx1); dy1 = nb_shift(R, 1, dy1, ny1); dz1 = nb_shift(R, 2, dz1, nz1);
-        const float r0 = dx0 * dx0 + dy0 * dy0 + dz0 * dz0, r1 = dx1 * dx1 + dy1 * dy1 + dz1 * dz1;
-        const bool in0 = r0 <= rmax2, in1 = hasb && r1 <= rmax2;
-        if (in0 || in1) {
-            const float4 a1 = woff[3 * j0 + 1], a2 = woff[3 * j0 + 2];
-            const float4 b1 = woff[3 * j1 + 1], b2 = woff[3 * j1 + 2];
-            if (!in0) { dx0 = 1.0e4f; dy0 = 0.f; dz0 = 0.f; }
-            if (!in1) { dx1 = 1.0e4f; dy1 = 0.f; dz1 = 0.f; }
-            // q[b] = (O_i - O_j - nL) - offset_j[b]; site displacement = offset_i[a] + q[b]
-            float2 eel = f2(0.f), elj = f2(0.f), vlj = f2(0.f);
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                float2 q[3];
-                if (b == 0) {
-                    q[0] = f2(dx0, dx1); q[1] = f2(dy0, dy1); q[2] = f2(dz0, dz1);
-                } else if (b == 1) {
-                    q[0] = f2(dx0 - a1.x, dx1 - b1.x); q[1] = f2(dy0 - a1.y, dy1 - b1.y);
-                    q[2] = f2(dz0 - a1.z, dz1 - b1.z);
-                } else {
-                    q[0] = f2(dx0 - a2.x, dx1 - b2.x); q[1] = f2(dy0 - a2.y, dy1 - b2.y);
-                    q[2] = f2(dz0 - a2.z, dz1 - b2.z);
-                }
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float2 ddx = a ? __fadd2_rn(hi[a - 1][0], q[0]) : q[0];
-                    const float2 ddy = a ? __fadd2_rn(hi[a - 1][1], q[1]) : q[1];
-                    const float2 ddz = a ? __fadd2_rn(hi[a - 1][2], q[2]) : q[2];
-                    const float2 rr2 = __ffma2_rn(ddx, ddx, __ffma2_rn(ddy, ddy, __fmul2_rn(ddz, ddz)));
-                    const float2 rinv = f2(nb_rsqrt_approx(rr2.x), nb_rsqrt_approx(rr2.y));
-                    const float2 s2 = __fmul2_rn(rinv, rinv);
-                    const float2 arg = __fmul2_rn(rr2, ex2c);
-                    // erfc(x) = exp(-x^2) * t * P(A t + B), t = 1 / (1 + P x), x = alpha r, with
-                    // no clamp to the fitted range x <= 4.5: beyond it the fit extrapolates
-                    // smoothly (relative error 1e-5 at x = 7, 2e-3 at x = 3500, the parked
-                    // entries) and exp(-x^2) < 1e-8 makes the term negligible
-                    const float2 den = __ffma2_rn(palpha, __fmul2_rn(rr2, rinv), f2(1.f));
-                    const float2 tt = f2(nb_rcp_approx(den.x), nb_rcp_approx(den.y));
-                    const float2 u = __ffma2_rn(f2(ERFCX_A), tt, f2(ERFCX_B));
-                    const float C[ERFCX_NC] = ERFCX_COEFS;
-                    float2 p = f2(C[ERFCX_NC - 1]);
-#pragma unroll
-                    for (int m = ERFCX_NC - 2; m >= 0; --m) p = __ffma2_rn(p, u, f2(C[m]));
-                    const float2 ex = f2(nb_ex2_approx(-arg.x), nb_ex2_approx(-arg.y));
-                    const float2 erfcv = __fmul2_rn(ex, __fmul2_rn(tt, p));
-                    const float qq = (a == 0 && b == 0) ? qqv[0] : ((a == 0 || b == 0) ? qqv[1] : qqv[2]);
-                    const float2 e = __fmul2_rn(__fmul2_rn(f2(qq), erfcv), rinv);
-                    // minus dE/dr / r
-                    float2 mdf = __fmul2_rn(__ffma2_rn(f2(qq * c2a), ex, e), s2);
-                    if (a == 0 && b == 0) {
-                        // LJ powers from a Newton-refined 1/r (r^-12 amplifies rsqrt's error 12 times)
-                        // rinv - rinv (r^2 rinv^2 - 1) / 2: the correction is formed as a small
-                        // number, so the result keeps round-to-nearest's lack of bias
-                        const float2 ri = __ffma2_rn(__fmul2_rn(f2(-0.5f), rinv), __ffma2_rn(rr2, s2, f2(-1.f)), rinv);
-                        const float2 sl = __fmul2_rn(ri, ri);
-                        const float2 s6 = __fmul2_rn(__fmul2_rn(sl, sl), sl);
-                        const float2 A = __fmul2_rn(__fmul2_rn(w12, s6), s6);
-                        // energy A (1 + c12) - B (1 + c6): c12, c6 restore the FP32 rounding of the
-                        // coefficients, whose relative error would otherwise bias every pair alike
-                        // (the force keeps A and B)
-                        float2 e1 = __ffma2_rn(nw6, __ffma2_rn(s6, c6, s6), __ffma2_rn(A, c12, A));
-                        // -df1 = 6 s2 (2A - B)
-                        float2 m1 = __fmul2_rn(__fmul2_rn(f2(6.f), sl), __ffma2_rn(nw6, s6, __fadd2_rn(A, A)));
-                        if (R.lj_switch) {
-                            float d0 = -m1.x, d1 = -m1.y;
-                            lj_switch_apply<float>(R, rr2.x, e1.x, d0);
-                            lj_switch_apply<float>(R, rr2.y, e1.y, d1);
-                            m1 = f2(-d0, -d1);
-                        }
-                        const bool l0 = rr2.x <= rv2, l1 = rr2.y <= rv2;
-                        e1 = f2(l0 ? e1.x : 0.f, l1 ? e1.y : 0.f);
-                        m1 = f2(l0 ? m1.x : 0.f, l1 ? m1.y : 0.f);
-                        elj = __fadd2_rn(elj, e1);
-                        if (VIR) vlj = __fmul2_rn(m1, rr2);   // -df1 r^2 (watwat_ewald_press.f:146-152)
-                        mdf = __fadd2_rn(mdf, m1);
+    for (int k = sub; k < n; k += LPW) {
+        const int j = j1;
+        const float4 oj = o1;
+        j1 = j2;
+        o1 = woff[3 * j1];
+        if (k + 2 * LPW < n) j2 = L1.at(k + 2 * LPW);
+        float dx = oi0.x - oj.x, dy = oi0.y - oj.y, dz = oi0.z - oj.z;
+        // (x + 1.5*2^23) - 1.5*2^23 rounds x to nearest (|x| < 2^22)
+        const float nx = fmaf(dx, iL0, 12582912.f) - 12582912.f, ny = fmaf(dy, iL1, 12582912.f) - 12582912.f,
+                    nz = fmaf(dz, iL2, 12582912.f) - 12582912.f;
+        dx = nb_shift(R, 0, dx, nx); dy = nb_shift(R, 1, dy, ny); dz = nb_shift(R, 2, dz, nz);
+        const float r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 <= rmax2) {
+            const float4 a = woff[3 * j + 1], b = woff[3 * j + 2];
+            float2 eel, e;
+            float eoo, elj = 0.f, vlj = 0.f;
+            {
+                // O-O: Coulomb and LJ (powers from a Newton-refined 1/r: r^-12 amplifies the
+                // approximate rsqrt's error 12 times; the correction is formed as a small number)
+                const float rr2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                const float rinv = nb_rsqrt_approx(rr2), s2 = rinv * rinv;
+                float mdf = ewald1(K, rr2, rinv, qOO, eoo);
+                if (rr2 <= rv2) {
+                    const float ri = fmaf(-0.5f * rinv, fmaf(rr2, s2, -1.f), rinv), sl = ri * ri;
+                    const float s6 = sl * sl * sl, A = w12 * s6 * s6;
+                    // c12, c6 restore the FP32 rounding of the coefficients in the energy (the force
+                    // keeps A and B)
+                    float e1 = fmaf(-w6, fmaf(s6, R.w6c, s6), fmaf(A, R.w12c, A));
+                    float m1 = 6.f * sl * fmaf(-w6, s6, A + A);
+                    if (R.lj_switch) {
+                        float d1 = -m1;
+                        lj_switch_apply<float>(R, rr2, e1, d1);
+                        m1 = -d1;
                     }
-                    eel = __fadd2_rn(eel, e);
-                    G[3 * a] = __ffma2_rn(mdf, ddx, G[3 * a]);
-                    G[3 * a + 1] = __ffma2_rn(mdf, ddy, G[3 * a + 1]);
-                    G[3 * a + 2] = __ffma2_rn(mdf, ddz, G[3 * a + 2]);
+                    elj = e1;
+                    if (VIR) vlj = m1 * rr2;   // -df1 r^2 (watwat_ewald_press.f:146-152)
+                    mdf += m1;
                 }
+                GO[0].x = fmaf(mdf, dx, GO[0].x); GO[1].x = fmaf(mdf, dy, GO[1].x); GO[2].x = fmaf(mdf, dz, GO[2].x);
             }
-            const bool img0 = (nx0 != 0.f) | (ny0 != 0.f) | (nz0 != 0.f);
-            const bool img1 = (nx1 != 0.f) | (ny1 != 0.f) | (nz1 != 0.f);
-            e4[img0 ? 1 : 0] += elj.x;
-            e4[img0 ? 3 : 2] += eel.x;
-            if (VIR) e4[img0 ? NE - 1 : NE - 2] += vlj.x;
-            e4[img1 ? 1 : 0] += elj.y;
-            e4[img1 ? 3 : 2] += eel.y;
-            if (VIR) e4[img1 ? NE - 1 : NE - 2] += vlj.y;
-            npair += 9 * ((int)in0 + (int)in1);
+            {
+                // O of i with (H1, H2) of j
+                const float2 x = f2(dx - a.x, dx - b.x), y = f2(dy - a.y, dy - b.y), z = f2(dz - a.z, dz - b.z);
+                const float2 m = ewald2(K, __ffma2_rn(x, x, __ffma2_rn(y, y, __fmul2_rn(z, z))), f2(qOH), eel);
+                GO[0] = __ffma2_rn(m, x, GO[0]); GO[1] = __ffma2_rn(m, y, GO[1]); GO[2] = __ffma2_rn(m, z, GO[2]);
+            }
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                // (H1, H2) of i with site s of j
+                const float qx = s == 0 ? dx : (s == 1 ? dx - a.x : dx - b.x);
+                const float qy = s == 0 ? dy : (s == 1 ? dy - a.y : dy - b.y);
+                const float qz = s == 0 ? dz : (s == 1 ? dz - a.z : dz - b.z);
+                const float2 x = __fadd2_rn(hx, f2(qx)), y = __fadd2_rn(hy, f2(qy)), z = __fadd2_rn(hz, f2(qz));
+                const float2 m = ewald2(K, __ffma2_rn(x, x, __ffma2_rn(y, y, __fmul2_rn(z, z))),
+                                        f2(s == 0 ? qOH : qHH), e);
+                eel = __fadd2_rn(eel, e);
+                GH[0] = __ffma2_rn(m, x, GH[0]); GH[1] = __ffma2_rn(m, y, GH[1]); GH[2] = __ffma2_rn(m, z, GH[2]);
+            }
+            const bool img = (nx != 0.f) | (ny != 0.f) | (nz != 0.f);
+            const float ec = eoo + (eel.x + eel.y);
+            e4[0] += img ? 0.f : elj; e4[1] += img ? elj : 0.f;
+            e4[2] += img ? 0.f : ec; e4[3] += img ? ec : 0.f;
+            if (VIR) { e4[NE - 2] += img ? 0.f : vlj; e4[NE - 1] += img ? vlj : 0.f; }
+            npair += 9;
         }
-        cnt += 2;
-        if (cnt >= CHUNK) { flush_all(); cnt = 0; }
+        if (++cnt == CHUNK) { flush_all(); cnt = 0; }
     }
-    flush_all();
-    water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, g, e4, npair, flush_all);
+    fold();
+    if (act) {
+        water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, sub, LPW, cnt, g, e4, npair, flush_all);
+    }
+    float ecorr = 0.f;
+    if (intra && sub == 0) {
+        // the molecule's own exclusion corrections (every water excludes exactly its three pairs)
+        const float qs[3] = {oi0.w, pos[3 * i + 1].w, pos[3 * i + 2].w};
+        ecorr = water_intra_f(R, oi1, oi2, qs, g);
+    }
+    flush_e();
 #pragma unroll
-    for (int k = 0; k < 9; ++k) grad[(size_t)9 * i + k] = sG[k][t];
-    double *eu = e_unit + NB_EU * (size_t)i;
+    for (int k = 0; k < 9; ++k)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) eu[k] = (double)sE[k][t].x + (double)sE[k][t].y;
-    eu[4] = (double)npair;
-    eu[5] = (double)ecorr;
-    eu[6] = VIR ? (double)sE[4][t].x + (double)sE[4][t].y : 0.0;
-    eu[7] = VIR ? (double)sE[5][t].x + (double)sE[5][t].y : 0.0;
+        for (int o = LPW / 2; o > 0; o >>= 1) g[k] += __shfl_xor_sync(0xffffffffu, g[k], o, LPW);
+    npair = sub_sum<LPW>(npair);
+    float2 es[NE];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) es[k] = sub_two_sum<LPW>(sE[k][t]);
+    if (!act) return;
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        if (sub == k % LPW) grad[(size_t)9 * i + k] = nb_fix(g[k]) + (long long)sG[w][k];
+    if (sub == 0) {
+        double *eu = e_unit + NB_EU * (size_t)i;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) eu[k] = (double)es[k].x + (double)es[k].y;
+        eu[4] = (double)npair;
+        eu[5] = (double)ecorr;
+        eu[6] = VIR ? (double)es[NE - 2].x + (double)es[NE - 2].y : 0.0;
+        eu[7] = VIR ? (double)es[NE - 1].x + (double)es[NE - 1].y : 0.0;
+    }
 }
 
 // ---------------------------------------------------------------------------------
 // FP32 water kernel over half lists (k_whalf): every water-water pair is evaluated once, by
-// its owner, with the pair arithmetic of k_water_f.  The owner keeps its own gradient as in
-// k_water_f; the partner's side of each pair (per partner site, summed over the owner's three
+// its owner, two list entries packed on the FP32x2 pipe (a molecule outside the O-O cutoff, or the
+// missing partner of an odd tail, is moved 1e4 Å away, where erfc and exp underflow to exactly
+// zero).  The owner keeps its own gradient in registers; the partner's side of each pair (per partner site, summed over the owner's three
 // sites) goes to an int32 accumulator in shared memory indexed by the partner's place in the
 // block's j-set, at 2^S units per kcal/mol/Å (S = 24 - log2 HB: HB contributions below
 // NB_HALF_CAP in magnitude fit); larger contributions go directly to the int64 gradient.
@@ -628,7 +640,7 @@ template <> struct HalfScale<128> { static constexpr int S = 17; };
 template <> struct HalfScale<256> { static constexpr int S = 16; };
 template <> struct HalfScale<512> { static constexpr int S = 15; };
 
-// VIR: also the water-water LJ virial terms (as k_water_f<true>)
+// VIR: also the water-water LJ virial terms (as k_water_s<.., true, ..>)
 template <int HB, bool VIR>
 __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict__ blocks, const RepDev *__restrict__ reps,
                                                           const float4 *__restrict__ pos, const float4 *__restrict__ woff,
@@ -858,7 +870,10 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
             if (cnt >= CHUNK) { flush(2.f); cnt = 0; }
         }
         flush(2.f);
-        water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, g, e4, npair, flush1);
+        if (wl2_off[i] < wl2_off[i + 1]) {
+            water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, 0, g, e4, npair, flush1);
+            flush1();
+        }
 #pragma unroll
         for (int k = 0; k < 4; ++k) eu[k] = (double)sE[k][t].x + (double)sE[k][t].y;
         eu[4] = (double)npair;
@@ -1210,6 +1225,27 @@ WaterHFn water_h_fn(int hb, bool vir)
     }
 }
 
+// Lanes per water of the full-list kernel, from the waters of the whole handle (all replica
+// groups, so a grouped handle gives the ungrouped one's bits): every lane of the GPU has work
+// from a few thousand waters at 32 lanes each, and from then on fewer lanes lose less to
+// partly filled rounds and to the sum over the lanes.  Water stage in us at 32 / 8 / 4 lanes:
+// 1,334 waters 16 / 26 / 38, 3,000 17 / 22 / 38, 7,000 32 / 24 / 40, 12,000 42 / 30 / 40, 32,000
+// 112 / 84 / 89, 110,860 (64 replicas) 339 / 206 / 194, 433,195 1304 / 743 / 678 (one water per
+// thread: 78, 79, 82, 79, 120, 204, 657).
+int water_lanes(const NbCtx *c) { return c->nw_handle <= 4096 ? 32 : (c->nw_handle <= 32768 ? 8 : 4); }
+
+using WaterSFn = decltype(&k_water_s<8, false, int>);
+WaterSFn water_s_fn(int lpw, bool vir, bool row16)
+{
+    // 32-bit rows belong to replicas of 65,536 waters or more
+    if (!row16) return vir ? k_water_s<4, true, int> : k_water_s<4, false, int>;
+    switch (lpw) {
+    case 32: return vir ? k_water_s<32, true, unsigned short> : k_water_s<32, false, unsigned short>;
+    case 8: return vir ? k_water_s<8, true, unsigned short> : k_water_s<8, false, unsigned short>;
+    default: return vir ? k_water_s<4, true, unsigned short> : k_water_s<4, false, unsigned short>;
+    }
+}
+
 template <typename T>
 void realspace_t(NbCtx *c)
 {
@@ -1224,14 +1260,13 @@ void realspace_t(NbCtx *c)
             cap_int(c->cap_wl2), c->d_grad_site, c->d_e_unit, c->water_excl_fast);
         c->launches++;
     } else if (c->nW > 0) {
-        const int nb = (int)((c->nW + WBLOCK - 1) / WBLOCK);
-        if constexpr (sizeof(T) == 4)
-            (c->virial ? (c->row16 ? k_water_f<true, unsigned short> : k_water_f<true, int>)
-                       : (c->row16 ? k_water_f<false, unsigned short> : k_water_f<false, int>))<<<nb, WBLOCK, 0, s>>>(
+        if constexpr (sizeof(T) == 4) {
+            const int lpw = water_lanes(c);
+            water_s_fn(lpw, c->virial, c->row16)<<<(int)((c->nW * lpw + WBLOCK - 1) / WBLOCK), WBLOCK, 0, s>>>(
                 (int)c->nW, c->d_reps, c->d_site_rep, (const float4 *)c->d_pos, (const float4 *)c->d_woff,
                 c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2,
                 cap_int(c->cap_wl2), c->d_grad_site, c->d_e_unit, c->water_excl_fast);
-        else {
+        } else {
             // both sides of every pair are added with atomics: the waters' gradient starts at zero
             cudaMemsetAsync(c->d_grad_site, 0, sizeof(long long) * 9 * (size_t)c->nW, s);
             (c->row16 ? k_water_d<unsigned short> : k_water_d<int>)<<<(int)((c->nW + WARPS64 - 1) / WARPS64),
@@ -1271,16 +1306,16 @@ static int carveout_pct(NbCtx *c, size_t bytes)
 
 int nb_realspace_configure(NbCtx *c)
 {
-    // full-list FP32 water kernels: four resident blocks of static shared memory each; the
-    // smallest carveout that holds them leaves the most L1 for the partner-record gathers
-    const void *fns[4] = {(const void *)k_water_f<false, unsigned short>, (const void *)k_water_f<false, int>,
-                          (const void *)k_water_f<true, unsigned short>, (const void *)k_water_f<true, int>};
-    for (const void *fn : fns) {
-        cudaFuncAttributes fa;
-        NB_CUDA_OK(c, cudaFuncGetAttributes(&fa, fn));
-        NB_CUDA_OK(c, cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           carveout_pct(c, 4 * fa.sharedSizeBytes)));
-    }
+    // full-list FP32 water kernel: five resident blocks of static shared memory; the smallest
+    // carveout that holds them leaves the most L1 for the partner-record gathers
+    for (int lpw : {32, 8, 4})
+        for (int k = 0; k < 4; ++k) {
+            const void *fn = (const void *)water_s_fn(lpw, k & 1, k & 2);
+            cudaFuncAttributes fa;
+            NB_CUDA_OK(c, cudaFuncGetAttributes(&fa, fn));
+            NB_CUDA_OK(c, cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               carveout_pct(c, 5 * (fa.sharedSizeBytes + 1024))));
+        }
     return MOIL_NB_OK;
 }
 
@@ -1323,7 +1358,7 @@ int nb_half_configure(NbCtx *c)
 void nb_launch_excl14(NbCtx *c, const double *d_coor)
 {
     const int fast = c->water_excl_fast && c->nW > 0;
-    // mixed path: the water kernel adds each water's own corrections (k_water_f)
+    // mixed path: the water kernels add each water's own corrections
     if (fast && c->precision == MOIL_NB_FP64) {
         k_excl_water<<<(int)((c->nW + 127) / 128), 128, 0, c->stream>>>(
             (int)c->nW, c->d_unit_atom, c->d_atom_rep, c->d_reps, d_coor, c->d_q, c->d_grad_ex, c->d_e_ex);

@@ -2,13 +2,13 @@
 where the sharing can go wrong: water counts that do not fill the last block, rows shorter and
 longer than a warp's buffer, solutes of a few atoms.  Each against the oracle in parity mode:
 the FP64 path to 2^-25 of the gradient (its 2 alpha / sqrt(pi) is an FP32 constant) and 1e-10 of
-the energy-term scale per term."""
+the energy-term scale per term, the mixed path to 1e-5 of the gradient and 1e-6 of that scale."""
 import numpy as np
 import pytest
 
 from conftest import ENERGY_TERMS, energy_scale, rel_rms
 from moil_fnrfd_gb300 import systems as S
-from moil_fnrfd_gb300.nb import MOIL_NB_FP64, Nonbonded
+from moil_fnrfd_gb300.nb import MOIL_NB_FP64, MOIL_NB_MIXED, WATER_FULL, Nonbonded
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -35,19 +35,39 @@ SYSTEMS = {
 }
 
 
+def close_to_oracle(dpot, e, ref, eref, precision):
+    scale = energy_scale(eref)
+    fp64 = precision == MOIL_NB_FP64
+    assert all(abs(e[k] - eref[k]) <= (1e-10 if fp64 else 1e-6) * scale for k in ENERGY_TERMS + ("e_total",))
+    if eref["site_pairs"] == 0:
+        # no pairs: the gradient is a small remainder of cancelling terms
+        assert np.abs(dpot - ref).max() <= 1e-6 * scale
+    else:
+        assert rel_rms(dpot, ref) <= (2.0 ** -25 if fp64 else 1e-5)
+
+
+@pytest.mark.parametrize("precision", [MOIL_NB_FP64, MOIL_NB_MIXED], ids=["fp64", "mixed"])
 @pytest.mark.parametrize("name", SYSTEMS)
-def test_split_rows_match_oracle(name, precision=MOIL_NB_FP64):
+def test_split_rows_match_oracle(name, precision):
     s = SYSTEMS[name]()
     ref, eref = O.eforce(s, mode="parity")
     nb = Nonbonded(s, precision=precision)
     for _ in range(2):                      # the build, then list reuse
         dpot, e = nb.eforce(s.coor)
-        if eref["site_pairs"] == 0:
-            # no pairs: gradient and total are small remainders of cancelling terms
-            assert np.abs(dpot - ref).max() <= 1e-6 * energy_scale(eref)
-            assert abs(e["e_total"] - eref["e_total"]) <= 1e-6 * energy_scale(eref)
-        else:
-            assert rel_rms(dpot, ref) <= 2.0 ** -25
-            assert all(abs(e[k] - eref[k]) <= 1e-10 * energy_scale(eref) for k in ENERGY_TERMS)
+        close_to_oracle(dpot, e, ref, eref, precision)
     assert nb.pair_stats()["site_pairs"] == eref["site_pairs"]
+    nb.close()
+
+
+@pytest.mark.parametrize("filler", [1, 11], ids=["8_lanes", "4_lanes"])
+def test_long_rows_on_full_lists(filler):
+    """Rows of more than 64 entries per lane, in handles of more than 4,096 and 32,768 waters (8
+    and 4 lanes per water), beside a replica that ends inside a block."""
+    dense = dense_cluster(1001, 9, 0.5)
+    box = S.water_box(3203, (3203 / S.WATER_DENSITY) ** (1 / 3), 10)
+    nb = Nonbonded([dense] + [box] * filler, shape=dict(water_kernel=WATER_FULL), groups=1)
+    dps, es = nb.eforce()
+    for k, s in ((0, dense), (filler, box)):
+        ref, eref = O.eforce(s, mode="parity")
+        close_to_oracle(dps[k], es[k], ref, eref, MOIL_NB_MIXED)
     nb.close()
