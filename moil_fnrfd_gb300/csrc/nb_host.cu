@@ -592,6 +592,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     NB_CUDA_OK(c, cudaMalloc(&c->d_site_q, ts * ns));
     NB_CUDA_OK(c, cudaMalloc(&c->d_wl1_cnt, sizeof(int2) * std::max<int64_t>(c->nW, 1)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_wl2_off, sizeof(int) * (c->nW + 1)));
+    NB_CUDA_OK(c, cudaMemset(c->d_wl2_off, 0, sizeof(int) * (c->nW + 1)));   // rebuilt where there are non-water atoms
     NB_CUDA_OK(c, cudaMalloc(&c->d_xl_off, sizeof(int) * (c->nA + 1)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_count_tmp, sizeof(int) * (3 * std::max(c->nW, c->nA) + 3)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_grad_site, sizeof(long long) * 3 * ns));
