@@ -893,14 +893,30 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
     }
 }
 
-// non-water atom per thread over its full site list
+// An energy sum: FP32 as an unevaluated hi + lo pair, FP64 plain.
+template <typename T> struct ESum;
+template <> struct ESum<float> {
+    float2 s = make_float2(0.f, 0.f);
+    __device__ void add(float v) { two_add(s, v); }
+    __device__ double total32() { const float2 a = sub_two_sum<32>(s); return (double)a.x + (double)a.y; }
+};
+template <> struct ESum<double> {
+    double s = 0.0;
+    __device__ void add(double v) { s += v; }
+    __device__ double total32() { return sub_sum<32>(s); }
+};
+
+// One warp per non-water atom over its full site list: the lanes take the list's entries in turn
+// (consecutive entries are mostly the sites of one water, so the position loads coalesce) and
+// their partial gradients and energies are summed over the warp at the end.  One atom per thread
+// ran its ~600 entries in series: 486 us for 2,496 atoms, 363 us for 203.
 template <typename T>
 __global__ void __launch_bounds__(128) k_atom(int nA, int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
                                               const void *pos_v, const void *lj_v, const unsigned *__restrict__ sflags,
                                               const int *__restrict__ xl_off, const int *__restrict__ xl, int capx,
                                               long long *__restrict__ grad, double *__restrict__ e_unit)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, k = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (k >= nA) return;
     typedef typename vec4<T>::type T4;
     typedef typename cplx<T>::type T2;
@@ -913,12 +929,11 @@ __global__ void __launch_bounds__(128) k_atom(int nA, int nW, const RepDev *__re
     unsigned fi = sflags[si];
     T g[3] = {0, 0, 0};
     long long G[3] = {0, 0, 0};
-    double elp = 0, eli = 0, eep = 0, eei = 0, vp = 0, vi = 0;
+    ESum<T> es[6];    // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
     int cnt = 0, npair = 0;
     // an overflowed list is read within the buffer (the evaluation is redone)
     const int q1 = min(xl_off[k + 1], capx);
-    for (int q = min(xl_off[k], capx); q < q1; ++q) {
-        nb_prefetch_l1(xl + min(q + 32, q1 - 1));
+    for (int q = min(xl_off[k], capx) + lane; q < q1; q += 32) {
         int s = xl[q];
         T4 xj = pos[s];
         T2 ljj = lj[s];
@@ -931,18 +946,27 @@ __global__ void __launch_bounds__(128) k_atom(int nA, int nW, const RepDev *__re
         g[0] += df * dx; g[1] += df * dy; g[2] += df * dz;
         // LJ virial: a water partner's side of the pair (its W2 list) adds none, so it counts
         // twice here; pairs of two non-water atoms are seen from both sides
-        const double wv = (double)vir * (s < 3 * nW ? 2.0 : 1.0);
-        if (img) { eei += (double)eel; eli += (double)elj; vi += wv; }
-        else { eep += (double)eel; elp += (double)elj; vp += wv; }
+        if (s < 3 * nW) vir += vir;
+        es[0].add(img ? (T)0 : elj); es[1].add(img ? elj : (T)0);
+        es[2].add(img ? (T)0 : eel); es[3].add(img ? eel : (T)0);
+        es[4].add(img ? (T)0 : vir); es[5].add(img ? vir : (T)0);
         if (++cnt == CHUNK) { flush(g, G, 3); cnt = 0; }
     }
     flush(g, G, 3);
-    grad[(size_t)3 * si] = G[0];
-    grad[(size_t)3 * si + 1] = G[1];
-    grad[(size_t)3 * si + 2] = G[2];
-    double *eu = e_unit + NB_EU * (size_t)(nW + k);
-    eu[0] = elp; eu[1] = eli; eu[2] = eep; eu[3] = eei; eu[4] = (double)npair; eu[5] = 0.0;
-    eu[6] = vp; eu[7] = vi;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const long long v = sub_sum<32>(G[d]);
+        if (lane == d) grad[(size_t)3 * si + d] = v;
+    }
+    double e[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) e[m] = es[m].total32();
+    npair = sub_sum<32>(npair);
+    if (lane == 0) {
+        double *eu = e_unit + NB_EU * (size_t)(nW + k);
+        eu[0] = e[0]; eu[1] = e[1]; eu[2] = e[2]; eu[3] = e[3]; eu[4] = (double)npair; eu[5] = 0.0;
+        eu[6] = e[4]; eu[7] = e[5];
+    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -1018,22 +1042,26 @@ __global__ void k_excl_water(int nW, const int *__restrict__ unit_atom, const in
 }
 
 // exclusion erf corrections (cdie_ewald.f:117-199) and 1-4 terms (ener14.f:38-95), FP64,
-// gathered per atom over both directions; raw (unimaged) displacements as MOIL uses.
-// With skip_water set, water atoms are left to k_excl_water.
-__global__ void k_excl14(int natom, const int *__restrict__ atom_rep, const RepDev *__restrict__ reps,
+// gathered per atom over both directions; raw (unimaged) displacements as MOIL uses.  Eight
+// lanes per atom share its exclusions and 1-4 pairs (an erf, exp, square root and division in
+// FP64 each: one atom per thread ran about eight in series, 33 us whatever the system's size).
+// atoms: the n atoms to take (NULL: atom k itself); those left out belong to k_excl_water or
+// the FP32 water kernels.
+#define EX_LANES 8
+__global__ void k_excl14(int n, const int *__restrict__ atoms, const int *__restrict__ atom_rep, const RepDev *__restrict__ reps,
                          const double *__restrict__ coor, const double *__restrict__ q, const int *__restrict__ ex_off,
                          const int *__restrict__ ex_j, const int *__restrict__ p_off, const int *__restrict__ p_j,
-                         const double *__restrict__ p_par, const unsigned *__restrict__ aflags, int skip_water,
-                         int fixed_out, double *__restrict__ grad, double *__restrict__ e_out)
+                         const double *__restrict__ p_par, int fixed_out, double *__restrict__ grad,
+                         double *__restrict__ e_out)
 {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= natom) return;
-    if (skip_water && (aflags[a] & SF_WATER)) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, sub = t & (EX_LANES - 1), u = t / EX_LANES;
+    const bool act = u < n;
+    const int a = act ? (atoms ? atoms[u] : u) : 0;
     const RepDev &R = reps[atom_rep[a]];
     double xa = coor[3 * (size_t)a], ya = coor[3 * (size_t)a + 1], za = coor[3 * (size_t)a + 2];
     double gx = 0, gy = 0, gz = 0, ecorr = 0, eel14 = 0, evdw14 = 0, vir14 = 0;
     double qa = q[a] * R.epstmp, al = R.alphad;
-    for (int k = ex_off[a]; k < ex_off[a + 1]; ++k) {
+    for (int k = ex_off[a] + sub; act && k < ex_off[a + 1]; k += EX_LANES) {
         int b = ex_j[k];
         double rx = xa - coor[3 * (size_t)b], ry = ya - coor[3 * (size_t)b + 1], rz = za - coor[3 * (size_t)b + 2];
         double r2 = rx * rx + ry * ry + rz * rz, s2 = 1.0 / r2, rij = sqrt(r2), s = 1.0 / rij;
@@ -1044,7 +1072,7 @@ __global__ void k_excl14(int natom, const int *__restrict__ atom_rep, const RepD
         gx += df * rx; gy += df * ry; gz += df * rz;
         ecorr += 0.5 * e2;
     }
-    for (int k = p_off[a]; k < p_off[a + 1]; ++k) {
+    for (int k = p_off[a] + sub; act && k < p_off[a + 1]; k += EX_LANES) {
         int b = p_j[k];
         const double *p = p_par + 3 * (size_t)k;
         double rx = xa - coor[3 * (size_t)b], ry = ya - coor[3 * (size_t)b + 1], rz = za - coor[3 * (size_t)b + 2];
@@ -1065,6 +1093,10 @@ __global__ void k_excl14(int natom, const int *__restrict__ atom_rep, const RepD
         evdw14 += 0.5 * e1;
         eel14 += 0.5 * e2;
     }
+    gx = sub_sum<EX_LANES>(gx); gy = sub_sum<EX_LANES>(gy); gz = sub_sum<EX_LANES>(gz);
+    ecorr = sub_sum<EX_LANES>(ecorr); eel14 = sub_sum<EX_LANES>(eel14); evdw14 = sub_sum<EX_LANES>(evdw14);
+    vir14 = sub_sum<EX_LANES>(vir14);
+    if (!act || sub != 0) return;
     if (fixed_out) {   // mixed path: 2^32 fixed point, as the site gradients
         long long *gf = (long long *)grad + 3 * (size_t)a;
         gf[0] = __double2ll_rn(gx * NB_FIX_SCALE);
@@ -1133,8 +1165,9 @@ __global__ void k_final_grad(int natom, const int *__restrict__ site_of, const i
 //  k_energy_part: one block per chunk (EChunk: up to NB_FE_SEG consecutive units, atoms or PME
 //    column items of one replica); every thread streams the chunk's flat array with a stride
 //    that keeps its slot fixed (coalesced reads), the slots are summed by a halving tree;
-//  k_energy_final: one thread per replica adds its chunks' slot sums in chunk order and forms
-//    MOIL's energy names (pot/eforce.f:122-204).
+//  k_energy_final: one warp per replica adds its chunks' slot sums (a lane per slot and
+//    chunk modulo four, then a fixed tree) and forms MOIL's energy names (pot/eforce.f:122-204);
+//    one thread per replica took 23 us over the 34 chunks of the solute system.
 #define NB_FE_THREADS 256
 static_assert(NB_FE_THREADS % NB_EU == 0 && NB_FE_THREADS % NB_EX == 0, "slot-preserving stride");
 __global__ void __launch_bounds__(NB_FE_THREADS) k_energy_part(const EChunk *__restrict__ chunks,
@@ -1179,23 +1212,37 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_energy_part(const EChunk *__r
     }
 }
 
-__global__ void k_energy_final(int nrep, const RepDev *__restrict__ reps, const EChunk *__restrict__ chunks,
-                               const int *__restrict__ chunk_begin, const double *__restrict__ part,
-                               double *__restrict__ e_rep)
+__global__ void __launch_bounds__(128) k_energy_final(int nrep, const RepDev *__restrict__ reps,
+                                                      const EChunk *__restrict__ chunks,
+                                                      const int *__restrict__ chunk_begin,
+                                                      const double *__restrict__ part, double *__restrict__ e_rep)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, r = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (r >= nrep) return;
     const RepDev &R = reps[r];
-    double pw[NB_EU] = {0, 0, 0, 0, 0, 0, 0, 0}, po[NB_EU] = {0, 0, 0, 0, 0, 0, 0, 0};
-    double px[NB_EX] = {0, 0, 0, 0}, cl = 0.0;
-    for (int c = chunk_begin[r]; c < chunk_begin[r + 1]; ++c) {
-        const double *q = part + (size_t)NB_EU * c;
+    const int slot = lane % NB_EU;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};    // by chunk kind: this lane's slot over every fourth chunk
+    const int c1 = chunk_begin[r + 1];
+    for (int c = chunk_begin[r] + lane / NB_EU; c < c1; c += 32 / NB_EU) {
+        const double v = part[(size_t)NB_EU * c + slot];
         const int kind = chunks[c].kind;
-        if (kind == 0) { for (int k = 0; k < NB_EU; ++k) pw[k] += q[k]; }
-        else if (kind == 1) { for (int k = 0; k < NB_EU; ++k) po[k] += q[k]; }
-        else if (kind == 2) { for (int k = 0; k < NB_EX; ++k) px[k] += q[k]; }
-        else cl += q[0];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] += kind == q ? v : 0.0;
     }
+    double pw[NB_EU], po[NB_EU], px[NB_EX];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int o = NB_EU; o < 32; o <<= 1) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+#pragma unroll
+    for (int k = 0; k < NB_EU; ++k) {
+        pw[k] = __shfl_sync(0xffffffffu, a[0], k);
+        po[k] = __shfl_sync(0xffffffffu, a[1], k);
+    }
+#pragma unroll
+    for (int k = 0; k < NB_EX; ++k) px[k] = __shfl_sync(0xffffffffu, a[2], k);
+    const double cl = __shfl_sync(0xffffffffu, a[3], 0);
+    if (lane != 0) return;
     const double elp = 0.5 * (pw[0] + po[0]), eli = 0.5 * (pw[1] + po[1]);
     const double eep = 0.5 * (pw[2] + po[2]), eei = 0.5 * (pw[3] + po[3]);
     const double npairs = 0.5 * (pw[4] + po[4]);
@@ -1279,7 +1326,7 @@ void realspace_t(NbCtx *c)
     }
     if (c->timing) cudaEventRecord(c->ev[3], s);
     if (c->nA > 0) {
-        k_atom<T><<<(int)((c->nA + 127) / 128), 128, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep,
+        k_atom<T><<<(int)((c->nA + 3) / 4), 128, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep,
                                                              c->d_pos, c->d_site_lj, c->d_site_flags, c->d_xl_off,
                                                              c->d_xl, cap_int(c->cap_xl), c->d_grad_site, c->d_e_unit);
         c->launches++;
@@ -1365,9 +1412,11 @@ void nb_launch_excl14(NbCtx *c, const double *d_coor)
         c->launches++;
     }
     if (!fast || c->nA > 0) {
-        k_excl14<<<(int)((c->natom + 127) / 128), 128, 0, c->stream>>>(
-            (int)c->natom, c->d_atom_rep, c->d_reps, d_coor, c->d_q, c->d_ex_off, c->d_ex_j, c->d_p14_off,
-            c->d_p14_j, c->d_p14_par, c->d_aflags, fast, c->precision != MOIL_NB_FP64, c->d_grad_ex, c->d_e_ex);
+        // the atoms outside waters (the units after the waters), or all of them
+        const int64_t n = fast ? c->nA : c->natom;
+        k_excl14<<<(int)((n * EX_LANES + 127) / 128), 128, 0, c->stream>>>(
+            (int)n, fast ? c->d_unit_atom + c->nW : nullptr, c->d_atom_rep, c->d_reps, d_coor, c->d_q, c->d_ex_off,
+            c->d_ex_j, c->d_p14_off, c->d_p14_j, c->d_p14_par, c->precision != MOIL_NB_FP64, c->d_grad_ex, c->d_e_ex);
         c->launches++;
     }
 }
@@ -1385,7 +1434,7 @@ void nb_launch_finalize(NbCtx *c, double *d_dpot)
             (const float *)c->d_part, c->d_q, c->water_excl_fast ? (int)(3 * c->nW) : 0, d_dpot, c->d_status);
     k_energy_part<<<(int)c->echunks.size(), NB_FE_THREADS, 0, s>>>(c->d_echunks, c->d_e_unit, c->d_e_ex, c->d_e_col,
                                                                     c->d_epart);
-    k_energy_final<<<(c->nrep + 127) / 128, 128, 0, s>>>(c->nrep, c->d_reps, c->d_echunks, c->d_echunk_begin,
+    k_energy_final<<<(c->nrep + 3) / 4, 128, 0, s>>>(c->nrep, c->d_reps, c->d_echunks, c->d_echunk_begin,
                                                          c->d_epart, c->d_e_rep);
     c->launches += 3;
 }
