@@ -100,9 +100,18 @@ __device__ __forceinline__ void atom_pair_adj(const RepDev &R, double r2, double
     }
 }
 
-// water molecule per thread: W1 (nine site pairs per molecule pair) and W2
+// Sum over the W lanes of a subgroup (all lanes of the warp present)
+template <int W> __device__ __forceinline__ double lane_sum(double v)
+{
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, W);
+    return v;
+}
+
+// one warp per water: W1 (nine site pairs per molecule pair) and W2, the lanes taking the
+// entries of both lists in turn
 template <typename T, typename E>
-__global__ void k_adj_water(int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
+__global__ void __launch_bounds__(128) k_adj_water(int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
                             const int *__restrict__ site_orig, const void *pos_v, const void *woff_v,
                             const void *lj_v, const unsigned *__restrict__ sflags, const int2 *__restrict__ wl1_cnt,
                             const void *__restrict__ wl1, int cap_row, const int *__restrict__ wl2_off,
@@ -110,7 +119,7 @@ __global__ void k_adj_water(int nW, const RepDev *__restrict__ reps, const int *
                             double *__restrict__ ds)
 {
     typedef typename vec4<T>::type T4;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (i >= nW) return;
     const T4 *pos = (const T4 *)pos_v;
     const T4 *woff = (const T4 *)woff_v;
@@ -126,7 +135,7 @@ __global__ void k_adj_water(int nW, const RepDev *__restrict__ reps, const int *
     const int nn = min(c.x, cap_row), n = min(c.x + c.y, cap_row);
     const E *row = (const E *)wl1 + (size_t)i * cap_row;
     const int base = sizeof(E) == 2 ? R.wat0 : 0;   // uint16 entries: offsets from the replica's first water
-    for (int v = 0; v < n; ++v) {
+    for (int v = lane; v < n; v += 32) {
         const int j = base + (int)row[v < nn ? v : cap_row - 1 - (v - nn)];
         const T4 oj = pos[3 * j];
         T dx = oi.x - oj.x, dy = oi.y - oj.y, dz = oi.z - oj.z;
@@ -157,7 +166,7 @@ __global__ void k_adj_water(int nW, const RepDev *__restrict__ reps, const int *
             lj_adj(R.arith, R.w12d * s6 * s6, R.w6d * s6, epsO, sigO, sj, dE[0], dS[0]);
         }
     }
-    for (int k = min(wl2_off[i], cap2); k < min(wl2_off[i + 1], cap2); ++k) {
+    for (int k = min(wl2_off[i], cap2) + lane; k < min(wl2_off[i + 1], cap2); k += 32) {
         const int s = wl2[k];
         const T4 xj = pos[s];
         const double2 ljj = lj_of<T>(lj_v, s);
@@ -174,6 +183,8 @@ __global__ void k_adj_water(int nW, const RepDev *__restrict__ reps, const int *
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+        phi[a] = lane_sum<32>(phi[a]); dE[a] = lane_sum<32>(dE[a]); dS[a] = lane_sum<32>(dS[a]);
+        if (lane != a) continue;
         const int o = site_orig[3 * i + a];
         dq[o] = phi[a];
         de[o] = dE[a];
@@ -181,16 +192,16 @@ __global__ void k_adj_water(int nW, const RepDev *__restrict__ reps, const int *
     }
 }
 
-// non-water atom per thread over its X list
+// one warp per non-water atom over its X list
 template <typename T>
-__global__ void k_adj_atom(int nA, int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
+__global__ void __launch_bounds__(128) k_adj_atom(int nA, int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
                            const int *__restrict__ site_orig, const void *pos_v, const void *lj_v,
                            const unsigned *__restrict__ sflags, const int *__restrict__ xl_off,
                            const int *__restrict__ xl, int capx, double *__restrict__ dq, double *__restrict__ de,
                            double *__restrict__ ds)
 {
     typedef typename vec4<T>::type T4;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, k = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (k >= nA) return;
     const T4 *pos = (const T4 *)pos_v;
     const int si = 3 * nW + k;
@@ -198,7 +209,7 @@ __global__ void k_adj_atom(int nA, int nW, const RepDev *__restrict__ reps, cons
     const T4 xi = pos[si];
     const double2 lji = lj_of<T>(lj_v, si);
     double phi = 0, dE = 0, dS = 0;
-    for (int q = min(xl_off[k], capx); q < min(xl_off[k + 1], capx); ++q) {
+    for (int q = min(xl_off[k], capx) + lane; q < min(xl_off[k + 1], capx); q += 32) {
         const int s = xl[q];
         const T4 xj = pos[s];
         T dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -208,6 +219,8 @@ __global__ void k_adj_atom(int nA, int nW, const RepDev *__restrict__ reps, cons
         atom_pair_adj<T>(R, (double)(dx * dx + dy * dy + dz * dz), (double)xi.w, (double)xj.w, lji,
                          lj_of<T>(lj_v, s), sflags[si], sflags[s], phi, dE, dS);
     }
+    phi = lane_sum<32>(phi); dE = lane_sum<32>(dE); dS = lane_sum<32>(dS);
+    if (lane != 0) return;
     const int o = site_orig[si];
     dq[o] = phi;
     de[o] = dE;
@@ -286,8 +299,10 @@ __device__ __forceinline__ void atom_pair_adj_f(const RepDev &R, float r2, float
     }
 }
 
-// water molecule per thread (FP32 pairs): W1 (nine site pairs per molecule pair, O-O LJ) and W2
-template <typename E>
+// LPW lanes per water (FP32 pairs): W1 (nine site pairs per molecule pair, O-O LJ) and W2, the
+// lanes taking the entries of both lists in turn; their FP64 sums are added at the end.  One
+// water per thread: 249 us for the 460 waters of a small solute system.
+template <int LPW, typename E>
 __global__ void __launch_bounds__(128) k_adj_water_f(int nW, const RepDev *__restrict__ reps,
                                                      const int *__restrict__ site_rep,
                                                      const int *__restrict__ site_orig,
@@ -299,8 +314,9 @@ __global__ void __launch_bounds__(128) k_adj_water_f(int nW, const RepDev *__res
                                                      const int *__restrict__ wl2, int cap2, double *__restrict__ dq,
                                                      double *__restrict__ de, double *__restrict__ ds)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nW) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, sub = t & (LPW - 1);
+    const bool act = t / LPW < nW;
+    const int i = act ? t / LPW : nW - 1;    // idle lanes of the last block: empty lists, no output
     const RepDev &R = reps[site_rep[3 * i]];
     const float4 oi = woff[3 * i];
     const float4 h1 = woff[3 * i + 1], h2 = woff[3 * i + 2];
@@ -320,12 +336,11 @@ __global__ void __launch_bounds__(128) k_adj_water_f(int nW, const RepDev *__res
     const float inv2eO = epsO > 0.f ? 0.5f / epsO : 0.f, invsO = sigO > 0.f ? 1.f / sigO : 0.f;
     const float alpha = R.alpha, ex2c = R.ex2c, rmax2 = R.rmax2, rv2 = R.rv2, w12 = R.w12, w6 = R.w6;
     const int2 c = wl1_cnt[i];
-    const int nn = min(c.x, cap_row), n = min(c.x + c.y, cap_row);
+    const int nn = min(c.x, cap_row), n = act ? min(c.x + c.y, cap_row) : 0;
     const E *row = (const E *)wl1 + (size_t)i * cap_row;
     const int base = sizeof(E) == 2 ? R.wat0 : 0;   // uint16 entries: offsets from the replica's first water
     int cnt = 0;
-    for (int v = 0; v < n; ++v) {
-        nb_prefetch_l1(row + min(v + 32, n - 1));
+    for (int v = sub; v < n; v += LPW) {
         const int j = base + (int)row[v < nn ? v : cap_row - 1 - (v - nn)];
         const float4 oj = woff[3 * j];
         float dx = oi.x - oj.x, dy = oi.y - oj.y, dz = oi.z - oj.z;
@@ -357,7 +372,7 @@ __global__ void __launch_bounds__(128) k_adj_water_f(int nW, const RepDev *__res
     }
     flush();
     cnt = 0;
-    const int q0 = min(wl2_off[i], cap2), q1 = min(wl2_off[i + 1], cap2);
+    const int q0 = min(wl2_off[i], cap2), q1 = act ? min(wl2_off[i + 1], cap2) : q0;
     float inv2e[3], sg[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -367,7 +382,7 @@ __global__ void __launch_bounds__(128) k_adj_water_f(int nW, const RepDev *__res
         inv2e[a] = ea > 0.f ? 0.5f / ea : 0.f;
         sg[a] = sa;
     }
-    for (int k = q0; k < q1; ++k) {
+    for (int k = q0 + sub; k < q1; k += LPW) {
         const int s = wl2[k];
         const float4 xj = pos[s];
         const float2 ljj = lj[s];
@@ -387,6 +402,8 @@ __global__ void __launch_bounds__(128) k_adj_water_f(int nW, const RepDev *__res
     flush();
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+        phi[a] = lane_sum<LPW>(phi[a]); dE[a] = lane_sum<LPW>(dE[a]); dS[a] = lane_sum<LPW>(dS[a]);
+        if (!act || sub != a) continue;
         const int o = site_orig[3 * i + a];
         dq[o] = R.epstmp * phi[a];
         de[o] = dE[a];
@@ -394,7 +411,7 @@ __global__ void __launch_bounds__(128) k_adj_water_f(int nW, const RepDev *__res
     }
 }
 
-// non-water atom per thread over its X list (FP32 pairs)
+// one warp per non-water atom over its X list (FP32 pairs); one atom per thread: 434 us for 209 atoms
 __global__ void __launch_bounds__(128) k_adj_atom_f(int nA, int nW, const RepDev *__restrict__ reps,
                                                     const int *__restrict__ site_rep,
                                                     const int *__restrict__ site_orig, const float4 *__restrict__ pos,
@@ -403,7 +420,7 @@ __global__ void __launch_bounds__(128) k_adj_atom_f(int nA, int nW, const RepDev
                                                     double *__restrict__ dq, double *__restrict__ de,
                                                     double *__restrict__ ds)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, k = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (k >= nA) return;
     const int si = 3 * nW + k;
     const RepDev &R = reps[site_rep[si]];
@@ -417,8 +434,7 @@ __global__ void __launch_bounds__(128) k_adj_atom_f(int nA, int nW, const RepDev
     float p = 0.f, e1 = 0.f, s1 = 0.f;
     int cnt = 0;
     const int q1 = min(xl_off[k + 1], capx);
-    for (int q = min(xl_off[k], capx); q < q1; ++q) {
-        nb_prefetch_l1(xl + min(q + 32, q1 - 1));
+    for (int q = min(xl_off[k], capx) + lane; q < q1; q += 32) {
         const int s = xl[q];
         const float4 xj = pos[s];
         float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -431,49 +447,111 @@ __global__ void __launch_bounds__(128) k_adj_atom_f(int nA, int nW, const RepDev
             p = 0.f; e1 = 0.f; s1 = 0.f; cnt = 0;
         }
     }
-    phi += (double)p; dE += (double)e1; dS += (double)s1;
+    phi = lane_sum<32>(phi + (double)p); dE = lane_sum<32>(dE + (double)e1); dS = lane_sum<32>(dS + (double)s1);
+    if (lane != 0) return;
     const int o = site_orig[si];
     dq[o] = R.epstmp * phi;
     de[o] = dE;
     ds[o] = dS;
 }
 
-// per caller atom: exclusion erf corrections, 1-4 terms, self energy (FP64 coordinates)
-__global__ void k_adj_excl14(int natom, const int *__restrict__ atom_rep, const RepDev *__restrict__ reps,
-                             const double *__restrict__ coor, const double *__restrict__ q,
-                             const double2 *__restrict__ lj, const int *__restrict__ ex_off,
-                             const int *__restrict__ ex_j, const int *__restrict__ p_off, const int *__restrict__ p_j,
-                             const double *__restrict__ p_par, double *__restrict__ dq, double *__restrict__ de,
-                             double *__restrict__ ds)
+// erf(alpha r) / r of a squared distance: 2 alpha / sqrt(pi) times the Taylor series of
+// erf(x)/x in u = x^2 (Abramowitz & Stegun 7.1.5; 16 terms, exact to rounding for u <= 0.5),
+// erf beyond it
+__device__ __forceinline__ double erf_over_r(double al, double r2)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= natom) return;
+    const double u = al * al * r2;
+    if (u > 0.5) {
+        const double r = sqrt(r2);
+        return erf(al * r) / r;
+    }
+    const double c[16] = {1.0, -1.0 / 3, 1.0 / 10, -1.0 / 42, 1.0 / 216, -1.0 / 1320, 1.0 / 9360, -1.0 / 75600,
+                          1.0 / 685440, -1.0 / 6894720, 1.0 / 76204800, -1.0 / 918086400, 1.0 / 11975040000.0,
+                          -1.0 / 168129561600.0, 1.0 / 2528170444800.0, -1.0 / 40537905408000.0};
+    double s = c[15];
+#pragma unroll
+    for (int k = 14; k >= 0; --k) s = fma(s, u, c[k]);
+    return al * NB_TWO_OVER_SQRTPI * s;
+}
+
+// Exclusion erf corrections, 1-4 terms and the self energy of n atoms (FP64 coordinates), eight
+// lanes per atom; atoms: which (NULL: atom k itself)
+#define ADJ_EX_LANES 8
+__global__ void __launch_bounds__(128) k_adj_excl14(int n, const int *__restrict__ atoms,
+                                                    const int *__restrict__ atom_rep, const RepDev *__restrict__ reps,
+                                                    const double *__restrict__ coor, const double *__restrict__ q,
+                                                    const double2 *__restrict__ lj, const int *__restrict__ ex_off,
+                                                    const int *__restrict__ ex_j, const int *__restrict__ p_off,
+                                                    const int *__restrict__ p_j, const double *__restrict__ p_par,
+                                                    double *__restrict__ dq, double *__restrict__ de,
+                                                    double *__restrict__ ds)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, sub = t & (ADJ_EX_LANES - 1), u = t / ADJ_EX_LANES;
+    const bool act = u < n;
+    const int a = act ? (atoms ? atoms[u] : u) : 0;
     const RepDev &R = reps[atom_rep[a]];
     const double xa = coor[3 * (size_t)a], ya = coor[3 * (size_t)a + 1], za = coor[3 * (size_t)a + 2];
-    double phi = -2.0 * R.alphad * (NB_TWO_OVER_SQRTPI * 0.5) * R.epstmp * q[a];   // self energy
-    double dE = 0, dS = 0, ea, sa;
-    lj_decode(R.arith, lj[a].x, lj[a].y, ea, sa);
-    for (int k = ex_off[a]; k < ex_off[a + 1]; ++k) {
+    double phi = 0, dE = 0, dS = 0;
+    for (int k = ex_off[a] + sub; act && k < ex_off[a + 1]; k += ADJ_EX_LANES) {
         const int b = ex_j[k];
         const double rx = xa - coor[3 * (size_t)b], ry = ya - coor[3 * (size_t)b + 1], rz = za - coor[3 * (size_t)b + 2];
-        const double r = sqrt(rx * rx + ry * ry + rz * rz);
-        phi -= R.epstmp * q[b] * erf(R.alphad * r) / r;
+        phi -= R.epstmp * q[b] * erf_over_r(R.alphad, rx * rx + ry * ry + rz * rz);
     }
-    for (int k = p_off[a]; k < p_off[a + 1]; ++k) {
-        const int b = p_j[k];
-        const double *p = p_par + 3 * (size_t)k;
-        const double rx = xa - coor[3 * (size_t)b], ry = ya - coor[3 * (size_t)b + 1], rz = za - coor[3 * (size_t)b + 2];
-        const double s2 = 1.0 / (rx * rx + ry * ry + rz * rz), s6 = s2 * s2 * s2;
-        if (p[0] > 1e-12) {
-            double eb, sb;
-            lj_decode(R.arith, lj[b].x, lj[b].y, eb, sb);
-            lj_adj(R.arith, p[0] * s6 * s6, p[1] * s6, ea, sa, sb, dE, dS);
+    const int p0 = p_off[a], p1 = p_off[a + 1];
+    if (act && p0 + sub < p1) {
+        double ea, sa;
+        lj_decode(R.arith, lj[a].x, lj[a].y, ea, sa);
+        for (int k = p0 + sub; k < p1; k += ADJ_EX_LANES) {
+            const int b = p_j[k];
+            const double *p = p_par + 3 * (size_t)k;
+            const double rx = xa - coor[3 * (size_t)b], ry = ya - coor[3 * (size_t)b + 1], rz = za - coor[3 * (size_t)b + 2];
+            const double s2 = 1.0 / (rx * rx + ry * ry + rz * rz), s6 = s2 * s2 * s2;
+            if (p[0] > 1e-12) {
+                double eb, sb;
+                lj_decode(R.arith, lj[b].x, lj[b].y, eb, sb);
+                lj_adj(R.arith, p[0] * s6 * s6, p[1] * s6, ea, sa, sb, dE, dS);
+            }
+            if (fabs(p[2]) > 1e-12 && fabs(q[a]) > 1e-12) phi += p[2] / q[a] * sqrt(s2);
         }
-        if (fabs(p[2]) > 1e-12 && fabs(q[a]) > 1e-12) phi += p[2] / q[a] * sqrt(s2);
     }
+    phi = lane_sum<ADJ_EX_LANES>(phi); dE = lane_sum<ADJ_EX_LANES>(dE); dS = lane_sum<ADJ_EX_LANES>(dS);
+    if (!act || sub != 0) return;
+    phi -= 2.0 * R.alphad * (NB_TWO_OVER_SQRTPI * 0.5) * R.epstmp * q[a];   // self energy
     dq[a] += phi;
     de[a] += dE;
     ds[a] += dS;
+}
+
+// The same for waters whose exclusions are exactly their three pairs (no 1-4 terms): one water
+// per thread, each pair's FP64 series once
+__global__ void __launch_bounds__(128) k_adj_excl_water(int nW, const int *__restrict__ unit_atom,
+                                                        const int *__restrict__ atom_rep,
+                                                        const RepDev *__restrict__ reps,
+                                                        const double *__restrict__ coor, const double *__restrict__ q,
+                                                        double *__restrict__ dq)
+{
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= nW) return;
+    const int a0 = unit_atom[u];
+    const RepDev &R = reps[atom_rep[a0]];
+    double x[3][3], qs[3], phi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x[k][d] = coor[3 * (size_t)(a0 + k) + d];
+        qs[k] = q[a0 + k];
+        phi[k] = -2.0 * R.alphad * (NB_TWO_OVER_SQRTPI * 0.5) * qs[k];          // self energy
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const int a = p < 2 ? 0 : 1, b = p < 1 ? 1 : 2;
+        const double rx = x[a][0] - x[b][0], ry = x[a][1] - x[b][1], rz = x[a][2] - x[b][2];
+        const double w = erf_over_r(R.alphad, rx * rx + ry * ry + rz * rz);
+        phi[a] -= qs[b] * w;
+        phi[b] -= qs[a] * w;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) dq[a0 + k] += R.epstmp * phi[k];
 }
 
 // PME: fc * sum(theta * potential grid) at each site, from the real planes k_plane_inv_f
@@ -499,23 +577,31 @@ __global__ void k_adj_pme_f(int nsite, const int *__restrict__ site_rep, const i
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double u = w[d], u2 = u * u, u3 = u2 * u, m = 1.0 - u;
-        th[d][0] = m * m * m / 6.0;
-        th[d][1] = (4.0 - 6.0 * u2 + 3.0 * u3) / 6.0;
-        th[d][2] = (1.0 + 3.0 * (u + u2 - u3)) / 6.0;
-        th[d][3] = u3 / 6.0;
+        th[d][0] = m * m * m;                       // 6 theta: 1/216 is applied to the sum
+        th[d][1] = 4.0 - 6.0 * u2 + 3.0 * u3;
+        th[d][2] = 1.0 + 3.0 * (u + u2 - u3);
+        th[d][3] = u3;
     }
     auto wrap = [](int k, int n) { return k < 0 ? k + n : (k >= n ? k - n : k); };
+    int xs[4];
+#pragma unroll
+    for (int t1 = 0; t1 < 4; ++t1) xs[t1] = wrap(i1 - 3 + t1, n1);
     double v = 0.0;
+#pragma unroll
     for (int t3 = 0; t3 < 4; ++t3) {
         const float *P = Q + wrap(i3 - 3 + t3, n3) * zs;
+        double sy = 0.0;
+#pragma unroll
         for (int t2 = 0; t2 < 4; ++t2) {
             const float *row = P + wrap(i2 - 3 + t2, n2) * n1;
             double sx = 0.0;
-            for (int t1 = 0; t1 < 4; ++t1) sx += th[0][t1] * (double)row[wrap(i1 - 3 + t1, n1)];
-            v += sx * th[1][t2] * th[2][t3];
+#pragma unroll
+            for (int t1 = 0; t1 < 4; ++t1) sx += th[0][t1] * (double)row[xs[t1]];
+            sy += sx * th[1][t2];
         }
+        v += sy * th[2][t3];
     }
-    dq[site_orig[s]] += R.fcd * v;
+    dq[site_orig[s]] += R.fcd * v * (1.0 / 216.0);
 }
 
 // PME on the plain path: fc * the four plane shares of the potential at each site
@@ -534,25 +620,29 @@ void adjoint_pairs(NbCtx *c, double *d_dq, double *d_de, double *d_ds)
     cudaStream_t s = c->stream;
     const int B = 128;
     if constexpr (sizeof(T) == 4) {
+        // lanes per water as the energy kernel (32-bit rows belong to replicas of 65,536 waters or more)
+        const int lpw = c->nw_handle <= 4096 ? 32 : 8;
         if (c->nW > 0)
-            (c->row16 ? k_adj_water_f<unsigned short> : k_adj_water_f<int>)<<<(int)((c->nW + B - 1) / B), B, 0, s>>>(
+            (!c->row16 ? k_adj_water_f<8, int>
+                       : (lpw == 32 ? k_adj_water_f<32, unsigned short> : k_adj_water_f<8, unsigned short>))<<<
+                (int)((c->nW * lpw + B - 1) / B), B, 0, s>>>(
                 (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, (const float4 *)c->d_pos,
                 (const float4 *)c->d_woff, (const float2 *)c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1,
                 c->cap_row1, c->d_wl2_off, c->d_wl2, cap_int(c->cap_wl2), d_dq, d_de, d_ds);
         if (c->nA > 0)
-            k_adj_atom_f<<<(int)((c->nA + B - 1) / B), B, 0, s>>>(
+            k_adj_atom_f<<<(int)((c->nA + 3) / 4), B, 0, s>>>(
                 (int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, (const float4 *)c->d_pos,
                 (const float2 *)c->d_site_lj, c->d_site_flags, c->d_xl_off, c->d_xl, cap_int(c->cap_xl), d_dq, d_de,
                 d_ds);
         return;
     }
     if (c->nW > 0)
-        (c->row16 ? k_adj_water<T, unsigned short> : k_adj_water<T, int>)<<<(int)((c->nW + B - 1) / B), B, 0, s>>>(
+        (c->row16 ? k_adj_water<T, unsigned short> : k_adj_water<T, int>)<<<(int)((c->nW + 3) / 4), B, 0, s>>>(
             (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_woff, c->d_site_lj,
             c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2, cap_int(c->cap_wl2), d_dq,
             d_de, d_ds);
     if (c->nA > 0)
-        k_adj_atom<T><<<(int)((c->nA + B - 1) / B), B, 0, s>>>(
+        k_adj_atom<T><<<(int)((c->nA + 3) / 4), B, 0, s>>>(
             (int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_site_lj,
             c->d_site_flags, c->d_xl_off, c->d_xl, cap_int(c->cap_xl), d_dq, d_de, d_ds);
 }
@@ -567,9 +657,15 @@ int nb_adjoint(NbCtx *c, double *d_dq, double *d_de, double *d_ds)
     const int B = 128;
     if (c->precision == MOIL_NB_FP64) adjoint_pairs<double>(c, d_dq, d_de, d_ds);
     else adjoint_pairs<float>(c, d_dq, d_de, d_ds);
-    k_adj_excl14<<<(int)((c->natom + B - 1) / B), B, 0, s>>>(
-        (int)c->natom, c->d_atom_rep, c->d_reps, c->d_coor, c->d_q, c->d_lj_d, c->d_ex_off, c->d_ex_j,
-        c->d_p14_off, c->d_p14_j, c->d_p14_par, d_dq, d_de, d_ds);
+    const bool fast = c->water_excl_fast && c->nW > 0;
+    if (fast)
+        k_adj_excl_water<<<(int)((c->nW + B - 1) / B), B, 0, s>>>((int)c->nW, c->d_unit_atom, c->d_atom_rep, c->d_reps,
+                                                                 c->d_coor, c->d_q, d_dq);
+    const int64_t n = fast ? c->nA : c->natom;
+    if (n > 0)
+        k_adj_excl14<<<(int)((n * ADJ_EX_LANES + B - 1) / B), B, 0, s>>>(
+            (int)n, fast ? c->d_unit_atom + c->nW : nullptr, c->d_atom_rep, c->d_reps, c->d_coor, c->d_q, c->d_lj_d,
+            c->d_ex_off, c->d_ex_j, c->d_p14_off, c->d_p14_j, c->d_p14_par, d_dq, d_de, d_ds);
     if (c->precision == MOIL_NB_FP64) {
         nb_launch_pme_potential(c, c->d_adj_phi);
         k_adj_pme_d<<<(int)((c->nsite + B - 1) / B), B, 0, s>>>((int)c->nsite, c->d_site_rep, c->d_site_orig,
