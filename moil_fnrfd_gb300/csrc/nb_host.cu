@@ -213,7 +213,9 @@ int alloc_half(NbCtx *c)
 // of 256 waters per multiprocessor leaves most of the GPU idle below it, while the full-list
 // kernel spreads each water over 8 or 32 lanes.  One evaluation in us, half / full lists:
 // 216 waters 116 / 98, 3,000 154 / 126, 12,000 210 / 177, 19,272 (24 replicas) 167 / 145,
-// 20,000 (one box) 200 / 214, 32,000 248 / 264.
+// 20,000 (one box) 200 / 214, 32,000 248 / 264.  Handles with atoms outside waters take full lists
+// at every size: the half-list kernel runs a water's list of them in one thread (water stage of
+// eight solute systems, 56,160 waters: 394 / 150 us).
 #define NB_FULL_MAX_WATERS 19500
 
 // Half-list set-up for the current shape: on for FP32 handles whose replicas all have fewer
@@ -226,7 +228,7 @@ int setup_half(NbCtx *c)
     free_ptr(c->d_hrow); free_ptr(c->d_jset);
     c->hblocks.clear();
     c->whalf = c->precision != MOIL_NB_FP64 && c->row16 && c->nW > 0 && c->want_whalf != MOIL_NB_WATER_FULL;
-    if (c->want_whalf == MOIL_NB_WATER_AUTO && c->nw_handle <= NB_FULL_MAX_WATERS) c->whalf = 0;
+    if (c->want_whalf == MOIL_NB_WATER_AUTO && (c->nw_handle <= NB_FULL_MAX_WATERS || c->na_handle > 0)) c->whalf = 0;
     if (!c->whalf) return MOIL_NB_OK;
     int maxw = 0;
     for (int r = 0; r < c->nrep; ++r) {
@@ -523,6 +525,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     c->nW = wat0;
     c->nA = oth0;
     c->nw_handle = std::max(c->nw_handle, c->nW);
+    c->na_handle = std::max(c->na_handle, c->nA);
     c->row16 = 1;
     for (int r = 0; r < nrep; ++r) c->row16 &= c->rd[r].nwat < 65536;
     c->nsite = 3 * c->nW + c->nA;
@@ -723,7 +726,8 @@ void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot)
     }
     if (c->timing) {
         // stage timing: one stream, stage after stage
-        nb_launch_realspace(c);
+        nb_launch_water(c);
+        nb_launch_atoms(c);
         nb_launch_excl14(c, d_coor);
         cudaEventRecord(c->ev[5], s);
         nb_launch_pme(c);
@@ -738,9 +742,19 @@ void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot)
         nb_launch_pme(c);
         std::swap(c->stream, c->stream2);
         cudaEventRecord(c->ev_join, c->stream2);
-        nb_launch_realspace(c);
-        nb_launch_excl14(c, d_coor);
+        // the non-water pair and the correction kernels (FP64) likewise, on a third
+        const bool third = c->nA > 0 || !c->water_excl_fast || c->precision == MOIL_NB_FP64;
+        if (third) {
+            cudaStreamWaitEvent(c->stream3, c->ev_fork, 0);
+            std::swap(c->stream, c->stream3);
+            nb_launch_atoms(c);
+            nb_launch_excl14(c, d_coor);
+            std::swap(c->stream, c->stream3);
+            cudaEventRecord(c->ev_join3, c->stream3);
+        }
+        nb_launch_water(c);
         cudaStreamWaitEvent(s, c->ev_join, 0);
+        if (third) cudaStreamWaitEvent(s, c->ev_join3, 0);
     }
     nb_launch_finalize(c, d_dpot);
 }
@@ -1007,6 +1021,7 @@ int eval_groups(NbCtx *h, const double *coor, double *dpot, moil_energies *e, bo
             if (c->pstream) {
                 std::swap(c->stream, c->pstream);
                 std::swap(c->stream2, c->pstream2);
+                std::swap(c->stream3, c->pstream3);
                 c->on_prio = on ? 1 : 0;
             }
     };
@@ -1114,6 +1129,7 @@ int init_groups(moil_nb_ctx *h, int nrep, const moil_replica *reps, int P)
         c->hb = h->hb;
         c->want_tiled = h->want_tiled;
         c->nw_handle = nwat;
+        c->na_handle = total - 3 * nwat;
         {
             // streams for host-buffer evaluations: earlier groups at higher priority finish
             // first, so their gradient copies overlap the later groups' kernels (device-
@@ -1122,7 +1138,8 @@ int init_groups(moil_nb_ctx *h, int nrep, const moil_replica *reps, int P)
             cudaDeviceGetStreamPriorityRange(&lo, &hi);
             const int prio = std::min(lo, hi + (int)g);
             if (cudaStreamCreateWithPriority(&c->pstream, cudaStreamNonBlocking, prio) != cudaSuccess ||
-                cudaStreamCreateWithPriority(&c->pstream2, cudaStreamNonBlocking, prio) != cudaSuccess) {
+                cudaStreamCreateWithPriority(&c->pstream2, cudaStreamNonBlocking, prio) != cudaSuccess ||
+                cudaStreamCreateWithPriority(&c->pstream3, cudaStreamNonBlocking, prio) != cudaSuccess) {
                 h->err = "creating replica group streams";
                 h->grp.push_back(c);
                 destroy_groups(h);
@@ -1163,11 +1180,15 @@ int moil_nb_create(moil_nb_ctx **out, int device)
     h->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&h->stream3, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&h->ev_join3, cudaEventDisableTiming) != cudaSuccess) {
         if (h->stream) cudaStreamDestroy(h->stream);
         if (h->stream2) cudaStreamDestroy(h->stream2);
+        if (h->stream3) cudaStreamDestroy(h->stream3);
         if (h->ev_fork) cudaEventDestroy(h->ev_fork);
+        if (h->ev_join) cudaEventDestroy(h->ev_join);
         delete h;
         return MOIL_NB_ERR_CUDA;
     }
@@ -1195,10 +1216,13 @@ void moil_nb_destroy(moil_nb_ctx *h)
     if (h->h_status) cudaFreeHost(h->h_status);
     if (h->d_status) cudaFree(h->d_status);
     if (h->stream2) { cudaStreamSynchronize(h->stream2); cudaStreamDestroy(h->stream2); }
+    if (h->stream3) { cudaStreamSynchronize(h->stream3); cudaStreamDestroy(h->stream3); }
     if (h->sbody) cudaStreamDestroy(h->sbody);
     if (h->sstep) cudaStreamDestroy(h->sstep);
     if (h->pstream) cudaStreamDestroy(h->pstream);
     if (h->pstream2) cudaStreamDestroy(h->pstream2);
+    if (h->pstream3) cudaStreamDestroy(h->pstream3);
+    if (h->ev_join3) cudaEventDestroy(h->ev_join3);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -1211,7 +1235,7 @@ int moil_nb_init(moil_nb_ctx *h, const moil_nb_params *p, const moil_topology *t
     moil_replica r = {p, t};
     cudaSetDevice(h->device);
     destroy_groups(h);
-    h->nw_handle = 0;
+    h->nw_handle = h->na_handle = 0;
     return init_impl(h, 1, &r);
 }
 
@@ -1228,7 +1252,7 @@ int moil_nb_init_batch(moil_nb_ctx *h, int nrep, const moil_replica *reps)
     }
     if (reps) nb_tune_cached_shape(h, nrep, reps);
     const int P = reps ? choose_groups(h, nrep, natom) : 1;
-    h->nw_handle = 0;
+    h->nw_handle = h->na_handle = 0;
     if (P <= 1) return init_impl(h, nrep, reps);
     if (h->inited) release_device(h);
     h->inited = 0;

@@ -37,11 +37,12 @@ struct NbCtx {
     int nsm = 152;                // multiprocessors: grids of the rebuild-gated kernels stay one wave
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;   // PME branch of an evaluation, concurrent with the pair kernels
+    cudaStream_t stream3 = nullptr;   // non-water pair and correction kernels, beside the water kernel
     cudaStream_t sbody = nullptr;     // captures the list rebuild into the conditional node's body
     cudaStream_t sstep = nullptr;     // captures an MD step into its gate node's body
     int capturing = 0;                // the evaluation is being captured into the handle's graph
-    cudaStream_t pstream = nullptr, pstream2 = nullptr;   // replica groups: prioritised by group index
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaStream_t pstream = nullptr, pstream2 = nullptr, pstream3 = nullptr;   // replica groups: prioritised by group index
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
     int precision = MOIL_NB_MIXED;
     int inited = 0;
     std::string err;
@@ -53,6 +54,7 @@ struct NbCtx {
     RepDev *d_reps = nullptr;
     int64_t natom = 0, nW = 0, nA = 0, nsite = 0, nunit = 0;
     int64_t nw_handle = 0;        // waters of the whole handle: all replica groups together
+    int64_t na_handle = 0;        // its atoms outside waters
     float skin = 1.0f, rwat = 1.1f;
     int list_period = 0;
     int water_excl_fast = 0;      // every water's exclusions are exactly O-H1, O-H2, H1-H2
@@ -243,7 +245,8 @@ void nb_launch_rebuild_cond(NbCtx *c, cudaGraphConditionalHandle h);
 void nb_launch_prepare(NbCtx *c, const double *d_coor, int check);
 void nb_exclusive_scan(NbCtx *c, const int *d_in, int *d_out, int n, int *d_total);
 // real space + corrections (nb_realspace.cu)
-void nb_launch_realspace(NbCtx *c);
+void nb_launch_water(NbCtx *c);      // water molecules: W1 and W2 lists
+void nb_launch_atoms(NbCtx *c);      // atoms outside waters: X lists
 // half-list water kernel: dynamic shared memory for c->jcap; MOIL_NB_OK if it fits the device
 int nb_half_configure(NbCtx *c);
 // the half-list kernel still fits its two (256-water) or four (128) resident blocks per SM

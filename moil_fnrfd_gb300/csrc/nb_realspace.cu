@@ -1278,8 +1278,9 @@ WaterHFn water_h_fn(int hb, bool vir)
 // partly filled rounds and to the sum over the lanes.  Water stage in us at 32 / 8 / 4 lanes:
 // 1,334 waters 16 / 26 / 38, 3,000 17 / 22 / 38, 7,000 32 / 24 / 40, 12,000 42 / 30 / 40, 32,000
 // 112 / 84 / 89, 110,860 (64 replicas) 339 / 206 / 194, 433,195 1304 / 743 / 678 (one water per
-// thread: 78, 79, 82, 79, 120, 204, 657).
-int water_lanes(const NbCtx *c) { return c->nw_handle <= 4096 ? 32 : (c->nw_handle <= 32768 ? 8 : 4); }
+// thread: 78, 79, 82, 79, 120, 204, 657).  With atoms outside waters a water also has a list of
+// those: 8 lanes for the large ones.
+int water_lanes(const NbCtx *c) { return c->nw_handle <= 4096 ? 32 : (c->nw_handle <= 32768 || c->na_handle > 0 ? 8 : 4); }
 
 using WaterSFn = decltype(&k_water_s<8, false, int>);
 WaterSFn water_s_fn(int lpw, bool vir, bool row16)
@@ -1294,7 +1295,7 @@ WaterSFn water_s_fn(int lpw, bool vir, bool row16)
 }
 
 template <typename T>
-void realspace_t(NbCtx *c)
+void water_t(NbCtx *c)
 {
     cudaStream_t s = c->stream;
     if (c->timing) cudaEventRecord(c->ev[2], s);
@@ -1325,6 +1326,12 @@ void realspace_t(NbCtx *c)
         c->launches++;
     }
     if (c->timing) cudaEventRecord(c->ev[3], s);
+}
+
+template <typename T>
+void atoms_t(NbCtx *c)
+{
+    cudaStream_t s = c->stream;
     if (c->nA > 0) {
         k_atom<T><<<(int)((c->nA + 3) / 4), 128, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep,
                                                              c->d_pos, c->d_site_lj, c->d_site_flags, c->d_xl_off,
@@ -1336,10 +1343,16 @@ void realspace_t(NbCtx *c)
 
 }  // namespace
 
-void nb_launch_realspace(NbCtx *c)
+void nb_launch_water(NbCtx *c)
 {
-    if (c->precision == MOIL_NB_FP64) realspace_t<double>(c);
-    else realspace_t<float>(c);
+    if (c->precision == MOIL_NB_FP64) water_t<double>(c);
+    else water_t<float>(c);
+}
+
+void nb_launch_atoms(NbCtx *c)
+{
+    if (c->precision == MOIL_NB_FP64) atoms_t<double>(c);
+    else atoms_t<float>(c);
 }
 
 // shared-memory carveout (percent of the per-SM maximum) for `bytes` of resident blocks
