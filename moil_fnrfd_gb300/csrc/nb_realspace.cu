@@ -439,6 +439,13 @@ __device__ __forceinline__ float ewald1(const WaterK &K, float rr2, float rinv, 
     e = qq * (ex * (tt * p)) * rinv;
     return fmaf(qq * K.c2a, ex, e) * (rinv * rinv);
 }
+// a value the compiler holds instead of loading it again (the replica's constants inside the pair
+// loops: 2.5% of the water stage)
+__device__ __forceinline__ float held(float x)
+{
+    asm volatile("" : "+f"(x));
+    return x;
+}
 // hi + lo += v (TwoSum, Knuth: the rounding error of hi + v collects in lo)
 __device__ __forceinline__ void two_add(float2 &a, float v)
 {
@@ -463,7 +470,7 @@ template <int W> __device__ __forceinline__ float2 sub_two_sum(float2 a)
 // partner site) -- and the O-O pair with its LJ part runs scalar, so one partner record is
 // live at a time.  VIR: also the water-water LJ virial terms.
 template <int LPW, bool VIR, typename E>
-__global__ void __launch_bounds__(WBLOCK, 5) k_water_s(int nW, const RepDev *__restrict__ reps,
+__global__ void __launch_bounds__(WBLOCK, 4) k_water_s(int nW, const RepDev *__restrict__ reps,
                                                        const int *__restrict__ site_rep, const float4 *__restrict__ pos,
                                                        const float4 *__restrict__ woff, const void *lj_v,
                                                        const unsigned *__restrict__ sflags,
@@ -512,30 +519,25 @@ __global__ void __launch_bounds__(WBLOCK, 5) k_water_s(int nW, const RepDev *__r
         flush_e();
     };
     int npair = 0;
-    const float iL0 = R.invL[0], iL1 = R.invL[1], iL2 = R.invL[2];
-    const float rmax2 = R.rmax2, rv2 = R.rv2;
-    const WaterK K = {ERFCX_P * R.alpha, R.ex2c, R.c2a};
-    const float qOO = R.qq[0], qOH = R.qq[1], qHH = R.qq[2], w12 = R.w12, w6 = R.w6;
-    const W1Row<E> L1(wl1_cnt, wl1, cap_row, i, R.wat0);
-    const int n = act ? L1.n : 0;
-    // two iterations ahead the entry, one ahead the partner's oxygen
-    int j1 = sub < n ? L1.at(sub) : i, j2 = sub + LPW < n ? L1.at(sub + LPW) : i;
-    float4 o1 = woff[3 * j1];
-    int cnt = 0;
-    for (int k = sub; k < n; k += LPW) {
-        const int j = j1;
-        const float4 oj = o1;
-        j1 = j2;
-        o1 = woff[3 * j1];
-        if (k + 2 * LPW < n) j2 = L1.at(k + 2 * LPW);
+    const float iL0 = held(R.invL[0]), iL1 = held(R.invL[1]), iL2 = held(R.invL[2]);
+    const float L0 = held(R.L[0]), L1 = held(R.L[1]), L2 = held(R.L[2]);
+    const float m0 = held(R.Llo[0]), m1 = held(R.Llo[1]), m2 = held(R.Llo[2]);
+    const float rmax2 = held(R.rmax2), rv2 = held(R.rv2);
+    const WaterK K = {held(ERFCX_P * R.alpha), held(R.ex2c), held(R.c2a)};
+    const float qOO = held(R.qq[0]), qOH = held(R.qq[1]), qHH = held(R.qq[2]), w12 = held(R.w12), w6 = held(R.w6);
+    const float w12c = held(R.w12c), w6c = held(R.w6c);
+    const bool sw = R.lj_switch != 0;
+    const W1Row<E> row(wl1_cnt, wl1, cap_row, i, R.wat0);
+    const int n = act ? row.n : 0;
+    // one molecule pair: the partner's record (O, then the H offsets)
+    auto pair = [&](float4 oj, float4 a, float4 b) {
         float dx = oi0.x - oj.x, dy = oi0.y - oj.y, dz = oi0.z - oj.z;
         // (x + 1.5*2^23) - 1.5*2^23 rounds x to nearest (|x| < 2^22)
         const float nx = fmaf(dx, iL0, 12582912.f) - 12582912.f, ny = fmaf(dy, iL1, 12582912.f) - 12582912.f,
                     nz = fmaf(dz, iL2, 12582912.f) - 12582912.f;
-        dx = nb_shift(R, 0, dx, nx); dy = nb_shift(R, 1, dy, ny); dz = nb_shift(R, 2, dz, nz);
+        dx = fmaf(-nx, m0, fmaf(-nx, L0, dx)); dy = fmaf(-ny, m1, fmaf(-ny, L1, dy)); dz = fmaf(-nz, m2, fmaf(-nz, L2, dz));
         const float r2 = dx * dx + dy * dy + dz * dz;
         if (r2 <= rmax2) {
-            const float4 a = woff[3 * j + 1], b = woff[3 * j + 2];
             float2 eel, e;
             float eoo, elj = 0.f, vlj = 0.f;
             {
@@ -549,9 +551,9 @@ __global__ void __launch_bounds__(WBLOCK, 5) k_water_s(int nW, const RepDev *__r
                     const float s6 = sl * sl * sl, A = w12 * s6 * s6;
                     // c12, c6 restore the FP32 rounding of the coefficients in the energy (the force
                     // keeps A and B)
-                    float e1 = fmaf(-w6, fmaf(s6, R.w6c, s6), fmaf(A, R.w12c, A));
+                    float e1 = fmaf(-w6, fmaf(s6, w6c, s6), fmaf(A, w12c, A));
                     float m1 = 6.f * sl * fmaf(-w6, s6, A + A);
-                    if (R.lj_switch) {
+                    if (sw) {
                         float d1 = -m1;
                         lj_switch_apply<float>(R, rr2, e1, d1);
                         m1 = -d1;
@@ -587,8 +589,29 @@ __global__ void __launch_bounds__(WBLOCK, 5) k_water_s(int nW, const RepDev *__r
             if (VIR) { e4[NE - 2] += img ? 0.f : vlj; e4[NE - 1] += img ? vlj : 0.f; }
             npair += 9;
         }
-        if (++cnt == CHUNK) { flush_all(); cnt = 0; }
+    };
+    // two record buffers in turn, as in k_water_h: the next entry's record is on its way while one is
+    // worked on, row entries two ahead of their records
+    int cnt = 0;
+    if (sub < n) {
+        auto entry = [&](int k) { return row.at(min(k, n - 1)); };
+        int ja = entry(sub), jb = entry(sub + LPW);
+        const float4 *r = woff + 3 * (size_t)ja;
+        float4 oa = r[0], ha = r[1], ia = r[2];
+        for (int k = sub; k < n; k += 2 * LPW) {
+            const int jc = entry(k + 2 * LPW), jd = entry(k + 3 * LPW);
+            r = woff + 3 * (size_t)jb;
+            const float4 ob = r[0], hb = r[1], ib = r[2];
+            pair(oa, ha, ia);
+            r = woff + 3 * (size_t)jc;
+            oa = r[0]; ha = r[1]; ia = r[2];
+            if (k + LPW < n) pair(ob, hb, ib);
+            jb = jd;
+            cnt += 2;
+            if (cnt >= CHUNK) { flush_all(); cnt = 0; }
+        }
     }
+    __syncwarp();     // rows differ in length: the lanes that end early wait here
     fold();
     if (act) {
         water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, sub, LPW, cnt, g, e4, npair, flush_all);
@@ -625,16 +648,24 @@ __global__ void __launch_bounds__(WBLOCK, 5) k_water_s(int nW, const RepDev *__r
 
 // ---------------------------------------------------------------------------------
 // FP32 water kernel over half lists (k_whalf): every water-water pair is evaluated once, by
-// its owner, two list entries packed on the FP32x2 pipe (a molecule outside the O-O cutoff, or the
-// missing partner of an odd tail, is moved 1e4 Å away, where erfc and exp underflow to exactly
-// zero).  The owner keeps its own gradient in registers; the partner's side of each pair (per partner site, summed over the owner's three
-// sites) goes to an int32 accumulator in shared memory indexed by the partner's place in the
-// block's j-set, at 2^S units per kcal/mol/Å (S = 24 - log2 HB: HB contributions below
-// NB_HALF_CAP in magnitude fit); larger contributions go directly to the int64 gradient.
-// At the end the block adds its j-set sums and its own waters' gradients to the int64 site
-// gradient with atomics (integer sums: the result does not depend on their order).  The
-// site gradient of the waters is cleared before the launch.  Water-water energies and pair
-// counts are doubled, as the energy reduction halves the full-list sums.
+// its owner, with the pair arithmetic of k_water_s (eight of the nine site pairs packed two by
+// two).  One water per thread, whose gradient stays in registers; the partner's side of each
+// pair goes to an int32 accumulator in shared memory indexed by the partner's place in the
+// block's j-set, at 2^S units per kcal/mol/Å (S = 24 - log2 HB).  A share is rounded to the unit by
+// adding 1.5 * 2^23 (a conversion would share the special-function pipe with rsqrt, rcp and
+// ex2), so it has to stay below 2^22 units, and HB of those cannot overflow; larger shares go
+// directly to the int64 gradient.  At the end the block adds its j-set sums and its own waters'
+// gradients to the int64 site gradient with atomics (integer sums: the result does not depend
+// on their order).  The site gradient of the waters is cleared before the launch.  Water-water
+// energies and pair counts are doubled, as the energy reduction halves the full-list sums.
+// Bound: instruction issue at the 16 warps that 128 registers allow, then the latency of the
+// partner gathers.  Two list entries per iteration packed on the FP32x2 pipe left 4 warps in 10
+// waiting for gathers (issue 35%): the hydrogens' loads depended on the O-O test, and lanes with
+// short rows ran the flush apart from the others.  Water stage, 256 replicas (433,195 waters):
+// 625 us; whole records one entry ahead and constants held in registers 543; the lanes together
+// before the tail, one gradient flush per row, loads without a branch 513; two record buffers in
+// turn 490; the rounding by addition 482.  Records staged in shared memory per block (a warp per
+// water, lanes over its row) took 50% more instructions and 750 us.
 template <int HB> struct HalfScale;
 template <> struct HalfScale<128> { static constexpr int S = 17; };
 template <> struct HalfScale<256> { static constexpr int S = 16; };
@@ -653,7 +684,7 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
                                                           double *__restrict__ e_unit, int intra)
 {
     constexpr int S = HalfScale<HB>::S;
-    constexpr float SC = (float)(1 << S);
+    constexpr float SC = (float)(1 << S), CAP = 4.19e6f / SC;   // (2^22 = 4,194,304)
     constexpr int NE = VIR ? 6 : 4;
     __shared__ float2 sE[NE][HB];
     extern __shared__ int sJ[];      // [9][jcap]: partner-site gradients, 2^S units
@@ -668,13 +699,13 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
     for (int k = 0; k < NE; ++k) sE[k][t] = make_float2(0.f, 0.f);
     __syncthreads();
     const int i = w.y + t;
+    const unsigned present = __ballot_sync(0xffffffffu, i - R.wat0 < R.nwat);
     if (i - R.wat0 < R.nwat) {
         const float4 oi0 = woff[3 * i];
         const float4 oi1 = woff[3 * i + 1], oi2 = woff[3 * i + 2];
-        const float2 hi[2][3] = {{f2(oi1.x), f2(oi1.y), f2(oi1.z)}, {f2(oi2.x), f2(oi2.y), f2(oi2.z)}};
-        float2 G[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) G[k] = f2(0.f);
+        const float2 hx = f2(oi1.x, oi2.x), hy = f2(oi1.y, oi2.y), hz = f2(oi1.z, oi2.z);   // (H1, H2) offsets
+        // minus the gradient: of O as two partials, of (H1, H2)
+        float2 GO[3] = {f2(0.f), f2(0.f), f2(0.f)}, GH[3] = {f2(0.f), f2(0.f), f2(0.f)};
         // the owner's gradient goes to the int64 site gradient with one atomic per component
         // and flush (no shared-memory slots: they would take the L1 that the gathers use)
         unsigned long long *gi = (unsigned long long *)(grad + 9 * (size_t)i);
@@ -686,189 +717,145 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
 #pragma unroll
         for (int k = 0; k < NE; ++k) e4[k] = 0.f;
         double *eu = e_unit + NB_EU * (size_t)i;
-        {
-            // the molecule's own exclusion corrections, flushed at once (fewer live registers
-            // in the pair loop)
-            float ecorr = 0.f;
-            if (intra) {
-                const float qs[3] = {oi0.w, pos[3 * i + 1].w, pos[3 * i + 2].w};
-                ecorr = water_intra_f(R, oi1, oi2, qs, g);
-#pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                    const long long v = nb_fix(g[k]);
-                    if (v != 0) atomicAdd(gi + k, (unsigned long long)v);
-                    g[k] = 0.f;
-                }
-            }
-            eu[5] = (double)ecorr;
-        }
         // ef: 2 for the water-water energies (each pair once), 1 for the W2 part (full list)
         auto flush = [&](float ef) {
 #pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                g[d] -= GO[d].x + GO[d].y; g[3 + d] -= GH[d].x; g[6 + d] -= GH[d].y;
+                GO[d] = f2(0.f); GH[d] = f2(0.f);
+            }
+#pragma unroll
             for (int k = 0; k < 9; ++k) {
-                const long long v = nb_fix(g[k] - (G[k].x + G[k].y));   // G holds minus the gradient
+                const long long v = nb_fix(g[k]);
                 if (v != 0) atomicAdd(gi + k, (unsigned long long)v);
                 g[k] = 0.f;
-                G[k] = f2(0.f);
             }
 #pragma unroll
-            for (int k = 0; k < NE; ++k) {
-                const float2 a = sE[k][t];
-                const float v = ef * e4[k];
-                const float sm = a.x + v, bb = sm - a.x, err = (a.x - (sm - bb)) + (v - bb);
-                sE[k][t] = make_float2(sm, a.y + err);
-                e4[k] = 0.f;
-            }
+            for (int k = 0; k < NE; ++k) { two_add(sE[k][t], ef * e4[k]); e4[k] = 0.f; }
         };
         auto flush1 = [&]() { flush(1.f); };
-        // partner site `site` of both entries: its gradient shares H (x: entry 0, y: entry 1).
-        // A parked entry's share is exactly zero, so it is added without a test; a share at or
-        // above NB_HALF_CAP (rare) takes the int64 path for that entry and component.
-        auto jadd = [&](int l0, int l1, int j0, int j1, int site, const float2 H[3]) {
-            bool big = false;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) big |= (fabsf(H[d].x) >= NB_HALF_CAP) | (fabsf(H[d].y) >= NB_HALF_CAP);
-            if (!big) {
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    atomicAdd(&sJ[(3 * site + d) * jcap + l0], __float2int_rn(H[d].x * SC));
-                    atomicAdd(&sJ[(3 * site + d) * jcap + l1], __float2int_rn(H[d].y * SC));
-                }
-            } else {
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const float fe[2] = {H[d].x, H[d].y};
-                    const int le[2] = {l0, l1}, je[2] = {j0, j1};
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        if (fabsf(fe[q]) < NB_HALF_CAP) atomicAdd(&sJ[(3 * site + d) * jcap + le[q]], __float2int_rn(fe[q] * SC));
-                        else atomicAdd((unsigned long long *)&grad[9 * (size_t)je[q] + 3 * site + d],
-                                       (unsigned long long)nb_fix(fe[q]));
-                    }
-                }
-            }
-        };
         int npair = 0;
-        const float iL0 = R.invL[0], iL1 = R.invL[1], iL2 = R.invL[2];
-        const float rmax2 = R.rmax2, rv2 = R.rv2;
-        const float2 palpha = f2(ERFCX_P * R.alpha), ex2c = f2(R.ex2c);
-        const float2 w12 = f2(R.w12), nw6 = f2(-R.w6);
-        const float2 c12 = f2(R.w12c), c6 = f2(R.w6c);
-        const float qqv[3] = {R.qq[0], R.qq[1], R.qq[2]};
-        const float c2a = R.c2a;
+        const float iL0 = held(R.invL[0]), iL1 = held(R.invL[1]), iL2 = held(R.invL[2]);
+        const float rmax2 = held(R.rmax2), rv2 = held(R.rv2);
+        const WaterK K = {held(ERFCX_P * R.alpha), held(R.ex2c), held(R.c2a)};
+        const float qOO = held(R.qq[0]), qOH = held(R.qq[1]), qHH = held(R.qq[2]), w12 = held(R.w12), w6 = held(R.w6);
+        const float w12c = held(R.w12c), w6c = held(R.w6c);
+        const float L0 = held(R.L[0]), L1 = held(R.L[1]), L2 = held(R.L[2]);
+        const float m0 = held(R.Llo[0]), m1 = held(R.Llo[1]), m2 = held(R.Llo[2]);
+        const bool sw = held(__int_as_float(R.lj_switch)) != 0.f;
         const unsigned *hr = hrow + (size_t)b * caph * HB + t;
         const int k1 = hcnt[i].y, wat0 = R.wat0;
         int cnt = 0;
-        // next pair of entries, loaded one iteration ahead
-        unsigned ea = k1 > 0 ? hr[0] : 0u;
-        unsigned eb = k1 > 1 ? hr[HB] : ea;
-        float4 oa = woff[3 * (wat0 + (int)(ea & 0xffffu))], ob = woff[3 * (wat0 + (int)(eb & 0xffffu))];
-        for (int k = 0; k < k1; k += 2) {
-            const bool hasb = k + 1 < k1;
-            const unsigned e0 = ea, e1 = eb;
-            const int j0 = wat0 + (int)(e0 & 0xffffu), j1 = wat0 + (int)(e1 & 0xffffu);
-            const int l0 = (int)(e0 >> 16), l1 = (int)(e1 >> 16);
-            const float4 o0 = oa, o1 = ob;
-            // the warp's row lines (one 128-byte line per entry) four iterations ahead (further
-            // ahead, the prefetched lines take L1 from the partner records)
-            nb_prefetch_l1(hr + (size_t)min(k + 8, k1 - 1) * HB);
-            if (k + 2 < k1) {
-                ea = hr[(size_t)(k + 2) * HB];
-                eb = k + 3 < k1 ? hr[(size_t)(k + 3) * HB] : ea;
-                oa = woff[3 * (wat0 + (int)(ea & 0xffffu))];
-                ob = woff[3 * (wat0 + (int)(eb & 0xffffu))];
-            }
-            float dx0 = oi0.x - o0.x, dy0 = oi0.y - o0.y, dz0 = oi0.z - o0.z;
-            float dx1 = oi0.x - o1.x, dy1 = oi0.y - o1.y, dz1 = oi0.z - o1.z;
-            const float nx0 = fmaf(dx0, iL0, 12582912.f) - 12582912.f, ny0 = fmaf(dy0, iL1, 12582912.f) - 12582912.f, nz0 = fmaf(dz0, iL2, 12582912.f) - 12582912.f;
-            const float nx1 = fmaf(dx1, iL0, 12582912.f) - 12582912.f, ny1 = fmaf(dy1, iL1, 12582912.f) - 12582912.f, nz1 = fmaf(dz1, iL2, 12582912.f) - 12582912.f;
-            dx0 = nb_shift(R, 0, dx0, nx0); dy0 = nb_shift(R, 1, dy0, ny0); dz0 = nb_shift(R, 2, dz0, nz0);
-            dx1 = nb_shift(R, 0, dx1, nx1); dy1 = nb_shift(R, 1, dy1, ny1); dz1 = nb_shift(R, 2, dz1, nz1);
-            const float r0 = dx0 * dx0 + dy0 * dy0 + dz0 * dz0, r1 = dx1 * dx1 + dy1 * dy1 + dz1 * dz1;
-            const bool in0 = r0 <= rmax2, in1 = hasb && r1 <= rmax2;
-            if (in0 || in1) {
-                const float4 a1 = woff[3 * j0 + 1], a2 = woff[3 * j0 + 2];
-                const float4 b1 = woff[3 * j1 + 1], b2 = woff[3 * j1 + 2];
-                if (!in0) { dx0 = 1.0e4f; dy0 = 0.f; dz0 = 0.f; }
-                if (!in1) { dx1 = 1.0e4f; dy1 = 0.f; dz1 = 0.f; }
-                float2 eel = f2(0.f), elj = f2(0.f), vlj = f2(0.f);
-#pragma unroll
-                for (int bs = 0; bs < 3; ++bs) {
-                    float2 q[3];
-                    if (bs == 0) {
-                        q[0] = f2(dx0, dx1); q[1] = f2(dy0, dy1); q[2] = f2(dz0, dz1);
-                    } else if (bs == 1) {
-                        q[0] = f2(dx0 - a1.x, dx1 - b1.x); q[1] = f2(dy0 - a1.y, dy1 - b1.y);
-                        q[2] = f2(dz0 - a1.z, dz1 - b1.z);
-                    } else {
-                        q[0] = f2(dx0 - a2.x, dx1 - b2.x); q[1] = f2(dy0 - a2.y, dy1 - b2.y);
-                        q[2] = f2(dz0 - a2.z, dz1 - b2.z);
-                    }
-                    float2 H[3] = {f2(0.f), f2(0.f), f2(0.f)};    // partner site bs: its gradient share
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const float2 ddx = a ? __fadd2_rn(hi[a - 1][0], q[0]) : q[0];
-                        const float2 ddy = a ? __fadd2_rn(hi[a - 1][1], q[1]) : q[1];
-                        const float2 ddz = a ? __fadd2_rn(hi[a - 1][2], q[2]) : q[2];
-                        const float2 rr2 = __ffma2_rn(ddx, ddx, __ffma2_rn(ddy, ddy, __fmul2_rn(ddz, ddz)));
-                        const float2 rinv = f2(nb_rsqrt_approx(rr2.x), nb_rsqrt_approx(rr2.y));
-                        const float2 s2 = __fmul2_rn(rinv, rinv);
-                        const float2 arg = __fmul2_rn(rr2, ex2c);
-                        const float2 den = __ffma2_rn(palpha, __fmul2_rn(rr2, rinv), f2(1.f));
-                        const float2 tt = f2(nb_rcp_approx(den.x), nb_rcp_approx(den.y));
-                        const float2 u = __ffma2_rn(f2(ERFCX_A), tt, f2(ERFCX_B));
-                        const float C[ERFCX_NC] = ERFCX_COEFS;
-                        float2 p = f2(C[ERFCX_NC - 1]);
-#pragma unroll
-                        for (int m = ERFCX_NC - 2; m >= 0; --m) p = __ffma2_rn(p, u, f2(C[m]));
-                        const float2 ex = f2(nb_ex2_approx(-arg.x), nb_ex2_approx(-arg.y));
-                        const float2 erfcv = __fmul2_rn(ex, __fmul2_rn(tt, p));
-                        const float qq = (a == 0 && bs == 0) ? qqv[0] : ((a == 0 || bs == 0) ? qqv[1] : qqv[2]);
-                        const float2 e = __fmul2_rn(__fmul2_rn(f2(qq), erfcv), rinv);
-                        float2 mdf = __fmul2_rn(__ffma2_rn(f2(qq * c2a), ex, e), s2);
-                        if (a == 0 && bs == 0) {
-                            const float2 ri = __ffma2_rn(__fmul2_rn(f2(-0.5f), rinv), __ffma2_rn(rr2, s2, f2(-1.f)), rinv);
-                            const float2 sl = __fmul2_rn(ri, ri);
-                            const float2 s6 = __fmul2_rn(__fmul2_rn(sl, sl), sl);
-                            const float2 A = __fmul2_rn(__fmul2_rn(w12, s6), s6);
-                            float2 e1 = __ffma2_rn(nw6, __ffma2_rn(s6, c6, s6), __ffma2_rn(A, c12, A));
-                            float2 m1 = __fmul2_rn(__fmul2_rn(f2(6.f), sl), __ffma2_rn(nw6, s6, __fadd2_rn(A, A)));
-                            if (R.lj_switch) {
-                                float d0 = -m1.x, d1 = -m1.y;
-                                lj_switch_apply<float>(R, rr2.x, e1.x, d0);
-                                lj_switch_apply<float>(R, rr2.y, e1.y, d1);
-                                m1 = f2(-d0, -d1);
-                            }
-                            const bool lj0 = rr2.x <= rv2, lj1 = rr2.y <= rv2;
-                            e1 = f2(lj0 ? e1.x : 0.f, lj1 ? e1.y : 0.f);
-                            m1 = f2(lj0 ? m1.x : 0.f, lj1 ? m1.y : 0.f);
-                            elj = __fadd2_rn(elj, e1);
-                            if (VIR) vlj = __fmul2_rn(m1, rr2);   // -df1 r^2 (watwat_ewald_press.f:146-152)
-                            mdf = __fadd2_rn(mdf, m1);
+        // one molecule pair: entry en, the partner's record
+        auto pair = [&](unsigned en, float4 oj, float4 A, float4 B) {
+            float dx = oi0.x - oj.x, dy = oi0.y - oj.y, dz = oi0.z - oj.z;
+            const float nx = fmaf(dx, iL0, 12582912.f) - 12582912.f, ny = fmaf(dy, iL1, 12582912.f) - 12582912.f,
+                        nz = fmaf(dz, iL2, 12582912.f) - 12582912.f;
+            dx = fmaf(-nx, m0, fmaf(-nx, L0, dx)); dy = fmaf(-ny, m1, fmaf(-ny, L1, dy)); dz = fmaf(-nz, m2, fmaf(-nz, L2, dz));
+            if (dx * dx + dy * dy + dz * dz <= rmax2) {
+                float H[9];      // the partner's gradient
+                float2 eel, e;
+                float eoo, elj = 0.f, vlj = 0.f;
+                {
+                    // O-O: Coulomb and LJ, as k_water_s
+                    const float rr2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    const float rinv = nb_rsqrt_approx(rr2), s2 = rinv * rinv;
+                    float mdf = ewald1(K, rr2, rinv, qOO, eoo);
+                    if (rr2 <= rv2) {
+                        const float ri = fmaf(-0.5f * rinv, fmaf(rr2, s2, -1.f), rinv), sl = ri * ri;
+                        const float s6 = sl * sl * sl, LA = w12 * s6 * s6;
+                        float e1 = fmaf(-w6, fmaf(s6, w6c, s6), fmaf(LA, w12c, LA));
+                        float m1 = 6.f * sl * fmaf(-w6, s6, LA + LA);
+                        if (sw) {
+                            float d1 = -m1;
+                            lj_switch_apply<float>(R, rr2, e1, d1);
+                            m1 = -d1;
                         }
-                        eel = __fadd2_rn(eel, e);
-                        G[3 * a] = __ffma2_rn(mdf, ddx, G[3 * a]);
-                        G[3 * a + 1] = __ffma2_rn(mdf, ddy, G[3 * a + 1]);
-                        G[3 * a + 2] = __ffma2_rn(mdf, ddz, G[3 * a + 2]);
-                        H[0] = __ffma2_rn(mdf, ddx, H[0]);
-                        H[1] = __ffma2_rn(mdf, ddy, H[1]);
-                        H[2] = __ffma2_rn(mdf, ddz, H[2]);
+                        elj = e1;
+                        if (VIR) vlj = m1 * rr2;   // -df1 r^2 (watwat_ewald_press.f:146-152)
+                        mdf += m1;
                     }
-                    jadd(l0, l1, j0, j1, bs, H);
+                    H[0] = mdf * dx; H[1] = mdf * dy; H[2] = mdf * dz;
+                    GO[0].x += H[0]; GO[1].x += H[1]; GO[2].x += H[2];
                 }
-                const bool img0 = (nx0 != 0.f) | (ny0 != 0.f) | (nz0 != 0.f);
-                const bool img1 = (nx1 != 0.f) | (ny1 != 0.f) | (nz1 != 0.f);
-                e4[img0 ? 1 : 0] += elj.x;
-                e4[img0 ? 3 : 2] += eel.x;
-                if (VIR) e4[img0 ? NE - 1 : NE - 2] += vlj.x;
-                e4[img1 ? 1 : 0] += elj.y;
-                e4[img1 ? 3 : 2] += eel.y;
-                if (VIR) e4[img1 ? NE - 1 : NE - 2] += vlj.y;
-                npair += 18 * ((int)in0 + (int)in1);
+                const float ax = dx - A.x, ay = dy - A.y, az = dz - A.z, bx = dx - B.x, by = dy - B.y, bz = dz - B.z;
+                {
+                    // O of i with (H1, H2) of j
+                    const float2 x = f2(ax, bx), y = f2(ay, by), z = f2(az, bz);
+                    const float2 m = ewald2(K, __ffma2_rn(x, x, __ffma2_rn(y, y, __fmul2_rn(z, z))), f2(qOH), eel);
+                    const float2 fx = __fmul2_rn(m, x), fy = __fmul2_rn(m, y), fz = __fmul2_rn(m, z);
+                    GO[0] = __fadd2_rn(GO[0], fx); GO[1] = __fadd2_rn(GO[1], fy); GO[2] = __fadd2_rn(GO[2], fz);
+                    H[3] = fx.x; H[4] = fy.x; H[5] = fz.x;
+                    H[6] = fx.y; H[7] = fy.y; H[8] = fz.y;
+                }
+#pragma unroll
+                for (int s = 0; s < 3; ++s) {
+                    // (H1, H2) of i with site s of j
+                    const float2 x = __fadd2_rn(hx, f2(s == 0 ? dx : (s == 1 ? ax : bx)));
+                    const float2 y = __fadd2_rn(hy, f2(s == 0 ? dy : (s == 1 ? ay : by)));
+                    const float2 z = __fadd2_rn(hz, f2(s == 0 ? dz : (s == 1 ? az : bz)));
+                    const float2 m = ewald2(K, __ffma2_rn(x, x, __ffma2_rn(y, y, __fmul2_rn(z, z))),
+                                            f2(s == 0 ? qOH : qHH), e);
+                    eel = __fadd2_rn(eel, e);
+                    const float2 fx = __fmul2_rn(m, x), fy = __fmul2_rn(m, y), fz = __fmul2_rn(m, z);
+                    GH[0] = __fadd2_rn(GH[0], fx); GH[1] = __fadd2_rn(GH[1], fy); GH[2] = __fadd2_rn(GH[2], fz);
+                    H[3 * s] += fx.x + fx.y; H[3 * s + 1] += fy.x + fy.y; H[3 * s + 2] += fz.x + fz.y;
+                }
+                const int l = (int)(en >> 16);
+                float hm = 0.f;
+#pragma unroll
+                for (int c = 0; c < 9; ++c) hm = fmaxf(hm, fabsf(H[c]));
+                if (hm < CAP) {
+#pragma unroll
+                    for (int c = 0; c < 9; ++c)
+                        atomicAdd(&sJ[c * jcap + l], __float_as_int(fmaf(H[c], SC, 12582912.f)) - 0x4b400000);
+                } else {
+                    // a large share (rare): straight to the int64 gradient
+                    unsigned long long *gj = (unsigned long long *)(grad + 9 * (size_t)(wat0 + (int)(en & 0xffffu)));
+#pragma unroll
+                    for (int c = 0; c < 9; ++c) atomicAdd(gj + c, (unsigned long long)nb_fix(H[c]));
+                }
+                const bool img = (nx != 0.f) | (ny != 0.f) | (nz != 0.f);
+                const float ec = eoo + (eel.x + eel.y);
+                e4[0] += img ? 0.f : elj; e4[1] += img ? elj : 0.f;
+                e4[2] += img ? 0.f : ec; e4[3] += img ? ec : 0.f;
+                if (VIR) { e4[NE - 2] += img ? 0.f : vlj; e4[NE - 1] += img ? vlj : 0.f; }
+                npair += 18;
             }
-            cnt += 2;
-            if (cnt >= CHUNK) { flush(2.f); cnt = 0; }
+        };
+        // The next entry's record is on its way while one is worked on: two record buffers in turn
+        // (a copy between them would tie a load to the end of the previous use of its registers),
+        // row entries two ahead of their records, the warp's row lines (one 128-byte line per
+        // entry) in L1 eight ahead.
+        auto rec = [&](unsigned en) { return woff + 3 * (wat0 + (int)(en & 0xffffu)); };
+        auto entry = [&](int k) { return hr[(size_t)min(k, k1 - 1) * HB]; };
+        if (k1 > 0) {
+            unsigned ea = entry(0), eb = entry(1);
+            const float4 *r = rec(ea);
+            float4 oa = r[0], ha = r[1], ia = r[2];
+            for (int k = 0; k < k1; k += 2) {
+                const unsigned ec = entry(k + 2), ed = entry(k + 3);
+                r = rec(eb);
+                const float4 ob = r[0], hb = r[1], ib = r[2];
+                nb_prefetch_l1(hr + (size_t)min(k + 8, k1 - 1) * HB);
+                nb_prefetch_l1(hr + (size_t)min(k + 9, k1 - 1) * HB);
+                pair(ea, oa, ha, ia);
+                r = rec(ec);
+                oa = r[0]; ha = r[1]; ia = r[2];
+                if (k + 1 < k1) pair(eb, ob, hb, ib);
+                ea = ec; eb = ed;
+                cnt += 2;
+                if (cnt >= 2 * CHUNK) { flush(2.f); cnt = 0; }
+            }
         }
+        __syncwarp(present);     // rows differ in length: without this, lanes that end early run the tail apart
+        // the molecule's own exclusion corrections join the last flush
+        float ecorr = 0.f;
+        if (intra) {
+            const float qs[3] = {oi0.w, pos[3 * i + 1].w, pos[3 * i + 2].w};
+            ecorr = water_intra_f(R, woff[3 * i + 1], woff[3 * i + 2], qs, g);
+        }
+        eu[5] = (double)ecorr;
         flush(2.f);
         if (wl2_off[i] < wl2_off[i + 1]) {
             water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, 0, g, e4, npair, flush1);
@@ -881,14 +868,19 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
         eu[7] = VIR ? (double)sE[NE - 1][t].x + (double)sE[NE - 1][t].y : 0.0;
     }
     __syncthreads();
-    // the block's partner shares of its j-set
+    // the block's partner shares of its j-set: a warp takes 32 partners, and its lanes the 288
+    // words of their gradients in order (nine consecutive words per partner, so a request
+    // touches 9 sectors instead of 32)
     const int *js = jset + (size_t)b * jcap;
-    for (int l = t; l < nJ; l += HB) {
-        const size_t jg = (size_t)js[l];
+    const int lane = t & 31;
+    for (int l0 = t - lane; l0 < nJ; l0 += HB) {
+        const int jl = l0 + lane < nJ ? js[l0 + lane] : -1;
 #pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            const int v = sJ[c * jcap + l];
-            if (v != 0) atomicAdd((unsigned long long *)&grad[9 * jg + c], (unsigned long long)((long long)v * (1LL << (32 - S))));
+        for (int q = 0; q < 9; ++q) {
+            const int f = 32 * q + lane, l = f / 9, c = f - 9 * l;
+            const int j = __shfl_sync(0xffffffffu, jl, l);
+            const int v = j >= 0 ? sJ[c * jcap + l0 + l] : 0;
+            if (v != 0) atomicAdd((unsigned long long *)&grad[9 * (size_t)j + c], (unsigned long long)((long long)v * (1LL << (32 - S))));
         }
     }
 }
@@ -1276,11 +1268,15 @@ WaterHFn water_h_fn(int hb, bool vir)
 // groups, so a grouped handle gives the ungrouped one's bits): every lane of the GPU has work
 // from a few thousand waters at 32 lanes each, and from then on fewer lanes lose less to
 // partly filled rounds and to the sum over the lanes.  Water stage in us at 32 / 8 / 4 lanes:
-// 1,334 waters 16 / 26 / 38, 3,000 17 / 22 / 38, 7,000 32 / 24 / 40, 12,000 42 / 30 / 40, 32,000
-// 112 / 84 / 89, 110,860 (64 replicas) 339 / 206 / 194, 433,195 1304 / 743 / 678 (one water per
+// 1,334 waters 14 / 19 / 27, 3,000 22 / 19 / 28, 7,000 32 / 21 / 30, 12,000 46 / 34 / 32, 32,000
+// 114 / 80 / 77, 110,860 (64 replicas) 366 / 197 / 175, 433,195 1418 / 733 / 633 (one water per
 // thread: 78, 79, 82, 79, 120, 204, 657).  With atoms outside waters a water also has a list of
-// those: 8 lanes for the large ones.
-int water_lanes(const NbCtx *c) { return c->nw_handle <= 4096 ? 32 : (c->nw_handle <= 32768 || c->na_handle > 0 ? 8 : 4); }
+// those (the solute system, 7,020 waters: 37 / 71 / 114).
+int water_lanes(const NbCtx *c)
+{
+    const bool atoms = c->na_handle > 0;
+    return c->nw_handle <= (atoms ? 8192 : 4096) ? 32 : (c->nw_handle <= 32768 || atoms ? 8 : 4);
+}
 
 using WaterSFn = decltype(&k_water_s<8, false, int>);
 WaterSFn water_s_fn(int lpw, bool vir, bool row16)
@@ -1300,8 +1296,6 @@ void water_t(NbCtx *c)
     cudaStream_t s = c->stream;
     if (c->timing) cudaEventRecord(c->ev[2], s);
     if (sizeof(T) == 4 && c->nW > 0 && c->whalf) {
-        // the water sites' gradients are sums of atomics: cleared first
-        cudaMemsetAsync(c->d_grad_site, 0, sizeof(long long) * 9 * (size_t)c->nW, s);
         water_h_fn(c->hb, c->virial)<<<(int)c->hblocks.size(), c->hb, (size_t)36 * c->jcap, s>>>(
             c->d_hblocks, c->d_reps, (const float4 *)c->d_pos, (const float4 *)c->d_woff, c->d_site_lj,
             c->d_site_flags, c->d_hrow, c->caph, c->d_hcnt, c->d_jset, c->d_jn, c->jcap, c->d_wl2_off, c->d_wl2,
@@ -1315,8 +1309,6 @@ void water_t(NbCtx *c)
                 c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2,
                 cap_int(c->cap_wl2), c->d_grad_site, c->d_e_unit, c->water_excl_fast);
         } else {
-            // both sides of every pair are added with atomics: the waters' gradient starts at zero
-            cudaMemsetAsync(c->d_grad_site, 0, sizeof(long long) * 9 * (size_t)c->nW, s);
             (c->row16 ? k_water_d<unsigned short> : k_water_d<int>)<<<(int)((c->nW + WARPS64 - 1) / WARPS64),
                                                                       32 * WARPS64, 0, s>>>(
                 (int)c->nW, c->d_reps, c->d_site_rep, (const double4 *)c->d_pos, (const double4 *)c->d_woff,
@@ -1345,6 +1337,10 @@ void atoms_t(NbCtx *c)
 
 void nb_launch_water(NbCtx *c)
 {
+    // the kernels that evaluate each water pair once add both sides with atomics: the water
+    // sites' gradient starts at zero
+    if (c->nW > 0 && (c->precision == MOIL_NB_FP64 || c->whalf))
+        cudaMemsetAsync(c->d_grad_site, 0, sizeof(long long) * 9 * (size_t)c->nW, c->stream);
     if (c->precision == MOIL_NB_FP64) water_t<double>(c);
     else water_t<float>(c);
 }
@@ -1366,7 +1362,7 @@ static int carveout_pct(NbCtx *c, size_t bytes)
 
 int nb_realspace_configure(NbCtx *c)
 {
-    // full-list FP32 water kernel: five resident blocks of static shared memory; the smallest
+    // full-list FP32 water kernel: four resident blocks of static shared memory; the smallest
     // carveout that holds them leaves the most L1 for the partner-record gathers
     for (int lpw : {32, 8, 4})
         for (int k = 0; k < 4; ++k) {
@@ -1374,7 +1370,7 @@ int nb_realspace_configure(NbCtx *c)
             cudaFuncAttributes fa;
             NB_CUDA_OK(c, cudaFuncGetAttributes(&fa, fn));
             NB_CUDA_OK(c, cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                               carveout_pct(c, 5 * (fa.sharedSizeBytes + 1024))));
+                                               carveout_pct(c, 4 * (fa.sharedSizeBytes + 1024))));
         }
     return MOIL_NB_OK;
 }
