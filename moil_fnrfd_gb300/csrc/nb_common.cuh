@@ -56,7 +56,6 @@ struct RepDev {
     double epstmp;           // kofdie / eps
     int n1, n2, n3, n1h;     // PME grid, n1h = n1/2 + 1
     long long g0;            // first complex element of this replica's half-complex grid
-    int zb0;                 // first z-bin of this replica
     int bsp0;                // bsp moduli: [bsp0, +n1) x, [+n1, +n2) y, [+n2, +n3) z
     float fc;                // sqrt(kofdie/eps)
     double fcd;
@@ -118,6 +117,49 @@ __device__ __forceinline__ void pme_fr_split(double v, int &i, double &w)
 {
     i = (int)v;
     w = v - (double)i;
+}
+
+// PME site record (fr1, fr2, fr3, q fc) of a position, and int(fr3) in [0, n3) as its z byte.
+// fr = n (u - anint(u) + 1/2), u = x / L.  FP32: carried as hi + lo through every step (1/L as
+// hi + lo, the product's rounding error by an FMA, the + 1/2 by Fast2Sum), so the fraction
+// within the grid cell keeps 2^-23 of a grid spacing.
+__device__ __forceinline__ float4 pme_site(const RepDev &R, const float xs[3], float q, unsigned char &zb)
+{
+    const int ns[3] = {R.n1, R.n2, R.n3};
+    float out[3];
+    int z = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float x = xs[d], ih = R.invL[d];
+        const float uh = x * ih, ul = fmaf(x, ih, -uh) + x * R.invL_lo[d];
+        const float a = uh - rintf(uh);              // exact (Sterbenz)
+        const float th = a + 0.5f, tl = (a - (th - 0.5f)) + ul;
+        const float n = (float)ns[d];
+        int i = (int)floorf(n * th);
+        float w = fmaf(n, th, -(float)i) + n * tl;
+        if (w < 0.f) { --i; w += 1.f; }
+        if (w >= 1.f) { ++i; w -= 1.f; }
+        if (i < 0) { i = 0; w = 0.f; }
+        out[d] = pme_fr_pack(i, w);
+        if (d == 2) z = i;
+    }
+    zb = (unsigned char)(z >= R.n3 ? z - R.n3 : z);
+    return make_float4(out[0], out[1], out[2], q * R.fc);
+}
+__device__ __forceinline__ double4 pme_site(const RepDev &R, const double x[3], double q, unsigned char &zb)
+{
+    double f[3];
+    const int ns[3] = {R.n1, R.n2, R.n3};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double w = x[d] * R.invLd[d];
+        f[d] = ns[d] * (w - round(w) + 0.5);
+    }
+    const int z = (int)f[2];
+    zb = (unsigned char)(z >= R.n3 ? z - R.n3 : (z < 0 ? 0 : z));
+    double4 o;
+    o.x = f[0]; o.y = f[1]; o.z = f[2]; o.w = q * R.fcd;
+    return o;
 }
 
 // site flags
@@ -254,11 +296,6 @@ __host__ __device__ __forceinline__ int nb_half_owner(int a, int b)
 {
     return ((a ^ b) & 1) ? min(a, b) : max(a, b);
 }
-
-// Half-list water kernel: j-side gradients are summed per block in int32 at 2^(24 - log2 HB)
-// units per kcal/mol/Å, so HB contributions of magnitude below NB_HALF_CAP cannot overflow;
-// a larger contribution goes straight to the int64 site gradient
-#define NB_HALF_CAP 127.0f
 
 // bounded-status helpers
 #define NB_DEV_ERR_OVERFLOW 1

@@ -7,7 +7,7 @@
 //   lists       (device-gated) unit sort + W1/W2/X list count/scan/fill
 //   real space  water-molecule kernel and non-water-atom kernel
 //   excl/1-4    FP64 corrections
-//   PME         bin, spread+FFT(x,y), FFT(z)+convolution, FFT(y,x)+gather
+//   PME         spread+FFT(x,y), FFT(z)+convolution, FFT(y,x)+gather
 //   finalize    gradient assembly in MOIL order, per-replica energies
 #include <math.h>
 #include <stdio.h>
@@ -90,7 +90,7 @@ void release_device(NbCtx *c)
     free_ptr(c->d_hblocks); free_ptr(c->d_hrow); free_ptr(c->d_hcnt); free_ptr(c->d_jset); free_ptr(c->d_jn);
     c->hblocks.clear();
     c->whalf = 0;
-    free_ptr(c->d_bsp); free_ptr(c->d_etab); free_ptr(c->d_zcount); free_ptr(c->d_zstart); free_ptr(c->d_zslot); free_ptr(c->d_zatoms);
+    free_ptr(c->d_bsp); free_ptr(c->d_etab); free_ptr(c->d_zidx);
     free_ptr(c->d_fr); free_ptr(c->d_grid); free_ptr(c->d_part); free_ptr(c->d_planes); free_ptr(c->d_cols);
     free_ptr(c->d_col_begin); free_ptr(c->d_e_col); free_ptr(c->d_e_rep);
     free_ptr(c->d_echunks); free_ptr(c->d_echunk_begin); free_ptr(c->d_epart);
@@ -211,12 +211,12 @@ int alloc_half(NbCtx *c)
 
 // The automatic shape takes full lists up to this many waters (of the whole handle): a block
 // of 256 waters per multiprocessor leaves most of the GPU idle below it, while the full-list
-// kernel spreads each water over 8 or 32 lanes.  One evaluation in us, half / full lists:
-// 216 waters 116 / 98, 3,000 154 / 126, 12,000 210 / 177, 19,272 (24 replicas) 167 / 145,
-// 20,000 (one box) 200 / 214, 32,000 248 / 264.  Handles with atoms outside waters take full lists
+// kernel spreads each water over 8 or 32 lanes.  One evaluation in us (lists rebuilt every 10),
+// half / full lists: 216 waters 98 / 80, 1,334 125 / 95, 7,000 124 / 104, 12,000 129 / 117, 32,000
+// 197 / 199, 110,860 (64 replicas) 385 / 402.  Handles with atoms outside waters take full lists
 // at every size: the half-list kernel runs a water's list of them in one thread (water stage of
-// eight solute systems, 56,160 waters: 394 / 150 us).
-#define NB_FULL_MAX_WATERS 19500
+// the solute system, 7,020 waters: 322 / 37 us).
+#define NB_FULL_MAX_WATERS 28672
 
 // Half-list set-up for the current shape: on for FP32 handles whose replicas all have fewer
 // than 65,536 waters (16-bit rows) unless full lists were asked for; blocks of hb waters
@@ -307,7 +307,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     std::vector<int> atom_rep, unit_atom_w, unit_atom_o, unit_rep_w, unit_rep_o;
     std::vector<std::vector<int>> exn, p14n;
     std::vector<std::vector<double>> p14p;
-    int64_t atom0 = 0, wat0 = 0, oth0 = 0, zb0 = 0, g0 = 0;
+    int64_t atom0 = 0, wat0 = 0, oth0 = 0, g0 = 0;
     int water_fast = 1;
     int cell0 = 0;
     for (int r = 0; r < nrep; ++r) {
@@ -432,8 +432,6 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
         R.n1h = R.n1 / 2 + 1;
         R.g0 = g0;
         g0 += (int64_t)R.n1h * R.n2 * R.n3;
-        R.zb0 = (int)zb0;
-        zb0 += R.n3;
         R.bsp0 = (int)c->bsp_h.size();
         {
             int ns[3] = {R.n1, R.n2, R.n3};
@@ -457,7 +455,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
         R.pivol = M_PI * p->a * p->b * p->c;
         nb_pme_fp32_consts(&R);
         {
-            // the FP32 path spreads fl(fl(q) fl(fc)) per site (k_pme_bin): the reciprocal energy,
+            // the FP32 path spreads fl(fl(q) fl(fc)) per site (pme_site): the reciprocal energy,
             // quadratic in the charges, is rescaled by sum (q fc)^2 / sum fl(..)^2, exact when
             // every charge has the same relative rounding (all waters: qH = -qO/2)
             double sd = 0.0, sf = 0.0;
@@ -532,7 +530,6 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     c->nunit = c->nW + c->nA;
     c->ncell = cell0;
     c->grid_elems = g0;
-    c->nzbin = (int)zb0;
     if (c->nsite != c->natom) { c->err = "internal: site count"; return MOIL_NB_ERR_ARG; }
     for (int r = 0; r < nrep; ++r) c->rd[r].oth0 = c->rd[r].oth0;   // already set
 
@@ -602,10 +599,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     NB_CUDA_OK(c, cudaMalloc(&c->d_e_unit, sizeof(double) * NB_EU * std::max<int64_t>(nu, 1)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_grad_ex, sizeof(double) * 3 * c->natom));
     NB_CUDA_OK(c, cudaMalloc(&c->d_e_ex, sizeof(double) * NB_EX * c->natom));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_zcount, sizeof(int) * (c->nzbin + 1)));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_zstart, sizeof(int) * (c->nzbin + 1)));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_zslot, sizeof(int) * ns));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_zatoms, sizeof(int) * ns));
+    NB_CUDA_OK(c, cudaMalloc(&c->d_zidx, ns + 16));
     NB_CUDA_OK(c, cudaMalloc(&c->d_e_rep, sizeof(double) * NB_EREP * nrep));
     NB_CUDA_OK(c, cudaMalloc(&c->d_coor, sizeof(double) * 3 * c->natom));
     NB_CUDA_OK(c, cudaMalloc(&c->d_dpot, sizeof(double) * 3 * c->natom));
@@ -636,8 +630,8 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     NB_TRY(nb_pme_configure(c));
     NB_TRY(setup_energy_chunks(c, water_fast));
     {
-        // tile sums for every scan: bins, per-water and per-atom counts, PME z-bins
-        int64_t nmax = std::max<int64_t>({2 * (int64_t)c->ncell, c->nW, c->nA, (int64_t)c->nzbin, 1});
+        // tile sums for every scan: bins, per-water and per-atom counts
+        int64_t nmax = std::max<int64_t>({2 * (int64_t)c->ncell, c->nW, c->nA, 1});
         NB_CUDA_OK(c, cudaMalloc(&c->d_scan_tmp, sizeof(long long) * (nmax / 4096 + 2)));
     }
     NB_CUDA_OK(c, cudaDeviceSynchronize());
@@ -732,16 +726,21 @@ void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot)
         cudaEventRecord(c->ev[5], s);
         nb_launch_pme(c);
     } else {
-        // the PME branch (binning, planes, columns, gather) runs on a second stream beside the
+        // the PME branch (planes, columns, gather) runs on a second stream beside the
         // pair and correction kernels: they read the same site positions and write disjoint
         // outputs, and the latency-bound plane kernels fill the multiprocessors the pair
         // kernel leaves idle
         cudaEventRecord(c->ev_fork, s);
-        cudaStreamWaitEvent(c->stream2, c->ev_fork, 0);
-        std::swap(c->stream, c->stream2);
+        // With full lists the water kernel's blocks would fill the GPU before the (few) blocks of
+        // each PME kernel, the longer chain: PME goes first then (an evaluation of 7,000 waters 104
+        // us, 135 at equal priorities).  The half-list kernel holds two blocks per multiprocessor
+        // anyway, and PME first costs it 4% at 256 replicas.
+        cudaStream_t &pme = c->whalf && !c->on_prio ? c->stream2n : c->stream2;
+        cudaStreamWaitEvent(pme, c->ev_fork, 0);
+        std::swap(c->stream, pme);
         nb_launch_pme(c);
-        std::swap(c->stream, c->stream2);
-        cudaEventRecord(c->ev_join, c->stream2);
+        std::swap(c->stream, pme);
+        cudaEventRecord(c->ev_join, pme);
         // the non-water pair and the correction kernels (FP64) likewise, on a third
         const bool third = c->nA > 0 || !c->water_excl_fast || c->precision == MOIL_NB_FP64;
         if (third) {
@@ -843,7 +842,7 @@ bool launch_graph(NbCtx *c, const double *d_coor, double *d_dpot)
         enqueue_eval(c, d_coor, d_dpot);
         c->capturing = 0;
         cudaError_t e1 = cudaStreamEndCapture(s, &g);
-        cudaError_t e2 = e1 == cudaSuccess ? cudaGraphInstantiate(&c->gexec, g, 0) : e1;
+        cudaError_t e2 = e1 == cudaSuccess ? cudaGraphInstantiate(&c->gexec, g, cudaGraphInstantiateFlagUseNodePriority) : e1;
         if (g) cudaGraphDestroy(g);
         if (e2 != cudaSuccess) {
             cudaGetLastError();
@@ -1178,14 +1177,17 @@ int moil_nb_create(moil_nb_ctx **out, int device)
     if (device < 0 || device >= ndev) return MOIL_NB_ERR_ARG;
     moil_nb_ctx *h = new moil_nb_ctx();
     h->device = device;
-    if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking) != cudaSuccess ||
+    int lo = 0, hi = 0;
+    if (cudaSetDevice(device) != cudaSuccess || cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess || cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&h->stream2, cudaStreamNonBlocking, hi) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&h->stream2n, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->stream3, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->ev_join3, cudaEventDisableTiming) != cudaSuccess) {
         if (h->stream) cudaStreamDestroy(h->stream);
         if (h->stream2) cudaStreamDestroy(h->stream2);
+        if (h->stream2n) cudaStreamDestroy(h->stream2n);
         if (h->stream3) cudaStreamDestroy(h->stream3);
         if (h->ev_fork) cudaEventDestroy(h->ev_fork);
         if (h->ev_join) cudaEventDestroy(h->ev_join);
@@ -1216,6 +1218,7 @@ void moil_nb_destroy(moil_nb_ctx *h)
     if (h->h_status) cudaFreeHost(h->h_status);
     if (h->d_status) cudaFree(h->d_status);
     if (h->stream2) { cudaStreamSynchronize(h->stream2); cudaStreamDestroy(h->stream2); }
+    if (h->stream2n) { cudaStreamSynchronize(h->stream2n); cudaStreamDestroy(h->stream2n); }
     if (h->stream3) { cudaStreamSynchronize(h->stream3); cudaStreamDestroy(h->stream3); }
     if (h->sbody) cudaStreamDestroy(h->sbody);
     if (h->sstep) cudaStreamDestroy(h->sstep);
@@ -1398,7 +1401,7 @@ int moil_nb_pressure(moil_nb_ctx *h, const double *coor, double *dpot, moil_ener
     }
     const size_t n = (size_t)h->natom;
     NB_CUDA_OK(h, cudaMemcpyAsync(h->d_coor, coor, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->stream));
-    int rc = eval_impl(h, h->d_coor, h->d_dpot, e);   // lists, positions, PME binning and shares
+    int rc = eval_impl(h, h->d_coor, h->d_dpot, e);   // lists, positions, PME records and shares
     if (rc != MOIL_NB_OK) return rc;
     if (!h->d_press_out) {
         NB_CUDA_OK(h, cudaMalloc(&h->d_press_unit, sizeof(double) * 6 * std::max<int64_t>(h->nW + h->nA, 1)));
@@ -1728,7 +1731,7 @@ int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *
         const bool built = enqueue_md_step(c, coor, vel, mass, dpot, dt, doh, dhh);
         c->capturing = 0;
         cudaError_t e1 = cudaStreamEndCapture(s, &g);
-        cudaError_t e2 = e1 == cudaSuccess ? (built ? cudaGraphInstantiate(&c->gexec_md, g, 0) : cudaErrorNotSupported) : e1;
+        cudaError_t e2 = e1 == cudaSuccess ? (built ? cudaGraphInstantiate(&c->gexec_md, g, cudaGraphInstantiateFlagUseNodePriority) : cudaErrorNotSupported) : e1;
         if (g) cudaGraphDestroy(g);
         if (e2 != cudaSuccess) {
             c->gexec_md = nullptr;

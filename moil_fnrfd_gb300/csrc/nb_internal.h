@@ -36,7 +36,8 @@ struct NbCtx {
     int device = 0;
     int nsm = 152;                // multiprocessors: grids of the rebuild-gated kernels stay one wave
     cudaStream_t stream = nullptr;
-    cudaStream_t stream2 = nullptr;   // PME branch of an evaluation, concurrent with the pair kernels
+    cudaStream_t stream2 = nullptr;   // PME branch of an evaluation, concurrent with the pair kernels: its
+    cudaStream_t stream2n = nullptr;  // blocks first (stream2), or at the pair kernels' priority (stream2n)
     cudaStream_t stream3 = nullptr;   // non-water pair and correction kernels, beside the water kernel
     cudaStream_t sbody = nullptr;     // captures the list rebuild into the conditional node's body
     cudaStream_t sstep = nullptr;     // captures an MD step into its gate node's body
@@ -131,8 +132,7 @@ struct NbCtx {
     std::vector<double> bsp_h;
     void *d_bsp = nullptr;             // float / double moduli
     float *d_etab = nullptr;           // FP32 path: exp(-pi^2 m^2 / (alpha L)^2) / B per dimension (bsp layout)
-    int nzbin = 0;
-    int *d_zcount = nullptr, *d_zstart = nullptr, *d_zslot = nullptr, *d_zatoms = nullptr;
+    unsigned char *d_zidx = nullptr;   // per site int(fr3): the last z plane of its stencil (16-byte tail)
     void *d_fr = nullptr;              // float4 / double4 per site (fr1, fr2, fr3, q*fc)
     void *d_grid = nullptr;            // half-complex grids, float2 / double2
     int64_t grid_elems = 0;
@@ -243,7 +243,6 @@ void nb_launch_build_lists(NbCtx *c, const double *d_coor);
 // one thread sets the conditional node of a captured evaluation to the device rebuild flag
 void nb_launch_rebuild_cond(NbCtx *c, cudaGraphConditionalHandle h);
 void nb_launch_prepare(NbCtx *c, const double *d_coor, int check);
-void nb_exclusive_scan(NbCtx *c, const int *d_in, int *d_out, int n, int *d_total);
 // real space + corrections (nb_realspace.cu)
 void nb_launch_water(NbCtx *c);      // water molecules: W1 and W2 lists
 void nb_launch_atoms(NbCtx *c);      // atoms outside waters: X lists
@@ -255,6 +254,11 @@ bool nb_half_two_blocks(NbCtx *c);
 int nb_realspace_configure(NbCtx *c);
 void nb_launch_excl14(NbCtx *c, const double *d_coor);
 // PME (nb_pme.cu)
+// Whether the coordinate preparation writes the PME records and z bytes itself: a launch less
+// before the first plane, up to this many units of the handle.  Larger handles write them in a
+// kernel at the head of the PME branch, beside the first blocks of the water kernel (256 replicas,
+// 433,195 waters: 1,156 against 1,168 us an evaluation).
+inline bool nb_fused_sites(const NbCtx *c) { return c->nw_handle + c->na_handle <= 65536; }
 void nb_launch_pme(NbCtx *c);
 int nb_pme_configure(NbCtx *c);
 // |DFT|^2 of the order-4 B-spline (pot/ewald_receip.f:413-481), n values

@@ -126,21 +126,30 @@ __global__ void k_site_build(int nunit, int nW, const int *__restrict__ sorted, 
     }
 }
 
-// 3. per-evaluation coordinate conversion into site order; displacement check.  One thread
+// 3. per-evaluation coordinate conversion into site order, with each site's PME record and z
+// byte; displacement check.  One thread
 // per sorted water (its three consecutive caller atoms, 72 contiguous bytes) or non-water
 // site, so every site-order array is read and written coalesced.
 // Sites that do not track (water hydrogens) neither read nor write their build position.
-template <typename T>
-__device__ __forceinline__ void prepare_site(int s, const double *x, const unsigned *__restrict__ site_flags,
-                                             const T *__restrict__ site_q, void *pos_v, float4 *__restrict__ posb,
-                                             float half_skin2, int snapshot, bool track, bool &moved)
+template <typename T, bool PME>
+__device__ __forceinline__ void prepare_site(const RepDev &R, int s, const double *x,
+                                             const unsigned *__restrict__ site_flags, const T *__restrict__ site_q,
+                                             void *pos_v, float4 *__restrict__ posb, void *fr_v,
+                                             unsigned char *__restrict__ zidx, float half_skin2, int snapshot,
+                                             bool track, bool &moved)
 {
     typedef typename vec4<T>::type T4;
     const unsigned f = site_flags[s];
+    const T q = site_q[s], xs[3] = {(T)x[0], (T)x[1], (T)x[2]};
     T4 p;
-    p.x = (T)x[0]; p.y = (T)x[1]; p.z = (T)x[2];
-    p.w = (f & SF_CHARGED) ? site_q[s] : (T)0;
+    p.x = xs[0]; p.y = xs[1]; p.z = xs[2];
+    p.w = (f & SF_CHARGED) ? q : (T)0;
     ((T4 *)pos_v)[s] = p;
+    if (PME) {
+        unsigned char z;
+        ((T4 *)fr_v)[s] = pme_site(R, xs, q, z);
+        zidx[s] = z;
+    }
     if (!track) return;
     const float4 pf = make_float4((float)x[0], (float)x[1], (float)x[2], 0.f);
     if (snapshot) {
@@ -169,10 +178,13 @@ __device__ __forceinline__ void load_atom(const double *__restrict__ coor, int a
     }
 }
 
-template <typename T>
-__global__ void k_prepare(int nW, int nA, const int *__restrict__ site_orig, const unsigned *__restrict__ site_flags,
+// PME: also each site's PME record (nb_fused_sites)
+template <typename T, bool PME>
+__global__ void __launch_bounds__(256, 5) k_prepare(int nW, int nA, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
+                          const int *__restrict__ site_orig, const unsigned *__restrict__ site_flags,
                           const void *site_q_v, const double *__restrict__ coor, void *pos_v, void *woff_v,
-                          float4 *__restrict__ posb, float half_skin2, float rwat2, int snapshot, int *st)
+                          float4 *__restrict__ posb, void *fr_v, unsigned char *__restrict__ zidx, float half_skin2,
+                          float rwat2, int snapshot, int *st)
 {
     // snapshot mode runs only on a rebuild; check mode only without one (the site order it
     // reads is the previous build's, which does not exist before the first build)
@@ -184,24 +196,25 @@ __global__ void k_prepare(int nW, int nA, const int *__restrict__ site_orig, con
         if (u < nW) {
             // a water's caller atoms are consecutive (O, H, H), as are its sites
             const int a = site_orig[3 * u];
-            double x[3][3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) load_atom(coor, a + m, x[m], st);
+            const RepDev &R = reps[site_rep[3 * u]];
+            double xo[3];
+            load_atom(coor, a, xo, st);
             // only the oxygen's displacement counts: every water list is built from oxygen
             // distances with radii that include the hydrogens' reach (rwat, checked below)
-#pragma unroll
-            for (int m = 0; m < 3; ++m)
-                prepare_site<T>(3 * u + m, x[m], site_flags, site_q, pos_v, posb, half_skin2, snapshot, m == 0,
-                                moved);
+            prepare_site<T, PME>(R, 3 * u, xo, site_flags, site_q, pos_v, posb, fr_v, zidx, half_skin2, snapshot, true, moved);
             // the molecule record of the water kernel: O position (and charge), then the offsets
             ((T4 *)woff_v)[3 * u] = ((const T4 *)pos_v)[3 * u];
-#pragma unroll
+#pragma unroll 1
             for (int m = 1; m < 3; ++m) {
+                double x[3];
+                load_atom(coor, a + m, x, st);
+                prepare_site<T, PME>(R, 3 * u + m, x, site_flags, site_q, pos_v, posb, fr_v, zidx, half_skin2, snapshot, false,
+                                moved);
                 // H offset from its O, formed in FP64 so the water kernel's site displacements
                 // inherit no extra rounding from absolute FP32 positions; water sites must stay
                 // within rwat of their oxygen (list radius assumption)
                 T4 off;
-                off.x = (T)(x[m][0] - x[0][0]); off.y = (T)(x[m][1] - x[0][1]); off.z = (T)(x[m][2] - x[0][2]);
+                off.x = (T)(x[0] - xo[0]); off.y = (T)(x[1] - xo[1]); off.z = (T)(x[2] - xo[2]);
                 off.w = (T)0;
                 if (off.x * off.x + off.y * off.y + off.z * off.z > (T)rwat2) atomicOr(&st[1], NB_DEV_ERR_RWAT);
                 ((T4 *)woff_v)[3 * u + m] = off;
@@ -210,7 +223,8 @@ __global__ void k_prepare(int nW, int nA, const int *__restrict__ site_orig, con
             const int s = 3 * nW + (u - nW);
             double x[3];
             load_atom(coor, site_orig[s], x, st);
-            prepare_site<T>(s, x, site_flags, site_q, pos_v, posb, half_skin2, snapshot, true, moved);
+            prepare_site<T, PME>(reps[site_rep[s]], s, x, site_flags, site_q, pos_v, posb, fr_v, zidx, half_skin2, snapshot,
+                            true, moved);
         }
     }
     if (moved) atomicOr(&st[0], 1);
@@ -932,9 +946,9 @@ void build_lists_t(NbCtx *c, const double *d_coor)
         (int)c->nunit, (int)c->nW, c->d_sorted_unit, c->d_unit_atom, c->d_atom_rep, c->d_aflags, c->d_lj_f,
         c->d_lj_d, c->d_q, c->d_site_orig, c->d_site_of, c->d_site_rep, c->d_site_flags, c->d_site_lj,
         c->d_site_q, c->d_status);
-    k_prepare<T><<<grid(c->nW + c->nA, B), B, 0, s>>>((int)c->nW, (int)c->nA, c->d_site_orig, c->d_site_flags,
-                                                      c->d_site_q, d_coor, c->d_pos, c->d_woff, c->d_posb, 0.f,
-                                                      c->rwat * c->rwat, 1, c->d_status);
+    (nb_fused_sites(c) ? k_prepare<T, true> : k_prepare<T, false>)<<<grid(c->nW + c->nA, B), B, 0, s>>>(
+        (int)c->nW, (int)c->nA, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_site_flags, c->d_site_q, d_coor,
+        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, 0.f, c->rwat * c->rwat, 1, c->d_status);
     c->launches += 5;
     // water lists with the row entry type of the handle (uint16 when every replica has fewer
     // than 65,536 waters)
@@ -995,9 +1009,10 @@ void prepare_t(NbCtx *c, const double *d_coor, int check)
     float hs = 0.5f * c->skin;
     const int64_t items = c->nW + c->nA;
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((items + B - 1) / B, (int64_t)c->nsm * 8));
-    k_prepare<T><<<g, B, 0, c->stream>>>((int)c->nW, (int)c->nA, c->d_site_orig, c->d_site_flags, c->d_site_q,
-                                         d_coor, c->d_pos, c->d_woff, c->d_posb, check ? hs * hs : 3.0e38f,
-                                         c->rwat * c->rwat, 0, c->d_status);
+    (nb_fused_sites(c) ? k_prepare<T, true> : k_prepare<T, false>)<<<g, B, 0, c->stream>>>(
+        (int)c->nW, (int)c->nA, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_site_flags, c->d_site_q, d_coor,
+        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, check ? hs * hs : 3.0e38f, c->rwat * c->rwat, 0,
+        c->d_status);
     c->launches += 1;
 }
 
@@ -1028,9 +1043,4 @@ void nb_launch_prepare(NbCtx *c, const double *d_coor, int check)
 {
     if (c->precision == MOIL_NB_FP64) prepare_t<double>(c, d_coor, check);
     else prepare_t<float>(c, d_coor, check);
-}
-
-void nb_exclusive_scan(NbCtx *c, const int *d_in, int *d_out, int n, int *d_total)
-{
-    nb_scan(c, d_in, d_out, n, d_total, 0);
 }

@@ -3,13 +3,14 @@
 // The reference spreads into a padded complex grid, runs two full 3D C2C FFTs
 // (pubz3d / FFTPACK) with the influence function in between (scalar_sum) and gathers.
 // Here the real-space charge grid never exists in HBM:
-//   k_pme_bin      fractional coordinates fr = n (w - anint(w) + 1/2) (:250-260), atoms
-//                  bucketed by int(fr3) (the last z plane of their stencil)
-//   plane_fwd      one CTA per (replica, z plane): the 4x4 x-y stencils of every atom whose
-//                  z stencil touches the plane are accumulated in shared memory in 64-bit
-//                  fixed point (order independent, hence deterministic), then R2C along x
-//                  and C2C along y in shared memory; the half-complex plane goes to HBM
-//                  as [z][kx][ky]
+//   pme_site       (in the coordinate preparation) fractional coordinates
+//                  fr = n (w - anint(w) + 1/2) (:250-260) and, one byte per site, int(fr3),
+//                  the last z plane of the site's stencil
+//   plane_fwd      one CTA per (replica, z plane): the sites whose z stencil touches the plane
+//                  are picked from the replica's z bytes (plane_sites), their 4x4 x-y stencils
+//                  accumulated in shared memory in 32-bit fixed point (order independent,
+//                  hence deterministic), then R2C along x and C2C along y in shared memory;
+//                  the half-complex plane goes to HBM as [z][kx][ky]
 //   zconv          one CTA per (replica, kx, run of ky): C2C along z, the influence function
 //                  exp(-pi^2 m^2 / alpha^2) / (pi V B(m) m^2) with the FP64 energy sum
 //                  (scalar_sum, :723-812), inverse C2C along z, written back in place
@@ -31,83 +32,126 @@
 
 namespace {
 
-__device__ __forceinline__ float nb_round(float x) { return roundf(x); }
-__device__ __forceinline__ double nb_round(double x) { return round(x); }
-
 __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // ---------------------------------------------------------------------------------
-// binning (both precisions)
-
+// PME records and z bytes of every site (handles whose coordinate preparation does not write
+// them, nb_fused_sites)
 template <typename T>
-__global__ void k_pme_bin(int nsite, const int *__restrict__ site_rep, const RepDev *__restrict__ reps,
-                          const void *pos_v, const void *q_v, void *fr_v, int *__restrict__ zcount,
-                          int *__restrict__ zslot)
+__global__ void __launch_bounds__(256) k_pme_sites(int nsite, const int *__restrict__ site_rep,
+                                                   const RepDev *__restrict__ reps, const void *pos_v, const void *q_v,
+                                                   void *fr_v, unsigned char *__restrict__ zidx)
 {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nsite) return;
     typedef typename vec4<T>::type T4;
-    const RepDev &R = reps[site_rep[s]];
-    T4 p = ((const T4 *)pos_v)[s];
-    T4 o;
-    int zb;
-    if constexpr (sizeof(T) == 4) {
-        // fr = n (u - anint(u) + 1/2), u = x / L, carried as hi + lo through every step (1/L as
-        // hi + lo, the product's rounding error by an FMA, the + 1/2 by Fast2Sum) so the
-        // fraction within the grid cell keeps 2^-23 of a grid spacing
-        const float xs[3] = {p.x, p.y, p.z};
-        const int ns[3] = {R.n1, R.n2, R.n3};
-        float out[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float x = xs[d], ih = R.invL[d];
-            const float uh = x * ih, ul = fmaf(x, ih, -uh) + x * R.invL_lo[d];
-            const float a = uh - rintf(uh);              // exact (Sterbenz)
-            const float th = a + 0.5f, tl = (a - (th - 0.5f)) + ul;
-            const float n = (float)ns[d];
-            int i = (int)floorf(n * th);
-            float w = fmaf(n, th, -(float)i) + n * tl;
-            if (w < 0.f) { --i; w += 1.f; }
-            if (w >= 1.f) { ++i; w -= 1.f; }
-            if (i < 0) { i = 0; w = 0.f; }
-            out[d] = pme_fr_pack(i, w);
-            if (d == 2) zb = i;
-        }
-        o.x = out[0]; o.y = out[1]; o.z = out[2];
-        o.w = ((const T *)q_v)[s] * (T)R.fc;
-    } else {
-        T w, f1, f2, f3;
-        w = p.x * rep_invL<T>(R, 0); f1 = (T)R.n1 * (w - nb_round(w) + (T)0.5);
-        w = p.y * rep_invL<T>(R, 1); f2 = (T)R.n2 * (w - nb_round(w) + (T)0.5);
-        w = p.z * rep_invL<T>(R, 2); f3 = (T)R.n3 * (w - nb_round(w) + (T)0.5);
-        o.x = f1; o.y = f2; o.z = f3;
-        o.w = ((const T *)q_v)[s] * (T)R.fcd;
-        zb = (int)f3;
-    }
-    ((T4 *)fr_v)[s] = o;
-    zb = zb >= R.n3 ? zb - R.n3 : (zb < 0 ? 0 : zb);
-    // one atomic per distinct bin of the warp (a warp's sites are neighbours in space)
-    const int key = R.zb0 + zb, lane = threadIdx.x & 31;
-    const unsigned same = __match_any_sync(__activemask(), key);
-    const int leader = __ffs(same) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(&zcount[key], __popc(same));
-    base = __shfl_sync(same, base, leader);
-    zslot[s] = base + __popc(same & ((1u << lane) - 1));
+    const T4 p = ((const T4 *)pos_v)[s];
+    const T x[3] = {p.x, p.y, p.z};
+    unsigned char z;
+    ((T4 *)fr_v)[s] = pme_site(reps[site_rep[s]], x, ((const T *)q_v)[s], z);
+    zidx[s] = z;
 }
 
-__global__ void k_pme_scatter(int nsite, const int *__restrict__ site_rep, const RepDev *__restrict__ reps,
-                              const void *fr_v, int is_double, const int *__restrict__ zstart,
-                              const int *__restrict__ zslot, int *__restrict__ zatoms)
+// ---------------------------------------------------------------------------------
+// Which of 16 sites' z bytes reach plane z: bit e set where (byte e - z) mod n3 < 4
+__device__ __forceinline__ unsigned z_hits(uint4 v, int z, int n3)
 {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsite) return;
-    const RepDev &R = reps[site_rep[s]];
-    int zb;
-    if (is_double) zb = (int)((const double4 *)fr_v)[s].z;
-    else zb = __float_as_int(((const float4 *)fr_v)[s].z) >> 23;   // pme_fr_split
-    zb = zb >= R.n3 ? zb - R.n3 : (zb < 0 ? 0 : zb);
-    zatoms[zstart[R.zb0 + zb] + zslot[s]] = s;
+    const unsigned u[4] = {v.x, v.y, v.z, v.w};
+    unsigned m = 0u;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        unsigned x;
+        if (z + 3 < n3) {
+            // bytes below 128 each: (b | 0x80) - z never borrows from its neighbour, and bits 2-6
+            // with the inverted top bit are zero exactly for 0 <= b - z < 4
+            x = (((u[w] | 0x80808080u) - 0x01010101u * (unsigned)z) ^ 0x80808080u) & 0xfcfcfcfcu;
+            x = ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);          // 0x80 in zero bytes
+        } else {
+            x = 0u;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                int d = (int)((u[w] >> (8 * e)) & 0xffu) - z;
+                d += d < 0 ? n3 : 0;
+                x |= (d < 4 ? 0x80u : 0u) << (8 * e);
+            }
+        }
+        m |= ((((x >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * w);
+    }
+    return m;
+}
+
+// The sites of replica R whose stencil reaches plane z: fn(n) is called by the whole block with n
+// entries (site << 2 | plane within the stencil, 0 = the last) in queue, cap ints of shared memory
+// that are free for this; several times when they do not fit at once or the replica has more
+// than 64 sites per thread.  A thread tests 16 sites' z bytes per load, so a block reads one byte
+// per site of its replica (5 KB for 5,000 sites, from L2) where lists of sites per plane took
+// four launches (binning, scan, scatter and a memset: 18 us before the planes of a small system
+// could start) and 70 bytes of traffic per site.  The order of the entries varies, which the
+// integer planes do not show.
+#define NB_ZLOADS 4
+template <typename Fn>
+__device__ __forceinline__ void plane_sites(const RepDev &R, int nW, int z, const unsigned char *__restrict__ zidx,
+                                            int *queue, int cap, Fn fn)
+{
+    __shared__ int count;
+    const int t = threadIdx.x, n3 = R.n3;
+    if (t == 0) count = 0;
+#pragma unroll 1
+    for (int r = 0; r < 2; ++r) {
+        // the water sites, then the others
+        const int s0 = r == 0 ? 3 * R.wat0 : 3 * nW + R.oth0, s1 = s0 + (r == 0 ? 3 * R.nwat : R.noth);
+#pragma unroll 1
+        for (int c = s0 & ~15; c < s1; c += 16 * NB_ZLOADS * blockDim.x) {
+            uint4 v[NB_ZLOADS];
+            unsigned m[NB_ZLOADS];
+#pragma unroll
+            for (int q = 0; q < NB_ZLOADS; ++q) {
+                const int s = c + 16 * (t + q * (int)blockDim.x);
+                v[q] = s < s1 ? *reinterpret_cast<const uint4 *>(zidx + s) : make_uint4(0u, 0u, 0u, 0u);
+            }
+            int hits = 0;
+#pragma unroll
+            for (int q = 0; q < NB_ZLOADS; ++q) {
+                const int s = c + 16 * (t + q * (int)blockDim.x);
+                m[q] = 0u;
+                if (s < s1) {
+                    m[q] = z_hits(v[q], z, n3);
+                    if (s < s0) m[q] &= 0xffffu << (s0 - s);
+                    if (s + 16 > s1) m[q] &= 0xffffu >> (s + 16 - s1);
+                    hits += __popc(m[q]);
+                }
+            }
+            __syncthreads();           // count is zero; the queue is free
+            const int p = hits ? atomicAdd(&count, hits) : 0;
+            __syncthreads();
+            const int total = count;
+#pragma unroll 1
+            for (int base = 0; base < total; base += cap) {
+                if (hits) {
+                    int k = p - base;
+#pragma unroll 1
+                    for (int q = 0; q < NB_ZLOADS; ++q) {
+                        const int s = c + 16 * (t + q * (int)blockDim.x);
+                        unsigned b = q == 0 ? m[0] : (q == 1 ? m[1] : (q == 2 ? m[2] : m[3]));
+                        while (b) {
+                            const int e = s + __ffs(b) - 1;
+                            b &= b - 1u;
+                            if (k >= 0 && k < cap) {
+                                int d = (int)zidx[e] - z;
+                                d += d < 0 ? n3 : 0;
+                                queue[k] = e << 2 | d;
+                            }
+                            ++k;
+                        }
+                    }
+                }
+                __syncthreads();
+                fn(min(cap, total - base));
+                __syncthreads();
+            }
+            if (t == 0) count = 0;     // everyone has read total (a barrier since, or it was zero)
+        }
+    }
 }
 
 // plane accumulation.  FP32: int32 fixed point; the caller pre-multiplies by the replica's
@@ -162,104 +206,94 @@ __device__ __forceinline__ void bsp4_dth(T w, T d[4])
 // grid index i in [-3, n] wrapped into [0, n)
 __device__ __forceinline__ int pme_wrap(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 
-// the 4x4 x-y stencil of every atom whose z stencil reaches plane z; one atom per thread
+// the 4x4 x-y stencil of n queued sites (plane_sites) into the plane; one site per thread
 template <typename T>
-__device__ __forceinline__ void spread_plane(const RepDev &R, int z, const int *__restrict__ zstart,
-                                             const int *__restrict__ zatoms, const typename vec4<T>::type *fr,
-                                             typename Acc<T>::type *acc, T scale)
+__device__ __forceinline__ void spread_sites(const RepDev &R, const int *queue, int n,
+                                             const typename vec4<T>::type *fr, typename Acc<T>::type *acc, T scale)
 {
     typedef typename vec4<T>::type T4;
-    const int n1 = R.n1, n2 = R.n2, n3 = R.n3;
-    for (int tp = 0; tp < 4; ++tp) {
-        int zb = z + tp;
-        zb = zb >= n3 ? zb - n3 : zb;
-        const int b0 = zstart[R.zb0 + zb], b1 = zstart[R.zb0 + zb + 1];
-        const int t3 = 3 - tp;
-        for (int idx = b0 + threadIdx.x; idx < b1; idx += blockDim.x) {
-            const T4 f = fr[zatoms[idx]];
-            int i1, i2, i3;
-            T w1, w2, w3;
-            pme_fr_split(f.x, i1, w1);
-            pme_fr_split(f.y, i2, w2);
-            pme_fr_split(f.z, i3, w3);
-            T th1[4], th2[4], th3[4];
-            if constexpr (sizeof(T) == 4) {
-                bsp4_th6(w1, th1);
-                bsp4_th6(w2, th2);
-                bsp4_th6(w3, th3);
-            } else {
-                bsp4_th<T>(w1, th1);
-                bsp4_th<T>(w2, th2);
-                bsp4_th<T>(w3, th3);
-            }
-            const T qz = th3[t3] * (f.w * scale);
-            int xs[4];
+    const int n1 = R.n1, n2 = R.n2;
+    for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+        const int e = queue[idx], t3 = 3 - (e & 3);
+        const T4 f = fr[e >> 2];
+        int i1, i2, i3;
+        T w1, w2, w3;
+        pme_fr_split(f.x, i1, w1);
+        pme_fr_split(f.y, i2, w2);
+        pme_fr_split(f.z, i3, w3);
+        T th1[4], th2[4], th3[4];
+        if constexpr (sizeof(T) == 4) {
+            bsp4_th6(w1, th1);
+            bsp4_th6(w2, th2);
+            bsp4_th6(w3, th3);
+        } else {
+            bsp4_th<T>(w1, th1);
+            bsp4_th<T>(w2, th2);
+            bsp4_th<T>(w3, th3);
+        }
+        const T qz = (t3 == 0 ? th3[0] : (t3 == 1 ? th3[1] : (t3 == 2 ? th3[2] : th3[3]))) * (f.w * scale);
+        int xs[4];
 #pragma unroll
-            for (int t1 = 0; t1 < 4; ++t1) xs[t1] = pme_wrap(i1 - 3 + t1, n1);
+        for (int t1 = 0; t1 < 4; ++t1) xs[t1] = pme_wrap(i1 - 3 + t1, n1);
 #pragma unroll
-            for (int t2 = 0; t2 < 4; ++t2) {
-                typename Acc<T>::type *row = acc + pme_wrap(i2 - 3 + t2, n2) * n1;
-                const T v = th2[t2] * qz;
+        for (int t2 = 0; t2 < 4; ++t2) {
+            typename Acc<T>::type *row = acc + pme_wrap(i2 - 3 + t2, n2) * n1;
+            const T v = th2[t2] * qz;
 #pragma unroll
-                for (int t1 = 0; t1 < 4; ++t1) Acc<T>::add(row + xs[t1], v * th1[t1]);
-            }
+            for (int t1 = 0; t1 < 4; ++t1) Acc<T>::add(row + xs[t1], v * th1[t1]);
         }
     }
 }
 
-// gradient share of plane z (real values Rp[ky][x]) for the atoms whose z stencil reaches it
+// gradient (or potential) share of one plane (real values Rp[ky][x]) for n queued sites
 template <typename T>
-__device__ __forceinline__ void gather_plane(const RepDev &R, int z, const int *__restrict__ zstart,
-                                             const int *__restrict__ zatoms, const typename vec4<T>::type *fr,
-                                             const T *Rp, T *__restrict__ part, bool pot = false)
+__device__ __forceinline__ void gather_sites(const RepDev &R, const int *queue, int n,
+                                             const typename vec4<T>::type *fr, const T *Rp, T *__restrict__ part,
+                                             bool pot)
 {
     typedef typename vec4<T>::type T4;
-    const int n1 = R.n1, n2 = R.n2, n3 = R.n3;
-    for (int tp = 0; tp < 4; ++tp) {
-        int zb = z + tp;
-        zb = zb >= n3 ? zb - n3 : zb;
-        const int b0 = zstart[R.zb0 + zb], b1 = zstart[R.zb0 + zb + 1];
-        const int t3 = 3 - tp;
-        for (int idx = b0 + threadIdx.x; idx < b1; idx += blockDim.x) {
-            const int s = zatoms[idx];
-            const T4 f = fr[s];
-            int i1, i2, i3;
-            T w1, w2, w3;
-            pme_fr_split(f.x, i1, w1);
-            pme_fr_split(f.y, i2, w2);
-            pme_fr_split(f.z, i3, w3);
-            T th1[4], dt1[4], th2[4], dt2[4], th3[4], dt3[4];
-            bsp4_th<T>(w1, th1); bsp4_dth<T>(w1, dt1);
-            bsp4_th<T>(w2, th2); bsp4_dth<T>(w2, dt2);
-            bsp4_th<T>(w3, th3); bsp4_dth<T>(w3, dt3);
-            int xs[4];
+    const int n1 = R.n1, n2 = R.n2;
+    for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+        const int e = queue[idx], s = e >> 2, t3 = 3 - (e & 3);
+        const T4 f = fr[s];
+        int i1, i2, i3;
+        T w1, w2, w3;
+        pme_fr_split(f.x, i1, w1);
+        pme_fr_split(f.y, i2, w2);
+        pme_fr_split(f.z, i3, w3);
+        T th1[4], dt1[4], th2[4], dt2[4], th3[4], dt3[4];
+        bsp4_th<T>(w1, th1); bsp4_dth<T>(w1, dt1);
+        bsp4_th<T>(w2, th2); bsp4_dth<T>(w2, dt2);
+        bsp4_th<T>(w3, th3); bsp4_dth<T>(w3, dt3);
+        const T z0 = t3 == 0 ? th3[0] : (t3 == 1 ? th3[1] : (t3 == 2 ? th3[2] : th3[3]));
+        const T z1 = t3 == 0 ? dt3[0] : (t3 == 1 ? dt3[1] : (t3 == 2 ? dt3[2] : dt3[3]));
+        int xs[4];
 #pragma unroll
-            for (int t1 = 0; t1 < 4; ++t1) xs[t1] = pme_wrap(i1 - 3 + t1, n1);
-            T gx = 0, gy = 0, gz = 0;
+        for (int t1 = 0; t1 < 4; ++t1) xs[t1] = pme_wrap(i1 - 3 + t1, n1);
+        T gx = 0, gy = 0, gz = 0;
 #pragma unroll
-            for (int t2 = 0; t2 < 4; ++t2) {
-                const T *row = Rp + pme_wrap(i2 - 3 + t2, n2) * n1;
-                T sx = 0, sy = 0;
+        for (int t2 = 0; t2 < 4; ++t2) {
+            const T *row = Rp + pme_wrap(i2 - 3 + t2, n2) * n1;
+            T sx = 0, sy = 0;
 #pragma unroll
-                for (int t1 = 0; t1 < 4; ++t1) {
-                    const T q = row[xs[t1]];
-                    sx += q * dt1[t1];
-                    sy += q * th1[t1];
-                }
-                gx += sx * th2[t2];
-                gy += sy * dt2[t2];
-                gz += sy * th2[t2];
+            for (int t1 = 0; t1 < 4; ++t1) {
+                const T q = row[xs[t1]];
+                sx += q * dt1[t1];
+                sy += q * th1[t1];
             }
-            if (pot) {
-                // the potential share of this plane (parameter derivatives): one slot per plane
-                part[4 * (size_t)s + t3] = gz * th3[t3];
-                continue;
-            }
-            T *o = part + 12 * (size_t)s + 3 * t3;
-            o[0] = gx * th3[t3];
-            o[1] = gy * th3[t3];
-            o[2] = gz * dt3[t3];
+            gx += sx * th2[t2];
+            gy += sy * dt2[t2];
+            gz += sy * th2[t2];
         }
+        if (pot) {
+            // the potential share of this plane (parameter derivatives): one slot per plane
+            part[4 * (size_t)s + t3] = gz * z0;
+            continue;
+        }
+        T *o = part + 12 * (size_t)s + 3 * t3;
+        o[0] = gx * z0;
+        o[1] = gy * z0;
+        o[2] = gz * z1;
     }
 }
 
@@ -432,10 +466,10 @@ __host__ __device__ __forceinline__ int zconv_buf_elems(int n3)
     return ((a > b ? a : b) + 1) & ~1;
 }
 
-__global__ void __launch_bounds__(256) k_plane_fwd_f(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
+__global__ void __launch_bounds__(256, 8) k_plane_fwd_f(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
                                                      const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
                                                      const float2 *__restrict__ tw, const int2 *__restrict__ tab,
-                                                     const int *__restrict__ zstart, const int *__restrict__ zatoms,
+                                                     int nW, const unsigned char *__restrict__ zidx,
                                                      const float4 *__restrict__ fr, float2 *__restrict__ grid)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -450,8 +484,8 @@ __global__ void __launch_bounds__(256) k_plane_fwd_f(const PlaneWork *__restrict
     ctx = fft_ctx_load(ctx, plans + rep_plan[3 * w.rep], tab, tw, c1);
     fft_ctx_load(ctx, plans + rep_plan[3 * w.rep + 1], tab, tw, c2);
     for (int k = threadIdx.x; k < n1 * n2; k += blockDim.x) acc[k] = 0;
-    __syncthreads();
-    spread_plane<float>(R, w.z, zstart, zatoms, fr, acc, R.spread216);
+    plane_sites(R, nW, w.z, zidx, (int *)B1, 2 * plane_buf_elems(n1, n2),
+                [&](int n) { spread_sites<float>(R, (const int *)B1, n, fr, acc, R.spread216); });
     __syncthreads();
     // x transform of real rows two at a time: line p carries row 2p as its real part and
     // row 2p+1 as its imaginary part
@@ -777,12 +811,14 @@ __device__ C *warp_fft(C *x, C *y, const FftPlanDev &p, const C *__restrict__ tw
 }
 
 #define NB_TK 16
+// ints in the line buffers of the one-warp-per-line kernels (two lines for each of 8 warps)
+template <typename C> constexpr int NB_SCR_INTS = (int)(sizeof(C) * 8 * 2 * NB_MAX_FFT / sizeof(int));
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_plane_fwd(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
                                                    const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                                   const void *tw_v, const int *__restrict__ zstart,
-                                                   const int *__restrict__ zatoms, const void *fr_v, void *grid_v)
+                                                   const void *tw_v, int nW, const unsigned char *__restrict__ zidx,
+                                                   const void *fr_v, void *grid_v)
 {
     typedef typename cplx<T>::type C;
     typedef typename Acc<T>::type A;
@@ -797,8 +833,10 @@ __global__ void __launch_bounds__(256) k_plane_fwd(const PlaneWork *__restrict__
     C *scr = P + n2 * pitch;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     for (int k = threadIdx.x; k < n1 * n2; k += blockDim.x) acc[k] = 0;
-    __syncthreads();
-    spread_plane<T>(R, w.z, zstart, zatoms, (const typename vec4<T>::type *)fr_v, acc, (T)1);
+    // the line buffers, free until the transforms, hold the queue
+    plane_sites(R, nW, w.z, zidx, (int *)scr, NB_SCR_INTS<C>, [&](int n) {
+        spread_sites<T>(R, (const int *)scr, n, (const typename vec4<T>::type *)fr_v, acc, (T)1);
+    });
     __syncthreads();
     C *x = scr + warp * 2 * NB_MAX_FFT, *y = x + NB_MAX_FFT;
     for (int j = warp; j < n2; j += nwarp) {
@@ -955,9 +993,8 @@ __global__ void __launch_bounds__(256) k_press_zvir(const ColWork *__restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) k_plane_inv(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
                                                    const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                                   const void *tw_v, const int *__restrict__ zstart,
-                                                   const int *__restrict__ zatoms, const void *fr_v,
-                                                   const void *grid_v, T *__restrict__ part, int pot)
+                                                   const void *tw_v, int nW, const unsigned char *__restrict__ zidx,
+                                                   const void *fr_v, const void *grid_v, T *__restrict__ part, int pot)
 {
     typedef typename cplx<T>::type C;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -996,7 +1033,9 @@ __global__ void __launch_bounds__(256) k_plane_inv(const PlaneWork *__restrict__
         __syncwarp();
     }
     __syncthreads();
-    gather_plane<T>(R, w.z, zstart, zatoms, (const typename vec4<T>::type *)fr_v, Rp, part, pot != 0);
+    plane_sites(R, nW, w.z, zidx, (int *)scr, NB_SCR_INTS<C>, [&](int n) {
+        gather_sites<T>(R, (const int *)scr, n, (const typename vec4<T>::type *)fr_v, Rp, part, pot != 0);
+    });
 }
 
 // ---------------------------------------------------------------------------------
@@ -1006,19 +1045,17 @@ template <typename T>
 void pme_t(NbCtx *c)
 {
     cudaStream_t s = c->stream;
-    const int B = 256;
     if (c->timing) cudaEventRecord(c->ev[6], s);
-    cudaMemsetAsync(c->d_zcount, 0, sizeof(int) * (c->nzbin + 1), s);
-    k_pme_bin<T><<<(int)((c->nsite + B - 1) / B), B, 0, s>>>((int)c->nsite, c->d_site_rep, c->d_reps, c->d_pos,
-                                                            c->d_site_q, c->d_fr, c->d_zcount, c->d_zslot);
-    nb_exclusive_scan(c, c->d_zcount, c->d_zstart, c->nzbin, nullptr);
-    k_pme_scatter<<<(int)((c->nsite + B - 1) / B), B, 0, s>>>((int)c->nsite, c->d_site_rep, c->d_reps, c->d_fr,
-                                                             sizeof(T) == 8, c->d_zstart, c->d_zslot, c->d_zatoms);
+    if (c->d_pos && !nb_fused_sites(c)) {
+        k_pme_sites<T><<<(int)((c->nsite + 255) / 256), 256, 0, s>>>((int)c->nsite, c->d_site_rep, c->d_reps, c->d_pos,
+                                                                    c->d_site_q, c->d_fr, c->d_zidx);
+        c->launches++;
+    }
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
     if (sizeof(T) == 4) {
         k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                           (const float2 *)c->d_tw, c->d_tab, c->d_zstart,
-                                                           c->d_zatoms, (const float4 *)c->d_fr, (float2 *)c->d_grid);
+                                                           (const float2 *)c->d_tw, c->d_tab, (int)c->nW, c->d_zidx,
+                                                           (const float4 *)c->d_fr, (float2 *)c->d_grid);
         if (c->timing) cudaEventRecord(c->ev[7], s);
         k_zconv_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan,
                                                   (const float2 *)c->d_tw, c->d_tab, c->d_etab,
@@ -1032,17 +1069,17 @@ void pme_t(NbCtx *c)
         c->launches++;
     } else {
         k_plane_fwd<T><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
-                                                          c->d_zstart, c->d_zatoms, c->d_fr, c->d_grid);
+                                                          (int)c->nW, c->d_zidx, c->d_fr, c->d_grid);
         if (c->timing) cudaEventRecord(c->ev[7], s);
         k_zconv<T><<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
                                                    c->d_bsp, c->d_grid, c->d_e_col);
         if (c->timing) cudaEventRecord(c->ev[8], s);
         k_plane_inv<T><<<np, 256, c->smem_plane_inv, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
-                                                          c->d_zstart, c->d_zatoms, c->d_fr, c->d_grid,
+                                                          (int)c->nW, c->d_zidx, c->d_fr, c->d_grid,
                                                           (T *)c->d_part, 0);
     }
     if (c->timing) cudaEventRecord(c->ev[9], s);
-    c->launches += 6;
+    c->launches += 3;
 }
 
 // radix plan and Stockham tables; returns 0 if n is not 2/3/5-smooth or too long.  Narrow
@@ -1290,7 +1327,7 @@ void nb_launch_pme(NbCtx *c)
     else pme_t<float>(c);
 }
 
-// pressure analysis: the charge planes of the evaluation's binning spread and transformed
+// pressure analysis: the charge planes of the evaluation's sites spread and transformed
 // again into grid (a copy beside the handle's own grid, whose potential planes stay valid),
 // and the reciprocal virial per column work item into v_col (mixed path)
 void nb_launch_pme_virial(NbCtx *c, void *grid, double *v_col)
@@ -1299,13 +1336,13 @@ void nb_launch_pme_virial(NbCtx *c, void *grid, double *v_col)
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
     if (c->precision == MOIL_NB_FP64) {
         k_plane_fwd<double><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                               c->d_tw, c->d_zstart, c->d_zatoms, c->d_fr, grid);
+                                                               c->d_tw, (int)c->nW, c->d_zidx, c->d_fr, grid);
         k_press_zvir<double><<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
                                                             c->d_bsp, grid, v_col);
         return;
     }
     k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                       (const float2 *)c->d_tw, c->d_tab, c->d_zstart, c->d_zatoms,
+                                                       (const float2 *)c->d_tw, c->d_tab, (int)c->nW, c->d_zidx,
                                                        (const float4 *)c->d_fr, (float2 *)grid);
     k_press_zvir_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan,
                                                    (const float2 *)c->d_tw, c->d_tab, (const float *)c->d_bsp,
@@ -1317,8 +1354,7 @@ void nb_launch_pme_virial(NbCtx *c, void *grid, double *v_col)
 void nb_launch_pme_potential(NbCtx *c, double *phi4)
 {
     k_plane_inv<double><<<(int)c->planes.size(), 256, c->smem_plane_inv, c->stream>>>(
-        c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw, c->d_zstart, c->d_zatoms, c->d_fr, c->d_grid,
-        phi4, 1);
+        c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw, (int)c->nW, c->d_zidx, c->d_fr, c->d_grid, phi4, 1);
 }
 
 int nb_pme_configure(NbCtx *c)
@@ -1381,16 +1417,11 @@ constexpr int NA_MAX_TAB = 3 * 8 * NA_MAX_N;
 constexpr size_t na_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // arena regions (byte offsets, 256-byte aligned)
-constexpr size_t NA_POS = 0;
-constexpr size_t NA_Q = NA_POS + na_up(sizeof(float4) * NA_MAX_ATOMS);
-constexpr size_t NA_REP = NA_Q + na_up(sizeof(float) * NA_MAX_ATOMS);
+constexpr size_t NA_REP = 0;
 constexpr size_t NA_FR = NA_REP + na_up(sizeof(int) * NA_MAX_ATOMS);
-constexpr size_t NA_ZSLOT = NA_FR + na_up(sizeof(float4) * NA_MAX_ATOMS);
-constexpr size_t NA_ZATOMS = NA_ZSLOT + na_up(sizeof(int) * NA_MAX_ATOMS);
-constexpr size_t NA_PART = NA_ZATOMS + na_up(sizeof(int) * NA_MAX_ATOMS);
-constexpr size_t NA_ZCOUNT = NA_PART + na_up(sizeof(float) * 12 * NA_MAX_ATOMS);
-constexpr size_t NA_ZSTART = NA_ZCOUNT + na_up(sizeof(int) * (NA_MAX_N + 1));
-constexpr size_t NA_GRID = NA_ZSTART + na_up(sizeof(int) * (NA_MAX_N + 1));
+constexpr size_t NA_ZIDX = NA_FR + na_up(sizeof(float4) * NA_MAX_ATOMS);
+constexpr size_t NA_PART = NA_ZIDX + na_up(NA_MAX_ATOMS + 16);
+constexpr size_t NA_GRID = NA_PART + na_up(sizeof(float) * 12 * NA_MAX_ATOMS);
 constexpr size_t NA_ECOL = NA_GRID + na_up(sizeof(float2) * ((NA_MAX_N / 2 + 1) * NA_MAX_N * NA_MAX_N + 2));
 constexpr size_t NA_PLANES = NA_ECOL + na_up(sizeof(double) * NA_MAX_COLS);
 constexpr size_t NA_COLS = NA_PLANES + na_up(sizeof(PlaneWork) * NA_MAX_N);
@@ -1412,13 +1443,14 @@ std::mutex g_na_mu;
 constexpr int NA_MAX_DEVICES = 64;
 unsigned char *g_na_base[NA_MAX_DEVICES] = {};
 
-__global__ void k_na_load(int natom, const double *__restrict__ coor, const double *__restrict__ q,
-                          float4 *__restrict__ pos, float *__restrict__ sq, int *__restrict__ srep)
+__global__ void k_na_load(int natom, const RepDev *__restrict__ reps, const double *__restrict__ coor,
+                          const double *__restrict__ q, float4 *__restrict__ fr, unsigned char *__restrict__ zidx,
+                          int *__restrict__ srep)
 {
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= natom) return;
-    pos[a] = make_float4((float)coor[3 * (size_t)a], (float)coor[3 * (size_t)a + 1], (float)coor[3 * (size_t)a + 2], 0.f);
-    sq[a] = (float)q[a];
+    const float x[3] = {(float)coor[3 * (size_t)a], (float)coor[3 * (size_t)a + 1], (float)coor[3 * (size_t)a + 2]};
+    fr[a] = pme_site(reps[0], x, (float)q[a], zidx[a]);
     srep[a] = 0;
 }
 
@@ -1539,7 +1571,7 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     R.pivol = M_PI * box[0] * box[1] * box[2];
     nb_pme_fp32_consts(&R);
     R.pme_qcorr = 1.0;    // the charges stay on the device: no rounding correction
-    R.natom = natom;
+    R.natom = R.noth = natom;   // every atom a non-water site
     FftPlanDev plans[3];
     int rep_plan[3];
     float2 tw[3 * NA_MAX_N];
@@ -1569,7 +1601,6 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     tmp.stream = stream;
     tmp.nrep = 1;
     tmp.nsite = natom;
-    tmp.nzbin = n3;
     for (int z = 0; z < n3; ++z) tmp.planes.push_back(PlaneWork{0, z});
     for (int kx = 0; kx < R.n1h; ++kx)
         push_col_runs(tmp.cols, 0, kx, n2, NB_TKF);
@@ -1577,15 +1608,10 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     tmp.smem_plane_fwd = plane_fwd_smem<float>(n1, n2);
     tmp.smem_plane_inv = plane_inv_smem<float>(n1, n2);
     tmp.smem_zconv = zconv_smem<float>(n3);
-    tmp.d_pos = base + NA_POS;
-    tmp.d_site_q = base + NA_Q;
     tmp.d_site_rep = (int *)(base + NA_REP);
     tmp.d_fr = base + NA_FR;
-    tmp.d_zslot = (int *)(base + NA_ZSLOT);
-    tmp.d_zatoms = (int *)(base + NA_ZATOMS);
+    tmp.d_zidx = base + NA_ZIDX;
     tmp.d_part = base + NA_PART;
-    tmp.d_zcount = (int *)(base + NA_ZCOUNT);
-    tmp.d_zstart = (int *)(base + NA_ZSTART);
     tmp.d_grid = base + NA_GRID;
     tmp.d_e_col = (double *)(base + NA_ECOL);
     tmp.d_planes = (PlaneWork *)(base + NA_PLANES);
@@ -1614,8 +1640,8 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     NA_CP(tmp.d_cols, tmp.cols.data(), sizeof(ColWork) * tmp.cols.size());
     NA_CP(tmp.d_col_begin, col_begin, sizeof(col_begin));
 #undef NA_CP
-    k_na_load<<<(natom + 255) / 256, 256, 0, stream>>>(natom, d_coor, d_q, (float4 *)tmp.d_pos,
-                                                       (float *)tmp.d_site_q, tmp.d_site_rep);
+    k_na_load<<<(natom + 255) / 256, 256, 0, stream>>>(natom, tmp.d_reps, d_coor, d_q, (float4 *)tmp.d_fr, tmp.d_zidx,
+                                                       tmp.d_site_rep);
     k_na_scale<<<1, 256, 0, stream>>>(natom, d_q, tmp.d_reps);
     pme_t<float>(&tmp);
     k_na_grad<<<(natom + 255) / 256, 256, 0, stream>>>(natom, tmp.d_reps, d_q, (const float *)tmp.d_part, d_dpot);

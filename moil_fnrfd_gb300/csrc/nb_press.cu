@@ -19,7 +19,7 @@
 // with checkANDmove, :985-1010), which needs consecutive atoms of a molecule closer than half
 // the box.
 //
-// The pass reuses the evaluation's lists, site positions, PME binning and PME gradient
+// The pass reuses the evaluation's lists, site positions, PME records and PME gradient
 // shares, with the pair predicates and the arithmetic of the energy kernels of the handle's
 // precision.  On the mixed path the products with the centre-of-mass separations are FP32
 // too, summed per thread in FP32 over chunks of NB_PCHUNK list entries and in FP64 across
