@@ -75,6 +75,16 @@ template <typename T> void free_ptr(T *&p)
     p = nullptr;
 }
 
+void drop_graph(NbCtx *c)
+{
+    for (NbCtx::EvalGraph &g : c->graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
+    if (c->gexec_md) cudaGraphExecDestroy(c->gexec_md);
+    c->gexec_md = nullptr;
+}
+
 void release_device(NbCtx *c)
 {
     free_ptr(c->d_reps); free_ptr(c->d_q); free_ptr(c->d_lj_f); free_ptr(c->d_lj_d); free_ptr(c->d_aflags);
@@ -92,7 +102,7 @@ void release_device(NbCtx *c)
     c->whalf = 0;
     free_ptr(c->d_bsp); free_ptr(c->d_etab); free_ptr(c->d_zidx);
     free_ptr(c->d_fr); free_ptr(c->d_grid); free_ptr(c->d_part); free_ptr(c->d_planes); free_ptr(c->d_cols);
-    free_ptr(c->d_col_begin); free_ptr(c->d_e_col); free_ptr(c->d_e_rep);
+    free_ptr(c->d_col_begin); free_ptr(c->d_e_col); free_ptr(c->d_edone);
     free_ptr(c->d_echunks); free_ptr(c->d_echunk_begin); free_ptr(c->d_epart);
     c->echunks.clear(); free_ptr(c->d_coor); free_ptr(c->d_dpot);
     free_ptr(c->d_adj); free_ptr(c->d_adj_phi); free_ptr(c->d_md_dpot); free_ptr(c->d_mdctl);
@@ -103,10 +113,7 @@ void release_device(NbCtx *c)
     c->nmol = 0;
     if (c->h_e_rep) cudaFreeHost(c->h_e_rep);
     c->h_e_rep = nullptr;
-    if (c->gexec) cudaGraphExecDestroy(c->gexec);
-    c->gexec = nullptr;
-    if (c->gexec_md) cudaGraphExecDestroy(c->gexec_md);
-    c->gexec_md = nullptr;
+    drop_graph(c);
     c->inited = 0;
 }
 
@@ -600,7 +607,8 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     NB_CUDA_OK(c, cudaMalloc(&c->d_grad_ex, sizeof(double) * 3 * c->natom));
     NB_CUDA_OK(c, cudaMalloc(&c->d_e_ex, sizeof(double) * NB_EX * c->natom));
     NB_CUDA_OK(c, cudaMalloc(&c->d_zidx, ns + 16));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_e_rep, sizeof(double) * NB_EREP * nrep));
+    NB_CUDA_OK(c, cudaMalloc(&c->d_edone, sizeof(int) * nrep));
+    NB_CUDA_OK(c, cudaMemset(c->d_edone, 0, sizeof(int) * nrep));
     NB_CUDA_OK(c, cudaMalloc(&c->d_coor, sizeof(double) * 3 * c->natom));
     NB_CUDA_OK(c, cudaMalloc(&c->d_dpot, sizeof(double) * 3 * c->natom));
     NB_CUDA_OK(c, cudaMemset(c->d_grad_site, 0, sizeof(long long) * 3 * ns));
@@ -642,28 +650,35 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     return MOIL_NB_OK;
 }
 
-// While an evaluation is captured: the list rebuild goes into the body of a conditional IF
-// node that a one-thread kernel sets from the device rebuild flag, so evaluations without a
-// rebuild launch none of the rebuild kernels.  Returns false (the gated kernels are then
-// captured in line) if the stream is not capturing or a graph call fails before the node is
-// added.
-bool enqueue_lists_conditional(NbCtx *c, const double *d_coor)
+// While an evaluation is captured: a conditional handle of its graph that the coordinate
+// preparation sets from the rebuild decision (0 if the stream is not capturing or the call fails)
+cudaGraphConditionalHandle rebuild_handle(NbCtx *c)
+{
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t g = nullptr;
+    cudaGraphConditionalHandle hc = 0;
+    if (cudaStreamGetCaptureInfo(c->stream, &cs, nullptr, &g, nullptr, nullptr, nullptr) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusActive ||
+        cudaGraphConditionalHandleCreate(&hc, g, 0, cudaGraphCondAssignDefault) != cudaSuccess)
+        return 0;
+    return hc;
+}
+
+// The list rebuild in the body of a conditional IF node on hc, so evaluations without a rebuild
+// launch none of its kernels.  Returns false (the gated kernels are then captured in line) if a
+// graph call fails before the node is added.
+bool enqueue_lists_conditional(NbCtx *c, const double *d_coor, cudaGraphConditionalHandle hc)
 {
     cudaStream_t s = c->stream;
     cudaStreamCaptureStatus cs;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t *deps = nullptr;
     size_t nd = 0;
-    if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, nullptr, &nd) != cudaSuccess ||
-        cs != cudaStreamCaptureStatusActive)
-        return false;
-    cudaGraphConditionalHandle hc;
-    if (cudaGraphConditionalHandleCreate(&hc, g, 0, cudaGraphCondAssignDefault) != cudaSuccess) return false;
+    if (!hc) return false;
     if (!c->sbody && cudaStreamCreateWithFlags(&c->sbody, cudaStreamNonBlocking) != cudaSuccess) {
         c->sbody = nullptr;
         return false;
     }
-    nb_launch_rebuild_cond(c, hc);
     if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, nullptr, &nd) != cudaSuccess) return false;
     cudaGraphNodeParams np = {};
     np.type = cudaGraphNodeTypeConditional;
@@ -689,19 +704,33 @@ bool enqueue_lists_conditional(NbCtx *c, const double *d_coor)
     return true;
 }
 
+// Handles whose evaluations the host decides on (EVAL_KEEP / EVAL_BUILD): the conditional node
+// and the copy of the initial status words cost 26 us of a 216-water evaluation's 77, a dropped
+// evaluation at most one per rebuild.  Larger handles lose more by a dropped evaluation (the
+// limit is about 150 us of work) and keep the device's decision; so do the prioritised streams,
+// and, after a rebuild because a site moved, the next two evaluations (calls on unrelated
+// coordinates rebuild every time).
+bool host_decides(const NbCtx *c) { return !c->on_prio && c->wary == 0 && c->nw_handle + c->na_handle <= 32768; }
+
 // The device part of one evaluation, in stream order.  The sequence does not depend on host
-// state beyond the handle's fixed buffers and the two caller pointers: the rebuild decision
-// travels through the pinned word h_status[8], read by the first copy.  That makes it
-// capturable as a CUDA graph.
+// state beyond the handle's fixed buffers and the two caller pointers, so it is capturable as a
+// CUDA graph; in EVAL_DEVICE the rebuild request travels through the pinned word h_status[8].
 // The evaluation between its status words: coordinate preparation, list rebuild, pair, PME
-// and correction kernels, gradient and energy assembly.
-void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot)
+// and correction kernels, gradient and energy assembly (ctl: as an MD step, see k_finalize).
+void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot, EvalMode mode, int *ctl)
 {
     cudaStream_t s = c->stream;
-    nb_launch_prepare(c, d_coor, 1);   // sets the rebuild flag when a site moved > skin/2
+    cudaGraphConditionalHandle hc = 0;
+    if (mode == EVAL_DEVICE && c->capturing && !c->on_prio) hc = rebuild_handle(c);
+    // sets the rebuild flag when a site moved > skin/2
+    if (mode != EVAL_BUILD) nb_launch_prepare(c, d_coor, hc, ctl);
     // every rebuild kernel is gated by the flag; a captured evaluation also skips their
     // launches through a conditional node
-    if (c->timing) {
+    if (mode == EVAL_BUILD) {
+        nb_launch_build_lists(c, d_coor);
+    } else if (mode == EVAL_KEEP) {
+        // none: a set flag comes back with the status words and the evaluation is redone
+    } else if (c->timing) {
         // stage timing (kernel by kernel): the host reads the flag and launches the rebuild
         // only when it is set, as the conditional node of a replayed evaluation does.  The
         // preparation stage (status upload, coordinate conversion with the skin check) ends
@@ -713,7 +742,7 @@ void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot)
         cudaEventRecord(c->ev[13], s);
         if (c->h_status[16]) nb_launch_build_lists(c, d_coor);
         cudaEventRecord(c->ev[1], s);
-    } else if (!(c->capturing && !c->on_prio && enqueue_lists_conditional(c, d_coor))) {
+    } else if (!enqueue_lists_conditional(c, d_coor, hc)) {
         // (on the prioritised streams of host-buffer group evaluations the conditional node
         // cost the copy/kernel overlap more than the skipped launches save: gated kernels)
         nb_launch_build_lists(c, d_coor);
@@ -755,83 +784,42 @@ void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot)
         cudaStreamWaitEvent(s, c->ev_join, 0);
         if (third) cudaStreamWaitEvent(s, c->ev_join3, 0);
     }
-    nb_launch_finalize(c, d_dpot);
+    nb_launch_finalize(c, d_dpot, ctl);
 }
 
-void enqueue_eval(NbCtx *c, const double *d_coor, double *d_dpot)
+void enqueue_eval(NbCtx *c, const double *d_coor, double *d_dpot, EvalMode mode)
 {
     cudaStream_t s = c->stream;
     c->launches = 0;
     if (c->timing) cudaEventRecord(c->ev[0], s);
-    cudaMemcpyAsync(c->d_status, c->h_status + 8, sizeof(int) * 8, cudaMemcpyHostToDevice, s);
-    enqueue_core(c, d_coor, d_dpot);
+    if (mode == EVAL_DEVICE) cudaMemcpyAsync(c->d_status, c->h_status + 8, sizeof(int) * 8, cudaMemcpyHostToDevice, s);
+    else if (mode == EVAL_BUILD) cudaMemsetAsync(c->d_status, 1, 1, s);    // the flag the rebuild kernels look at
+    enqueue_core(c, d_coor, d_dpot, mode, nullptr);
     if (c->timing) cudaEventRecord(c->ev[10], s);
-    cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int) * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(c->h_e_rep, c->d_e_rep, sizeof(double) * NB_EREP * c->nrep, cudaMemcpyDeviceToHost, s);
 }
 
-// one whole MD step of a context, as captured into its step graph: a gate kernel sets an IF
-// node that runs the step only while no error has been raised in the call; the step is the
-// step-control kernel, the evaluation, the error bits and rebuild counter, the leapfrog +
-// SETTLE integrator.  Returns false if the gate could not be built (nothing captured then).
-bool enqueue_md_step(NbCtx *c, double *coor, double *vel, const double *mass, double *dpot, double dt, double doh,
+// one whole MD step of a context, as captured into its step graph: the evaluation, whose last
+// kernel keeps the error bits and sets the next step's rebuild request, and the leapfrog + SETTLE
+// integrator.  After an error the coordinate preparation of the remaining steps returns at
+// once, so no list is rebuilt from what those steps move (the call is then redone from its
+// starting state).
+void enqueue_md_step(NbCtx *c, double *coor, double *vel, const double *mass, double *dpot, double dt, double doh,
                      double dhh)
 {
-    cudaStream_t s = c->stream;
     c->launches = 0;
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t nd = 0;
-    if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, nullptr, &nd) != cudaSuccess ||
-        cs != cudaStreamCaptureStatusActive)
-        return false;
-    cudaGraphConditionalHandle hc;
-    if (cudaGraphConditionalHandleCreate(&hc, g, 0, cudaGraphCondAssignDefault) != cudaSuccess) return false;
-    if (!c->sstep && cudaStreamCreateWithFlags(&c->sstep, cudaStreamNonBlocking) != cudaSuccess) {
-        c->sstep = nullptr;
-        return false;
-    }
-    nb_launch_md_gate(c, s, hc);
-    if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, nullptr, &nd) != cudaSuccess) return false;
-    cudaGraphNodeParams np = {};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = hc;
-    np.conditional.type = cudaGraphCondTypeIf;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    if (cudaGraphAddNode(&node, g, deps, nullptr, nd, &np) != cudaSuccess) return false;
-    if (cudaStreamBeginCaptureToGraph(c->sstep, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                      cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-        return false;
-    std::swap(c->stream, c->sstep);
-    nb_launch_md_begin(c, c->stream);
-    enqueue_core(c, coor, dpot);
-    nb_launch_md_end(c, c->stream);
+    enqueue_core(c, coor, dpot, EVAL_DEVICE, c->d_mdctl);
     nb_launch_integrate(c, c->stream, coor, vel, mass, dpot, dt, doh, dhh);
-    std::swap(c->stream, c->sstep);
-    cudaGraph_t done = nullptr;
-    cudaStreamEndCapture(c->sstep, &done);
-    cudaStreamUpdateCaptureDependencies(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
-    return true;
-}
-
-void drop_graph(NbCtx *c)
-{
-    if (c->gexec) cudaGraphExecDestroy(c->gexec);
-    c->gexec = nullptr;
-    if (c->gexec_md) cudaGraphExecDestroy(c->gexec_md);
-    c->gexec_md = nullptr;
 }
 
 // replay the captured evaluation, capturing it first when the caller pointers or the list
 // buffers changed; returns false (graph mode switched off) if capture is not possible
-bool launch_graph(NbCtx *c, const double *d_coor, double *d_dpot)
+bool launch_graph(NbCtx *c, const double *d_coor, double *d_dpot, EvalMode mode)
 {
     cudaStream_t s = c->stream;
-    if (!c->gexec || c->g_coor != d_coor || c->g_dpot != d_dpot || c->g_gen != c->list_gen ||
-        c->g_prio != c->on_prio) {
-        drop_graph(c);
+    NbCtx::EvalGraph &G = c->graphs[mode];
+    if (!G.exec || G.coor != d_coor || G.dpot != d_dpot || G.gen != c->list_gen || G.prio != c->on_prio) {
+        if (G.exec) cudaGraphExecDestroy(G.exec);
+        G.exec = nullptr;
         cudaGraph_t g = nullptr;
         if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
@@ -839,35 +827,47 @@ bool launch_graph(NbCtx *c, const double *d_coor, double *d_dpot)
             return false;
         }
         c->capturing = 1;
-        enqueue_eval(c, d_coor, d_dpot);
+        enqueue_eval(c, d_coor, d_dpot, mode);
         c->capturing = 0;
         cudaError_t e1 = cudaStreamEndCapture(s, &g);
-        cudaError_t e2 = e1 == cudaSuccess ? cudaGraphInstantiate(&c->gexec, g, cudaGraphInstantiateFlagUseNodePriority) : e1;
+        cudaError_t e2 = e1 == cudaSuccess ? cudaGraphInstantiate(&G.exec, g, cudaGraphInstantiateFlagUseNodePriority) : e1;
         if (g) cudaGraphDestroy(g);
         if (e2 != cudaSuccess) {
             cudaGetLastError();
-            c->gexec = nullptr;
+            G.exec = nullptr;
             c->use_graph = 0;
             return false;
         }
-        c->g_coor = d_coor;
-        c->g_dpot = d_dpot;
-        c->g_prio = c->on_prio;
-        c->g_gen = c->list_gen;
-        c->graph_launches = c->launches;
+        G.coor = d_coor;
+        G.dpot = d_dpot;
+        G.prio = c->on_prio;
+        G.gen = c->list_gen;
+        G.launches = c->launches;
     }
-    c->launches = c->graph_launches;
-    return cudaGraphLaunch(c->gexec, s) == cudaSuccess;
+    c->launches = G.launches;
+    return cudaGraphLaunch(G.exec, s) == cudaSuccess;
 }
 
 // queue one evaluation on the context's stream (no synchronisation)
 void eval_launch(NbCtx *c, const double *d_coor, double *d_dpot)
 {
     bool forced = c->need_rebuild || (c->list_period > 0 && c->evals_since_build >= c->list_period);
+    c->eval_forced = forced;
     c->h_status[8] = forced ? 1 : 0;
     for (int k = 9; k < 16; ++k) c->h_status[k] = 0;
-    if (!(c->use_graph && !c->timing && launch_graph(c, d_coor, d_dpot))) enqueue_eval(c, d_coor, d_dpot);
+    c->h_status[23] = 0;
+    EvalMode mode = EVAL_DEVICE;
+    if (c->use_graph && !c->timing) {
+        if (host_decides(c)) mode = forced ? EVAL_BUILD : EVAL_KEEP;
+        c->eval_mode = mode;
+        if (launch_graph(c, d_coor, d_dpot, mode)) return;
+    }
+    c->eval_mode = EVAL_DEVICE;
+    enqueue_eval(c, d_coor, d_dpot, EVAL_DEVICE);
 }
+
+// internal status of an evaluation without the rebuild it turned out to need (redone with it)
+constexpr int kStale = -1;
 
 // wait for the queued evaluation and read its status words
 int eval_complete(NbCtx *c)
@@ -875,6 +875,9 @@ int eval_complete(NbCtx *c)
     NB_CUDA_OK(c, cudaStreamSynchronize(c->stream));
     NB_CUDA_OK(c, cudaGetLastError());
     int rebuilt = c->h_status[0] != 0;
+    if (rebuilt && !c->eval_forced) c->wary = 2;
+    else if (c->wary > 0 && c->eval_mode == EVAL_DEVICE) --c->wary;
+    if (rebuilt && c->eval_mode == EVAL_KEEP) return kStale;
     if (rebuilt) {
         c->evals_since_build = 0;
         c->last_water_pairs = c->h_status[2];
@@ -903,7 +906,7 @@ int eval_complete(NbCtx *c)
         t.list_rebuilt = rebuilt;
         t.launches = c->launches;
     }
-    int err = c->h_status[1];
+    int err = c->h_status[1] | (c->h_status[23] ? NB_DEV_ERR_NAN : 0);
     if (err & NB_DEV_ERR_OVERFLOW) return MOIL_NB_ERR_OVERFLOW;
     if (err & NB_DEV_ERR_NAN) { c->err = "non-finite coordinate or gradient"; return MOIL_NB_ERR_NAN; }
     if (err & NB_DEV_ERR_RWAT) { c->err = "a water hydrogen moved more than 1.1 A from its oxygen"; return MOIL_NB_ERR_TOPOLOGY; }
@@ -933,12 +936,16 @@ void read_energies(NbCtx *c, moil_energies *e)
     c->last_site_pairs = (int64_t)(np + 0.5);
 }
 
-// an evaluation whose first attempt (if any) has completed with status rc: on a list
-// overflow, grow the lists from the counts and redo
+// an evaluation whose first attempt (if any) has completed with status rc: redone with a rebuild
+// if it was stale; on a list overflow, grow the lists from the counts and redo
 int eval_retry(NbCtx *c, const double *d_coor, double *d_dpot, moil_energies *e, int rc, bool done)
 {
     for (int attempt = 0; attempt < 4; ++attempt) {
         if (!done || attempt > 0) rc = eval_once(c, d_coor, d_dpot);
+        if (rc == kStale) {
+            c->need_rebuild = 1;
+            rc = eval_once(c, d_coor, d_dpot);
+        }
         if (rc != MOIL_NB_ERR_OVERFLOW) break;
         // grow from the exact totals the count pass produced, then redo with a fresh build
         int64_t need1 = c->h_status[6], need2 = c->h_status[3], need3 = c->h_status[4];
@@ -1005,8 +1012,8 @@ int eval_groups(NbCtx *h, const double *coor, double *dpot, moil_energies *e, bo
         double *dd = host ? c->d_dpot : dpot + 3 * h->grp_atom0[g];
         const int first = eval_complete(c);
         int rc = eval_retry(c, dc, dd, e ? e + h->grp_rep0[g] : nullptr, first, true);
-        if (rc == MOIL_NB_OK && host && first == MOIL_NB_ERR_OVERFLOW) {
-            // redone after an overflow: the gradient copied with the first attempt is stale
+        if (rc == MOIL_NB_OK && host && first != MOIL_NB_OK) {
+            // redone: the gradient copied with the first attempt is not this evaluation's
             NB_CUDA_OK(c, cudaMemcpyAsync(dpot + 3 * h->grp_atom0[g], c->d_dpot, slice_bytes(g),
                                           cudaMemcpyDeviceToHost, c->stream));
             NB_CUDA_OK(c, cudaStreamSynchronize(c->stream));
@@ -1221,7 +1228,6 @@ void moil_nb_destroy(moil_nb_ctx *h)
     if (h->stream2n) { cudaStreamSynchronize(h->stream2n); cudaStreamDestroy(h->stream2n); }
     if (h->stream3) { cudaStreamSynchronize(h->stream3); cudaStreamDestroy(h->stream3); }
     if (h->sbody) cudaStreamDestroy(h->sbody);
-    if (h->sstep) cudaStreamDestroy(h->sstep);
     if (h->pstream) cudaStreamDestroy(h->pstream);
     if (h->pstream2) cudaStreamDestroy(h->pstream2);
     if (h->pstream3) cudaStreamDestroy(h->pstream3);
@@ -1716,9 +1722,12 @@ int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *
     if (!c->d_mdctl) NB_CUDA_OK(c, cudaMalloc(&c->d_mdctl, sizeof(int) * 4));
     // the host's list schedule goes to the device once per call
     c->h_status[17] = c->evals_since_build;
-    c->h_status[18] = c->need_rebuild ? 1 : 0;
-    c->h_status[19] = 0;
+    c->h_status[18] = c->h_status[19] = 0;
+    c->h_status[8] = c->need_rebuild || (c->list_period > 0 && c->evals_since_build >= c->list_period) ? 1 : 0;
+    for (int k = 9; k < 16; ++k) c->h_status[k] = 0;
+    c->h_status[23] = 0;
     NB_CUDA_OK(c, cudaMemcpyAsync(c->d_mdctl, c->h_status + 17, sizeof(int) * 3, cudaMemcpyHostToDevice, s));
+    NB_CUDA_OK(c, cudaMemcpyAsync(c->d_status, c->h_status + 8, sizeof(int) * 8, cudaMemcpyHostToDevice, s));
     const bool same = c->gexec_md && c->gmd_key[0] == coor && c->gmd_key[1] == vel && c->gmd_key[2] == mass &&
                       c->gmd_dt == dt && c->gmd_doh == doh && c->gmd_dhh == dhh && c->gmd_gen == c->list_gen &&
                       c->gmd_dpot == dpot;
@@ -1728,10 +1737,10 @@ int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *
         cudaGraph_t g = nullptr;
         NB_CUDA_OK(c, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         c->capturing = 1;
-        const bool built = enqueue_md_step(c, coor, vel, mass, dpot, dt, doh, dhh);
+        enqueue_md_step(c, coor, vel, mass, dpot, dt, doh, dhh);
         c->capturing = 0;
         cudaError_t e1 = cudaStreamEndCapture(s, &g);
-        cudaError_t e2 = e1 == cudaSuccess ? (built ? cudaGraphInstantiate(&c->gexec_md, g, cudaGraphInstantiateFlagUseNodePriority) : cudaErrorNotSupported) : e1;
+        cudaError_t e2 = e1 == cudaSuccess ? cudaGraphInstantiate(&c->gexec_md, g, cudaGraphInstantiateFlagUseNodePriority) : e1;
         if (g) cudaGraphDestroy(g);
         if (e2 != cudaSuccess) {
             c->gexec_md = nullptr;
@@ -1744,10 +1753,9 @@ int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *
         c->gmd_gen = c->list_gen;
     }
     for (int k = 0; k < nsteps; ++k) NB_CUDA_OK(c, cudaGraphLaunch(c->gexec_md, s));
-    // the last step's status words and energies, and the step control, in one wait
-    NB_CUDA_OK(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
-    NB_CUDA_OK(c, cudaMemcpyAsync(c->h_e_rep, c->d_e_rep, sizeof(double) * NB_EREP * c->nrep,
-                                  cudaMemcpyDeviceToHost, s));
+    // the step control in one wait (the last step's status words and energies are on the host
+    // already); the rebuild request it left for a step that does not come is withdrawn
+    NB_CUDA_OK(c, cudaMemsetAsync(c->d_status, 0, sizeof(int) * 8, s));
     NB_CUDA_OK(c, cudaMemcpyAsync(c->h_status + 20, c->d_mdctl, sizeof(int) * 3, cudaMemcpyDeviceToHost, s));
     return MOIL_NB_OK;
 }

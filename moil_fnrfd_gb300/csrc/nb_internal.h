@@ -21,6 +21,11 @@ struct FftPlanDev {
     unsigned magic[8];
 };
 
+// How an evaluation decides on the list rebuild: on the device (a conditional graph node, or gated
+// kernels), or on the host -- a graph without the rebuild, whose result is dropped and the
+// evaluation redone when a site turns out to have moved too far, and one with it
+enum EvalMode { EVAL_DEVICE = 0, EVAL_KEEP = 1, EVAL_BUILD = 2 };
+
 struct RepHost {
     moil_nb_params p;
     int npt;
@@ -40,7 +45,6 @@ struct NbCtx {
     cudaStream_t stream2n = nullptr;  // blocks first (stream2), or at the pair kernels' priority (stream2n)
     cudaStream_t stream3 = nullptr;   // non-water pair and correction kernels, beside the water kernel
     cudaStream_t sbody = nullptr;     // captures the list rebuild into the conditional node's body
-    cudaStream_t sstep = nullptr;     // captures an MD step into its gate node's body
     int capturing = 0;                // the evaluation is being captured into the handle's graph
     cudaStream_t pstream = nullptr, pstream2 = nullptr, pstream3 = nullptr;   // replica groups: prioritised by group index
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
@@ -152,8 +156,8 @@ struct NbCtx {
     EChunk *d_echunks = nullptr;
     int *d_echunk_begin = nullptr;     // first chunk of each replica, then the count
     double *d_epart = nullptr;         // NB_EU slot sums per chunk
-    double *d_e_rep = nullptr;         // nrep * 16
-    double *h_e_rep = nullptr;         // pinned mirror
+    int *d_edone = nullptr;            // finished chunks per replica (zero between evaluations)
+    double *h_e_rep = nullptr;         // pinned, NB_EREP per replica, written by k_finalize
 
     // caller buffers used by host-pointer evaluations
     double *d_coor = nullptr, *d_dpot = nullptr;
@@ -185,12 +189,13 @@ struct NbCtx {
     double *d_press_out = nullptr;     // 12 per replica
 
     // device status: [0] rebuild flag, [1] error bits, [2..4] W1 / W2 / X entry totals,
-    // [5] largest half-list j-set, [6] longest W1 row, [7] longest half row; all reset at the
-    // start of every evaluation
+    // [5] largest half-list j-set, [6] longest W1 row, [7] longest half row; zero at the start of
+    // every evaluation but for a requested rebuild (k_finalize clears them)
     int *d_status = nullptr;
-    int *h_status = nullptr;           // pinned: [0..7] mirror, [8..15] initial words of an evaluation,
-                                       // [16] the rebuild flag read back in stage-timing mode,
-                                       // [17..19] / [20..22] MD step control written / read back
+    int *h_status = nullptr;           // pinned: [0..7] the last evaluation's words (k_finalize),
+                                       // [8..15] initial words of an evaluation, [16] the rebuild
+                                       // flag read back in stage-timing mode, [17..19] / [20..22] MD
+                                       // step control written / read back, [23] non-finite gradient
     int need_rebuild = 1;
     int evals_since_build = 0;
     int64_t last_list_entries = 0, last_water_pairs = 0, last_atom_pairs = 0, last_site_pairs = 0;
@@ -217,15 +222,20 @@ struct NbCtx {
     std::string tune_cache;            // autotuner cache file read by moil_nb_init_batch ("" none)
     int tuning = 0;                    // moil_nb_autotune is re-initialising the handle
     int tune_mode = 0;                 // MOIL_NB_TUNE_DEVICE / MOIL_NB_TUNE_HOST
-    cudaGraphExec_t gexec = nullptr;
-    const double *g_coor = nullptr;
-    double *g_dpot = nullptr;
-    int g_gen = -1, list_gen = 0, graph_launches = 0;
+    struct EvalGraph {
+        cudaGraphExec_t exec = nullptr;
+        const double *coor = nullptr;
+        double *dpot = nullptr;
+        int gen = -1, prio = 0, launches = 0;
+    } graphs[3];                       // by EvalMode
+    int eval_mode = 0, eval_forced = 0;   // of the evaluation last queued: EvalMode, rebuild requested
+    int wary = 0;                      // evaluations to leave to the device's decision (host_decides)
+    int list_gen = 0;
     // an asynchronous evaluation queued by moil_nb_eval_device_async and not yet waited for
     int pending = 0, pend_rc = 0;
     const double *pend_coor = nullptr;
     double *pend_dpot = nullptr;
-    int on_prio = 0, g_prio = 0;       // running on the prioritised group streams (now / when captured)
+    int on_prio = 0;                   // running on the prioritised group streams
 };
 
 // the public handle is the context itself
@@ -240,9 +250,9 @@ inline int cap_int(int64_t cap) { return cap > 0x7fffffff ? 0x7fffffff : (int)ca
 // ---- launchers implemented in the kernel files -------------------------------------
 // lists (nb_lists.cu)
 void nb_launch_build_lists(NbCtx *c, const double *d_coor);
-// one thread sets the conditional node of a captured evaluation to the device rebuild flag
-void nb_launch_rebuild_cond(NbCtx *c, cudaGraphConditionalHandle h);
-void nb_launch_prepare(NbCtx *c, const double *d_coor, int check);
+// coordinate preparation and skin check; cond: the conditional node around the rebuild (0: none);
+// ctl: the step control of an MD step (d_mdctl) or NULL
+void nb_launch_prepare(NbCtx *c, const double *d_coor, cudaGraphConditionalHandle cond, const int *ctl);
 // real space + corrections (nb_realspace.cu)
 void nb_launch_water(NbCtx *c);      // water molecules: W1 and W2 lists
 void nb_launch_atoms(NbCtx *c);      // atoms outside waters: X lists
@@ -271,12 +281,9 @@ void nb_pme_fp32_consts(RepDev *R);
 // FP64 B-spline moduli
 void nb_pme_etab(const RepDev &R, const double *bsp, float *out);
 // finalize (nb_realspace.cu)
-void nb_launch_finalize(NbCtx *c, double *d_dpot);
-// MD step loop (nb_md.cu / nb_host.cu): the step-control kernels around an evaluation, the
-// integrator of one context, and the graph replay of nsteps whole steps (no host wait)
-void nb_launch_md_begin(NbCtx *c, cudaStream_t s);
-void nb_launch_md_gate(NbCtx *c, cudaStream_t s, cudaGraphConditionalHandle h);
-void nb_launch_md_end(NbCtx *c, cudaStream_t s);
+void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl);   // ctl: as nb_launch_prepare
+// MD step loop (nb_md.cu / nb_host.cu): the integrator of one context, and the graph replay of
+// nsteps whole steps (no host wait)
 int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, const double *dpot,
                         double dt, double doh, double dhh);
 int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *dpot, double dt, double doh,

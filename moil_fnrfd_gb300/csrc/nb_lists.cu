@@ -178,17 +178,23 @@ __device__ __forceinline__ void load_atom(const double *__restrict__ coor, int a
     }
 }
 
-// PME: also each site's PME record (nb_fused_sites)
+// PME: also each site's PME record (nb_fused_sites).  cond (0: none): the conditional node around
+// the list rebuild, set when the host asked for one or a site moved.
 template <typename T, bool PME>
 __global__ void __launch_bounds__(256, 5) k_prepare(int nW, int nA, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
                           const int *__restrict__ site_orig, const unsigned *__restrict__ site_flags,
                           const void *site_q_v, const double *__restrict__ coor, void *pos_v, void *woff_v,
                           float4 *__restrict__ posb, void *fr_v, unsigned char *__restrict__ zidx, float half_skin2,
-                          float rwat2, int snapshot, int *st)
+                          float rwat2, int snapshot, int *st, cudaGraphConditionalHandle cond, const int *ctl)
 {
+    // after an error in an MD step the rest of the call's steps do no work on new positions
+    if (ctl && ctl[2] != 0) return;
     // snapshot mode runs only on a rebuild; check mode only without one (the site order it
     // reads is the previous build's, which does not exist before the first build)
-    if (snapshot ? rebuild_off(st) : !rebuild_off(st)) return;
+    if (snapshot ? rebuild_off(st) : !rebuild_off(st)) {
+        if (cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 1);
+        return;
+    }
     typedef typename vec4<T>::type T4;
     const T *site_q = (const T *)site_q_v;
     bool moved = false;
@@ -227,7 +233,10 @@ __global__ void __launch_bounds__(256, 5) k_prepare(int nW, int nA, const RepDev
                             true, moved);
         }
     }
-    if (moved) atomicOr(&st[0], 1);
+    if (moved) {
+        atomicOr(&st[0], 1);
+        if (cond) cudaGraphSetConditional(cond, 1);
+    }
 }
 
 // unique neighbour cells along one axis
@@ -948,7 +957,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
         c->d_site_q, c->d_status);
     (nb_fused_sites(c) ? k_prepare<T, true> : k_prepare<T, false>)<<<grid(c->nW + c->nA, B), B, 0, s>>>(
         (int)c->nW, (int)c->nA, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_site_flags, c->d_site_q, d_coor,
-        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, 0.f, c->rwat * c->rwat, 1, c->d_status);
+        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, 0.f, c->rwat * c->rwat, 1, c->d_status, 0, nullptr);
     c->launches += 5;
     // water lists with the row entry type of the handle (uint16 when every replica has fewer
     // than 65,536 waters)
@@ -1003,7 +1012,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
 }
 
 template <typename T>
-void prepare_t(NbCtx *c, const double *d_coor, int check)
+void prepare_t(NbCtx *c, const double *d_coor, cudaGraphConditionalHandle cond, const int *ctl)
 {
     const int B = 256;
     float hs = 0.5f * c->skin;
@@ -1011,27 +1020,12 @@ void prepare_t(NbCtx *c, const double *d_coor, int check)
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((items + B - 1) / B, (int64_t)c->nsm * 8));
     (nb_fused_sites(c) ? k_prepare<T, true> : k_prepare<T, false>)<<<g, B, 0, c->stream>>>(
         (int)c->nW, (int)c->nA, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_site_flags, c->d_site_q, d_coor,
-        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, check ? hs * hs : 3.0e38f, c->rwat * c->rwat, 0,
-        c->d_status);
+        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, hs * hs, c->rwat * c->rwat, 0, c->d_status, cond,
+        ctl);
     c->launches += 1;
 }
 
 }  // namespace
-
-namespace {
-// the rebuild decision of a captured evaluation: the IF node around the list rebuild runs its
-// body only when the coordinate preparation (or the host) set the device rebuild flag
-__global__ void k_rebuild_cond(cudaGraphConditionalHandle h, const int *st)
-{
-    cudaGraphSetConditional(h, st[0] != 0 ? 1u : 0u);
-}
-}  // namespace
-
-void nb_launch_rebuild_cond(NbCtx *c, cudaGraphConditionalHandle h)
-{
-    k_rebuild_cond<<<1, 1, 0, c->stream>>>(h, c->d_status);
-    c->launches++;
-}
 
 void nb_launch_build_lists(NbCtx *c, const double *d_coor)
 {
@@ -1039,8 +1033,8 @@ void nb_launch_build_lists(NbCtx *c, const double *d_coor)
     else build_lists_t<float>(c, d_coor);
 }
 
-void nb_launch_prepare(NbCtx *c, const double *d_coor, int check)
+void nb_launch_prepare(NbCtx *c, const double *d_coor, cudaGraphConditionalHandle cond, const int *ctl)
 {
-    if (c->precision == MOIL_NB_FP64) prepare_t<double>(c, d_coor, check);
-    else prepare_t<float>(c, d_coor, check);
+    if (c->precision == MOIL_NB_FP64) prepare_t<double>(c, d_coor, cond, ctl);
+    else prepare_t<float>(c, d_coor, cond, ctl);
 }

@@ -138,30 +138,6 @@ __global__ void __launch_bounds__(256) k_kinetic(int natom, const double *__rest
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0] / kAccel;
 }
 
-// Step control of the device-side step loop (d_mdctl = {evaluations since the last rebuild,
-// rebuild requested, sticky error bits}).  Before an evaluation: the status words the host
-// writes before a normal evaluation, with the rebuild forced when the list period is reached
-// or a rebuild was requested (the skin check of the coordinate preparation adds its own).
-__global__ void k_md_begin(int *__restrict__ st, int *__restrict__ ctl, int list_period)
-{
-    st[0] = (ctl[1] || (list_period > 0 && ctl[0] >= list_period)) ? 1 : 0;
-    for (int k = 1; k < 8; ++k) st[k] = 0;
-    ctl[1] = 0;
-}
-// the gate of a step: its body runs only while no step of the call has raised an error (after
-// one, the call is redone from its starting state by the per-step path)
-__global__ void k_md_gate(cudaGraphConditionalHandle h, const int *__restrict__ ctl)
-{
-    cudaGraphSetConditional(h, ctl[2] == 0 ? 1u : 0u);
-}
-// after it: the error bits kept across steps, the rebuild counter advanced
-__global__ void k_md_end(const int *__restrict__ st, int *__restrict__ ctl)
-{
-    if (st[0]) ctl[0] = 0;
-    ctl[0] += 1;
-    ctl[2] |= st[1];
-}
-
 // the integrator kernels of one (ungrouped) context over its caller-atom range
 int integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, const double *dpot,
               double dt, double doh, double dhh)
@@ -177,24 +153,6 @@ int integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double 
 }
 
 }  // namespace
-
-void nb_launch_md_begin(NbCtx *c, cudaStream_t s)
-{
-    k_md_begin<<<1, 1, 0, s>>>(c->d_status, c->d_mdctl, c->list_period);
-    c->launches++;
-}
-
-void nb_launch_md_gate(NbCtx *c, cudaStream_t s, cudaGraphConditionalHandle h)
-{
-    k_md_gate<<<1, 1, 0, s>>>(h, c->d_mdctl);
-    c->launches++;
-}
-
-void nb_launch_md_end(NbCtx *c, cudaStream_t s)
-{
-    k_md_end<<<1, 1, 0, s>>>(c->d_status, c->d_mdctl);
-    c->launches++;
-}
 
 int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, const double *dpot,
                         double dt, double doh, double dhh)

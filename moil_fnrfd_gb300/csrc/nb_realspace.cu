@@ -1102,15 +1102,17 @@ __global__ void k_excl14(int n, const int *__restrict__ atoms, const int *__rest
 }
 
 // ---------------------------------------------------------------------------------
-// gradient assembly in MOIL order: fixed-point real space + FP64 corrections + PME
+// End of an evaluation, one launch (k_finalize): gradient assembly in MOIL order, per-replica
+// energies, and the status words and energies written to the host's page-locked copies by the
+// blocks that have them.  Three launches and two copies took 22 us of a 216-water evaluation.
+
+// one atom's gradient: fixed-point real space + FP64 corrections + PME; false if not finite
 template <typename T>
-__global__ void k_final_grad(int natom, const int *__restrict__ site_of, const int *__restrict__ atom_rep,
-                             const RepDev *__restrict__ reps, const long long *__restrict__ grad_site,
-                             const double *__restrict__ grad_ex, const T *__restrict__ part,
-                             const double *__restrict__ q, int nsw, double *__restrict__ dpot, int *st)
+__device__ __forceinline__ bool final_grad(int a, const int *__restrict__ site_of, const int *__restrict__ atom_rep,
+                                           const RepDev *__restrict__ reps, const long long *__restrict__ grad_site,
+                                           const double *__restrict__ grad_ex, const T *__restrict__ part,
+                                           const double *__restrict__ q, int nsw, double *__restrict__ dpot)
 {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= natom) return;
     const RepDev &R = reps[atom_rep[a]];
     int s = site_of[a];
     bool bad = false;
@@ -1149,28 +1151,25 @@ __global__ void k_final_grad(int natom, const int *__restrict__ site_of, const i
             dpot[3 * (size_t)a + d] = v;
         }
     }
-    if (bad) atomicOr(&st[1], NB_DEV_ERR_NAN);
+    return !bad;
 }
 
 // Per-replica energies in two passes with a fixed partition, so large replicas spread over
 // many blocks and the sums stay in a fixed order (deterministic):
-//  k_energy_part: one block per chunk (EChunk: up to NB_FE_SEG consecutive units, atoms or PME
+//  energy_chunk: one block per chunk (EChunk: up to NB_FE_SEG consecutive units, atoms or PME
 //    column items of one replica); every thread streams the chunk's flat array with a stride
 //    that keeps its slot fixed (coalesced reads), the slots are summed by a halving tree;
-//  k_energy_final: one warp per replica adds its chunks' slot sums (a lane per slot and
-//    chunk modulo four, then a fixed tree) and forms MOIL's energy names (pot/eforce.f:122-204);
-//    one thread per replica took 23 us over the 34 chunks of the solute system.
+//  energy_replica: the warp of the replica's last finished block adds its chunks' slot sums (a
+//    lane per slot and chunk modulo four, then a fixed tree) and forms MOIL's energy names
+//    (pot/eforce.f:122-204).
 #define NB_FE_THREADS 256
 static_assert(NB_FE_THREADS % NB_EU == 0 && NB_FE_THREADS % NB_EX == 0, "slot-preserving stride");
-__global__ void __launch_bounds__(NB_FE_THREADS) k_energy_part(const EChunk *__restrict__ chunks,
-                                                               const double *__restrict__ e_unit,
-                                                               const double *__restrict__ e_ex,
-                                                               const double *__restrict__ e_col,
-                                                               double *__restrict__ part)
+__device__ __forceinline__ void energy_chunk(int chunk, EChunk ch, const double *__restrict__ e_unit,
+                                             const double *__restrict__ e_ex, const double *__restrict__ e_col,
+                                             double *__restrict__ part)
 {
     __shared__ double sh[NB_FE_THREADS];
     const int t = threadIdx.x;
-    const EChunk ch = chunks[blockIdx.x];
     const int width = ch.kind <= 1 ? NB_EU : (ch.kind == 2 ? NB_EX : 1);
     const double *b = ch.kind <= 1 ? e_unit + (size_t)NB_EU * ch.begin
                                    : (ch.kind == 2 ? e_ex + (size_t)NB_EX * ch.begin : e_col + ch.begin);
@@ -1200,23 +1199,21 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_energy_part(const EChunk *__r
         double w = 0.0;
         if (t < width)
             for (int q = t; q < live; q += width) w += sh[q];
-        part[(size_t)NB_EU * blockIdx.x + t] = w;
+        part[(size_t)NB_EU * chunk + t] = w;
     }
 }
 
-__global__ void __launch_bounds__(128) k_energy_final(int nrep, const RepDev *__restrict__ reps,
-                                                      const EChunk *__restrict__ chunks,
-                                                      const int *__restrict__ chunk_begin,
-                                                      const double *__restrict__ part, double *__restrict__ e_rep)
+
+__device__ __forceinline__ void energy_replica(int r, int lane, const RepDev *__restrict__ reps,
+                                               const EChunk *__restrict__ chunks, const int *__restrict__ chunk_begin,
+                                               const double *part, double *__restrict__ e_rep)
 {
-    const int lane = threadIdx.x & 31, r = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (r >= nrep) return;
     const RepDev &R = reps[r];
     const int slot = lane % NB_EU;
     double a[4] = {0.0, 0.0, 0.0, 0.0};    // by chunk kind: this lane's slot over every fourth chunk
     const int c1 = chunk_begin[r + 1];
     for (int c = chunk_begin[r] + lane / NB_EU; c < c1; c += 32 / NB_EU) {
-        const double v = part[(size_t)NB_EU * c + slot];
+        const double v = __ldcg(part + (size_t)NB_EU * c + slot);
         const int kind = chunks[c].kind;
 #pragma unroll
         for (int q = 0; q < 4; ++q) a[q] += kind == q ? v : 0.0;
@@ -1261,6 +1258,59 @@ WaterHFn water_h_fn(int hb, bool vir)
     case 128: return vir ? k_water_h<128, true> : k_water_h<128, false>;
     case 512: return vir ? k_water_h<512, true> : k_water_h<512, false>;
     default: return vir ? k_water_h<256, true> : k_water_h<256, false>;
+    }
+}
+
+// Blocks [0, nchunk): energy chunks; the others: gradients of 256 atoms each.  st: status words
+// (the kernels before this one are done with them), copied to the host's st_h and cleared
+// for the next evaluation; a non-finite gradient sets *nan_h.  done: finished chunks per replica
+// (zero between launches).  ctl: in an MD step, {evaluations since the last rebuild, -, sticky
+// error bits}: the step's outcome goes there, and st[0] becomes the next step's rebuild request.
+template <typename T>
+__global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
+    int nchunk, const EChunk *__restrict__ chunks, const int *__restrict__ chunk_begin,
+    const double *__restrict__ e_unit, const double *__restrict__ e_ex, const double *__restrict__ e_col,
+    double *__restrict__ epart, int *__restrict__ done, double *__restrict__ e_rep_h, int natom,
+    const int *__restrict__ site_of, const int *__restrict__ atom_rep, const RepDev *__restrict__ reps,
+    const long long *__restrict__ grad_site, const double *__restrict__ grad_ex, const T *__restrict__ part,
+    const double *__restrict__ q, int nsw, double *__restrict__ dpot, int *__restrict__ st, int *__restrict__ st_h,
+    int *__restrict__ nan_h, int *__restrict__ ctl, int list_period)
+{
+    const int t = threadIdx.x, b = blockIdx.x;
+    if (b >= nchunk) {
+        const int a = (b - nchunk) * NB_FE_THREADS + t;
+        if (a < natom && !final_grad<T>(a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, dpot)) {
+            *nan_h = 1;
+            if (ctl) atomicOr(&ctl[2], NB_DEV_ERR_NAN);
+        }
+        return;
+    }
+    const EChunk ch = chunks[b];
+    energy_chunk(b, ch, e_unit, e_ex, e_col, epart);
+    if (t < 32) {
+        // the chunk's sums are visible before it counts as finished
+        __threadfence();
+        __syncwarp();
+        int last = 0;
+        if (t == 0) last = atomicAdd(&done[ch.rep], 1) == chunk_begin[ch.rep + 1] - chunk_begin[ch.rep] - 1;
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (last) {
+            __threadfence();
+            energy_replica(ch.rep, t, reps, chunks, chunk_begin, epart, e_rep_h);
+            if (t == 0) done[ch.rep] = 0;
+        }
+    }
+    if (b == 0 && t == 0) {
+        int s[8];
+        for (int k = 0; k < 8; ++k) s[k] = st[k];
+        for (int k = 0; k < 8; ++k) { st_h[k] = s[k]; st[k] = 0; }
+        if (ctl) {
+            if (s[0]) ctl[0] = 0;
+            ctl[0] += 1;
+            if (s[1]) atomicOr(&ctl[2], s[1]);
+            // (no rebuild after an error)
+            st[0] = list_period > 0 && ctl[0] >= list_period && (s[1] | ctl[2]) == 0 ? 1 : 0;
+        }
     }
 }
 
@@ -1430,20 +1480,16 @@ void nb_launch_excl14(NbCtx *c, const double *d_coor)
     }
 }
 
-void nb_launch_finalize(NbCtx *c, double *d_dpot)
+void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl)
 {
-    cudaStream_t s = c->stream;
-    if (c->precision == MOIL_NB_FP64)
-        k_final_grad<double><<<(int)((c->natom + 255) / 256), 256, 0, s>>>(
-            (int)c->natom, c->d_site_of, c->d_atom_rep, c->d_reps, c->d_grad_site, c->d_grad_ex,
-            (const double *)c->d_part, c->d_q, 0, d_dpot, c->d_status);
-    else
-        k_final_grad<float><<<(int)((c->natom + 255) / 256), 256, 0, s>>>(
-            (int)c->natom, c->d_site_of, c->d_atom_rep, c->d_reps, c->d_grad_site, c->d_grad_ex,
-            (const float *)c->d_part, c->d_q, c->water_excl_fast ? (int)(3 * c->nW) : 0, d_dpot, c->d_status);
-    k_energy_part<<<(int)c->echunks.size(), NB_FE_THREADS, 0, s>>>(c->d_echunks, c->d_e_unit, c->d_e_ex, c->d_e_col,
-                                                                    c->d_epart);
-    k_energy_final<<<(c->nrep + 3) / 4, 128, 0, s>>>(c->nrep, c->d_reps, c->d_echunks, c->d_echunk_begin,
-                                                         c->d_epart, c->d_e_rep);
-    c->launches += 3;
+    const int nchunk = (int)c->echunks.size(), nb = nchunk + (int)((c->natom + NB_FE_THREADS - 1) / NB_FE_THREADS);
+    auto launch = [&](auto kernel, auto part, int nsw) {
+        kernel<<<nb, NB_FE_THREADS, 0, c->stream>>>(
+            nchunk, c->d_echunks, c->d_echunk_begin, c->d_e_unit, c->d_e_ex, c->d_e_col, c->d_epart, c->d_edone,
+            c->h_e_rep, (int)c->natom, c->d_site_of, c->d_atom_rep, c->d_reps, c->d_grad_site, c->d_grad_ex, part,
+            c->d_q, nsw, d_dpot, c->d_status, c->h_status, c->h_status + 23, ctl, c->list_period);
+    };
+    if (c->precision == MOIL_NB_FP64) launch(k_finalize<double>, (const double *)c->d_part, 0);
+    else launch(k_finalize<float>, (const float *)c->d_part, c->water_excl_fast ? (int)(3 * c->nW) : 0);
+    c->launches++;
 }
