@@ -249,7 +249,9 @@ int setup_half(NbCtx *c)
     NB_CUDA_OK(c, cudaMemset(c->d_hcnt, 0, sizeof(int2) * c->nW));
     NB_CUDA_OK(c, cudaMemset(c->d_jn, 0, sizeof(int) * c->hblocks.size()));
     c->caph = ((c->cap_row1 * 5 / 8 + 32) + 31) & ~31;
-    c->jcap = std::min(maxw, 7 * c->hb);
+    // A block of 256 waters at liquid density has 1,000-2,500 partners: with 7 hb every large handle's
+    // first evaluation overflowed and ran twice (16 replicas x 500 steps: 5050 us, 2830 with 10 hb).
+    c->jcap = std::min(maxw, (c->hb <= 256 ? 10 : 7) * c->hb);
     c->need_rebuild = 1;
     return alloc_half(c);
 }

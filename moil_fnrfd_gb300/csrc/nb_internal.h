@@ -114,6 +114,7 @@ struct NbCtx {
     int *d_jset = nullptr;        // per block: jcap sorted water indices (the block's partners)
     int *d_jn = nullptr;          // per block: j-set size
     int caph = 0, jcap = 0;
+    int jsh = 0;                  // partners of a block with accumulators in shared memory
 
     // exclusion / 1-4 lists per caller atom (both directions)
     int *d_ex_off = nullptr, *d_ex_j = nullptr;

@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
                                                           const void *lj_v, const unsigned *__restrict__ sflags,
                                                           const unsigned *__restrict__ hrow, int caph,
                                                           const int2 *__restrict__ hcnt, const int *__restrict__ jset,
-                                                          const int *__restrict__ jn, int jcap,
+                                                          const int *__restrict__ jn, int jcap, int jsh,
                                                           const int *__restrict__ wl2_off, const int *__restrict__ wl2,
                                                           int cap2, long long *__restrict__ grad,
                                                           double *__restrict__ e_unit, int intra)
@@ -687,14 +687,14 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
     constexpr float SC = (float)(1 << S), CAP = 4.19e6f / SC;   // (2^22 = 4,194,304)
     constexpr int NE = VIR ? 6 : 4;
     __shared__ float2 sE[NE][HB];
-    extern __shared__ int sJ[];      // [9][jcap]: partner-site gradients, 2^S units
+    extern __shared__ int sJ[];      // [9][jsh]: partner-site gradients, 2^S units
     const int t = threadIdx.x, b = blockIdx.x;
     const int2 w = blocks[b];
     const RepDev &R = reps[w.x];
-    const int nJ = jn[b];
+    const int nJ = min(jn[b], jsh);
     for (int k = t; k < nJ; k += HB)
 #pragma unroll
-        for (int c = 0; c < 9; ++c) sJ[c * jcap + k] = 0;
+        for (int c = 0; c < 9; ++c) sJ[c * jsh + k] = 0;
 #pragma unroll
     for (int k = 0; k < NE; ++k) sE[k][t] = make_float2(0.f, 0.f);
     __syncthreads();
@@ -805,12 +805,12 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
                 float hm = 0.f;
 #pragma unroll
                 for (int c = 0; c < 9; ++c) hm = fmaxf(hm, fabsf(H[c]));
-                if (hm < CAP) {
+                if (hm < CAP && l < jsh) {
 #pragma unroll
                     for (int c = 0; c < 9; ++c)
-                        atomicAdd(&sJ[c * jcap + l], __float_as_int(fmaf(H[c], SC, 12582912.f)) - 0x4b400000);
+                        atomicAdd(&sJ[c * jsh + l], __float_as_int(fmaf(H[c], SC, 12582912.f)) - 0x4b400000);
                 } else {
-                    // a large share (rare): straight to the int64 gradient
+                    // a large share (rare), or a partner past the shared memory: to the int64 gradient
                     unsigned long long *gj = (unsigned long long *)(grad + 9 * (size_t)(wat0 + (int)(en & 0xffffu)));
 #pragma unroll
                     for (int c = 0; c < 9; ++c) atomicAdd(gj + c, (unsigned long long)nb_fix(H[c]));
@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
         for (int q = 0; q < 9; ++q) {
             const int f = 32 * q + lane, l = f / 9, c = f - 9 * l;
             const int j = __shfl_sync(0xffffffffu, jl, l);
-            const int v = j >= 0 ? sJ[c * jcap + l0 + l] : 0;
+            const int v = j >= 0 ? sJ[c * jsh + l0 + l] : 0;
             if (v != 0) atomicAdd((unsigned long long *)&grad[9 * (size_t)j + c], (unsigned long long)((long long)v * (1LL << (32 - S))));
         }
     }
@@ -1346,9 +1346,9 @@ void water_t(NbCtx *c)
     cudaStream_t s = c->stream;
     if (c->timing) cudaEventRecord(c->ev[2], s);
     if (sizeof(T) == 4 && c->nW > 0 && c->whalf) {
-        water_h_fn(c->hb, c->virial)<<<(int)c->hblocks.size(), c->hb, (size_t)36 * c->jcap, s>>>(
+        water_h_fn(c->hb, c->virial)<<<(int)c->hblocks.size(), c->hb, (size_t)36 * c->jsh, s>>>(
             c->d_hblocks, c->d_reps, (const float4 *)c->d_pos, (const float4 *)c->d_woff, c->d_site_lj,
-            c->d_site_flags, c->d_hrow, c->caph, c->d_hcnt, c->d_jset, c->d_jn, c->jcap, c->d_wl2_off, c->d_wl2,
+            c->d_site_flags, c->d_hrow, c->caph, c->d_hcnt, c->d_jset, c->d_jn, c->jcap, c->jsh, c->d_wl2_off, c->d_wl2,
             cap_int(c->cap_wl2), c->d_grad_site, c->d_e_unit, c->water_excl_fast);
         c->launches++;
     } else if (c->nW > 0) {
@@ -1444,11 +1444,16 @@ int nb_half_configure(NbCtx *c)
     int optin = 0;
     NB_CUDA_OK(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     const void *fns[2] = {(const void *)water_h_fn(c->hb, false), (const void *)water_h_fn(c->hb, true)};
-    const size_t dyn = (size_t)36 * c->jcap;
+    // Accumulators in shared memory: 9.5 per water of the block.  The blocks of an SM then take 175 KB; the
+    // next carveout leaves too little L1 for the partner records (256 waters a block, 512 replicas,
+    // evaluation in us: 2,430 partners 2179, 2,560 2453, 1,560 2196), and the few partners beyond go
+    // straight to the gradient (32,000 waters: 2,230 and 2,430 167, 1,780 212).
+    c->jsh = nb_half_two_blocks(c) ? std::min(c->jcap, 19 * c->hb / 2) : c->jcap;
+    const size_t dyn = (size_t)36 * c->jsh;
     for (const void *fn : fns) {
         cudaFuncAttributes fa;
         NB_CUDA_OK(c, cudaFuncGetAttributes(&fa, fn));
-        if (c->jcap > 65535 || dyn + fa.sharedSizeBytes > (size_t)optin) return MOIL_NB_ERR_OVERFLOW;
+        if (c->jcap > 65535 || (size_t)36 * c->jcap + fa.sharedSizeBytes > (size_t)optin) return MOIL_NB_ERR_OVERFLOW;
         // the limit belongs to the kernel, not to the handle: other handles (replica groups)
         // may launch it with larger j-sets, so it only ever grows
         if ((int)dyn > fa.maxDynamicSharedSizeBytes)

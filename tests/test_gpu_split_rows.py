@@ -8,7 +8,7 @@ import pytest
 
 from conftest import ENERGY_TERMS, energy_scale, rel_rms
 from moil_fnrfd_gb300 import systems as S
-from moil_fnrfd_gb300.nb import MOIL_NB_FP64, MOIL_NB_MIXED, WATER_FULL, Nonbonded
+from moil_fnrfd_gb300.nb import MOIL_NB_FP64, MOIL_NB_MIXED, WATER_FULL, WATER_HALF, Nonbonded
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -70,4 +70,18 @@ def test_long_rows_on_full_lists(filler):
     for k, s in ((0, dense), (filler, box)):
         ref, eref = O.eforce(s, mode="parity")
         close_to_oracle(dps[k], es[k], ref, eref, MOIL_NB_MIXED)
+    nb.close()
+
+
+@pytest.mark.parametrize("n", [1215, 1217, 1275])
+def test_more_partners_than_shared_accumulators(n):
+    """Half lists keep 9.5 partner accumulators per water of a block in shared memory: with blocks
+    of 128 waters 1,216, and the shares of the partners beyond go straight to the gradient."""
+    s = dense_cluster(n, 11, 0.55)
+    ref, eref = O.eforce(s, mode="parity")
+    nb = Nonbonded(s, shape=dict(water_kernel=WATER_HALF, half_block=128))
+    for _ in range(2):
+        dpot, e = nb.eforce(s.coor)
+        close_to_oracle(dpot, e, ref, eref, MOIL_NB_MIXED)
+    assert nb.shape()["water_kernel"] == WATER_HALF
     nb.close()
