@@ -108,7 +108,7 @@ void release_device(NbCtx *c)
     free_ptr(c->d_adj); free_ptr(c->d_adj_phi); free_ptr(c->d_md_dpot); free_ptr(c->d_mdctl);
     free_ptr(c->d_md_save);
     free_ptr(c->d_mol_off); free_ptr(c->d_mol_atom); free_ptr(c->d_mass); free_ptr(c->d_xrel);
-    free_ptr(c->d_xsite); free_ptr(c->d_press_unit); free_ptr(c->d_press_site); free_ptr(c->d_press_col); free_ptr(c->d_press_grid);
+    free_ptr(c->d_xsite); free_ptr(c->d_press_unit); free_ptr(c->d_press_part); free_ptr(c->d_press_col); free_ptr(c->d_press_grid);
     free_ptr(c->d_press_out);
     c->nmol = 0;
     if (c->h_e_rep) cudaFreeHost(c->h_e_rep);
@@ -1413,7 +1413,8 @@ int moil_nb_pressure(moil_nb_ctx *h, const double *coor, double *dpot, moil_ener
     if (rc != MOIL_NB_OK) return rc;
     if (!h->d_press_out) {
         NB_CUDA_OK(h, cudaMalloc(&h->d_press_unit, sizeof(double) * 6 * std::max<int64_t>(h->nW + h->nA, 1)));
-        NB_CUDA_OK(h, cudaMalloc(&h->d_press_site, sizeof(double) * 3 * std::max<int64_t>(h->nsite, 1)));
+        h->press_split = nb_press_split(h);
+        NB_CUDA_OK(h, cudaMalloc(&h->d_press_part, sizeof(double) * 12 * h->nrep * h->press_split));
         const size_t fp = h->precision == MOIL_NB_FP64 ? sizeof(double) : sizeof(float);
         NB_CUDA_OK(h, cudaMalloc(&h->d_xsite, 4 * fp * std::max<int64_t>(h->nsite, 1)));
         NB_CUDA_OK(h, cudaMalloc(&h->d_press_col, sizeof(double) * 3 * std::max<size_t>(h->cols.size(), 1)));
@@ -1422,10 +1423,13 @@ int moil_nb_pressure(moil_nb_ctx *h, const double *coor, double *dpot, moil_ener
     }
     rc = nb_pressure(h, h->d_coor, h->d_press_out);
     if (rc != MOIL_NB_OK) return rc;
+    // the gradient is complete (the evaluation has ended): its copy runs beside the kernels above
+    if (dpot) {
+        NB_CUDA_OK(h, cudaMemcpyAsync(dpot, h->d_dpot, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream3));
+        NB_CUDA_OK(h, cudaStreamSynchronize(h->stream3));
+    }
     NB_CUDA_OK(h, cudaMemcpyAsync(press, h->d_press_out, sizeof(double) * 12 * h->nrep, cudaMemcpyDeviceToHost,
                                   h->stream));
-    if (dpot)
-        NB_CUDA_OK(h, cudaMemcpyAsync(dpot, h->d_dpot, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream));
     NB_CUDA_OK(h, cudaStreamSynchronize(h->stream));
     return MOIL_NB_OK;
 }

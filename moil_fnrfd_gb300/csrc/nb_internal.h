@@ -181,10 +181,11 @@ struct NbCtx {
     int nmol = 0;
     int *d_mol_off = nullptr, *d_mol_atom = nullptr;   // molecules as CSR over caller atoms
     double *d_mass = nullptr;          // per caller atom
-    double *d_xrel = nullptr;          // position relative to the molecule's centre of mass, 3 per atom
-    void *d_xsite = nullptr;           // the same in site order, float4 / double4 (pair kernels)
+    double *d_xrel = nullptr;          // scratch: atoms placed beside their molecule's first, 3 per atom
+    void *d_xsite = nullptr;           // positions relative to the centre of mass, site order, float4 / double4
     double *d_press_unit = nullptr;    // 6 per unit: LJ and real-space Coulomb terms
-    double *d_press_site = nullptr;    // 3 per site: PME force x xrel
+    double *d_press_part = nullptr;    // 12 per replica and block of the reduction
+    int press_split = 1;               // (press_split blocks at most)
     double *d_press_col = nullptr;     // 3 per PME column work item: reciprocal virial
     void *d_press_grid = nullptr;      // second half-complex grid for the reciprocal virial (float2 / double2)
     double *d_press_out = nullptr;     // 12 per replica
@@ -295,6 +296,7 @@ void read_energies_of(NbCtx *c, moil_energies *e);
 int nb_adjoint(NbCtx *c, double *d_dq, double *d_de, double *d_ds);
 // pressure analysis terms after an evaluation of d_coor (nb_press.cu): 12 per replica
 int nb_pressure(NbCtx *c, const double *d_coor, double *d_out);
+int nb_press_split(const NbCtx *c);     // most blocks a replica's reduction takes
 
 #define NB_CUDA_OK(c, call)                                                         \
     do {                                                                            \

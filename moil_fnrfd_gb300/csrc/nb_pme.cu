@@ -1330,9 +1330,8 @@ void nb_launch_pme(NbCtx *c)
 // pressure analysis: the charge planes of the evaluation's sites spread and transformed
 // again into grid (a copy beside the handle's own grid, whose potential planes stay valid),
 // and the reciprocal virial per column work item into v_col (mixed path)
-void nb_launch_pme_virial(NbCtx *c, void *grid, double *v_col)
+void nb_launch_pme_virial(NbCtx *c, cudaStream_t s, void *grid, double *v_col)
 {
-    cudaStream_t s = c->stream;
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
     if (c->precision == MOIL_NB_FP64) {
         k_plane_fwd<double><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,

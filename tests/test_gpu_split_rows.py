@@ -85,3 +85,18 @@ def test_more_partners_than_shared_accumulators(n):
         close_to_oracle(dpot, e, ref, eref, MOIL_NB_MIXED)
     assert nb.shape()["water_kernel"] == WATER_HALF
     nb.close()
+
+
+@pytest.mark.parametrize("precision", [MOIL_NB_FP64, MOIL_NB_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("name", ["lone_water", "197_waters", "dense_rows", "solute"])
+def test_pressure_rows_match_oracle(name, precision):
+    """Pressure terms where a water's owned pairs end inside eight lanes and where they fill its
+    buffer of 64 more than once: 1e-5 (mixed) and 1e-9 (FP64) of the tensor's magnitude sum."""
+    s = SYSTEMS[name]()
+    mol, mass = S.molecules(s)
+    want = O.pressure(s, mol, mass, mode="mi")[2]
+    nb = Nonbonded(s, precision=precision)
+    nb.set_molecules(mol, mass)
+    press = nb.pressure(s.coor)[2]
+    nb.close()
+    assert np.abs(press - want).max() <= (1e-9 if precision == MOIL_NB_FP64 else 1e-5) * np.abs(want).sum()
