@@ -33,65 +33,45 @@ __device__ __forceinline__ void lj_switch_apply(const RepDev &R, T r2, T &e1, T 
     }
 }
 
-template <typename T> struct Consts;
-template <> struct Consts<float> {
-    __device__ static float qq(const RepDev &R, int k) { return R.qq[k]; }
-    __device__ static float w12(const RepDev &R) { return R.w12; }
-    __device__ static float w6(const RepDev &R) { return R.w6; }
-    __device__ static float alpha(const RepDev &R) { return R.alpha; }
-    __device__ static float epstmp(const RepDev &R) { return (float)R.epstmp; }
-};
-template <> struct Consts<double> {
-    __device__ static double qq(const RepDev &R, int k) { return R.qqd[k]; }
-    __device__ static double w12(const RepDev &R) { return R.w12d; }
-    __device__ static double w6(const RepDev &R) { return R.w6d; }
-    __device__ static double alpha(const RepDev &R) { return R.alphad; }
-    __device__ static double epstmp(const RepDev &R) { return R.epstmp; }
-};
-
-// one non-water-type pair (cdie_ewald list1/2/3 semantics); d already minimum-imaged
+// FP64 path: one non-water-type pair (cdie_ewald list1/2/3 semantics); d already minimum-imaged
 // vir receives MOIL's LJ virial term of the pair, -df1 r^2 (cdie_ewald_press.f:413-419)
-template <typename T>
-__device__ __forceinline__ T atom_pair(const RepDev &R, T r2, T qi, T qj, T e12i, T e6i, T e12j, T e6j,
-                                       unsigned fi, unsigned fj, T &eel, T &elj, T &vir, int &npair)
+__device__ __forceinline__ double atom_pair(const RepDev &R, double r2, double qi, double qj, double e12i, double e6i,
+                                            double e12j, double e6j, unsigned fi, unsigned fj, double &eel, double &elj,
+                                            double &vir, int &npair)
 {
-    bool hr = !R.arith && R.hvdw0 && ((fi | fj) & SF_HTINY) && r2 < (T)R.re2;
-    bool lj = r2 < (T)R.rv2 && !hr;
-    T qq = qi * qj;
-    bool el = r2 < (T)R.rmax2 && qq != (T)0;
-    if (!lj && !el) return (T)0;
+    bool hr = !R.arith && R.hvdw0 && ((fi | fj) & SF_HTINY) && r2 < (double)R.re2;
+    bool lj = r2 < (double)R.rv2 && !hr;
+    double qq = qi * qj;
+    bool el = r2 < (double)R.rmax2 && qq != 0.0;
+    if (!lj && !el) return 0.0;
     ++npair;
-    T rinv = nb_rsqrt(r2);
-    T s2 = rinv * rinv;
-    T df = 0;
+    double rinv = nb_rsqrt(r2);
+    double s2 = rinv * rinv;
+    double df = 0;
     if (el) {
-        T x = Consts<T>::alpha(R) * r2 * rinv;
-        T ex;
-        T erfcv = nb_erfc_ex(x, r2 * (T)R.ex2c, &ex);
-        qq *= Consts<T>::epstmp(R);
-        T e = qq * erfcv * rinv;
-        df = -(e + qq * (T)R.c2a * ex) * s2;
+        double x = R.alphad * r2 * rinv;
+        double ex;
+        double erfcv = nb_erfc_ex(x, r2 * (double)R.ex2c, &ex);
+        qq *= R.epstmp;
+        double e = qq * erfcv * rinv;
+        df = -(e + qq * (double)R.c2a * ex) * s2;
         eel += e;
     }
     if (lj) {
-        // r^-6 and r^-12 amplify the approximate FP32 rsqrt's error 6 and 12 times: one
-        // Newton step (FP32) first
-        const T rl = sizeof(T) == 4 ? fma((T)-0.5 * rinv, fma(r2, s2, (T)-1), rinv) : rinv;
-        s2 = rl * rl;
-        T s6 = s2 * s2 * s2, A, B;
+        double s6 = s2 * s2 * s2, A, B;
         if (!R.arith) {
             A = e12i * e12j * s6 * s6;
             B = e6i * e6j * s6;
         } else {
-            T aa = e12i * e12j, sg = (T)0.5 * (e6i + e6j);
-            T b1 = sg * sg * sg;
+            double aa = e12i * e12j, sg = 0.5 * (e6i + e6j);
+            double b1 = sg * sg * sg;
             b1 = b1 * b1;
             B = aa * b1 * s6;
             A = aa * b1 * b1 * s6 * s6;
         }
-        T e1 = A - B;
-        T df1 = (T)-6 * s2 * (A + e1);
-        lj_switch_apply<T>(R, r2, e1, df1);
+        double e1 = A - B;
+        double df1 = -6.0 * s2 * (A + e1);
+        lj_switch_apply<double>(R, r2, e1, df1);
         elj += e1;
         vir -= df1 * r2;
         df += df1;
@@ -99,14 +79,13 @@ __device__ __forceinline__ T atom_pair(const RepDev &R, T r2, T qi, T qj, T e12i
     return df;
 }
 
-template <typename T>
-__device__ __forceinline__ void min_image(const RepDev &R, T &dx, T &dy, T &dz, bool &img)
+__device__ __forceinline__ void min_image(const RepDev &R, double &dx, double &dy, double &dz, bool &img)
 {
-    T nx = nb_rint(dx * rep_invL<T>(R, 0)), ny = nb_rint(dy * rep_invL<T>(R, 1)), nz = nb_rint(dz * rep_invL<T>(R, 2));
+    const double nx = nb_rint(dx * R.invLd[0]), ny = nb_rint(dy * R.invLd[1]), nz = nb_rint(dz * R.invLd[2]);
     dx = nb_shift(R, 0, dx, nx);
     dy = nb_shift(R, 1, dy, ny);
     dz = nb_shift(R, 2, dz, nz);
-    img = (nx != (T)0) | (ny != (T)0) | (nz != (T)0);
+    img = (nx != 0.0) | (ny != 0.0) | (nz != 0.0);
 }
 
 __device__ __forceinline__ void flush(float g[], long long G[], int n)
@@ -127,42 +106,192 @@ __device__ __forceinline__ void flush(double g[], long long G[], int n)
 // water sites of molecule i against its W2 list of non-water atoms (entries first, first +
 // stride, ...): atom semantics per site pair; partial gradients and energies go to g / e4, which
 // already hold cnt entries, flushed every CHUNK entries and left to the caller after the last
-template <typename T, typename Flush>
-__device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const typename vec4<T>::type *pos,
+template <typename Flush>
+__device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const double4 *pos,
                                                const void *lj_v, const unsigned *__restrict__ sflags,
                                                const int *__restrict__ wl2_off, const int *__restrict__ wl2, int cap2,
-                                               int first, int stride, int cnt, T g[9], T e4[4], int &npair, Flush &flush_all)
+                                               int first, int stride, int cnt, double g[9], double e4[4], int &npair,
+                                               Flush &flush_all)
 {
-    typedef typename vec4<T>::type T4;
-    typedef typename cplx<T>::type T2;
     // an overflowed list (offsets past the capacity) is read within the buffer; the
     // evaluation reports the overflow and is redone with a larger one
     const int q0 = min(wl2_off[i], cap2), q1 = min(wl2_off[i + 1], cap2);
     if (q0 >= q1) return;
-    const T2 *lj = (const T2 *)lj_v;
-    const T4 si[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-    const T2 lji[3] = {lj[3 * i], lj[3 * i + 1], lj[3 * i + 2]};
+    const double2 *lj = (const double2 *)lj_v;
+    const double4 si[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+    const double2 lji[3] = {lj[3 * i], lj[3 * i + 1], lj[3 * i + 2]};
     const unsigned fi[3] = {sflags[3 * i], sflags[3 * i + 1], sflags[3 * i + 2]};
     for (int k = q0 + first; k < q1; k += stride) {
         nb_prefetch_l1(wl2 + min(k + 32, q1 - 1));
         int s = wl2[k];
-        T4 xj = pos[s];
-        T2 ljj = lj[s];
+        double4 xj = pos[s];
+        double2 ljj = lj[s];
         unsigned fj = sflags[s];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            T dx = si[a].x - xj.x, dy = si[a].y - xj.y, dz = si[a].z - xj.z;
+            double dx = si[a].x - xj.x, dy = si[a].y - xj.y, dz = si[a].z - xj.z;
             bool img;
-            min_image<T>(R, dx, dy, dz, img);
-            T r2 = dx * dx + dy * dy + dz * dz;
-            T eel = 0, elj = 0, vir = 0;   // the virial of these pairs is counted by k_atom
-            T df = atom_pair<T>(R, r2, si[a].w, xj.w, lji[a].x, lji[a].y, ljj.x, ljj.y, fi[a], fj, eel, elj, vir,
+            min_image(R, dx, dy, dz, img);
+            double r2 = dx * dx + dy * dy + dz * dz;
+            double eel = 0, elj = 0, vir = 0;   // the virial of these pairs is counted by k_atom
+            double df = atom_pair(R, r2, si[a].w, xj.w, lji[a].x, lji[a].y, ljj.x, ljj.y, fi[a], fj, eel, elj, vir,
                                 npair);
             g[3 * a] += df * dx;
             g[3 * a + 1] += df * dy;
             g[3 * a + 2] += df * dz;
             e4[img ? 1 : 0] += elj;
             e4[img ? 3 : 2] += eel;
+        }
+        if (++cnt == CHUNK) { flush_all(); cnt = 0; }
+    }
+}
+
+// FP32 pairs of non-water semantics (atom_pair): a replica's constants held in registers, since a
+// pair's arithmetic is no longer than loading them again each time.
+struct AtomK {
+    float iL0, iL1, iL2, L0, L1, L2, m0, m1, m2, rmax2, rv2, re2, ke;
+    WaterK K;
+    bool arith, tiny, sw;        // tiny: the hvdw0 rule applies (geometric rule, small-sigma hydrogens)
+    __device__ void rules(const RepDev &R)
+    {
+        re2 = R.re2; ke = held((float)R.epstmp);
+        arith = R.arith != 0; tiny = !R.arith && R.hvdw0; sw = R.lj_switch != 0;
+    }
+    __device__ AtomK(const RepDev &R)
+        : iL0(held(R.invL[0])), iL1(held(R.invL[1])), iL2(held(R.invL[2])), L0(held(R.L[0])), L1(held(R.L[1])),
+          L2(held(R.L[2])), m0(held(R.Llo[0])), m1(held(R.Llo[1])), m2(held(R.Llo[2])), rmax2(held(R.rmax2)),
+          rv2(held(R.rv2)), K{held(ERFCX_P * R.alpha), held(R.ex2c), held(R.c2a)}
+    {
+        rules(R);
+    }
+    // values that the caller holds already
+    __device__ AtomK(const RepDev &R, float a0, float a1, float a2, float b0, float b1, float b2, float c0, float c1,
+                     float c2, float rm, float rv, WaterK k)
+        : iL0(a0), iL1(a1), iL2(a2), L0(b0), L1(b1), L2(b2), m0(c0), m1(c1), m2(c2), rmax2(rm), rv2(rv), K(k)
+    {
+        rules(R);
+    }
+    // (x + 1.5*2^23) - 1.5*2^23 rounds x to nearest (|x| < 2^22)
+    __device__ void image(float &dx, float &dy, float &dz, bool &img) const
+    {
+        const float nx = fmaf(dx, iL0, 12582912.f) - 12582912.f, ny = fmaf(dy, iL1, 12582912.f) - 12582912.f,
+                    nz = fmaf(dz, iL2, 12582912.f) - 12582912.f;
+        dx = fmaf(-nx, m0, fmaf(-nx, L0, dx)); dy = fmaf(-ny, m1, fmaf(-ny, L1, dy)); dz = fmaf(-nz, m2, fmaf(-nz, L2, dz));
+        img = (nx != 0.f) | (ny != 0.f) | (nz != 0.f);
+    }
+    // LJ of a pair inside the LJ cutoff: its energy, and minus (dE/dr)/r as the result.  r^-6 and r^-12
+    // amplify the approximate rsqrt's error 6 and 12 times: one Newton step first
+    __device__ float lj(const RepDev &R, float r2, float rinv, float2 a, float2 b, float &e1) const
+    {
+        const float ri = fmaf(-0.5f * rinv, fmaf(r2, rinv * rinv, -1.f), rinv), s2 = ri * ri, s6 = s2 * s2 * s2;
+        float A, B;
+        if (!arith) {
+            A = a.x * b.x * s6 * s6;
+            B = a.y * b.y * s6;
+        } else {
+            const float aa = a.x * b.x, sg = 0.5f * (a.y + b.y);
+            float b1 = sg * sg * sg;
+            b1 = b1 * b1;
+            B = aa * b1 * s6;
+            A = B * b1 * s6;
+        }
+        e1 = A - B;
+        float df = -6.f * s2 * (A + e1);
+        if (sw) lj_switch_apply<float>(R, r2, e1, df);
+        return -df;
+    }
+    // one pair (charges times each other and ke in qq): minus (dE/dr)/r
+    __device__ float pair(const RepDev &R, float r2, float qq, float2 a, float2 b, bool t, float &eel, float &elj,
+                          float &vir, int &npair) const
+    {
+        const bool in_lj = r2 < rv2 && !(t && r2 < re2), in_el = r2 < rmax2 && qq != 0.f;
+        eel = 0.f; elj = 0.f; vir = 0.f;
+        float m = 0.f;
+        if (in_lj || in_el) {
+            ++npair;
+            const float rinv = nb_rsqrt_approx(r2);
+            if (in_el) m = ewald1(K, r2, rinv, qq, eel);
+            if (in_lj) {
+                const float l = lj(R, r2, rinv, a, b, elj);
+                vir = l * r2;
+                m += l;
+            }
+        }
+        return m;
+    }
+};
+
+// FP32: the H sites packed two by two on the FP32x2 pipe, their LJ part skipped for waters whose
+// hydrogens carry none.  Water stage of 8 systems of 7,020 waters and 2,496 atoms: three scalar pairs
+// per entry 208 us, this 182, with records one entry ahead 170.
+template <typename Flush>
+__device__ __forceinline__ void water_vs_atoms(const RepDev &R, const AtomK &A, int i, const float4 *pos, const void *lj_v,
+                                               const unsigned *__restrict__ sflags, const int *__restrict__ wl2_off,
+                                               const int *__restrict__ wl2, int cap2, int first, int stride, int cnt,
+                                               float g[9], float e4[4], int &npair, Flush &flush_all)
+{
+    const int q0 = min(wl2_off[i], cap2), q1 = min(wl2_off[i + 1], cap2);
+    if (q0 >= q1) return;
+    const float2 *lj = (const float2 *)lj_v;
+    const float4 o = pos[3 * i], h1 = pos[3 * i + 1], h2 = pos[3 * i + 2];
+    const float2 ljo = lj[3 * i], lj1 = lj[3 * i + 1], lj2 = lj[3 * i + 2];
+    const float qo = o.w * A.ke;
+    const float2 qh = f2(h1.w * A.ke, h2.w * A.ke);
+    const unsigned to = A.tiny ? sflags[3 * i] & SF_HTINY : 0, t1 = A.tiny ? sflags[3 * i + 1] & SF_HTINY : 0,
+                   t2 = A.tiny ? sflags[3 * i + 2] & SF_HTINY : 0;
+    const bool hlj = lj1.x != 0.f || lj2.x != 0.f || (!A.arith && (lj1.y != 0.f || lj2.y != 0.f));
+    if (q0 + first >= q1) return;
+    // the next entry's record is on its way while one is worked on, its index one further ahead
+    auto entry = [&](int k) { return wl2[min(k, q1 - 1)]; };
+    int sb = entry(q0 + first), sn = entry(q0 + first + stride);
+    float4 xb = pos[sb];
+    float2 lb = lj[sb];
+    for (int k = q0 + first; k < q1; k += stride) {
+        const int s = sb;
+        const float4 xj = xb;
+        const float2 ljj = lb;
+        sb = sn;
+        xb = pos[sb]; lb = lj[sb];
+        sn = entry(k + 2 * stride);
+        const unsigned fj = A.tiny ? sflags[s] & SF_HTINY : 0;
+        float eel, elj, vir;      // the virial of these pairs is counted by k_atom
+        bool img;
+        {
+            float dx = o.x - xj.x, dy = o.y - xj.y, dz = o.z - xj.z;
+            A.image(dx, dy, dz, img);
+            const float m = A.pair(R, dx * dx + dy * dy + dz * dz, qo * xj.w, ljo, ljj, (to | fj) != 0, eel, elj, vir, npair);
+            g[0] = fmaf(-m, dx, g[0]); g[1] = fmaf(-m, dy, g[1]); g[2] = fmaf(-m, dz, g[2]);
+            e4[0] += img ? 0.f : elj; e4[1] += img ? elj : 0.f;
+            e4[2] += img ? 0.f : eel; e4[3] += img ? eel : 0.f;
+        }
+        float2 x = f2(h1.x - xj.x, h2.x - xj.x), y = f2(h1.y - xj.y, h2.y - xj.y), z = f2(h1.z - xj.z, h2.z - xj.z);
+        const float2 mg = f2(12582912.f), nm = f2(-12582912.f);
+        const float2 nx = __fadd2_rn(__ffma2_rn(x, f2(A.iL0), mg), nm), ny = __fadd2_rn(__ffma2_rn(y, f2(A.iL1), mg), nm),
+                     nz = __fadd2_rn(__ffma2_rn(z, f2(A.iL2), mg), nm);
+        x = __ffma2_rn(nx, f2(-A.m0), __ffma2_rn(nx, f2(-A.L0), x));
+        y = __ffma2_rn(ny, f2(-A.m1), __ffma2_rn(ny, f2(-A.L1), y));
+        z = __ffma2_rn(nz, f2(-A.m2), __ffma2_rn(nz, f2(-A.L2), z));
+        const float2 r2 = __ffma2_rn(x, x, __ffma2_rn(y, y, __fmul2_rn(z, z)));
+        const float2 qq = __fmul2_rn(qh, f2(xj.w));
+        const bool el1 = r2.x < A.rmax2 && qq.x != 0.f, el2 = r2.y < A.rmax2 && qq.y != 0.f;
+        const bool v1 = r2.x < A.rv2 && !((t1 | fj) && r2.x < A.re2), v2 = r2.y < A.rv2 && !((t2 | fj) && r2.y < A.re2);
+        npair += (int)(el1 || v1) + (int)(el2 || v2);
+        if (el1 || el2 || (hlj && (v1 || v2))) {
+            float2 e, m = ewald2(A.K, r2, qq, e);
+            m = f2(el1 ? m.x : 0.f, el2 ? m.y : 0.f);
+            e = f2(el1 ? e.x : 0.f, el2 ? e.y : 0.f);
+            const bool i1 = (nx.x != 0.f) | (ny.x != 0.f) | (nz.x != 0.f), i2 = (nx.y != 0.f) | (ny.y != 0.f) | (nz.y != 0.f);
+            if (hlj) {
+                float l1 = 0.f, l2 = 0.f;
+                if (v1) m.x += A.lj(R, r2.x, nb_rsqrt_approx(r2.x), lj1, ljj, l1);
+                if (v2) m.y += A.lj(R, r2.y, nb_rsqrt_approx(r2.y), lj2, ljj, l2);
+                e4[0] += (i1 ? 0.f : l1) + (i2 ? 0.f : l2);
+                e4[1] += (i1 ? l1 : 0.f) + (i2 ? l2 : 0.f);
+            }
+            e4[2] += (i1 ? 0.f : e.x) + (i2 ? 0.f : e.y);
+            e4[3] += (i1 ? e.x : 0.f) + (i2 ? e.y : 0.f);
+            g[3] = fmaf(-m.x, x.x, g[3]); g[4] = fmaf(-m.x, y.x, g[4]); g[5] = fmaf(-m.x, z.x, g[5]);
+            g[6] = fmaf(-m.y, x.y, g[6]); g[7] = fmaf(-m.y, y.y, g[7]); g[8] = fmaf(-m.y, z.y, g[8]);
         }
         if (++cnt == CHUNK) { flush_all(); cnt = 0; }
     }
@@ -271,7 +400,7 @@ __global__ void __launch_bounds__(32 * WARPS64) k_water_d(int nW, const RepDev *
             if (nb_half_owner(il, j - R.wat0) == il) {
                 const double4 oj = pos[3 * (size_t)j];
                 dx = oi0.x - oj.x; dy = oi0.y - oj.y; dz = oi0.z - oj.z;
-                min_image<double>(R, dx, dy, dz, img);
+                min_image(R, dx, dy, dz, img);
                 in = dx * dx + dy * dy + dz * dz <= rmax2;
             }
         }
@@ -290,7 +419,7 @@ __global__ void __launch_bounds__(32 * WARPS64) k_water_d(int nW, const RepDev *
     for (int k = 0; k < 6; ++k) e4[k] *= 2.0;   // each pair once; the energy reduction halves
     // water sites against non-water atoms (W2, full list): a lane's share of the entries
     auto none = []() {};
-    water_vs_atoms<double>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, lane, 32, 0, g, e4, npair, none);
+    water_vs_atoms(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, lane, 32, 0, g, e4, npair, none);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const long long v = sub_sum<32>(nb_fix(g[k]));
@@ -514,7 +643,8 @@ __global__ void __launch_bounds__(WBLOCK, 4) k_water_s(int nW, const RepDev *__r
     __syncwarp();     // rows differ in length: the lanes that end early wait here
     fold();
     if (act) {
-        water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, sub, LPW, cnt, g, e4, npair, flush_all);
+        const AtomK A(R, iL0, iL1, iL2, L0, L1, L2, m0, m1, m2, rmax2, rv2, K);
+        water_vs_atoms(R, A, i, pos, lj_v, sflags, wl2_off, wl2, cap2, sub, LPW, cnt, g, e4, npair, flush_all);
     }
     float ecorr = 0.f;
     if (intra && sub == 0) {
@@ -758,7 +888,8 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
         eu[5] = (double)ecorr;
         flush(2.f);
         if (wl2_off[i] < wl2_off[i + 1]) {
-            water_vs_atoms<float>(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, 0, g, e4, npair, flush1);
+            const AtomK A(R, iL0, iL1, iL2, L0, L1, L2, m0, m1, m2, rmax2, rv2, K);
+            water_vs_atoms(R, A, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, 0, g, e4, npair, flush1);
             flush1();
         }
 #pragma unroll
@@ -785,33 +916,103 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
     }
 }
 
-// An energy sum: FP32 as an unevaluated hi + lo pair, FP64 plain.
-template <typename T> struct ESum;
-template <> struct ESum<float> {
-    float2 s = make_float2(0.f, 0.f);
-    __device__ void add(float v) { two_add(s, v); }
-    __device__ double total32() { const float2 a = sub_two_sum<32>(s); return (double)a.x + (double)a.y; }
-};
-template <> struct ESum<double> {
-    double s = 0.0;
-    __device__ void add(double v) { s += v; }
-    __device__ double total32() { return sub_sum<32>(s); }
-};
-
 // One warp per non-water atom over its full site list: the lanes take the list's entries in turn
 // (consecutive entries are mostly the sites of one water, so the position loads coalesce) and
-// their partial gradients and energies are summed over the warp at the end.  One atom per thread
-// ran its ~600 entries in series: 486 us for 2,496 atoms, 363 us for 203.
-template <typename T>
-__global__ void __launch_bounds__(128) k_atom(int nA, int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
+// their partial gradients and energies are summed over the warp at the end, energies as hi + lo
+// pairs.  One atom per thread ran its ~600 entries in series: 486 us for 2,496 atoms, 363 us for
+// 203.  Bound: instruction issue; with the constants loaded again for every pair and six hi + lo
+// sums per pair 19,968 atoms took 90 us, with held constants, records one entry ahead and six blocks
+// per multiprocessor 68.
+#define CHUNK_ATOM 16
+__global__ void __launch_bounds__(128, 6) k_atom_f(int nA, int nW, const RepDev *__restrict__ reps,
+                                                const int *__restrict__ site_rep, const float4 *__restrict__ pos,
+                                                const float2 *__restrict__ lj, const unsigned *__restrict__ sflags,
+                                                const int *__restrict__ xl_off, const int *__restrict__ xl, int capx,
+                                                long long *__restrict__ grad, double *__restrict__ e_unit)
+{
+    const int lane = threadIdx.x & 31, k = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (k >= nA) return;
+    const int si = 3 * nW + k;
+    const RepDev &R = reps[site_rep[si]];
+    const AtomK A(R);
+    const float4 xi = pos[si];
+    const float2 lji = lj[si];
+    const float qi = xi.w * A.ke;
+    const unsigned fi = A.tiny ? sflags[si] & SF_HTINY : 0;
+    float g[3] = {0.f, 0.f, 0.f}, e6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    long long G[3] = {0, 0, 0};
+    float2 es[6];    // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
+#pragma unroll
+    for (int m = 0; m < 6; ++m) es[m] = f2(0.f);
+    auto flush6 = [&]() {
+        flush(g, G, 3);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) { two_add(es[m], e6[m]); e6[m] = 0.f; }
+    };
+    int cnt = 0, npair = 0;
+    // an overflowed list is read within the buffer (the evaluation is redone)
+    const int q0 = min(xl_off[k], capx), q1 = min(xl_off[k + 1], capx);
+    if (q0 + lane < q1) {
+        // the next entry's record is on its way while one is worked on, its index one further ahead
+        auto entry = [&](int q) { return xl[min(q, q1 - 1)]; };
+        int s = entry(q0 + lane), sn = entry(q0 + lane + 32);
+        float4 xj = pos[s];
+        float2 ljj = lj[s];
+        for (int q = q0 + lane; q < q1; q += 32) {
+            const int sc = s;
+            const float4 xc = xj;
+            const float2 lc = ljj;
+            s = sn;
+            xj = pos[s]; ljj = lj[s];
+            sn = entry(q + 64);
+            float dx = xi.x - xc.x, dy = xi.y - xc.y, dz = xi.z - xc.z;
+            bool img;
+            A.image(dx, dy, dz, img);
+            const bool t = A.tiny && ((fi | (sflags[sc] & SF_HTINY)) != 0);
+            float eel, elj, vir;
+            const float m = A.pair(R, dx * dx + dy * dy + dz * dz, qi * xc.w, lji, lc, t, eel, elj, vir, npair);
+            g[0] = fmaf(-m, dx, g[0]); g[1] = fmaf(-m, dy, g[1]); g[2] = fmaf(-m, dz, g[2]);
+            // LJ virial: a water partner's side of the pair (its W2 list) adds none, so it counts
+            // twice here; pairs of two non-water atoms are seen from both sides
+            if (sc < 3 * nW) vir += vir;
+            e6[0] += img ? 0.f : elj; e6[1] += img ? elj : 0.f;
+            e6[2] += img ? 0.f : eel; e6[3] += img ? eel : 0.f;
+            e6[4] += img ? 0.f : vir; e6[5] += img ? vir : 0.f;
+            if (++cnt == CHUNK_ATOM) { flush6(); cnt = 0; }
+        }
+    }
+    __syncwarp();
+    flush6();
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const long long v = sub_sum<32>(G[d]);
+        if (lane == d) grad[(size_t)3 * si + d] = v;
+    }
+    double e[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+        const float2 v = sub_two_sum<32>(es[m]);
+        e[m] = (double)v.x + (double)v.y;
+    }
+    npair = sub_sum<32>(npair);
+    if (lane == 0) {
+        double *eu = e_unit + NB_EU * (size_t)(nW + k);
+        eu[0] = e[0]; eu[1] = e[1]; eu[2] = e[2]; eu[3] = e[3]; eu[4] = (double)npair; eu[5] = 0.0;
+        eu[6] = e[4]; eu[7] = e[5];
+    }
+}
+
+// The same on the plain FP64 path
+__global__ void __launch_bounds__(128) k_atom_d(int nA, int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
                                               const void *pos_v, const void *lj_v, const unsigned *__restrict__ sflags,
                                               const int *__restrict__ xl_off, const int *__restrict__ xl, int capx,
                                               long long *__restrict__ grad, double *__restrict__ e_unit)
 {
     const int lane = threadIdx.x & 31, k = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (k >= nA) return;
-    typedef typename vec4<T>::type T4;
-    typedef typename cplx<T>::type T2;
+    typedef double T;
+    typedef double4 T4;
+    typedef double2 T2;
     const T4 *pos = (const T4 *)pos_v;
     const T2 *lj = (const T2 *)lj_v;
     int si = 3 * nW + k;
@@ -821,7 +1022,7 @@ __global__ void __launch_bounds__(128) k_atom(int nA, int nW, const RepDev *__re
     unsigned fi = sflags[si];
     T g[3] = {0, 0, 0};
     long long G[3] = {0, 0, 0};
-    ESum<T> es[6];    // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
+    T es[6] = {0, 0, 0, 0, 0, 0};    // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
     int cnt = 0, npair = 0;
     // an overflowed list is read within the buffer (the evaluation is redone)
     const int q1 = min(xl_off[k + 1], capx);
@@ -831,17 +1032,17 @@ __global__ void __launch_bounds__(128) k_atom(int nA, int nW, const RepDev *__re
         T2 ljj = lj[s];
         T dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
         bool img;
-        min_image<T>(R, dx, dy, dz, img);
+        min_image(R, dx, dy, dz, img);
         T r2 = dx * dx + dy * dy + dz * dz;
         T eel = 0, elj = 0, vir = 0;
-        T df = atom_pair<T>(R, r2, xi.w, xj.w, lji.x, lji.y, ljj.x, ljj.y, fi, sflags[s], eel, elj, vir, npair);
+        T df = atom_pair(R, r2, xi.w, xj.w, lji.x, lji.y, ljj.x, ljj.y, fi, sflags[s], eel, elj, vir, npair);
         g[0] += df * dx; g[1] += df * dy; g[2] += df * dz;
         // LJ virial: a water partner's side of the pair (its W2 list) adds none, so it counts
         // twice here; pairs of two non-water atoms are seen from both sides
         if (s < 3 * nW) vir += vir;
-        es[0].add(img ? (T)0 : elj); es[1].add(img ? elj : (T)0);
-        es[2].add(img ? (T)0 : eel); es[3].add(img ? eel : (T)0);
-        es[4].add(img ? (T)0 : vir); es[5].add(img ? vir : (T)0);
+        es[0] += img ? (T)0 : elj; es[1] += img ? elj : (T)0;
+        es[2] += img ? (T)0 : eel; es[3] += img ? eel : (T)0;
+        es[4] += img ? (T)0 : vir; es[5] += img ? vir : (T)0;
         if (++cnt == CHUNK) { flush(g, G, 3); cnt = 0; }
     }
     flush(g, G, 3);
@@ -852,7 +1053,7 @@ __global__ void __launch_bounds__(128) k_atom(int nA, int nW, const RepDev *__re
     }
     double e[6];
 #pragma unroll
-    for (int m = 0; m < 6; ++m) e[m] = es[m].total32();
+    for (int m = 0; m < 6; ++m) e[m] = sub_sum<32>(es[m]);
     npair = sub_sum<32>(npair);
     if (lane == 0) {
         double *eu = e_unit + NB_EU * (size_t)(nW + k);
@@ -1270,19 +1471,6 @@ void water_t(NbCtx *c)
     if (c->timing) cudaEventRecord(c->ev[3], s);
 }
 
-template <typename T>
-void atoms_t(NbCtx *c)
-{
-    cudaStream_t s = c->stream;
-    if (c->nA > 0) {
-        k_atom<T><<<(int)((c->nA + 3) / 4), 128, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep,
-                                                             c->d_pos, c->d_site_lj, c->d_site_flags, c->d_xl_off,
-                                                             c->d_xl, cap_int(c->cap_xl), c->d_grad_site, c->d_e_unit);
-        c->launches++;
-    }
-    if (c->timing) cudaEventRecord(c->ev[4], s);
-}
-
 }  // namespace
 
 void nb_launch_water(NbCtx *c)
@@ -1297,8 +1485,20 @@ void nb_launch_water(NbCtx *c)
 
 void nb_launch_atoms(NbCtx *c)
 {
-    if (c->precision == MOIL_NB_FP64) atoms_t<double>(c);
-    else atoms_t<float>(c);
+    cudaStream_t s = c->stream;
+    if (c->nA > 0) {
+        const int nb = (int)((c->nA + 3) / 4);
+        if (c->precision == MOIL_NB_FP64)
+            k_atom_d<<<nb, 128, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_site_lj,
+                                        c->d_site_flags, c->d_xl_off, c->d_xl, cap_int(c->cap_xl), c->d_grad_site,
+                                        c->d_e_unit);
+        else
+            k_atom_f<<<nb, 128, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, (const float4 *)c->d_pos,
+                                        (const float2 *)c->d_site_lj, c->d_site_flags, c->d_xl_off, c->d_xl,
+                                        cap_int(c->cap_xl), c->d_grad_site, c->d_e_unit);
+        c->launches++;
+    }
+    if (c->timing) cudaEventRecord(c->ev[4], s);
 }
 
 // shared-memory carveout (percent of the per-SM maximum) for `bytes` of resident blocks

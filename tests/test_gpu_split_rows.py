@@ -23,6 +23,14 @@ def dense_cluster(n, seed, shrink):
     return s
 
 
+def hydrogens_with_lj(s):
+    """The same system with LJ coefficients on the waters' hydrogens, which meet non-water atoms."""
+    h = np.arange(s.npt - 3 * 150, s.npt).reshape(-1, 3)[:, 1:].ravel()
+    s.epsgm12, s.epsgm6 = s.epsgm12.copy(), s.epsgm6.copy()
+    s.epsgm12[h], s.epsgm6[h] = 0.4, 0.6
+    return s
+
+
 SYSTEMS = {
     "lone_water": lambda: S.water_box(1, 20.0, 3),
     "three_waters": lambda: S.water_box(3, 18.7, 4),
@@ -32,6 +40,7 @@ SYSTEMS = {
     "solute": lambda: S.config1(seed=7, n_solute=61, n_ions=7, n_waters=299, box=24.0),
     "solute_geometric": lambda: S.config1(seed=8, n_solute=45, n_ions=7, n_waters=150, box=24.0, arith=False,
                                           tiny_h=True),
+    "solute_hydrogen_lj": lambda: hydrogens_with_lj(S.config1(seed=9, n_solute=45, n_ions=7, n_waters=150, box=24.0)),
 }
 
 
