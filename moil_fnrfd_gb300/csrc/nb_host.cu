@@ -1319,10 +1319,11 @@ int moil_nb_adjoint(moil_nb_ctx *h, const double *coor, double *dEdq, double *dE
     NB_CUDA_OK(h, cudaMemcpyAsync(h->d_coor, coor, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->stream));
     int rc = eval_impl(h, h->d_coor, h->d_dpot, e);   // lists, positions and the potential grid
     if (rc != MOIL_NB_OK) return rc;
-    if (!h->d_adj) NB_CUDA_OK(h, cudaMalloc(&h->d_adj, sizeof(double) * 3 * std::max<size_t>(n, 1)));
+    const bool mixed = h->precision != MOIL_NB_FP64;      // with a second set of sums (nb_adjoint)
+    if (!h->d_adj) NB_CUDA_OK(h, cudaMalloc(&h->d_adj, sizeof(double) * (mixed ? 6 : 3) * std::max<size_t>(n, 1)));
     if (h->precision == MOIL_NB_FP64 && !h->d_adj_phi)
         NB_CUDA_OK(h, cudaMalloc(&h->d_adj_phi, sizeof(double) * 4 * std::max<int64_t>(h->nsite, 1)));
-    rc = nb_adjoint(h, h->d_adj, h->d_adj + n, h->d_adj + 2 * n);
+    rc = nb_adjoint(h, h->d_adj, mixed ? h->d_adj + 3 * n : nullptr);
     if (rc != MOIL_NB_OK) return rc;
     double *out[3] = {dEdq, dEdeps, dEdsig};
     for (int k = 0; k < 3; ++k)

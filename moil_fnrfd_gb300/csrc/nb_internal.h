@@ -84,8 +84,8 @@ struct NbCtx {
     unsigned *d_site_flags = nullptr;
     void *d_pos = nullptr;        // float4 / double4 (x, y, z, q_eff)
     float4 *d_posb = nullptr;     // positions at the last list build
-    void *d_woff = nullptr;       // float4 / double4 per water, 3 in a row: O position (and charge),
-                                  // then the two H offsets from O (FP64-computed)
+    void *d_woff = nullptr;       // float4 / double4 per water, 3 in a row: O position, then the two H
+                                  // offsets from O (FP64-computed), each with its charge
     void *d_site_lj = nullptr;    // float2 / double2
     void *d_site_q = nullptr;     // float / double (PME charge)
 
@@ -162,7 +162,7 @@ struct NbCtx {
 
     // caller buffers used by host-pointer evaluations
     double *d_coor = nullptr, *d_dpot = nullptr;
-    double *d_adj = nullptr;           // parameter derivatives, 3 x natom (allocated on first use)
+    double *d_adj = nullptr;           // parameter derivatives, 3 x natom (mixed path: and as many beside them; on first use)
     double *d_adj_phi = nullptr;       // plain path: PME potential share of 4 planes per site (first use)
     double *d_md_dpot = nullptr;       // gradient of the MD steps (moil_nb_md_step, first use)
     // device-side MD step loop (moil_nb_md_step): one graph per context holds a whole step
@@ -292,8 +292,9 @@ int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *
                double dhh, int nsteps);
 // per-replica energies and pair count of the last completed evaluation (e may be NULL)
 void read_energies_of(NbCtx *c, moil_energies *e);
-// parameter derivatives after an evaluation of c->d_coor (nb_adjoint.cu), mixed path
-int nb_adjoint(NbCtx *c, double *d_dq, double *d_de, double *d_ds);
+// parameter derivatives after an evaluation of c->d_coor (nb_adjoint.cu): dq, de, ds one after another;
+// out2: room for as many (mixed path), or NULL
+int nb_adjoint(NbCtx *c, double *out, double *out2);
 // pressure analysis terms after an evaluation of d_coor (nb_press.cu): 12 per replica
 int nb_pressure(NbCtx *c, const double *d_coor, double *d_out);
 int nb_press_split(const NbCtx *c);     // most blocks a replica's reduction takes

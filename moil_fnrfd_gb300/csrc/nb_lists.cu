@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256, 5) k_prepare(int nW, int nA, const RepDev
                 // within rwat of their oxygen (list radius assumption)
                 T4 off;
                 off.x = (T)(x[0] - xo[0]); off.y = (T)(x[1] - xo[1]); off.z = (T)(x[2] - xo[2]);
-                off.w = (T)0;
+                off.w = ((const T4 *)pos_v)[3 * u + m].w;
                 if (off.x * off.x + off.y * off.y + off.z * off.z > (T)rwat2) atomicOr(&st[1], NB_DEV_ERR_RWAT);
                 ((T4 *)woff_v)[3 * u + m] = off;
             }
