@@ -173,8 +173,20 @@ struct EChunk { int rep, kind, begin, end; };
 #define NB_FE_SEG 1024
 
 // work descriptors for the PME plane / column kernels
-struct PlaneWork { int rep, z; };
-struct ColWork { int rep, kx, ky0, nky; };   // z columns at fixed kx for ky in [ky0, ky0 + nky)
+// Work items of the PME kernels.  They carry their replica's grid (sizes, first complex element) and
+// the place and length of the plans' tables (FP32 path, in 16-byte units of d_blob): a block's loads
+// then depend on one load, not on four in a row.
+struct alignas(16) PlaneWork {
+    int rep, z, n1, n2;
+    int bx, lx, by, ly;          // x and y tables
+    long long g0;
+};
+struct alignas(16) ColWork {
+    int rep, kx, ky0, nky;       // z columns at fixed kx for ky in [ky0, ky0 + nky)
+    int n1, n2, n3, bsp0;
+    int bz, lz;                  // z tables
+    long long g0;
+};
 
 // ---------------------------------------------------------------------------------
 // precision traits

@@ -11,9 +11,9 @@
 
 // FFT plan for one length: radices (4, 2, 3, 5 in that order), twiddles exp(-2 pi i k / n)
 // at tw0, and per Stockham stage s: the span Ns, the butterfly count nb = n/R, the magic
-// multiplier for dividing by nb, and nb (twiddle step, destination index) entries at tab0+off[s]
+// multiplier for dividing by nb, and nb (twiddle step, destination index) entries at off[s]
 struct FftPlanDev {
-    int n, nst, tw0, tab0;
+    int n, nst, tw0;
     int rad[8];
     int ns[8];
     int nb[8];
@@ -133,7 +133,7 @@ struct NbCtx {
     std::vector<int> rep_plan;         // 3 plan indices per replica
     int *d_rep_plan = nullptr;
     void *d_tw = nullptr;              // float2 / double2 twiddles
-    int2 *d_tab = nullptr;             // Stockham stage tables (twiddle step, destination index)
+    int4 *d_blob = nullptr;            // FP32 path: per plan its constants, twiddles and stage table
     std::vector<double> bsp_h;
     void *d_bsp = nullptr;             // float / double moduli
     float *d_etab = nullptr;           // FP32 path: exp(-pi^2 m^2 / (alpha L)^2) / B per dimension (bsp layout)

@@ -383,7 +383,7 @@ __device__ __forceinline__ void fft_pass(int R, const float2 *src, float2 *dst, 
     }
 }
 
-// A plan with its stage table and twiddles, staged in shared memory by fft_ctx_load so the
+// A plan with its twiddles and stage table, staged in shared memory by fft_ctx_load so the
 // butterflies read them without global-memory latency.
 struct FftCtx {
     const FftPlanDev *p;
@@ -394,23 +394,27 @@ struct FftCtx {
 // shared-memory bytes of one staged plan of length n
 size_t fft_ctx_bytes(int n, bool wide);
 
-__device__ __forceinline__ unsigned char *fft_ctx_load(unsigned char *dst, const FftPlanDev *__restrict__ gp,
-                                                       const int2 *__restrict__ gtab, const float2 *__restrict__ gtw,
+// copies from global to shared memory that no register and no thread waits for until async_wait
+__device__ __forceinline__ void async_copy16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_copy8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// the tables of a plan of length n: len 16-byte units (plan, twiddles, stage table); complete after
+// async_wait and a barrier
+__device__ __forceinline__ unsigned char *fft_ctx_load(unsigned char *dst, const int4 *__restrict__ src, int len, int n,
                                                        FftCtx &ctx)
 {
-    const int n = gp->n, nst = gp->nst;
-    const int ntab = gp->off[nst - 1] + gp->nb[nst - 1];
-    FftPlanDev *sp = (FftPlanDev *)dst;
-    int2 *st = (int2 *)(dst + align16(sizeof(FftPlanDev)));
-    float2 *stw = (float2 *)((unsigned char *)st + align16(ntab * sizeof(int2)));
-    for (int k = threadIdx.x; k < (int)(sizeof(FftPlanDev) / 4); k += blockDim.x)
-        ((int *)sp)[k] = ((const int *)gp)[k];
-    for (int k = threadIdx.x; k < ntab; k += blockDim.x) st[k] = gtab[gp->tab0 + k];
-    for (int k = threadIdx.x; k < n; k += blockDim.x) stw[k] = gtw[gp->tw0 + k];
-    ctx.p = sp;
-    ctx.tab = st;
-    ctx.tw = stw;
-    return (unsigned char *)stw + align16(n * sizeof(float2));
+    for (int k = threadIdx.x; k < len; k += blockDim.x) async_copy16(dst + 16 * k, src + k);
+    ctx.p = (const FftPlanDev *)dst;
+    ctx.tw = (const float2 *)(dst + align16(sizeof(FftPlanDev)));
+    ctx.tab = (const int2 *)((const unsigned char *)ctx.tw + align16(n * sizeof(float2)));
+    return dst + 16 * (size_t)len;
 }
 
 // Full forward FFT of L lines of length n held in a (line stride in_ss); b is scratch.  The
@@ -467,25 +471,25 @@ __host__ __device__ __forceinline__ int zconv_buf_elems(int n3)
 }
 
 __global__ void __launch_bounds__(256, 8) k_plane_fwd_f(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                                     const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                                     const float2 *__restrict__ tw, const int2 *__restrict__ tab,
+                                                     const int4 *__restrict__ blob,
                                                      int nW, const unsigned char *__restrict__ zidx,
                                                      const float4 *__restrict__ fr, float2 *__restrict__ grid)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const PlaneWork w = work[blockIdx.x];
     const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n1h = R.n1h, n2p = (n2 + 1) >> 1;
+    const int n1 = w.n1, n2 = w.n2, n1h = n1 / 2 + 1, n2p = (n2 + 1) >> 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     float2 *B0 = (float2 *)smem, *B1 = B0 + plane_buf_elems(n1, n2);
     int *acc = (int *)B0;                        // the int32 plane lives in B0 until it is packed
     FftCtx c1, c2;
     unsigned char *ctx = (unsigned char *)(B1 + plane_buf_elems(n1, n2));
-    ctx = fft_ctx_load(ctx, plans + rep_plan[3 * w.rep], tab, tw, c1);
-    fft_ctx_load(ctx, plans + rep_plan[3 * w.rep + 1], tab, tw, c2);
+    ctx = fft_ctx_load(ctx, blob + w.bx, w.lx, n1, c1);
+    fft_ctx_load(ctx, blob + w.by, w.ly, n2, c2);
     for (int k = threadIdx.x; k < n1 * n2; k += blockDim.x) acc[k] = 0;
     plane_sites(R, nW, w.z, zidx, (int *)B1, 2 * plane_buf_elems(n1, n2),
                 [&](int n) { spread_sites<float>(R, (const int *)B1, n, fr, acc, R.spread216); });
+    async_wait();
     __syncthreads();
     // x transform of real rows two at a time: line p carries row 2p as its real part and
     // row 2p+1 as its imaginary part
@@ -512,13 +516,12 @@ __global__ void __launch_bounds__(256, 8) k_plane_fwd_f(const PlaneWork *__restr
     __syncthreads();
     // y: n1h lines of n2
     float2 *Y = fft_lines<0, false>(c2, T, Z, nullptr, n1h, 0, sT, n2);
-    float2 *g = grid + R.g0 + (size_t)w.z * n1h * n2;
+    float2 *g = grid + w.g0 + (size_t)w.z * n1h * n2;
     for (int k = threadIdx.x; k < n1h * n2; k += blockDim.x) g[k] = Y[k];
 }
 
 __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                                 const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                                 const float2 *__restrict__ tw, const int2 *__restrict__ tab,
+                                                 const int4 *__restrict__ blob,
                                                  const float *__restrict__ etab_all, float2 *__restrict__ grid,
                                                  double *__restrict__ e_col)
 {
@@ -526,18 +529,19 @@ __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ 
     __shared__ double red[8];
     const ColWork w = work[blockIdx.x];
     const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n3 = R.n3, n1h = R.n1h;
+    const int n1 = w.n1, n2 = w.n2, n3 = w.n3, n1h = n1 / 2 + 1;
     const int tk = w.nky;
-    const float *etab = etab_all + R.bsp0;
+    const float *etab = etab_all + w.bsp0;
     float2 *A = (float2 *)smem, *B = A + zconv_buf_elems(n3);
     FftCtx c3;
-    fft_ctx_load((unsigned char *)(B + zconv_buf_elems(n3)), plans + rep_plan[3 * w.rep + 2], tab, tw, c3);
+    fft_ctx_load((unsigned char *)(B + zconv_buf_elems(n3)), blob + w.bz, w.lz, n3, c3);
     const int sA = n3 | 1;    // odd line stride of the columns as loaded and stored
-    float2 *g = grid + R.g0 + (size_t)w.kx * n2 + w.ky0;
+    float2 *g = grid + w.g0 + (size_t)w.kx * n2 + w.ky0;
     const size_t zs = (size_t)n1h * n2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int kz = warp; kz < n3; kz += 8)
-        if (lane < tk) A[lane * sA + kz] = g[kz * zs + lane];
+        if (lane < tk) async_copy8(A + lane * sA + kz, g + kz * zs + lane);
+    async_wait();
     __syncthreads();
     float2 *F = fft_lines<0, false, true>(c3, A, B, nullptr, tk, 0, sA, n3);
     float2 *Fo = F == A ? B : A;
@@ -596,27 +600,26 @@ __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ 
 // E(m) (1 - 2 (1 + pi^2 m^2 / alpha^2) m_a^2 / m^2) with E(m) = wgt * eterm * |S(m)|^2 as the
 // energy sum forms it; three FP64 partial sums per column work item (fixed-order reduction)
 __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                                      const FftPlanDev *__restrict__ plans,
-                                                      const int *__restrict__ rep_plan, const float2 *__restrict__ tw,
-                                                      const int2 *__restrict__ tab, const float *__restrict__ bsp_all,
+                                                      const int4 *__restrict__ blob, const float *__restrict__ bsp_all,
                                                       const float2 *__restrict__ grid, double *__restrict__ v_col)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double red[3][8];
     const ColWork w = work[blockIdx.x];
     const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n3 = R.n3, n1h = R.n1h;
+    const int n1 = w.n1, n2 = w.n2, n3 = w.n3, n1h = n1 / 2 + 1;
     const int tk = w.nky;
-    const float *bsp = bsp_all + R.bsp0;
+    const float *bsp = bsp_all + w.bsp0;
     float2 *A = (float2 *)smem, *B = A + zconv_buf_elems(n3);
     FftCtx c3;
-    fft_ctx_load((unsigned char *)(B + zconv_buf_elems(n3)), plans + rep_plan[3 * w.rep + 2], tab, tw, c3);
+    fft_ctx_load((unsigned char *)(B + zconv_buf_elems(n3)), blob + w.bz, w.lz, n3, c3);
     const int sA = n3 | 1;
-    const float2 *g = grid + R.g0 + (size_t)w.kx * n2 + w.ky0;
+    const float2 *g = grid + w.g0 + (size_t)w.kx * n2 + w.ky0;
     const size_t zs = (size_t)n1h * n2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int kz = warp; kz < n3; kz += 8)
-        if (lane < tk) A[lane * sA + kz] = g[kz * zs + lane];
+        if (lane < tk) async_copy8(A + lane * sA + kz, g + kz * zs + lane);
+    async_wait();
     __syncthreads();
     const float2 *F = fft_lines<0, false, true>(c3, A, B, nullptr, tk, 0, sA, n3);
     const float wgt = (w.kx == 0 || 2 * w.kx == n1) ? 1.f : 2.f;
@@ -658,24 +661,23 @@ __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict_
 
 // inverse y and x transforms of plane z; the real potential plane (n1 x n2 floats) is stored
 // over the plane's own complex storage, which this block alone reads, for k_pme_gather_f
-__global__ void __launch_bounds__(256) k_plane_inv_f(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                                     const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                                     const float2 *__restrict__ tw, const int2 *__restrict__ tab,
+__global__ void __launch_bounds__(256) k_plane_inv_f(const PlaneWork *__restrict__ work,
+                                                     const int4 *__restrict__ blob,
                                                      float2 *__restrict__ grid)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const PlaneWork w = work[blockIdx.x];
-    const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n1h = R.n1h, n2p = (n2 + 1) >> 1;
+    const int n1 = w.n1, n2 = w.n2, n1h = n1 / 2 + 1, n2p = (n2 + 1) >> 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     float2 *B0 = (float2 *)smem, *B1 = B0 + plane_buf_elems(n1, n2);
     FftCtx c1, c2;
     unsigned char *ctx = (unsigned char *)(B1 + plane_buf_elems(n1, n2));
-    ctx = fft_ctx_load(ctx, plans + rep_plan[3 * w.rep], tab, tw, c1);
-    fft_ctx_load(ctx, plans + rep_plan[3 * w.rep + 1], tab, tw, c2);
-    float2 *g = grid + R.g0 + (size_t)w.z * n1h * n2;
+    ctx = fft_ctx_load(ctx, blob + w.bx, w.lx, n1, c1);
+    fft_ctx_load(ctx, blob + w.by, w.ly, n2, c2);
+    float2 *g = grid + w.g0 + (size_t)w.z * n1h * n2;
     // [kx][ky] lines of n2, conjugated (inverse through the forward transform)
     for (int k = threadIdx.x; k < n1h * n2; k += blockDim.x) B0[k] = cconj(g[k]);
+    async_wait();
     __syncthreads();
     // y: n1h lines; last pass conjugates back and stores transposed to H[ky][kx] at the odd
     // row stride hs
@@ -1053,16 +1055,13 @@ void pme_t(NbCtx *c)
     }
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
     if (sizeof(T) == 4) {
-        k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                           (const float2 *)c->d_tw, c->d_tab, (int)c->nW, c->d_zidx,
+        k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
                                                            (const float4 *)c->d_fr, (float2 *)c->d_grid);
         if (c->timing) cudaEventRecord(c->ev[7], s);
-        k_zconv_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                  (const float2 *)c->d_tw, c->d_tab, c->d_etab,
+        k_zconv_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, c->d_etab,
                                                   (float2 *)c->d_grid, c->d_e_col);
         if (c->timing) cudaEventRecord(c->ev[8], s);
-        k_plane_inv_f<<<np, 256, c->smem_plane_inv, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                           (const float2 *)c->d_tw, c->d_tab, (float2 *)c->d_grid);
+        k_plane_inv_f<<<np, 256, c->smem_plane_inv, s>>>(c->d_planes, c->d_blob, (float2 *)c->d_grid);
         k_pme_gather_f<<<(int)((c->nsite + 255) / 256), 256, 0, s>>>(
             (int)c->nsite, c->d_site_rep, c->d_reps, (const float4 *)c->d_fr, (const float2 *)c->d_grid,
             (float4 *)c->d_part);
@@ -1180,15 +1179,35 @@ template <typename T> int col_tile() { return sizeof(T) == 4 ? NB_TKF : NB_TK; }
 // (within one), so no block of the column kernels works on a short remainder alone (n2 = 36
 // gives two runs of 18, not 32 and 4: every Stockham pass of a run then fits one sweep of the
 // block's threads)
-void push_col_runs(std::vector<ColWork> &cols, int rep, int kx, int n2, int tile)
+void push_col_runs(std::vector<ColWork> &cols, ColWork w, int tile)
 {
+    const int n2 = w.n2;
     const int nrun = (n2 + tile - 1) / tile, base = n2 / nrun, extra = n2 % nrun;
     int ky0 = 0;
     for (int k = 0; k < nrun; ++k) {
         const int len = base + (k < extra ? 1 : 0);
-        cols.push_back(ColWork{rep, kx, ky0, len});
+        w.ky0 = ky0;
+        w.nky = len;
+        cols.push_back(w);
         ky0 += len;
     }
+}
+
+// one plan's tables as the FP32 kernels stage them (fft_ctx_load), appended to blob; its offset and
+// length in 16-byte units
+void push_blob(std::vector<int4> &blob, const FftPlanDev &p, const std::vector<int2> &tab, const std::vector<float2> &tw,
+               int *off, int *len)
+{
+    const size_t b0 = align16(sizeof(FftPlanDev)), b1 = b0 + align16(p.n * sizeof(float2)),
+                 b2 = b1 + align16(tab.size() * sizeof(int2));
+    *off = (int)blob.size();
+    *len = (int)(b2 / 16);
+    blob.resize(blob.size() + b2 / 16);
+    unsigned char *d = (unsigned char *)(blob.data() + *off);
+    memset(d, 0, b2);
+    memcpy(d, &p, sizeof(p));
+    memcpy(d + b0, tw.data(), p.n * sizeof(float2));
+    memcpy(d + b1, tab.data(), tab.size() * sizeof(int2));
 }
 
 // raise a kernel's dynamic shared-memory limit to at least `bytes` (never lower it)
@@ -1225,7 +1244,8 @@ int configure_t(NbCtx *c)
     c->plans.clear();
     c->rep_plan.assign(3 * c->nrep, 0);
     std::vector<double> twr, twi;
-    std::vector<int2> tab;
+    std::vector<int4> blob;
+    std::vector<int> boff, blen;   // per plan (FP32 path)
     std::vector<char> wide_of;     // per plan: wide radix set (the FP32 z columns)
     for (int r = 0; r < c->nrep; ++r) {
         int ns[3] = {c->rd[r].n1, c->rd[r].n2, c->rd[r].n3};
@@ -1236,15 +1256,19 @@ int configure_t(NbCtx *c)
                 if (c->plans[k].n == ns[d] && (bool)wide_of[k] == wide) found = (int)k;
             if (found < 0) {
                 FftPlanDev p;
-                int tab0 = (int)tab.size();
+                std::vector<int2> tab;
+                std::vector<float2> tw;
                 if (!make_plan(ns[d], &p, &tab, wide)) return MOIL_NB_ERR_GRID;
-                p.tab0 = tab0;
                 p.tw0 = (int)twr.size();
                 for (int t = 0; t < ns[d]; ++t) {
                     double ang = -2.0 * M_PI * (double)t / (double)ns[d];
                     twr.push_back(cos(ang));
                     twi.push_back(sin(ang));
+                    tw.push_back(make_float2((float)twr.back(), (float)twi.back()));
                 }
+                boff.push_back(0);
+                blen.push_back(0);
+                if (sizeof(T) == 4) push_blob(blob, p, tab, tw, &boff.back(), &blen.back());
                 c->plans.push_back(p);
                 wide_of.push_back(wide);
                 found = (int)c->plans.size() - 1;
@@ -1260,8 +1284,10 @@ int configure_t(NbCtx *c)
     NB_CUDA_OK(c, cudaMemcpy(c->d_rep_plan, c->rep_plan.data(), sizeof(int) * c->rep_plan.size(), cudaMemcpyHostToDevice));
     NB_CUDA_OK(c, cudaMalloc(&c->d_tw, sizeof(C) * tw.size()));
     NB_CUDA_OK(c, cudaMemcpy(c->d_tw, tw.data(), sizeof(C) * tw.size(), cudaMemcpyHostToDevice));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_tab, sizeof(int2) * tab.size()));
-    NB_CUDA_OK(c, cudaMemcpy(c->d_tab, tab.data(), sizeof(int2) * tab.size(), cudaMemcpyHostToDevice));
+    if (sizeof(T) == 4) {
+        NB_CUDA_OK(c, cudaMalloc(&c->d_blob, sizeof(int4) * blob.size()));
+        NB_CUDA_OK(c, cudaMemcpy(c->d_blob, blob.data(), sizeof(int4) * blob.size(), cudaMemcpyHostToDevice));
+    }
     std::vector<T> bsp(c->bsp_h.size());
     for (size_t k = 0; k < bsp.size(); ++k) bsp[k] = (T)c->bsp_h[k];
     NB_CUDA_OK(c, cudaMalloc(&c->d_bsp, sizeof(T) * bsp.size()));
@@ -1283,10 +1309,12 @@ int configure_t(NbCtx *c)
     const int tk = col_tile<T>();
     for (int r = 0; r < c->nrep; ++r) {
         const RepDev &R = c->rd[r];
-        for (int z = 0; z < R.n3; ++z) c->planes.push_back(PlaneWork{r, z});
+        const int *pl = &c->rep_plan[3 * r];
+        for (int z = 0; z < R.n3; ++z)
+            c->planes.push_back(PlaneWork{r, z, R.n1, R.n2, boff[pl[0]], blen[pl[0]], boff[pl[1]], blen[pl[1]], R.g0});
         c->col_begin[r] = (int)c->cols.size();
         for (int kx = 0; kx < R.n1h; ++kx)
-            push_col_runs(c->cols, r, kx, R.n2, tk);
+            push_col_runs(c->cols, ColWork{r, kx, 0, 0, R.n1, R.n2, R.n3, R.bsp0, boff[pl[2]], blen[pl[2]], R.g0}, tk);
         sf = std::max(sf, plane_fwd_smem<T>(R.n1, R.n2));
         si = std::max(si, plane_inv_smem<T>(R.n1, R.n2));
         sz = std::max(sz, zconv_smem<T>(R.n3));
@@ -1340,11 +1368,9 @@ void nb_launch_pme_virial(NbCtx *c, cudaStream_t s, void *grid, double *v_col)
                                                             c->d_bsp, grid, v_col);
         return;
     }
-    k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                       (const float2 *)c->d_tw, c->d_tab, (int)c->nW, c->d_zidx,
+    k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
                                                        (const float4 *)c->d_fr, (float2 *)grid);
-    k_press_zvir_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                   (const float2 *)c->d_tw, c->d_tab, (const float *)c->d_bsp,
+    k_press_zvir_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, (const float *)c->d_bsp,
                                                    (const float2 *)grid, v_col);
 }
 
@@ -1412,7 +1438,11 @@ namespace {
 constexpr int NA_MAX_ATOMS = 65536;
 constexpr int NA_MAX_N = 64;
 constexpr int NA_MAX_COLS = (NA_MAX_N / 2 + 1) * ((NA_MAX_N + NB_TKF - 1) / NB_TKF);
-constexpr int NA_MAX_TAB = 3 * 8 * NA_MAX_N;
+struct alignas(16) NaParams {
+    RepDev R;
+    unsigned long long qmax;     // largest |charge| (bits of a non-negative double order as integers)
+    unsigned done;               // blocks of k_na_load that have finished
+};
 constexpr size_t na_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // arena regions (byte offsets, 256-byte aligned)
@@ -1422,19 +1452,17 @@ constexpr size_t NA_ZIDX = NA_FR + na_up(sizeof(float4) * NA_MAX_ATOMS);
 constexpr size_t NA_PART = NA_ZIDX + na_up(NA_MAX_ATOMS + 16);
 constexpr size_t NA_GRID = NA_PART + na_up(sizeof(float) * 12 * NA_MAX_ATOMS);
 constexpr size_t NA_ECOL = NA_GRID + na_up(sizeof(float2) * ((NA_MAX_N / 2 + 1) * NA_MAX_N * NA_MAX_N + 2));
-constexpr size_t NA_PLANES = NA_ECOL + na_up(sizeof(double) * NA_MAX_COLS);
-constexpr size_t NA_COLS = NA_PLANES + na_up(sizeof(PlaneWork) * NA_MAX_N);
-constexpr size_t NA_COLBEG = NA_COLS + na_up(sizeof(ColWork) * NA_MAX_COLS);
-constexpr size_t NA_PLANS = NA_COLBEG + na_up(sizeof(int) * 2);
-constexpr size_t NA_REPPLAN = NA_PLANS + na_up(sizeof(FftPlanDev) * 3);
-constexpr size_t NA_TW = NA_REPPLAN + na_up(sizeof(int) * 3);
-constexpr size_t NA_TAB = NA_TW + na_up(sizeof(float2) * 3 * NA_MAX_N);
-constexpr size_t NA_BSP = NA_TAB + na_up(sizeof(int2) * NA_MAX_TAB);
-constexpr size_t NA_ETAB = NA_BSP + na_up(sizeof(float) * 3 * NA_MAX_N);
-constexpr size_t NA_REPS = NA_ETAB + na_up(sizeof(float) * 3 * NA_MAX_N);
-constexpr size_t NA_EOUT = NA_REPS + na_up(sizeof(RepDev));
-constexpr size_t NA_STATUS = NA_EOUT + na_up(sizeof(double));
-constexpr size_t NA_BYTES = NA_STATUS + na_up(sizeof(int) * 8);
+constexpr size_t NA_ETAB = NA_ECOL + na_up(sizeof(double) * NA_MAX_COLS);
+constexpr size_t NA_EOUT = NA_ETAB + na_up(sizeof(float) * 3 * NA_MAX_N);
+// what the host lays out, one copy per call: constants (with the charge maximum and the block count
+// of k_na_load, zero), planes, columns, tables
+constexpr size_t NA_HOST = NA_EOUT + na_up(sizeof(double));
+constexpr size_t NA_PLANES = sizeof(NaParams);
+constexpr size_t NA_COLS = NA_PLANES + sizeof(PlaneWork) * NA_MAX_N;
+constexpr size_t NA_BLOB = NA_COLS + sizeof(ColWork) * NA_MAX_COLS;
+constexpr size_t NA_HOST_BYTES = NA_BLOB + 3 * (512 + sizeof(float2) * NA_MAX_N + sizeof(int2) * 8 * NA_MAX_N);
+static_assert(sizeof(FftPlanDev) + 32 <= 512, "room of a plan in the tables");
+constexpr size_t NA_BYTES = NA_HOST + na_up(NA_HOST_BYTES);
 
 static __device__ __align__(256) unsigned char g_pme_scratch[NA_BYTES];
 
@@ -1442,44 +1470,76 @@ std::mutex g_na_mu;
 constexpr int NA_MAX_DEVICES = 64;
 unsigned char *g_na_base[NA_MAX_DEVICES] = {};
 
-__global__ void k_na_load(int natom, const RepDev *__restrict__ reps, const double *__restrict__ coor,
-                          const double *__restrict__ q, float4 *__restrict__ fr, unsigned char *__restrict__ zidx,
-                          int *__restrict__ srep)
+// Records of the atoms, and beside them the spread scale from the largest charge (same rule as the
+// handle path), set by the last block to finish, and the influence function's tables (last
+// block; order-4 B-spline moduli |1/6 + 2/3 w + 1/6 w^2|^2 = (2/3 + cos(2 pi k / n) / 3)^2,
+// ewald_receip.f:413-481).  The charge maximum in a block of its own took 49 us for 23,556 atoms, and
+// the moduli on the host 100.
+__global__ void __launch_bounds__(256) k_na_load(int natom, NaParams *__restrict__ P, const double *__restrict__ coor,
+                                                 const double *__restrict__ q, float4 *__restrict__ fr,
+                                                 unsigned char *__restrict__ zidx, int *__restrict__ srep,
+                                                 float *__restrict__ etab)
 {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= natom) return;
-    const float x[3] = {(float)coor[3 * (size_t)a], (float)coor[3 * (size_t)a + 1], (float)coor[3 * (size_t)a + 2]};
-    fr[a] = pme_site(reps[0], x, (float)q[a], zidx[a]);
-    srep[a] = 0;
+    __shared__ unsigned long long smax;
+    RepDev &R = P->R;
+    if (threadIdx.x == 0) smax = 0ull;
+    __syncthreads();
+    if (blockIdx.x == gridDim.x - 1) {
+        const int n[3] = {R.n1, R.n2, R.n3};
+        for (int t = threadIdx.x; t < n[0] + n[1] + n[2]; t += blockDim.x) {
+            const int d = t < n[0] ? 0 : (t < n[0] + n[1] ? 1 : 2), k = t - (d > 0 ? n[0] : 0) - (d > 1 ? n[1] : 0);
+            const int nd = d == 0 ? n[0] : (d == 1 ? n[1] : n[2]);
+            const int m = k < (nd + 1) / 2 ? k : k - nd;
+            const double b = 2.0 / 3.0 + cospi(2.0 * k / nd) / 3.0, mh = m * R.invLd[d];
+            etab[t] = (float)(exp(-R.pme_fac * mh * mh) / (b * b));
+        }
+    } else {
+        const int a = blockIdx.x * blockDim.x + threadIdx.x;
+        double qa = 0.0;
+        if (a < natom) {
+            qa = q[a];
+            const float x[3] = {(float)coor[3 * (size_t)a], (float)coor[3 * (size_t)a + 1], (float)coor[3 * (size_t)a + 2]};
+            fr[a] = pme_site(R, x, (float)qa, zidx[a]);
+            srep[a] = 0;
+        }
+        // (a NaN charge is left out, as fmax leaves it out)
+        atomicMax(&smax, qa == qa ? (unsigned long long)__double_as_longlong(fabs(qa)) : 0ull);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(&P->qmax, smax);
+        __threadfence();
+        if (atomicAdd(&P->done, 1u) == gridDim.x - 1) {
+            const double m = __longlong_as_double((long long)atomicMax(&P->qmax, 0ull));
+            const int k = nb_spread_exp(m * R.fcd);
+            R.spread_scale = (float)ldexp(1.0, k);
+            R.spread_inv = (float)ldexp(1.0, -k);
+            const double s216 = ldexp(1.0, k) / 216.0;
+            R.spread216 = (float)s216;
+            const double c = s216 / (double)R.spread216;
+            R.pme_qcorr = c * c;
+        }
+    }
 }
 
-// int32 plane scale from the largest charge (same rule as the handle path)
-__global__ void k_na_scale(int natom, const double *__restrict__ q, RepDev *__restrict__ reps)
+// gradient (grad_sum, pot/ewald_receip.f:815-970), overwriting dpot, and in the last block the energy
+__global__ void __launch_bounds__(256) k_na_grad(int natom, const RepDev *__restrict__ reps, const double *__restrict__ q,
+                                                 const float *__restrict__ part, double *__restrict__ dpot, int ncol,
+                                                 const double *__restrict__ e_col, double *__restrict__ out)
 {
     __shared__ double sh[256];
-    double m = 0;
-    for (int a = threadIdx.x; a < natom; a += blockDim.x) m = fmax(m, fabs(q[a]));
-    sh[threadIdx.x] = m;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] = fmax(sh[threadIdx.x], sh[threadIdx.x + o]);
+    if (blockIdx.x == gridDim.x - 1) {
+        double v = 0;
+        for (int w = threadIdx.x; w < ncol; w += blockDim.x) v += e_col[w];
+        sh[threadIdx.x] = v;
         __syncthreads();
+        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+            if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) *out = 0.5 * sh[0];
+        return;
     }
-    if (threadIdx.x == 0) {
-        const int k = nb_spread_exp(sh[0] * reps[0].fcd);
-        reps[0].spread_scale = (float)ldexp(1.0, k);
-        reps[0].spread_inv = (float)ldexp(1.0, -k);
-        const double s216 = ldexp(1.0, k) / 216.0;
-        reps[0].spread216 = (float)s216;
-        const double c = s216 / (double)reps[0].spread216;
-        reps[0].pme_qcorr = c * c;
-    }
-}
-
-// gradient from the four per-plane slots (grad_sum, pot/ewald_receip.f:815-970); overwrites dpot
-__global__ void k_na_grad(int natom, const RepDev *__restrict__ reps, const double *__restrict__ q,
-                          const float *__restrict__ part, double *__restrict__ dpot)
-{
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= natom) return;
     const RepDev &R = reps[0];
@@ -1489,20 +1549,6 @@ __global__ void k_na_grad(int natom, const RepDev *__restrict__ reps, const doub
     dpot[3 * (size_t)a] = qf * R.n1 * R.invLd[0] * pg[0];
     dpot[3 * (size_t)a + 1] = qf * R.n2 * R.invLd[1] * pg[1];
     dpot[3 * (size_t)a + 2] = qf * R.n3 * R.invLd[2] * pg[2];
-}
-
-__global__ void k_na_energy(int ncol, const double *__restrict__ e_col, double *__restrict__ out)
-{
-    __shared__ double sh[256];
-    double v = 0;
-    for (int w = threadIdx.x; w < ncol; w += blockDim.x) v += e_col[w];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = 0.5 * sh[0];
 }
 
 }  // namespace
@@ -1550,9 +1596,10 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     if (raise_pme_limits<float>(plane_fwd_smem<float>(n1, n2), zconv_smem<float>(n3),
                                 plane_inv_smem<float>(n1, n2)) != cudaSuccess)
         return MOIL_NB_ERR_CUDA;
-    // one-replica constants, FFT plans and tables, B-spline moduli, work lists (host side)
-    RepDev R;
-    memset(&R, 0, sizeof(R));
+    // one-replica constants, FFT plans and tables, work lists (host side)
+    NaParams P;
+    memset((void *)&P, 0, sizeof(P));
+    RepDev &R = P.R;
     for (int d = 0; d < 3; ++d) {
         R.Ld[d] = box[d];
         R.L[d] = (float)box[d];
@@ -1571,39 +1618,27 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     nb_pme_fp32_consts(&R);
     R.pme_qcorr = 1.0;    // the charges stay on the device: no rounding correction
     R.natom = R.noth = natom;   // every atom a non-water site
-    FftPlanDev plans[3];
-    int rep_plan[3];
-    float2 tw[3 * NA_MAX_N];
-    std::vector<int2> tab;
-    float bsp[3 * NA_MAX_N];
-    int ntw = 0;
+    std::vector<int4> blob;
+    int boff[3], blen[3];
     for (int d = 0; d < 3; ++d) {
-        int tab0 = (int)tab.size();
-        make_plan(grid[d], &plans[d], &tab, d == 2);     // the z columns take the wide radix set
-        plans[d].tab0 = tab0;
-        plans[d].tw0 = ntw;
+        FftPlanDev plan;
+        std::vector<int2> tab;
+        std::vector<float2> tw(grid[d]);
+        make_plan(grid[d], &plan, &tab, d == 2);     // the z columns take the wide radix set
         for (int t = 0; t < grid[d]; ++t) {
-            double ang = -2.0 * M_PI * (double)t / (double)grid[d];
-            tw[ntw++] = make_float2((float)cos(ang), (float)sin(ang));
+            const double ang = -2.0 * M_PI * (double)t / (double)grid[d];
+            tw[t] = make_float2((float)cos(ang), (float)sin(ang));
         }
-        rep_plan[d] = d;
+        push_blob(blob, plan, tab, tw, &boff[d], &blen[d]);
     }
-    if ((int)tab.size() > NA_MAX_TAB) return MOIL_NB_ERR_GRID;
-    double bspd[3 * NA_MAX_N];
-    nb_bsp_moduli(n1, bspd);
-    nb_bsp_moduli(n2, bspd + n1);
-    nb_bsp_moduli(n3, bspd + n1 + n2);
-    for (int k = 0; k < n1 + n2 + n3; ++k) bsp[k] = (float)bspd[k];
-    float etab[3 * NA_MAX_N];
-    nb_pme_etab(R, bspd, etab);
     NbCtx tmp;
     tmp.stream = stream;
     tmp.nrep = 1;
     tmp.nsite = natom;
-    for (int z = 0; z < n3; ++z) tmp.planes.push_back(PlaneWork{0, z});
+    for (int z = 0; z < n3; ++z) tmp.planes.push_back(PlaneWork{0, z, n1, n2, boff[0], blen[0], boff[1], blen[1], 0});
     for (int kx = 0; kx < R.n1h; ++kx)
-        push_col_runs(tmp.cols, 0, kx, n2, NB_TKF);
-    int col_begin[2] = {0, (int)tmp.cols.size()};
+        push_col_runs(tmp.cols, ColWork{0, kx, 0, 0, n1, n2, n3, 0, boff[2], blen[2], 0}, NB_TKF);
+    if (NA_BLOB + sizeof(int4) * blob.size() > NA_HOST_BYTES) return MOIL_NB_ERR_GRID;
     tmp.smem_plane_fwd = plane_fwd_smem<float>(n1, n2);
     tmp.smem_plane_inv = plane_inv_smem<float>(n1, n2);
     tmp.smem_zconv = zconv_smem<float>(n3);
@@ -1613,38 +1648,26 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     tmp.d_part = base + NA_PART;
     tmp.d_grid = base + NA_GRID;
     tmp.d_e_col = (double *)(base + NA_ECOL);
-    tmp.d_planes = (PlaneWork *)(base + NA_PLANES);
-    tmp.d_cols = (ColWork *)(base + NA_COLS);
-    tmp.d_col_begin = (int *)(base + NA_COLBEG);
-    tmp.d_plans = (FftPlanDev *)(base + NA_PLANS);
-    tmp.d_rep_plan = (int *)(base + NA_REPPLAN);
-    tmp.d_tw = base + NA_TW;
-    tmp.d_tab = (int2 *)(base + NA_TAB);
-    tmp.d_bsp = base + NA_BSP;
+    tmp.d_planes = (PlaneWork *)(base + NA_HOST + NA_PLANES);
+    tmp.d_cols = (ColWork *)(base + NA_HOST + NA_COLS);
+    tmp.d_blob = (int4 *)(base + NA_HOST + NA_BLOB);
     tmp.d_etab = (float *)(base + NA_ETAB);
-    tmp.d_reps = (RepDev *)(base + NA_REPS);
-    tmp.d_status = (int *)(base + NA_STATUS);
+    NaParams *d_P = (NaParams *)(base + NA_HOST);
+    tmp.d_reps = &d_P->R;
     double *d_eout = (double *)(base + NA_EOUT);
-#define NA_CP(dst, src, bytes)                                                                       \
-    if (cudaMemcpyAsync((dst), (src), (bytes), cudaMemcpyHostToDevice, stream) != cudaSuccess)      \
+    std::vector<unsigned char> host(NA_BLOB + sizeof(int4) * blob.size());
+    memcpy(host.data(), &P, sizeof(P));
+    memcpy(host.data() + NA_PLANES, tmp.planes.data(), sizeof(PlaneWork) * tmp.planes.size());
+    memcpy(host.data() + NA_COLS, tmp.cols.data(), sizeof(ColWork) * tmp.cols.size());
+    memcpy(host.data() + NA_BLOB, blob.data(), sizeof(int4) * blob.size());
+    // (pageable memory: copied out before the call returns)
+    if (cudaMemcpyAsync(d_P, host.data(), host.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess)
         return MOIL_NB_ERR_CUDA;
-    NA_CP(tmp.d_reps, &R, sizeof(R));
-    NA_CP(tmp.d_plans, plans, sizeof(plans));
-    NA_CP(tmp.d_rep_plan, rep_plan, sizeof(rep_plan));
-    NA_CP(tmp.d_tw, tw, sizeof(float2) * ntw);
-    NA_CP(tmp.d_tab, tab.data(), sizeof(int2) * tab.size());
-    NA_CP(tmp.d_bsp, bsp, sizeof(float) * (n1 + n2 + n3));
-    NA_CP(tmp.d_etab, etab, sizeof(float) * (n1 + n2 + n3));
-    NA_CP(tmp.d_planes, tmp.planes.data(), sizeof(PlaneWork) * tmp.planes.size());
-    NA_CP(tmp.d_cols, tmp.cols.data(), sizeof(ColWork) * tmp.cols.size());
-    NA_CP(tmp.d_col_begin, col_begin, sizeof(col_begin));
-#undef NA_CP
-    k_na_load<<<(natom + 255) / 256, 256, 0, stream>>>(natom, tmp.d_reps, d_coor, d_q, (float4 *)tmp.d_fr, tmp.d_zidx,
-                                                       tmp.d_site_rep);
-    k_na_scale<<<1, 256, 0, stream>>>(natom, d_q, tmp.d_reps);
+    const int nb = (natom + 255) / 256 + 1;      // the last block: tables, energy
+    k_na_load<<<nb, 256, 0, stream>>>(natom, d_P, d_coor, d_q, (float4 *)tmp.d_fr, tmp.d_zidx, tmp.d_site_rep, tmp.d_etab);
     pme_t<float>(&tmp);
-    k_na_grad<<<(natom + 255) / 256, 256, 0, stream>>>(natom, tmp.d_reps, d_q, (const float *)tmp.d_part, d_dpot);
-    k_na_energy<<<1, 256, 0, stream>>>((int)tmp.cols.size(), tmp.d_e_col, d_eout);
+    k_na_grad<<<nb, 256, 0, stream>>>(natom, tmp.d_reps, d_q, (const float *)tmp.d_part, d_dpot, (int)tmp.cols.size(),
+                                      tmp.d_e_col, d_eout);
     // a launch that failed is reported before waiting for the stream (the error stays pending
     // for the caller to read)
     if (cudaPeekAtLastError() != cudaSuccess) return MOIL_NB_ERR_CUDA;
