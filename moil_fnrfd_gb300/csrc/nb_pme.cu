@@ -324,16 +324,26 @@ __host__ __device__ __forceinline__ int swz(int e) { return e + (e >> 4); }
 // float2 slots that hold m elements in the spread layout
 __host__ __device__ __forceinline__ int swz_elems(int m) { return m + (m >> 4) + 1; }
 
-// One Stockham stage over L lines of length n.  Source line l at src + l*ss (contiguous),
-// or in the spread layout (SW_IN).  Destination: MODE 0 natural (dst + l*ds, spread if
-// SW_OUT), MODE 1 transposed (dst[k*ds + l] for k < keep), MODE 2 real part natural
-// (rdst + l*ds).  CONJ_OUT conjugates the stored values.  tab / tw point into shared memory
-// (fft_ctx_load).
-template <int RADIX, int MODE, bool CONJ_OUT, bool SW_IN, bool SW_OUT>
-__device__ __forceinline__ void fft_pass_r(const float2 *__restrict__ src, float2 *__restrict__ dst,
-                                           float *__restrict__ rdst, int L, int ss, int ds, int keep,
-                                           int Ns, int nb, unsigned magic, const int2 *__restrict__ tab,
-                                           const float2 *__restrict__ tw)
+// Where a transform's first stage reads and its last one writes, besides the shared-memory buffers
+enum FftIn { IN_LINES, IN_SPREAD, IN_CONJ, IN_PLANE };
+enum FftOut { OUT_LINES, OUT_SPREAD, OUT_TRANSPOSED, OUT_ROWS };
+struct FftEnds {
+    const float2 *in = nullptr;   // IN_CONJ: lines in global memory, conjugated
+    const int *acc = nullptr;     // IN_PLANE: the int32 charge plane, rows 2l and 2l + 1 as line l
+    float inv = 0.f;
+    int rows = 0;                 // rows of the plane (IN_PLANE, OUT_ROWS)
+    float2 *out = nullptr;        // OUT_LINES: to global memory
+    float *real = nullptr;        // OUT_ROWS: Re and -Im of line l as rows 2l and 2l + 1, in global memory
+};
+
+// One Stockham stage over L lines of length n = RADIX * nb.  Source line l at src + l*ss (contiguous)
+// or in the spread layout (IN_SPREAD); destination dst + l*ds, in the spread layout (OUT_SPREAD) or
+// transposed (dst[k*ds + l]); or the ends above.  CONJ_OUT conjugates the stored values.  tab / tw
+// point into shared memory (fft_ctx_load).
+template <int RADIX, int IN, int OUT, bool CONJ_OUT>
+__device__ __forceinline__ void fft_pass_r(const float2 *__restrict__ src, float2 *__restrict__ dst, const FftEnds &E,
+                                           int L, int ss, int ds, int Ns, int nb, unsigned magic,
+                                           const int2 *__restrict__ tab, const float2 *__restrict__ tw)
 {
     const int total = L * nb;
     for (int b = threadIdx.x; b < total; b += blockDim.x) {
@@ -342,44 +352,53 @@ __device__ __forceinline__ void fft_pass_r(const float2 *__restrict__ src, float
         int2 e = tab[j];
         const int s0 = line * ss + j;
         float2 v[RADIX];
+        if (IN == IN_PLANE) {
+            const int *a0 = E.acc + 2 * line * ss + j, *a1 = a0 + ss;
+            const bool two = 2 * line + 1 < E.rows;
 #pragma unroll
-        for (int r = 0; r < RADIX; ++r) v[r] = src[SW_IN ? swz(s0 + r * nb) : s0 + r * nb];
+            for (int r = 0; r < RADIX; ++r)
+                v[r] = make_float2(Acc<float>::get(a0[r * nb], E.inv), two ? Acc<float>::get(a1[r * nb], E.inv) : 0.f);
+        } else {
 #pragma unroll
-        for (int r = 1; r < RADIX; ++r) v[r] = cmul(v[r], tw[r * e.x]);
+            for (int r = 0; r < RADIX; ++r)
+                v[r] = IN == IN_CONJ ? cconj(E.in[s0 + r * nb]) : src[IN == IN_SPREAD ? swz(s0 + r * nb) : s0 + r * nb];
+        }
+        if (IN == IN_SPREAD) {          // (a first stage's twiddles are all one)
+#pragma unroll
+            for (int r = 1; r < RADIX; ++r) v[r] = cmul(v[r], tw[r * e.x]);
+        }
         bfly<RADIX>(v);
 #pragma unroll
         for (int r = 0; r < RADIX; ++r) {
             float2 o = CONJ_OUT ? cconj(v[r]) : v[r];
             int k = e.y + r * Ns;
-            if (MODE == 0) { const int d = line * ds + k; dst[SW_OUT ? swz(d) : d] = o; }
-            else if (MODE == 1) { if (k < keep) dst[k * ds + line] = o; }
-            else rdst[line * ds + k] = o.x;
+            if (OUT == OUT_TRANSPOSED) {
+                dst[k * ds + line] = o;
+            } else if (OUT == OUT_ROWS) {
+                E.real[2 * line * ds + k] = o.x;
+                if (2 * line + 1 < E.rows) E.real[(2 * line + 1) * ds + k] = -o.y;
+            } else {
+                const int d = line * ds + k;
+                dst[OUT == OUT_SPREAD ? swz(d) : d] = o;
+            }
         }
     }
     __syncthreads();
 }
 
-// WIDE: the radix set of a wide plan (2..10); otherwise 2, 3, 4, 5 only, so the kernel keeps
-// the register count of the small butterflies
-template <int MODE, bool CONJ_OUT, bool SW_IN, bool SW_OUT, bool WIDE>
-__device__ __forceinline__ void fft_pass(int R, const float2 *src, float2 *dst, float *rdst, int L, int ss, int ds,
-                                         int keep, int Ns, int nb, unsigned magic, const int2 *tab, const float2 *tw)
+template <int IN, int OUT, bool CONJ_OUT>
+__device__ __forceinline__ void fft_pass(int R, const float2 *src, float2 *dst, const FftEnds &E, int L, int ss, int ds,
+                                         int Ns, int nb, unsigned magic, const int2 *tab, const float2 *tw)
 {
     switch (R) {
-    case 4: fft_pass_r<4, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-    case 2: fft_pass_r<2, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-    case 3: fft_pass_r<3, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-    case 5: fft_pass_r<5, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-    default:
-        if constexpr (WIDE) {
-            switch (R) {
-            case 6: fft_pass_r<6, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-            case 8: fft_pass_r<8, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-            case 9: fft_pass_r<9, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-            default: fft_pass_r<10, MODE, CONJ_OUT, SW_IN, SW_OUT>(src, dst, rdst, L, ss, ds, keep, Ns, nb, magic, tab, tw); break;
-            }
-        }
-        break;
+    case 2: fft_pass_r<2, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
+    case 3: fft_pass_r<3, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
+    case 4: fft_pass_r<4, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
+    case 5: fft_pass_r<5, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
+    case 6: fft_pass_r<6, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
+    case 8: fft_pass_r<8, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
+    case 9: fft_pass_r<9, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
+    default: fft_pass_r<10, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
     }
 }
 
@@ -417,32 +436,28 @@ __device__ __forceinline__ unsigned char *fft_ctx_load(unsigned char *dst, const
     return dst + 16 * (size_t)len;
 }
 
-// Full forward FFT of L lines of length n held in a (line stride in_ss); b is scratch.  The
-// last pass is stored in the mode given with stride out_ds (MODE 1: the transposed row
-// stride); the stages between keep the spread layout.  Returns the buffer holding the
-// result; CONJ_LAST conjugates the final output (second half of an inverse transform).
-template <int LAST_MODE, bool CONJ_LAST, bool WIDE = false>
-__device__ float2 *fft_lines(const FftCtx &c, float2 *a, float2 *b, float *rdst, int L, int keep, int in_ss,
-                             int out_ds)
+// Full forward FFT of L lines of length n held in a (line stride in_ss), or read as IN says; b is
+// scratch.  The last pass stores as OUT says with stride out_ds (OUT_TRANSPOSED: the transposed row
+// stride); the stages between keep the spread layout.  Returns the buffer holding the result;
+// CONJ_LAST conjugates the final output (second half of an inverse transform).
+template <int IN, int OUT, bool CONJ_LAST>
+__device__ float2 *fft_lines(const FftCtx &c, float2 *a, float2 *b, const FftEnds &E, int L, int in_ss, int out_ds)
 {
     const FftPlanDev &p = *c.p;
     float2 *src = a, *dst = b;
     const int n = p.n, nst = p.nst;
     for (int s = 0; s < nst; ++s) {
         const int2 *t = c.tab + p.off[s];
+        float2 *o = s + 1 == nst && E.out ? E.out : dst;
         if (s + 1 < nst) {
             if (s == 0)
-                fft_pass<0, false, false, true, WIDE>(p.rad[s], src, dst, nullptr, L, in_ss, n, 0, p.ns[s], p.nb[s],
-                                                p.magic[s], t, c.tw);
+                fft_pass<IN, OUT_SPREAD, false>(p.rad[s], src, o, E, L, in_ss, n, p.ns[s], p.nb[s], p.magic[s], t, c.tw);
             else
-                fft_pass<0, false, true, true, WIDE>(p.rad[s], src, dst, nullptr, L, n, n, 0, p.ns[s], p.nb[s], p.magic[s],
-                                               t, c.tw);
+                fft_pass<IN_SPREAD, OUT_SPREAD, false>(p.rad[s], src, o, E, L, n, n, p.ns[s], p.nb[s], p.magic[s], t, c.tw);
         } else if (s == 0) {
-            fft_pass<LAST_MODE, CONJ_LAST, false, false, WIDE>(p.rad[s], src, dst, rdst, L, in_ss, out_ds, keep, p.ns[s],
-                                                         p.nb[s], p.magic[s], t, c.tw);
+            fft_pass<IN, OUT, CONJ_LAST>(p.rad[s], src, o, E, L, in_ss, out_ds, p.ns[s], p.nb[s], p.magic[s], t, c.tw);
         } else {
-            fft_pass<LAST_MODE, CONJ_LAST, true, false, WIDE>(p.rad[s], src, dst, rdst, L, n, out_ds, keep, p.ns[s],
-                                                        p.nb[s], p.magic[s], t, c.tw);
+            fft_pass<IN_SPREAD, OUT, CONJ_LAST>(p.rad[s], src, o, E, L, n, out_ds, p.ns[s], p.nb[s], p.magic[s], t, c.tw);
         }
         float2 *x = src; src = dst; dst = x;
     }
@@ -470,6 +485,11 @@ __host__ __device__ __forceinline__ int zconv_buf_elems(int n3)
     return ((a > b ? a : b) + 1) & ~1;
 }
 
+// Charge plane z: the sites' stencils into an int32 plane, then the x and y transforms.  Bound: instruction
+// issue and the shared-memory pipe; of 180 us for 9,535 planes of about 37 x 37 (256 replicas) the
+// transforms take 65, the selection of the sites 48, their stencils 42.  Two passes per axis (wide
+// radices), the first from the int32 plane and the last to the grid, without a staging copy at either
+// end: 512 replicas 1981 -> 1939 us per evaluation with the inverse's, 24 images 94.5 -> 90.6.
 __global__ void __launch_bounds__(256, 8) k_plane_fwd_f(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
                                                      const int4 *__restrict__ blob,
                                                      int nW, const unsigned char *__restrict__ zidx,
@@ -492,16 +512,10 @@ __global__ void __launch_bounds__(256, 8) k_plane_fwd_f(const PlaneWork *__restr
     async_wait();
     __syncthreads();
     // x transform of real rows two at a time: line p carries row 2p as its real part and
-    // row 2p+1 as its imaginary part
-    const float inv = R.spread_inv;
-    for (int p = warp; p < n2p; p += nwarp)
-        for (int x = lane; x < n1; x += 32) {
-            const float re = Acc<float>::get(acc[2 * p * n1 + x], inv);
-            const float im = 2 * p + 1 < n2 ? Acc<float>::get(acc[(2 * p + 1) * n1 + x], inv) : 0.f;
-            B1[p * n1 + x] = make_float2(re, im);
-        }
-    __syncthreads();
-    float2 *Z = fft_lines<0, false>(c1, B1, B0, nullptr, n2p, 0, n1, n1);
+    // row 2p+1 as its imaginary part, read from the int32 plane
+    FftEnds ex, ey;
+    ex.acc = acc; ex.inv = R.spread_inv; ex.rows = n2;
+    float2 *Z = fft_lines<IN_PLANE, OUT_LINES, false>(c1, B0, B1, ex, n2p, n1, n1);
     float2 *T = Z == B1 ? B0 : B1;
     // separate the two real transforms (X_2p = (Z_k + conj Z_-k)/2, X_2p+1 = -i (Z_k - conj Z_-k)/2)
     // and keep kx < n1h, transposed to [kx][y] lines of n2 at the odd row stride sT (the lanes'
@@ -514,10 +528,9 @@ __global__ void __launch_bounds__(256, 8) k_plane_fwd_f(const PlaneWork *__restr
             if (2 * p + 1 < n2) T[k * sT + 2 * p + 1] = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
         }
     __syncthreads();
-    // y: n1h lines of n2
-    float2 *Y = fft_lines<0, false>(c2, T, Z, nullptr, n1h, 0, sT, n2);
-    float2 *g = grid + w.g0 + (size_t)w.z * n1h * n2;
-    for (int k = threadIdx.x; k < n1h * n2; k += blockDim.x) g[k] = Y[k];
+    // y: n1h lines of n2, to the grid
+    ey.out = grid + w.g0 + (size_t)w.z * n1h * n2;
+    fft_lines<IN_LINES, OUT_LINES, false>(c2, T, Z, ey, n1h, sT, n2);
 }
 
 __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
@@ -543,7 +556,7 @@ __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ 
         if (lane < tk) async_copy8(A + lane * sA + kz, g + kz * zs + lane);
     async_wait();
     __syncthreads();
-    float2 *F = fft_lines<0, false, true>(c3, A, B, nullptr, tk, 0, sA, n3);
+    float2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds(), tk, sA, n3);
     float2 *Fo = F == A ? B : A;
     const float wgt = (w.kx == 0 || 2 * w.kx == n1) ? 1.f : 2.f;
     // influence function exp(-pi^2 m^2 / alpha^2) / (pi V B(m) m^2): the exponential and the
@@ -577,7 +590,7 @@ __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ 
         }
     }
     __syncthreads();
-    float2 *I = fft_lines<0, true, true>(c3, F, Fo, nullptr, tk, 0, n3, sA);
+    float2 *I = fft_lines<IN_LINES, OUT_LINES, true>(c3, F, Fo, FftEnds(), tk, n3, sA);
     for (int kz = warp; kz < n3; kz += 8)
         if (lane < tk) g[kz * zs + lane] = I[lane * sA + kz];
     // fixed-order reduction: each thread's few terms in FP32, then FP64 across the warp and
@@ -621,7 +634,7 @@ __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict_
         if (lane < tk) async_copy8(A + lane * sA + kz, g + kz * zs + lane);
     async_wait();
     __syncthreads();
-    const float2 *F = fft_lines<0, false, true>(c3, A, B, nullptr, tk, 0, sA, n3);
+    const float2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds(), tk, sA, n3);
     const float wgt = (w.kx == 0 || 2 * w.kx == n1) ? 1.f : 2.f;
     const float fac2 = R.pme_fac2f, pivol = R.pivolf, fac = (float)R.pme_fac;
     const int nf2 = (n2 + 1) / 2, nf3 = (n3 + 1) / 2;
@@ -661,7 +674,9 @@ __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict_
 
 // inverse y and x transforms of plane z; the real potential plane (n1 x n2 floats) is stored
 // over the plane's own complex storage, which this block alone reads, for k_pme_gather_f
-__global__ void __launch_bounds__(256) k_plane_inv_f(const PlaneWork *__restrict__ work,
+// Inverse y and x transforms of plane z (the comment above): the first pass reads the grid and the last
+// one stores the real rows.
+__global__ void __launch_bounds__(256, 8) k_plane_inv_f(const PlaneWork *__restrict__ work,
                                                      const int4 *__restrict__ blob,
                                                      float2 *__restrict__ grid)
 {
@@ -675,16 +690,14 @@ __global__ void __launch_bounds__(256) k_plane_inv_f(const PlaneWork *__restrict
     ctx = fft_ctx_load(ctx, blob + w.bx, w.lx, n1, c1);
     fft_ctx_load(ctx, blob + w.by, w.ly, n2, c2);
     float2 *g = grid + w.g0 + (size_t)w.z * n1h * n2;
-    // [kx][ky] lines of n2, conjugated (inverse through the forward transform)
-    for (int k = threadIdx.x; k < n1h * n2; k += blockDim.x) B0[k] = cconj(g[k]);
     async_wait();
     __syncthreads();
-    // y: n1h lines; last pass conjugates back and stores transposed to H[ky][kx] at the odd
-    // row stride hs
+    // y: n1h lines [kx][ky] of n2 from the grid, conjugated (inverse through the forward transform); the
+    // last pass conjugates back and stores transposed to H[ky][kx] at the odd row stride hs
     const int hs = n1h | 1;
-    fft_lines<1, true>(c2, B0, B1, nullptr, n1h, n2, n2, hs);
-    // which buffer got the transposed result depends on the pass count
-    float2 *H = (c2.p->nst & 1) ? B1 : B0;
+    FftEnds ey, ex;
+    ey.in = g;
+    float2 *H = fft_lines<IN_CONJ, OUT_TRANSPOSED, true>(c2, B1, B0, ey, n1h, n2, hs);
     float2 *Zc = H == B0 ? B1 : B0;
     // x inverse of two real rows at a time: Z = H_2p + i H_2p+1 over the full Hermitian line of
     // n1, conjugated so the forward transform inverts it; row 2p = Re, row 2p+1 = -Im of the result
@@ -698,15 +711,9 @@ __global__ void __launch_bounds__(256) k_plane_inv_f(const PlaneWork *__restrict
             Zc[p * n1 + k] = make_float2(a.x - b.y, -(a.y + b.x));
         }
     __syncthreads();
-    const float2 *W = fft_lines<0, false>(c1, Zc, H, nullptr, n2p, 0, n1, n1);
     // the real potential plane over the plane's own complex storage (this block alone reads it)
-    float *gr = (float *)g;
-    for (int p = warp; p < n2p; p += nwarp)
-        for (int x = lane; x < n1; x += 32) {
-            const float2 v = W[p * n1 + x];
-            gr[2 * p * n1 + x] = v.x;
-            if (2 * p + 1 < n2) gr[(2 * p + 1) * n1 + x] = -v.y;
-        }
+    ex.real = (float *)g; ex.rows = n2;
+    fft_lines<IN_LINES, OUT_ROWS, false>(c1, Zc, H, ex, n2p, n1, n1);
 }
 
 // PME gradient of each site from the real potential grid (grad_sum,
@@ -1101,25 +1108,29 @@ void pme_t(NbCtx *c)
 }
 
 // radix plan and Stockham tables; returns 0 if n is not 2/3/5-smooth or too long.  Narrow
-// plans (the plane kernels and the FP64 one-warp-per-line transform) take 4s first, then 2, 3,
-// 5.  Wide plans (the FP32 z columns) also have the composite codelets 6, 8, 9, 10 and take
-// the fewest passes (a line of up to 100 points in two), larger radices first on ties.  tab
+// plans (the FP64 one-warp-per-line transform) take 4s first, then 2, 3, 5.  Wide plans (FP32)
+// also have the composite codelets 6, 8, 9, 10 and take the fewest passes (a line of up to 100
+// points in two), the most even split on ties.  tab
 // receives (twiddle step, destination index) per butterfly.
-// fewest factors of m from the wide radix set, at most `left` of them (-1: none)
+// fewest factors of m from the wide radix set, at most `left` of them, and of those the smallest sum
+// (the most even split: the longest butterfly sets the time of a pass); its count, -1 if none
 int wide_factors(int m, int left, int *out)
 {
     static const int R[8] = {10, 9, 8, 6, 5, 4, 3, 2};
     if (m == 1) return 0;
     if (left == 0) return -1;
-    int best = -1, tmp[8];
+    int best = -1, sum = 0, tmp[8];
     for (int k = 0; k < 8; ++k) {
         if (m % R[k]) continue;
-        const int f = wide_factors(m / R[k], best < 0 ? left - 1 : best - 2, tmp);
+        const int f = wide_factors(m / R[k], best < 0 ? left - 1 : best - 1, tmp);
         if (f < 0) continue;
+        int s = R[k];
+        for (int q = 0; q < f; ++q) s += tmp[q];
+        if (best >= 0 && f + 1 == best && s >= sum) continue;
         best = f + 1;
+        sum = s;
         out[0] = R[k];
         for (int q = 0; q < f; ++q) out[1 + q] = tmp[q];
-        if (best == 1) break;
     }
     return best;
 }
@@ -1172,7 +1183,7 @@ size_t fft_ctx_bytes(int n, bool wide)
 template <typename T>
 size_t plane_fwd_smem(int n1, int n2)
 {
-    if (sizeof(T) == 4) return (size_t)2 * plane_buf_elems(n1, n2) * sizeof(float2) + fft_ctx_bytes(n1, false) + fft_ctx_bytes(n2, false);
+    if (sizeof(T) == 4) return (size_t)2 * plane_buf_elems(n1, n2) * sizeof(float2) + fft_ctx_bytes(n1, true) + fft_ctx_bytes(n2, true);
     typedef typename cplx<T>::type C;
     size_t acc = (sizeof(typename Acc<T>::type) * n1 * n2 + 15) & ~(size_t)15;
     return acc + sizeof(C) * n2 * ((n1 / 2 + 1) | 1) + sizeof(C) * 8 * 2 * NB_MAX_FFT;
@@ -1180,7 +1191,7 @@ size_t plane_fwd_smem(int n1, int n2)
 template <typename T>
 size_t plane_inv_smem(int n1, int n2)
 {
-    if (sizeof(T) == 4) return (size_t)2 * plane_buf_elems(n1, n2) * sizeof(float2) + fft_ctx_bytes(n1, false) + fft_ctx_bytes(n2, false);
+    if (sizeof(T) == 4) return (size_t)2 * plane_buf_elems(n1, n2) * sizeof(float2) + fft_ctx_bytes(n1, true) + fft_ctx_bytes(n2, true);
     typedef typename cplx<T>::type C;
     size_t r = (sizeof(T) * n1 * n2 + 15) & ~(size_t)15;
     return r + sizeof(C) * n2 * ((n1 / 2 + 1) | 1) + sizeof(C) * 8 * 2 * NB_MAX_FFT;
@@ -1269,7 +1280,7 @@ int configure_t(NbCtx *c)
     for (int r = 0; r < c->nrep; ++r) {
         int ns[3] = {c->rd[r].n1, c->rd[r].n2, c->rd[r].n3};
         for (int d = 0; d < 3; ++d) {
-            const bool wide = sizeof(T) == 4 && d == 2;
+            const bool wide = sizeof(T) == 4;
             int found = -1;
             for (size_t k = 0; k < c->plans.size(); ++k)
                 if (c->plans[k].n == ns[d] && (bool)wide_of[k] == wide) found = (int)k;
@@ -1643,7 +1654,7 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
         FftPlanDev plan;
         std::vector<int2> tab;
         std::vector<float2> tw(grid[d]);
-        make_plan(grid[d], &plan, &tab, d == 2);     // the z columns take the wide radix set
+        make_plan(grid[d], &plan, &tab, true);
         for (int t = 0; t < grid[d]; ++t) {
             const double ang = -2.0 * M_PI * (double)t / (double)grid[d];
             tw[t] = make_float2((float)cos(ang), (float)sin(ang));

@@ -29,6 +29,19 @@ def test_small_and_long_planes(cfg0, grid, precision):
     nb.close()
 
 
+@pytest.mark.parametrize("grid", [(10, 9, 8), (27, 50, 36), (96, 20, 6), (6, 75, 45), (40, 25, 24)])
+def test_transform_lengths(cfg0, grid):
+    """Lines of one, two and three passes along each axis, radices 2 to 10."""
+    s = cfg0.copy()
+    s.nfft = grid
+    ref, eref = O.eforce(s, mode="parity")
+    nb = Nonbonded(s)
+    dpot, e = nb.eforce(s.coor)
+    assert rel_rms(dpot, ref) <= 1e-5
+    assert abs(e["e_ew_receip"] - eref["e_ew_receip"]) <= 1e-5 * abs(eref["e_ew_receip"])
+    nb.close()
+
+
 @pytest.mark.parametrize("natom", [1, 255, 16384, 16401, 33001])
 def test_sites_past_one_round(natom):
     """The allocation-free sum on natom random charges (a block tests 16,384 sites per round)."""
