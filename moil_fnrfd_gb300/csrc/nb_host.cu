@@ -173,11 +173,17 @@ template <typename V> int upload(NbCtx *c, V *&dst, const std::vector<V> &src)
 
 // Water-water rows by all-pairs tiles (k_wlist_tiled) or by cell search (k_wlist).  By
 // default the tiles take replicas where the 27-cell stencil already covers at least 40% of
-// the box (2-4 cells per side); moil_nb_set_shape can switch them off or on everywhere.
+// the box (2-4 cells per side), in handles of many waters: a tile block runs through its whole
+// replica, and the search's warp per water is faster until such blocks fill the GPU.  Rebuild in us by
+// tiles / by search: 1,334 waters 149 / 71, 4,000 235 / 79, 24 replicas of 800 134 / 119, 16 of 500-
+// 4,000 (28,900 waters) 279 / 281, 48 (82,500) 362 / 633, 512 2547 / 5578.  moil_nb_set_shape can
+// switch them off or on everywhere.
+#define NB_TILED_MIN_WATERS 28672
 int tiled_choice(const NbCtx *c, const RepDev &R)
 {
     if (R.nwat <= 0 || R.nwat > 16384 || c->want_tiled == MOIL_NB_TILED_OFF) return 0;
     if (c->want_tiled == MOIL_NB_TILED_ALL) return 1;
+    if (c->nw_handle <= NB_TILED_MIN_WATERS) return 0;
     double frac = 1.0;
     for (int d = 0; d < 3; ++d) frac *= (double)std::min(R.nc[d], 3) / R.nc[d];
     return frac >= 0.4 ? 1 : 0;
@@ -493,7 +499,6 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
         }
         R.nwat = nwat; R.noth = noth;
         wat0 += nwat; oth0 += noth;
-        R.wtiled = tiled_choice(c, R);
         for (int i = 0; i < t->npt; ++i) {
             q.push_back(t->ptchg[i]);
             lj_e12.push_back(t->epsgm12[i]);
@@ -532,6 +537,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     c->nW = wat0;
     c->nA = oth0;
     c->nw_handle = std::max(c->nw_handle, c->nW);
+    for (RepDev &R : c->rd) R.wtiled = tiled_choice(c, R);
     c->na_handle = std::max(c->na_handle, c->nA);
     c->row16 = 1;
     for (int r = 0; r < nrep; ++r) c->row16 &= c->rd[r].nwat < 65536;
