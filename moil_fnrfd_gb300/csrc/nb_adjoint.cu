@@ -765,11 +765,11 @@ int nb_adjoint(NbCtx *c, double *out, double *out2)
     const bool fast = c->water_excl_fast && c->nW > 0;
     const int64_t n = fast ? c->nA : na;
     if (n > 0)
-        k_adj_excl14<<<(int)((n * ADJ_EX_LANES + B - 1) / B), B, 0, s2>>>(
+        k_adj_excl14<<<(int)((n * ADJ_EX_LANES + 31) / 32), 32, 0, s2>>>(
             (int)n, fast ? c->d_unit_atom + c->nW : nullptr, c->d_atom_rep, c->d_reps, c->d_coor, c->d_q, c->d_lj_d,
             c->d_ex_off, c->d_ex_j, c->d_p14_off, c->d_p14_j, c->d_p14_par, x, x + na, x + 2 * na);
     if (fast)
-        k_adj_excl_water<<<(int)((c->nW + B - 1) / B), B, 0, s2>>>((int)c->nW, c->d_unit_atom, c->d_atom_rep, c->d_reps,
+        k_adj_excl_water<<<(int)((c->nW + 31) / 32), 32, 0, s2>>>((int)c->nW, c->d_unit_atom, c->d_atom_rep, c->d_reps,
                                                                   c->d_coor, c->d_q, x);
     if (c->precision == MOIL_NB_FP64) {
         nb_launch_pme_potential(c, c->d_adj_phi);

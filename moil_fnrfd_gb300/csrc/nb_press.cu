@@ -480,7 +480,7 @@ void pressure_t(NbCtx *c, const double *d_coor, double *d_out)
     nb_launch_pme_virial(c, pme, c->d_press_grid, c->d_press_col);
     cudaEventRecord(c->ev_join, pme);
     if (c->nmol > 0)
-        k_press_xrel<T><<<(c->nmol + B - 1) / B, B, 0, s>>>(c->nmol, c->d_mol_off, c->d_mol_atom, c->d_atom_rep, c->d_reps,
+        k_press_xrel<T><<<(c->nmol + 31) / 32, 32, 0, s>>>(c->nmol, c->d_mol_off, c->d_mol_atom, c->d_atom_rep, c->d_reps,
                                                            d_coor, c->d_mass, c->d_site_of, c->d_xrel, c->d_xsite);
     if (c->nW > 0) {
         const int wpb = PW_BLOCK / PW_LANES;
