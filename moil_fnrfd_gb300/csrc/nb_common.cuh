@@ -314,3 +314,4 @@ __host__ __device__ __forceinline__ int nb_half_owner(int a, int b)
 #define NB_DEV_ERR_NAN 2
 #define NB_DEV_ERR_BIGFORCE 4
 #define NB_DEV_ERR_RWAT 8
+#define NB_DEV_STALE 16         // an MD step whose rebuild was not foreseen (EVAL_KEEP)

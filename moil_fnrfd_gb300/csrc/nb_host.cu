@@ -81,8 +81,10 @@ void drop_graph(NbCtx *c)
         if (g.exec) cudaGraphExecDestroy(g.exec);
         g.exec = nullptr;
     }
-    if (c->gexec_md) cudaGraphExecDestroy(c->gexec_md);
-    c->gexec_md = nullptr;
+    for (cudaGraphExec_t &g : c->gexec_md) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
 }
 
 void release_device(NbCtx *c)
@@ -792,7 +794,7 @@ void enqueue_core(NbCtx *c, const double *d_coor, double *d_dpot, EvalMode mode,
         cudaStreamWaitEvent(s, c->ev_join, 0);
         if (third) cudaStreamWaitEvent(s, c->ev_join3, 0);
     }
-    nb_launch_finalize(c, d_dpot, ctl);
+    nb_launch_finalize(c, d_dpot, ctl, mode);
 }
 
 void enqueue_eval(NbCtx *c, const double *d_coor, double *d_dpot, EvalMode mode)
@@ -807,15 +809,15 @@ void enqueue_eval(NbCtx *c, const double *d_coor, double *d_dpot, EvalMode mode)
 }
 
 // one whole MD step of a context, as captured into its step graph: the evaluation, whose last
-// kernel keeps the error bits and sets the next step's rebuild request, and the leapfrog + SETTLE
-// integrator.  After an error the coordinate preparation of the remaining steps returns at
-// once, so no list is rebuilt from what those steps move (the call is then redone from its
-// starting state).
+// kernel keeps the error bits and (EVAL_DEVICE) sets the next step's rebuild request, and the
+// leapfrog + SETTLE integrator.  After an error the coordinate preparation of the remaining steps
+// returns at once; the call is then redone from its starting state.
 void enqueue_md_step(NbCtx *c, double *coor, double *vel, const double *mass, double *dpot, double dt, double doh,
-                     double dhh)
+                     double dhh, EvalMode mode)
 {
     c->launches = 0;
-    enqueue_core(c, coor, dpot, EVAL_DEVICE, c->d_mdctl);
+    if (mode == EVAL_BUILD) cudaMemsetAsync(c->d_status, 1, 1, c->stream);
+    enqueue_core(c, coor, dpot, mode, c->d_mdctl);
     nb_launch_integrate(c, c->stream, coor, vel, mass, dpot, dt, doh, dhh);
 }
 
@@ -1728,44 +1730,57 @@ void eforce_nb_press_gpu_(const int *npt, const double *coor, double *dpot, doub
 // ---- device-side MD step loop (moil_nb_md_step) -----------------------------------------
 void read_energies_of(NbCtx *c, moil_energies *e) { read_energies(c, e); }
 
+// Replays nsteps step graphs without waiting for any.  host: the lists are rebuilt every list_period
+// steps, in steps that the host knows beforehand, and a step of the others that finds a site moved
+// too far ends the loop with NB_DEV_STALE; otherwise each step carries the rebuild behind a
+// conditional node, which costs a step of 28,900 waters 12 us of 204 and one of 32,000 15 of 234.
 int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *dpot, double dt, double doh,
-               double dhh, int nsteps)
+               double dhh, int nsteps, bool host)
 {
     cudaStream_t s = c->stream;
     if (!c->d_mdctl) NB_CUDA_OK(c, cudaMalloc(&c->d_mdctl, sizeof(int) * 4));
     // the host's list schedule goes to the device once per call
+    const bool first = c->need_rebuild || (c->list_period > 0 && c->evals_since_build >= c->list_period);
     c->h_status[17] = c->evals_since_build;
     c->h_status[18] = c->h_status[19] = 0;
-    c->h_status[8] = c->need_rebuild || (c->list_period > 0 && c->evals_since_build >= c->list_period) ? 1 : 0;
+    c->h_status[8] = first && !host ? 1 : 0;
     for (int k = 9; k < 16; ++k) c->h_status[k] = 0;
     c->h_status[23] = 0;
     NB_CUDA_OK(c, cudaMemcpyAsync(c->d_mdctl, c->h_status + 17, sizeof(int) * 3, cudaMemcpyHostToDevice, s));
     NB_CUDA_OK(c, cudaMemcpyAsync(c->d_status, c->h_status + 8, sizeof(int) * 8, cudaMemcpyHostToDevice, s));
-    const bool same = c->gexec_md && c->gmd_key[0] == coor && c->gmd_key[1] == vel && c->gmd_key[2] == mass &&
-                      c->gmd_dt == dt && c->gmd_doh == doh && c->gmd_dhh == dhh && c->gmd_gen == c->list_gen &&
-                      c->gmd_dpot == dpot;
-    if (!same) {
-        if (c->gexec_md) cudaGraphExecDestroy(c->gexec_md);
-        c->gexec_md = nullptr;
-        cudaGraph_t g = nullptr;
-        NB_CUDA_OK(c, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        c->capturing = 1;
-        enqueue_md_step(c, coor, vel, mass, dpot, dt, doh, dhh);
-        c->capturing = 0;
-        cudaError_t e1 = cudaStreamEndCapture(s, &g);
-        cudaError_t e2 = e1 == cudaSuccess ? cudaGraphInstantiate(&c->gexec_md, g, cudaGraphInstantiateFlagUseNodePriority) : e1;
-        if (g) cudaGraphDestroy(g);
-        if (e2 != cudaSuccess) {
-            c->gexec_md = nullptr;
-            c->err = std::string("capturing the MD step graph: ") + cudaGetErrorString(e2);
-            return MOIL_NB_ERR_CUDA;
+    NbCtx::MdKey key;
+    key.coor = coor; key.vel = vel; key.mass = mass; key.dpot = dpot;
+    key.dt = dt; key.doh = doh; key.dhh = dhh;
+    key.gen = c->list_gen;
+    auto launch = [&](EvalMode mode) -> int {
+        cudaGraphExec_t &exec = c->gexec_md[mode];
+        if (!exec || !(c->gmd_key[mode] == key)) {
+            if (exec) cudaGraphExecDestroy(exec);
+            exec = nullptr;
+            cudaGraph_t g = nullptr;
+            NB_CUDA_OK(c, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+            c->capturing = 1;
+            enqueue_md_step(c, coor, vel, mass, dpot, dt, doh, dhh, mode);
+            c->capturing = 0;
+            cudaError_t e1 = cudaStreamEndCapture(s, &g);
+            cudaError_t e2 = e1 == cudaSuccess ? cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority) : e1;
+            if (g) cudaGraphDestroy(g);
+            if (e2 != cudaSuccess) {
+                exec = nullptr;
+                c->err = std::string("capturing the MD step graph: ") + cudaGetErrorString(e2);
+                return MOIL_NB_ERR_CUDA;
+            }
+            c->gmd_key[mode] = key;
         }
-        c->gmd_key[0] = coor; c->gmd_key[1] = vel; c->gmd_key[2] = mass;
-        c->gmd_dpot = dpot;
-        c->gmd_dt = dt; c->gmd_doh = doh; c->gmd_dhh = dhh;
-        c->gmd_gen = c->list_gen;
+        NB_CUDA_OK(c, cudaGraphLaunch(exec, s));
+        return MOIL_NB_OK;
+    };
+    bool build = first;
+    for (int k = 0, evals = c->evals_since_build; k < nsteps; ++k) {
+        NB_TRY(launch(!host ? EVAL_DEVICE : (build ? EVAL_BUILD : EVAL_KEEP)));
+        evals = build ? 1 : evals + 1;
+        build = evals >= c->list_period;
     }
-    for (int k = 0; k < nsteps; ++k) NB_CUDA_OK(c, cudaGraphLaunch(c->gexec_md, s));
     // the step control in one wait (the last step's status words and energies are on the host
     // already); the rebuild request it left for a step that does not come is withdrawn
     NB_CUDA_OK(c, cudaMemsetAsync(c->d_status, 0, sizeof(int) * 8, s));

@@ -168,11 +168,18 @@ struct NbCtx {
     // device-side MD step loop (moil_nb_md_step): one graph per context holds a whole step
     // (evaluation, then leapfrog + SETTLE); d_mdctl = {evaluations since the last rebuild,
     // rebuild requested, sticky error bits}, read back once per call
-    cudaGraphExec_t gexec_md = nullptr;
-    const void *gmd_key[3] = {nullptr, nullptr, nullptr};
-    double gmd_dt = 0.0, gmd_doh = 0.0, gmd_dhh = 0.0;
-    int gmd_gen = -1;
-    double *gmd_dpot = nullptr;
+    cudaGraphExec_t gexec_md[3] = {nullptr, nullptr, nullptr};    // by EvalMode
+    struct MdKey {
+        const void *coor = nullptr, *vel = nullptr, *mass = nullptr, *dpot = nullptr;
+        double dt = 0.0, doh = 0.0, dhh = 0.0;
+        int gen = -1;
+        bool operator==(const MdKey &o) const
+        {
+            return coor == o.coor && vel == o.vel && mass == o.mass && dpot == o.dpot && dt == o.dt && doh == o.doh &&
+                   dhh == o.dhh && gen == o.gen;
+        }
+    } gmd_key[3];
+    int md_wary = 0, md_backoff = 0;   // step loops left to the device's decision after a stale one
     int *d_mdctl = nullptr;
     double *d_md_save = nullptr;       // the call's starting coordinates and velocities (the
                                        // per-step path redoes the call from them after an error)
@@ -283,13 +290,13 @@ void nb_pme_fp32_consts(RepDev *R);
 // FP64 B-spline moduli
 void nb_pme_etab(const RepDev &R, const double *bsp, float *out);
 // finalize (nb_realspace.cu)
-void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl);   // ctl: as nb_launch_prepare
+void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl, EvalMode mode);   // ctl: as nb_launch_prepare
 // MD step loop (nb_md.cu / nb_host.cu): the integrator of one context, and the graph replay of
 // nsteps whole steps (no host wait)
 int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, const double *dpot,
                         double dt, double doh, double dhh);
 int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *dpot, double dt, double doh,
-               double dhh, int nsteps);
+               double dhh, int nsteps, bool host);
 // per-replica energies and pair count of the last completed evaluation (e may be NULL)
 void read_energies_of(NbCtx *c, moil_energies *e);
 // parameter derivatives after an evaluation of c->d_coor (nb_adjoint.cu): dq, de, ds one after another;

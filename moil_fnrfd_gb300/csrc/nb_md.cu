@@ -13,6 +13,7 @@
 // outside waters move unconstrained (this library holds no bonded terms).  FP64 throughout.
 // The trajectory writer follows dynamics/wdyncrd.f's binary branch: Fortran unformatted
 // sequential records (4-byte length before and after each record).
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
@@ -197,20 +198,26 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
     const double dhh = water_geom ? water_geom[1] : 2.0 * 0.9572 * sin(104.52 * M_PI / 360.0);
     const size_t n = (size_t)h->natom;
     if (!h->d_md_dpot) NB_CUDA_OK(h, cudaMalloc(&h->d_md_dpot, sizeof(double) * 3 * std::max<size_t>(n, 1)));
-    // Device-side loop: every context replays a graph of whole steps nsteps times with no host
-    // wait between them; the error bits are read once at the end.  Any error (a list overflow
-    // to regrow, a non-finite coordinate) sends the call back to the saved state and through
+    // Device-side loop: every context replays graphs of whole steps with no host wait between them;
+    // the error bits are read once at the end.  With a list period the host decides which steps
+    // rebuild, in runs of at most 64 steps; a run whose lists were outrun before their time goes back
+    // to its saved state and leaves the decision to the device, as do some of the next runs (twice
+    // as many after each such run, 64 at most).  Any other error (a list overflow to regrow, a
+    // non-finite coordinate) sends the run back to the saved state and the rest of the call through
     // the per-step path below, which handles it as a single evaluation does.
     int first = 0;
     const bool loop = nsteps > 1 && h->use_graph && !h->timing;
-    if (loop) {
-        if (!h->d_md_save) NB_CUDA_OK(h, cudaMalloc(&h->d_md_save, sizeof(double) * 6 * std::max<size_t>(n, 1)));
+    std::vector<NbCtx *> ctxs;
+    if (h->grp.empty()) ctxs.push_back(h);
+    else for (NbCtx *c : h->grp) ctxs.push_back(c);
+    if (loop && !h->d_md_save) NB_CUDA_OK(h, cudaMalloc(&h->d_md_save, sizeof(double) * 6 * std::max<size_t>(n, 1)));
+    while (loop && first < nsteps) {
+        const bool host = h->list_period > 0 && h->md_wary == 0;
+        const int run = host ? std::min(nsteps - first, 64) : nsteps - first;
+        if (h->md_wary > 0) --h->md_wary;
         NB_CUDA_OK(h, cudaMemcpyAsync(h->d_md_save, d_coor, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, h->stream));
         NB_CUDA_OK(h, cudaMemcpyAsync(h->d_md_save + 3 * n, d_vel, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice,
                                       h->stream));
-        std::vector<NbCtx *> ctxs;
-        if (h->grp.empty()) ctxs.push_back(h);
-        else for (NbCtx *c : h->grp) ctxs.push_back(c);
         int rc = MOIL_NB_OK;
         for (size_t g = 0; g < ctxs.size() && rc == MOIL_NB_OK; ++g) {
             NbCtx *c = ctxs[g];
@@ -219,8 +226,8 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
                 NB_CUDA_OK(h, cudaEventRecord(h->ev[11], h->stream));            // the snapshot copies
                 NB_CUDA_OK(h, cudaStreamWaitEvent(c->stream, h->ev[11], 0));
             }
-            rc = nb_md_loop(c, d_coor + 3 * a0, d_vel + 3 * a0, d_mass + a0, h->d_md_dpot + 3 * a0, dt, doh, dhh,
-                            nsteps);
+            rc = nb_md_loop(c, d_coor + 3 * a0, d_vel + 3 * a0, d_mass + a0, h->d_md_dpot + 3 * a0, dt, doh, dhh, run,
+                            host);
         }
         int err = 0;
         for (NbCtx *c : ctxs) {
@@ -236,23 +243,26 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
             }
         }
         if (rc == MOIL_NB_OK && !err) {
-            if (!h->grp.empty()) {
-                h->last_site_pairs = 0;
-                for (NbCtx *c : ctxs) h->last_site_pairs += c->last_site_pairs;
-            }
-            if (energies) {
-                for (size_t g = 0; g < ctxs.size(); ++g)
-                    read_energies_of(ctxs[g], energies + (h->grp.empty() ? 0 : h->grp_rep0[g]));
-            }
-            first = nsteps;
-        } else {
-            NB_CUDA_OK(h, cudaMemcpyAsync(d_coor, h->d_md_save, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice,
-                                          h->stream));
-            NB_CUDA_OK(h, cudaMemcpyAsync(d_vel, h->d_md_save + 3 * n, sizeof(double) * 3 * n,
-                                          cudaMemcpyDeviceToDevice, h->stream));
-            NB_CUDA_OK(h, cudaStreamSynchronize(h->stream));
-            for (NbCtx *c : ctxs) c->need_rebuild = 1;
-            if (rc != MOIL_NB_OK) cudaGetLastError();
+            first += run;
+            continue;
+        }
+        NB_CUDA_OK(h, cudaMemcpyAsync(d_coor, h->d_md_save, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, h->stream));
+        NB_CUDA_OK(h, cudaMemcpyAsync(d_vel, h->d_md_save + 3 * n, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice,
+                                      h->stream));
+        NB_CUDA_OK(h, cudaStreamSynchronize(h->stream));
+        for (NbCtx *c : ctxs) c->need_rebuild = 1;
+        if (rc != MOIL_NB_OK) cudaGetLastError();
+        if (rc != MOIL_NB_OK || err != NB_DEV_STALE) break;
+        h->md_wary = h->md_backoff = std::min(64, 2 * h->md_backoff + 2);
+    }
+    if (loop && first == nsteps) {
+        if (!h->grp.empty()) {
+            h->last_site_pairs = 0;
+            for (NbCtx *c : ctxs) h->last_site_pairs += c->last_site_pairs;
+        }
+        if (energies) {
+            for (size_t g = 0; g < ctxs.size(); ++g)
+                read_energies_of(ctxs[g], energies + (h->grp.empty() ? 0 : h->grp_rep0[g]));
         }
     }
     for (int step = first; step < nsteps; ++step) {

@@ -1278,7 +1278,9 @@ WaterHFn water_h_fn(int hb, bool vir)
 // (the kernels before this one are done with them), copied to the host's st_h and cleared
 // for the next evaluation; a non-finite gradient sets *nan_h.  done: finished chunks per replica
 // (zero between launches).  ctl: in an MD step, {evaluations since the last rebuild, -, sticky
-// error bits}: the step's outcome goes there, and st[0] becomes the next step's rebuild request.
+// error bits}: the step's outcome goes there, and st[0] becomes the next step's rebuild request where
+// the device decides on it (list_period > 0); list_period < 0: a step without a rebuild, whose lists a
+// site has outrun (st[0]).
 template <typename T>
 __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
     int nchunk, const EChunk *__restrict__ chunks, const int *__restrict__ chunk_begin,
@@ -1320,9 +1322,10 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
         if (ctl) {
             if (s[0]) ctl[0] = 0;
             ctl[0] += 1;
-            if (s[1]) atomicOr(&ctl[2], s[1]);
+            const int err = s[1] | (s[0] && list_period < 0 ? NB_DEV_STALE : 0);
+            if (err) atomicOr(&ctl[2], err);
             // (no rebuild after an error)
-            st[0] = list_period > 0 && ctl[0] >= list_period && (s[1] | ctl[2]) == 0 ? 1 : 0;
+            st[0] = list_period > 0 && ctl[0] >= list_period && (err | ctl[2]) == 0 ? 1 : 0;
         }
     }
 }
@@ -1497,14 +1500,15 @@ void nb_launch_excl14(NbCtx *c, const double *d_coor)
     }
 }
 
-void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl)
+void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl, EvalMode mode)
 {
+    const int period = mode == EVAL_DEVICE ? c->list_period : (mode == EVAL_KEEP ? -1 : 0);
     const int nchunk = (int)c->echunks.size(), nb = nchunk + (int)((c->natom + NB_FE_THREADS - 1) / NB_FE_THREADS);
     auto launch = [&](auto kernel, auto part, int nsw) {
         kernel<<<nb, NB_FE_THREADS, 0, c->stream>>>(
             nchunk, c->d_echunks, c->d_echunk_begin, c->d_e_unit, c->d_e_ex, c->d_e_col, c->d_epart, c->d_edone,
             c->h_e_rep, (int)c->natom, c->d_site_of, c->d_atom_rep, c->d_reps, c->d_grad_site, c->d_grad_ex, part,
-            c->d_q, nsw, d_dpot, c->d_status, c->h_status, c->h_status + 23, ctl, c->list_period);
+            c->d_q, nsw, d_dpot, c->d_status, c->h_status, c->h_status + 23, ctl, period);
     };
     if (c->precision == MOIL_NB_FP64) launch(k_finalize<double>, (const double *)c->d_part, 0);
     else launch(k_finalize<float>, (const float *)c->d_part, c->water_excl_fast ? (int)(3 * c->nW) : 0);
