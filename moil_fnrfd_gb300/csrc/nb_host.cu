@@ -93,7 +93,7 @@ void release_device(NbCtx *c)
     free_ptr(c->d_atom_rep); free_ptr(c->d_unit_atom); free_ptr(c->d_unit_rep); free_ptr(c->d_unit_key);
     free_ptr(c->d_unit_slot); free_ptr(c->d_bin_count); free_ptr(c->d_bin_start); free_ptr(c->d_sorted_unit);
     free_ptr(c->d_site_orig); free_ptr(c->d_site_of); free_ptr(c->d_site_rep); free_ptr(c->d_site_flags);
-    free_ptr(c->d_pos); free_ptr(c->d_posb); free_ptr(c->d_woff); free_ptr(c->d_site_lj); free_ptr(c->d_site_q);
+    free_ptr(c->d_pos); free_ptr(c->d_posb); free_ptr(c->d_opos); free_ptr(c->d_woff); free_ptr(c->d_site_lj); free_ptr(c->d_site_q);
     free_ptr(c->d_wl1_cnt); free_ptr(c->d_wl1); free_ptr(c->d_wl2_off); free_ptr(c->d_wl2); free_ptr(c->d_xl_off);
     free_ptr(c->d_xl); free_ptr(c->d_count_tmp); free_ptr(c->d_ex_off); free_ptr(c->d_ex_j); free_ptr(c->d_p14_off);
     free_ptr(c->d_p14_j); free_ptr(c->d_p14_par); free_ptr(c->d_grad_site); free_ptr(c->d_e_unit);
@@ -177,10 +177,10 @@ template <typename V> int upload(NbCtx *c, V *&dst, const std::vector<V> &src)
 // default the tiles take replicas where the 27-cell stencil already covers at least 40% of
 // the box (2-4 cells per side), in handles of many waters: a tile block runs through its whole
 // replica, and the search's warp per water is faster until such blocks fill the GPU.  Rebuild in us by
-// tiles / by search: 1,334 waters 149 / 71, 4,000 235 / 79, 24 replicas of 800 134 / 119, 16 of 500-
-// 4,000 (28,900 waters) 279 / 281, 48 (82,500) 362 / 633, 512 2547 / 5578.  moil_nb_set_shape can
+// tiles / by search: 1,334 waters 149 / 67, 4,000 235 / 74, 24 replicas of 800 134 / 107, 16 of 500-
+// 4,000 (28,900 waters) 277 / 233, 32 (42,300) 296 / 297, 48 (82,500) 362 / 496, 512 2550 / 4300.  moil_nb_set_shape can
 // switch them off or on everywhere.
-#define NB_TILED_MIN_WATERS 28672
+#define NB_TILED_MIN_WATERS 40960
 int tiled_choice(const NbCtx *c, const RepDev &R)
 {
     if (R.nwat <= 0 || R.nwat > 16384 || c->want_tiled == MOIL_NB_TILED_OFF) return 0;
@@ -603,6 +603,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     NB_CUDA_OK(c, cudaMalloc(&c->d_site_rep, sizeof(int) * ns));
     NB_CUDA_OK(c, cudaMalloc(&c->d_site_flags, sizeof(unsigned) * ns));
     NB_CUDA_OK(c, cudaMalloc(&c->d_pos, 4 * ts * ns));
+    NB_CUDA_OK(c, cudaMalloc(&c->d_opos, 4 * ts * std::max<int64_t>(c->nW, 1)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_posb, sizeof(float4) * ns));
     NB_CUDA_OK(c, cudaMalloc(&c->d_woff, 4 * ts * 3 * std::max<int64_t>(c->nW, 1)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_site_lj, 2 * ts * ns));

@@ -84,6 +84,7 @@ struct NbCtx {
     unsigned *d_site_flags = nullptr;
     void *d_pos = nullptr;        // float4 / double4 (x, y, z, q_eff)
     float4 *d_posb = nullptr;     // positions at the last list build
+    void *d_opos = nullptr;       // water oxygens at the last list build, as d_pos
     void *d_woff = nullptr;       // float4 / double4 per water, 3 in a row: O position, then the two H
                                   // offsets from O (FP64-computed), each with its charge
     void *d_site_lj = nullptr;    // float2 / double2

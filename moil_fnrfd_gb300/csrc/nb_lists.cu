@@ -184,8 +184,8 @@ template <typename T, bool PME>
 __global__ void __launch_bounds__(256, 5) k_prepare(int nW, int nA, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
                           const int *__restrict__ site_orig, const unsigned *__restrict__ site_flags,
                           const void *site_q_v, const double *__restrict__ coor, void *pos_v, void *woff_v,
-                          float4 *__restrict__ posb, void *fr_v, unsigned char *__restrict__ zidx, float half_skin2,
-                          float rwat2, int snapshot, int *st, cudaGraphConditionalHandle cond, const int *ctl)
+                          float4 *__restrict__ posb, void *opos_v, void *fr_v, unsigned char *__restrict__ zidx,
+                          float half_skin2, float rwat2, int snapshot, int *st, cudaGraphConditionalHandle cond, const int *ctl)
 {
     // after an error in an MD step the rest of the call's steps do no work on new positions
     if (ctl && ctl[2] != 0) return;
@@ -209,7 +209,9 @@ __global__ void __launch_bounds__(256, 5) k_prepare(int nW, int nA, const RepDev
             // distances with radii that include the hydrogens' reach (rwat, checked below)
             prepare_site<T, PME>(R, 3 * u, xo, site_flags, site_q, pos_v, posb, fr_v, zidx, half_skin2, snapshot, true, moved);
             // the molecule record of the water kernel: O position (and charge), then the offsets
-            ((T4 *)woff_v)[3 * u] = ((const T4 *)pos_v)[3 * u];
+            const T4 po = ((const T4 *)pos_v)[3 * u];
+            ((T4 *)woff_v)[3 * u] = po;
+            if (snapshot) ((T4 *)opos_v)[u] = po;      // oxygens in a row for the searches
 #pragma unroll 1
             for (int m = 1; m < 3; ++m) {
                 double x[3];
@@ -275,6 +277,27 @@ __device__ __forceinline__ T mi_r2(const RepDev &R, T dx, T dy, T dz)
     return dx * dx + dy * dy + dz * dz;
 }
 
+// two at once: FP32 packed, the rounding by the 1.5 * 2^23 shift (|d / L| < 2^22; a rounding
+// instruction shares the special-function pipe)
+__device__ __forceinline__ void mi_r2x2(const RepDev &R, float4 o, float4 a, float4 b, float &ra, float &rb)
+{
+    const float2 mg = make_float2(12582912.f, 12582912.f), nm = make_float2(-12582912.f, -12582912.f);
+    float2 d[3] = {make_float2(o.x - a.x, o.x - b.x), make_float2(o.y - a.y, o.y - b.y), make_float2(o.z - a.z, o.z - b.z)};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float2 n = __fadd2_rn(__ffma2_rn(d[k], make_float2(R.invL[k], R.invL[k]), mg), nm);
+        d[k] = __ffma2_rn(n, make_float2(-R.L[k], -R.L[k]), d[k]);
+    }
+    const float2 r = __ffma2_rn(d[0], d[0], __ffma2_rn(d[1], d[1], __fmul2_rn(d[2], d[2])));
+    ra = r.x;
+    rb = r.y;
+}
+__device__ __forceinline__ void mi_r2x2(const RepDev &R, double4 o, double4 a, double4 b, double &ra, double &rb)
+{
+    ra = mi_r2<double>(R, o.x - a.x, o.y - a.y, o.z - a.z);
+    rb = mi_r2<double>(R, o.x - b.x, o.y - b.y, o.z - b.z);
+}
+
 __device__ __forceinline__ bool nb_excluded(const int *__restrict__ ex_off, const int *__restrict__ ex_j, int a, int b)
 {
     for (int k = ex_off[a]; k < ex_off[a + 1]; ++k)
@@ -338,11 +361,13 @@ __device__ __forceinline__ void cell_runs(const RepDev &R, T x, T y, T z, Fn fn)
 // pass, W2 (non-water sites, CSR) counted in the FILL = 0 pass and written in the FILL = 1 pass.
 // The lanes test 32 consecutive sorted units at a time and the hits are placed by a ballot, so
 // the rows are in the order of the search.  One water per thread scanned its 1,700 candidates
-// in series: 493 us for the 7,020 waters of the solute system (count pass), 357 (fill).
+// in series: 493 us for the 7,020 waters of the solute system (count pass), 357 (fill).  Bound:
+// instruction issue; two candidates per lane and round on the packed FP32 pipe, from a row of oxygens
+// of their own (the site positions hold them 48 bytes apart): rebuild of 32,000 waters 281 -> 236 us.
 #define NB_LW 4      // warps per block
 template <typename T, int FILL, typename E>
 __global__ void __launch_bounds__(32 * NB_LW) k_wlist(int nW, const RepDev *__restrict__ reps,
-                                                      const int *__restrict__ site_rep, const void *pos_v,
+                                                      const int *__restrict__ site_rep, const void *pos_v, const void *opos_v,
                                                       const int *__restrict__ bin_start, int ncell,
                                                       int2 *__restrict__ wcnt, int *__restrict__ cnt2,
                                                       const int *__restrict__ off2, void *__restrict__ l1, int cap_row,
@@ -350,7 +375,7 @@ __global__ void __launch_bounds__(32 * NB_LW) k_wlist(int nW, const RepDev *__re
 {
     if (rebuild_off(st)) return;
     typedef typename vec4<T>::type T4;
-    const T4 *pos = (const T4 *)pos_v;
+    const T4 *pos = (const T4 *)pos_v, *opos = (const T4 *)opos_v;
     __shared__ int sum1, max1;
     if (threadIdx.x == 0) { sum1 = 0; max1 = 0; }
     __syncthreads();
@@ -363,49 +388,49 @@ __global__ void __launch_bounds__(32 * NB_LW) k_wlist(int nW, const RepDev *__re
             if (!FILL && lane == 0) cnt2[i] = 0;
             continue;
         }
-        const T4 oi = pos[3 * (size_t)i];
+        const T4 oi = opos[i];
         const T rl2 = (T)R.rlist2, rw2 = (T)R.rlistw2, rc2 = (T)R.rmax2;
         const int w2 = FILL ? off2[i] : 0, base = row_base<E>(R), noth = R.noth;
         E *row = (E *)l1 + (size_t)i * cap_row;
         int n2 = 0, nn = 0, nf = 0;
+        auto put = [&](int p, bool in, bool close) {
+            const unsigned mn = __ballot_sync(0xffffffffu, in && close), mf = __ballot_sync(0xffffffffu, in && !close);
+            if (in) {
+                const int k = close ? nn + __popc(mn & below) : cap_row - 1 - nf - __popc(mf & below);
+                if (close ? k < cap_row : k >= 0) row[k] = (E)(p - base);
+            }
+            nn += __popc(mn);
+            nf += __popc(mf);
+        };
         cell_runs<T>(R, oi.x, oi.y, oi.z, [&](int c0, int c1) {
             if (do_w1) {
                 const int p1 = bin_start[c1];
-                for (int p0 = bin_start[c0]; p0 < p1; p0 += 32) {
-                    const int p = p0 + lane;
-                    bool in = false, near = false;
-                    if (p < p1 && p != i) {
-                        const T4 oj = pos[3 * (size_t)p];
-                        const T r2 = mi_r2<T>(R, oi.x - oj.x, oi.y - oj.y, oi.z - oj.z);
-                        in = r2 < rl2;
-                        near = in && r2 <= rc2;
-                    }
-                    const unsigned mn = __ballot_sync(0xffffffffu, near), mf = __ballot_sync(0xffffffffu, in && !near);
-                    if (near) {
-                        const int k = nn + __popc(mn & below);
-                        if (k < cap_row) row[k] = (E)(p - base);
-                    } else if (in) {
-                        const int k = nf + __popc(mf & below);
-                        if (k < cap_row) row[cap_row - 1 - k] = (E)(p - base);
-                    }
-                    nn += __popc(mn);
-                    nf += __popc(mf);
+                // two candidates per lane and round, both loads on their way together
+                for (int p0 = bin_start[c0]; p0 < p1; p0 += 64) {
+                    const int pa = p0 + lane, pb = pa + 32;
+                    const T4 oa = opos[min(pa, p1 - 1)], ob = opos[min(pb, p1 - 1)];
+                    T ra, rb;
+                    mi_r2x2(R, oi, oa, ob, ra, rb);
+                    put(pa, pa < p1 && pa != i && ra < rl2, ra <= rc2);
+                    if (p0 + 32 < p1) put(pb, pb < p1 && pb != i && rb < rl2, rb <= rc2);
                 }
             }
             if (noth > 0) {
                 // non-water atoms of the run
                 const int p1 = bin_start[ncell + c1];
-                for (int p0 = bin_start[ncell + c0]; p0 < p1; p0 += 32) {
-                    const int p = p0 + lane, s = 3 * nW + (p - nW);
-                    bool in = false;
-                    if (p < p1) {
-                        const T4 xj = pos[s];
-                        in = mi_r2<T>(R, oi.x - xj.x, oi.y - xj.y, oi.z - xj.z) < rw2;
-                    }
+                auto put2 = [&](int s, bool in) {
                     const unsigned m = __ballot_sync(0xffffffffu, in);
                     const int64_t k = (int64_t)w2 + n2 + __popc(m & below);
                     if (FILL && in && k < cap2) l2[k] = s;
                     n2 += __popc(m);
+                };
+                for (int p0 = bin_start[ncell + c0]; p0 < p1; p0 += 64) {
+                    const int pa = p0 + lane, pb = pa + 32, s0 = 2 * nW;      // site 3 nW + (p - nW)
+                    const T4 xa = pos[s0 + min(pa, p1 - 1)], xb = pos[s0 + min(pb, p1 - 1)];
+                    T ra, rb;
+                    mi_r2x2(R, oi, xa, xb, ra, rb);
+                    put2(s0 + pa, pa < p1 && ra < rw2);
+                    if (p0 + 32 < p1) put2(s0 + pb, pb < p1 && rb < rw2);
                 }
             }
         });
@@ -698,6 +723,7 @@ template <typename T, int FILL>
 __global__ void __launch_bounds__(32 * NB_LW) k_xlist(int nA, int nW, const RepDev *__restrict__ reps,
                                                       const int *__restrict__ site_rep,
                                                       const int *__restrict__ site_orig, const void *pos_v,
+                                                      const void *opos_v,
                                                       const int *__restrict__ bin_start, int ncell,
                                                       const int *__restrict__ ex_off, const int *__restrict__ ex_j,
                                                       int *__restrict__ cnt, const int *__restrict__ off,
@@ -705,7 +731,7 @@ __global__ void __launch_bounds__(32 * NB_LW) k_xlist(int nA, int nW, const RepD
 {
     if (rebuild_off(st)) return;
     typedef typename vec4<T>::type T4;
-    const T4 *pos = (const T4 *)pos_v;
+    const T4 *pos = (const T4 *)pos_v, *opos = (const T4 *)opos_v;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     for (int k = blockIdx.x * NB_LW + (threadIdx.x >> 5); k < nA; k += gridDim.x * NB_LW) {
@@ -718,13 +744,7 @@ __global__ void __launch_bounds__(32 * NB_LW) k_xlist(int nA, int nW, const RepD
         int n = 0;
         cell_runs<T>(R, xi.x, xi.y, xi.z, [&](int c0, int c1) {
             int p1 = bin_start[c1];
-            for (int p0 = bin_start[c0]; p0 < p1; p0 += 32) {
-                const int p = p0 + lane;
-                bool in = false;
-                if (p < p1) {
-                    const T4 oj = pos[3 * (size_t)p];
-                    in = mi_r2<T>(R, xi.x - oj.x, xi.y - oj.y, xi.z - oj.z) < rw2;
-                }
+            auto put_water = [&](int p, bool in) {
                 const unsigned m = __ballot_sync(0xffffffffu, in);
                 if (FILL && in) {
                     const int64_t q = (int64_t)w + n + 3 * __popc(m & below);
@@ -733,20 +753,30 @@ __global__ void __launch_bounds__(32 * NB_LW) k_xlist(int nA, int nW, const RepD
                         if (q + t < cap) l[q + t] = 3 * p + t;
                 }
                 n += 3 * __popc(m);
+            };
+            for (int p0 = bin_start[c0]; p0 < p1; p0 += 64) {
+                const int pa = p0 + lane, pb = pa + 32;
+                const T4 oa = opos[min(pa, p1 - 1)], ob = opos[min(pb, p1 - 1)];
+                T ra, rb;
+                mi_r2x2(R, xi, oa, ob, ra, rb);
+                put_water(pa, pa < p1 && ra < rw2);
+                if (p0 + 32 < p1) put_water(pb, pb < p1 && rb < rw2);
             }
             p1 = bin_start[ncell + c1];
-            for (int p0 = bin_start[ncell + c0]; p0 < p1; p0 += 32) {
-                const int p = p0 + lane, sj = 3 * nW + (p - nW);
-                bool in = false;
-                if (p < p1 && sj != si) {
-                    const T4 xj = pos[sj];
-                    in = mi_r2<T>(R, xi.x - xj.x, xi.y - xj.y, xi.z - xj.z) < rl2 &&
-                         !nb_excluded(ex_off, ex_j, ai, site_orig[sj]);
-                }
+            auto put_atom = [&](int sj, bool in) {
+                in = in && sj != si && !nb_excluded(ex_off, ex_j, ai, site_orig[sj]);
                 const unsigned m = __ballot_sync(0xffffffffu, in);
                 const int64_t q = (int64_t)w + n + __popc(m & below);
                 if (FILL && in && q < cap) l[q] = sj;
                 n += __popc(m);
+            };
+            for (int p0 = bin_start[ncell + c0]; p0 < p1; p0 += 64) {
+                const int pa = p0 + lane, pb = pa + 32, s0 = 2 * nW;          // site 3 nW + (p - nW)
+                const T4 xa = pos[s0 + min(pa, p1 - 1)], xb = pos[s0 + min(pb, p1 - 1)];
+                T ra, rb;
+                mi_r2x2(R, xi, xa, xb, ra, rb);
+                put_atom(s0 + pa, pa < p1 && ra < rl2);
+                if (p0 + 32 < p1) put_atom(s0 + pb, pb < p1 && rb < rl2);
             }
         });
         if (lane != 0) continue;
@@ -957,7 +987,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
         c->d_site_q, c->d_status);
     (nb_fused_sites(c) ? k_prepare<T, true> : k_prepare<T, false>)<<<grid(c->nW + c->nA, B), B, 0, s>>>(
         (int)c->nW, (int)c->nA, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_site_flags, c->d_site_q, d_coor,
-        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, 0.f, c->rwat * c->rwat, 1, c->d_status, 0, nullptr);
+        c->d_pos, c->d_woff, c->d_posb, c->d_opos, c->d_fr, c->d_zidx, 0.f, c->rwat * c->rwat, 1, c->d_status, 0, nullptr);
     c->launches += 5;
     // water lists with the row entry type of the handle (uint16 when every replica has fewer
     // than 65,536 waters)
@@ -971,7 +1001,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
         // are non-water atoms (the W2 offsets are zero from the start otherwise)
         bool search = c->nA > 0;
         for (const RepDev &R : c->rd) search |= R.nwat > 0 && !R.wtiled;
-        if (search) k_wlist<T, 0, E><<<gw, 32 * NB_LW, 0, s>>>((int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_bin_start,
+        if (search) k_wlist<T, 0, E><<<gw, 32 * NB_LW, 0, s>>>((int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_opos, c->d_bin_start,
                                             c->ncell, c->d_wl1_cnt, cnt2, nullptr, c->d_wl1, c->cap_row1, nullptr, 0,
                                             c->d_status);
         if (nt > 0)
@@ -980,7 +1010,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
         c->launches += (search ? 1 : 0) + (nt > 0 ? 1 : 0);
         if (c->nA == 0) return;
         nb_scan(c, cnt2, c->d_wl2_off, (int)c->nW, c->d_status + 3, 1);
-        k_wlist<T, 1, E><<<gw, 32 * NB_LW, 0, s>>>((int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_bin_start,
+        k_wlist<T, 1, E><<<gw, 32 * NB_LW, 0, s>>>((int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_opos, c->d_bin_start,
                                             c->ncell, nullptr, nullptr, c->d_wl2_off, nullptr, 0, c->d_wl2, c->cap_wl2,
                                             c->d_status);
         c->launches++;
@@ -1000,11 +1030,11 @@ void build_lists_t(NbCtx *c, const double *d_coor)
     }
     if (c->nA > 0) {
         const int ga = warp_grid(c->nA);
-        k_xlist<T, 0><<<ga, 32 * NB_LW, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos,
+        k_xlist<T, 0><<<ga, 32 * NB_LW, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_opos,
                                          c->d_bin_start, c->ncell, c->d_ex_off, c->d_ex_j, c->d_count_tmp, nullptr,
                                          nullptr, 0, c->d_status);
         nb_scan(c, c->d_count_tmp, c->d_xl_off, (int)c->nA, c->d_status + 4, 1);
-        k_xlist<T, 1><<<ga, 32 * NB_LW, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos,
+        k_xlist<T, 1><<<ga, 32 * NB_LW, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_opos,
                                          c->d_bin_start, c->ncell, c->d_ex_off, c->d_ex_j, nullptr, c->d_xl_off,
                                          c->d_xl, c->cap_xl, c->d_status);
         c->launches += 2;
@@ -1020,7 +1050,7 @@ void prepare_t(NbCtx *c, const double *d_coor, cudaGraphConditionalHandle cond, 
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((items + B - 1) / B, (int64_t)c->nsm * 8));
     (nb_fused_sites(c) ? k_prepare<T, true> : k_prepare<T, false>)<<<g, B, 0, c->stream>>>(
         (int)c->nW, (int)c->nA, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_site_flags, c->d_site_q, d_coor,
-        c->d_pos, c->d_woff, c->d_posb, c->d_fr, c->d_zidx, hs * hs, c->rwat * c->rwat, 0, c->d_status, cond,
+        c->d_pos, c->d_woff, c->d_posb, c->d_opos, c->d_fr, c->d_zidx, hs * hs, c->rwat * c->rwat, 0, c->d_status, cond,
         ctl);
     c->launches += 1;
 }
