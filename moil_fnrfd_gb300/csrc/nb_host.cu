@@ -880,10 +880,11 @@ void eval_launch(NbCtx *c, const double *d_coor, double *d_dpot)
 // internal status of an evaluation without the rebuild it turned out to need (redone with it)
 constexpr int kStale = -1;
 
-// wait for the queued evaluation and read its status words
-int eval_complete(NbCtx *c)
+// wait for the queued evaluation (end: the event after it, where more work has been queued) and read its
+// status words
+int eval_complete(NbCtx *c, cudaEvent_t end = nullptr)
 {
-    NB_CUDA_OK(c, cudaStreamSynchronize(c->stream));
+    NB_CUDA_OK(c, end ? cudaEventSynchronize(end) : cudaStreamSynchronize(c->stream));
     NB_CUDA_OK(c, cudaGetLastError());
     int rebuilt = c->h_status[0] != 0;
     if (rebuilt && !c->eval_forced) c->wary = 2;
@@ -981,6 +982,24 @@ int eval_retry(NbCtx *c, const double *d_coor, double *d_dpot, moil_energies *e,
 int eval_impl(NbCtx *c, const double *d_coor, double *d_dpot, moil_energies *e)
 {
     return eval_retry(c, d_coor, d_dpot, e, MOIL_NB_OK, false);
+}
+
+// One evaluation of h->d_coor and the pass that follows it (queue), whose launches do not wait for the
+// evaluation's status words: their host time (8 to 12 launches and events, about 25 us) passes while
+// it runs.  An evaluation that has to be redone takes the pass with it.
+template <typename F>
+int eval_and(NbCtx *h, moil_energies *e, F queue)
+{
+    eval_launch(h, h->d_coor, h->d_dpot);
+    NB_CUDA_OK(h, cudaEventRecord(h->ev[11], h->stream));
+    const int queued = queue();
+    const int first = eval_complete(h, h->ev[11]);
+    const int rc = eval_retry(h, h->d_coor, h->d_dpot, e, first, true);
+    if (rc != MOIL_NB_OK) {
+        cudaStreamSynchronize(h->stream);       // (the pass reads the handle's buffers)
+        return rc;
+    }
+    return first != MOIL_NB_OK && queued == MOIL_NB_OK ? queue() : queued;
 }
 
 // ---- replica groups ------------------------------------------------------------------
@@ -1301,11 +1320,16 @@ int moil_nb_eval(moil_nb_ctx *h, const double *coor, double *dpot, moil_energies
     // the coordinates in and the gradient out took 0.7 ms together
     size_t bytes = sizeof(double) * 3 * h->natom;
     NB_CUDA_OK(h, cudaMemcpyAsync(h->d_coor, coor, bytes, cudaMemcpyHostToDevice, h->stream));
-    int rc = eval_impl(h, h->d_coor, h->d_dpot, e);
-    if (rc != MOIL_NB_OK) return rc;
+    eval_launch(h, h->d_coor, h->d_dpot);
+    // queued behind the evaluation, as a group's copy is; copied again if that had to be redone
     NB_CUDA_OK(h, cudaMemcpyAsync(dpot, h->d_dpot, bytes, cudaMemcpyDeviceToHost, h->stream));
-    NB_CUDA_OK(h, cudaStreamSynchronize(h->stream));
-    return MOIL_NB_OK;
+    const int first = eval_complete(h);
+    int rc = eval_retry(h, h->d_coor, h->d_dpot, e, first, true);
+    if (rc == MOIL_NB_OK && first != MOIL_NB_OK) {
+        NB_CUDA_OK(h, cudaMemcpyAsync(dpot, h->d_dpot, bytes, cudaMemcpyDeviceToHost, h->stream));
+        NB_CUDA_OK(h, cudaStreamSynchronize(h->stream));
+    }
+    return rc;
 }
 
 int moil_nb_adjoint(moil_nb_ctx *h, const double *coor, double *dEdq, double *dEdeps, double *dEdsig,
@@ -1326,13 +1350,12 @@ int moil_nb_adjoint(moil_nb_ctx *h, const double *coor, double *dEdq, double *dE
     }
     const size_t n = (size_t)h->natom;
     NB_CUDA_OK(h, cudaMemcpyAsync(h->d_coor, coor, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->stream));
-    int rc = eval_impl(h, h->d_coor, h->d_dpot, e);   // lists, positions and the potential grid
-    if (rc != MOIL_NB_OK) return rc;
     const bool mixed = h->precision != MOIL_NB_FP64;      // with a second set of sums (nb_adjoint)
     if (!h->d_adj) NB_CUDA_OK(h, cudaMalloc(&h->d_adj, sizeof(double) * (mixed ? 6 : 3) * std::max<size_t>(n, 1)));
     if (h->precision == MOIL_NB_FP64 && !h->d_adj_phi)
         NB_CUDA_OK(h, cudaMalloc(&h->d_adj_phi, sizeof(double) * 4 * std::max<int64_t>(h->nsite, 1)));
-    rc = nb_adjoint(h, h->d_adj, mixed ? h->d_adj + 3 * n : nullptr);
+    // lists, positions and the potential grid from an evaluation
+    const int rc = eval_and(h, e, [&] { return nb_adjoint(h, h->d_adj, mixed ? h->d_adj + 3 * n : nullptr); });
     if (rc != MOIL_NB_OK) return rc;
     double *out[3] = {dEdq, dEdeps, dEdsig};
     for (int k = 0; k < 3; ++k)
@@ -1419,8 +1442,6 @@ int moil_nb_pressure(moil_nb_ctx *h, const double *coor, double *dpot, moil_ener
     }
     const size_t n = (size_t)h->natom;
     NB_CUDA_OK(h, cudaMemcpyAsync(h->d_coor, coor, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->stream));
-    int rc = eval_impl(h, h->d_coor, h->d_dpot, e);   // lists, positions, PME records and shares
-    if (rc != MOIL_NB_OK) return rc;
     if (!h->d_press_out) {
         NB_CUDA_OK(h, cudaMalloc(&h->d_press_unit, sizeof(double) * 6 * std::max<int64_t>(h->nW + h->nA, 1)));
         h->press_split = nb_press_split(h);
@@ -1431,7 +1452,8 @@ int moil_nb_pressure(moil_nb_ctx *h, const double *coor, double *dpot, moil_ener
         NB_CUDA_OK(h, cudaMalloc(&h->d_press_grid, 2 * fp * (h->grid_elems + 2)));
         NB_CUDA_OK(h, cudaMalloc(&h->d_press_out, sizeof(double) * 12 * h->nrep));
     }
-    rc = nb_pressure(h, h->d_coor, h->d_press_out);
+    // lists, positions, PME records and shares from an evaluation
+    const int rc = eval_and(h, e, [&] { return nb_pressure(h, h->d_coor, h->d_press_out); });
     if (rc != MOIL_NB_OK) return rc;
     // the gradient is complete (the evaluation has ended): its copy runs beside the kernels above
     if (dpot) {

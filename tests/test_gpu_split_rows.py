@@ -109,3 +109,16 @@ def test_pressure_rows_match_oracle(name, precision):
     press = nb.pressure(s.coor)[2]
     nb.close()
     assert np.abs(press - want).max() <= (1e-9 if precision == MOIL_NB_FP64 else 1e-5) * np.abs(want).sum()
+
+
+def test_pass_is_redone_with_its_evaluation():
+    """Derivatives and pressure as a handle's first call, on rows that overflow their first capacity
+    (the evaluation and the pass queued behind it are redone), and again on the lists then built."""
+    s = dense_cluster(900, 12, 0.55)
+    mol, mass = S.molecules(s)
+    for call in (lambda nb: np.stack(nb.adjoint(s.coor)), lambda nb: nb.pressure(s.coor)[2]):
+        nb = Nonbonded(s)
+        nb.set_molecules(mol, mass)
+        first, again = call(nb), call(nb)
+        nb.close()
+        assert np.isfinite(first).all() and np.abs(first - again).max() <= 1e-9 * np.abs(again).max()
