@@ -227,11 +227,11 @@ int alloc_half(NbCtx *c)
 // The automatic shape takes full lists up to this many waters (of the whole handle): a block
 // of 256 waters per multiprocessor leaves most of the GPU idle below it, while the full-list
 // kernel spreads each water over 8 or 32 lanes.  One evaluation in us (lists rebuilt every 10),
-// half / full lists: 216 waters 98 / 80, 1,334 125 / 95, 7,000 124 / 104, 12,000 129 / 117, 32,000
-// 197 / 199, 110,860 (64 replicas) 385 / 402.  Handles with atoms outside waters take full lists
-// at every size: the half-list kernel runs a water's list of them in one thread (water stage of
-// the solute system, 7,020 waters: 322 / 37 us).
-#define NB_FULL_MAX_WATERS 28672
+// half / full lists: 216 waters 75 / 46, 1,334 94 / 52, 7,000 102 / 68, 12,000 105 / 79, 28,800 (16
+// replicas) 130 / 125, 32,000 149 / 154, 110,860 (64 replicas) 340 / 371.  Handles with atoms outside
+// waters take full lists at every size: the half-list kernel runs a water's list of them in one
+// thread (water stage of the solute system, 7,020 waters: 322 / 37 us).
+#define NB_FULL_MAX_WATERS 30000
 
 // Half-list set-up for the current shape: on for FP32 handles whose replicas all have fewer
 // than 65,536 waters (16-bit rows) unless full lists were asked for; blocks of hb waters

@@ -1337,7 +1337,7 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
 // 1,334 waters 14 / 19 / 27, 3,000 22 / 19 / 28, 7,000 32 / 21 / 30, 12,000 46 / 34 / 32, 32,000
 // 114 / 80 / 77, 110,860 (64 replicas) 366 / 197 / 175, 433,195 1418 / 733 / 633 (one water per
 // thread: 78, 79, 82, 79, 120, 204, 657).  With atoms outside waters a water also has a list of
-// those (the solute system, 7,020 waters: 37 / 71 / 114).
+// those (the solute system, 7,020 waters: 37 / 71 / 114; 34 at 32 lanes since its loop is packed).
 int water_lanes(const NbCtx *c)
 {
     const bool atoms = c->na_handle > 0;
