@@ -44,14 +44,14 @@ F_PAIR = 50            # FP32 operations per in-cutoff site pair (FMA = 2, MUFU 
 LIST_PERIOD = 10
 SKIN = 1.0
 # DRAM bytes per water molecule of one water-kernel launch (ncu dram__bytes_read.sum +
-# dram__bytes_write.sum, 48-replica captures over 74,171 waters): full lists (one water per thread)
-# 37.44 MB, k_water_h (half lists, 256-water blocks) 38.48 MB
-WATER_KERNEL_DRAM_BYTES_PER_WATER = {1: 504.9, 2: 518.8}
+# dram__bytes_write.sum): full lists (an earlier build, 74,171 waters) 37.44 MB, k_water_h (half
+# lists, 256-water blocks, 48 replicas of 500-4,000 waters, 82,496 waters) 38.79 MB
+WATER_KERNEL_DRAM_BYTES_PER_WATER = {1: 504.9, 2: 470.2}
 WATER_KERNEL_NAME = {1: "k_water_s (full lists)", 2: "k_water_h (half lists)"}
-# DRAM bytes per atom of one evaluation's PME kernels (k_pme_bin, k_plane_fwd_f, k_zconv_f,
-# k_plane_inv_f, k_pme_gather_f: 5.37 + 4.55 + 10.86 + 10.82 + 15.00 MB, 48-replica capture over
-# 222,513 atoms, caches flushed before each launch, so an upper bound)
-PME_DRAM_BYTES_PER_ATOM = 209.8
+# DRAM bytes per atom of one evaluation's PME kernels (k_pme_sites, k_plane_fwd_f, k_zconv_f,
+# k_plane_inv_f, k_pme_gather_f: 5.96 + 4.42 + 12.05 + 12.02 + 16.59 MB, the same capture, 247,488
+# atoms, caches flushed before each launch, so an upper bound)
+PME_DRAM_BYTES_PER_ATOM = 206.3
 
 
 ACCEL = 418.4                 # (kcal/mol/Å) / amu in Å/ps^2
@@ -564,7 +564,7 @@ def main():
     b = 56 * natoms + 64 * ng
     t_pme = (avg["pme_spread_fft_ms"] + avg["pme_conv_ms"] + avg["pme_gather_ms"]) / 1e3
     traffic_pme = PME_DRAM_BYTES_PER_ATOM * natoms
-    roof_pme = {"kernel": "PME (bin+spread+FFT, convolution, gather)", "bound": "hbm",
+    roof_pme = {"kernel": "PME (spread+FFT, convolution, gather)", "bound": "hbm",
                 "achieved": b / t_pme / 1e9, "peak": hbm, "unit": "GB/s", "frac": b / t_pme / 1e9 / hbm,
                 "traffic": traffic_pme,
                 "traffic_note": "ncu DRAM read+write of the five PME kernels per atom on a 48-replica capture "
@@ -632,11 +632,8 @@ def main():
                                        f"{max(s.npt for s in sample)} atoms ({sum(s.npt for s in sample)} in all), "
                                        f"one per handle/launch sequence, {LIST_PERIOD} evaluations each "
                                        f"(one list build)",
-                             "note": "the FP64 water kernel takes 93% of a small replica's evaluation (launch "
-                                     "list of a 2,151-atom replica: 3.4 of 3.7 ms): one water per thread runs "
-                                     "its ~900 FP64 site pairs (erfc, square root, division) in series, and "
-                                     "spreading a replica over 4x more multiprocessors gained 6%, so it is "
-                                     "latency-bound per thread, not launch-bound; the 96,000-atom FP64 rate is "
+                             "note": "the FP64 water kernel (a warp per water, each pair once) is bound by the "
+                                     "FP64 pipe, 1/64 of the FP32 rate; the 96,000-atom FP64 rate is "
                                      "in single_system_md.plain_fp64_atom_evals_per_s"}
         out["speedup_vs_plain_fp64"] = value / fp64_value
         out["force_err_vs_fp64"] = {"max_rel_rms": max(errs), "replicas": len(errs)}
