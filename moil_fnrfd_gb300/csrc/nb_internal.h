@@ -171,13 +171,13 @@ struct NbCtx {
     // rebuild requested, sticky error bits}, read back once per call
     cudaGraphExec_t gexec_md[3] = {nullptr, nullptr, nullptr};    // by EvalMode
     struct MdKey {
-        const void *coor = nullptr, *vel = nullptr, *mass = nullptr, *dpot = nullptr;
+        const void *coor = nullptr, *vel = nullptr, *mass = nullptr;
         double dt = 0.0, doh = 0.0, dhh = 0.0;
         int gen = -1;
         bool operator==(const MdKey &o) const
         {
-            return coor == o.coor && vel == o.vel && mass == o.mass && dpot == o.dpot && dt == o.dt && doh == o.doh &&
-                   dhh == o.dhh && gen == o.gen;
+            return coor == o.coor && vel == o.vel && mass == o.mass && dt == o.dt && doh == o.doh && dhh == o.dhh &&
+                   gen == o.gen;
         }
     } gmd_key[3];
     int md_wary = 0, md_backoff = 0;   // step loops left to the device's decision after a stale one
@@ -294,10 +294,10 @@ void nb_pme_etab(const RepDev &R, const double *bsp, float *out);
 void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl, EvalMode mode);   // ctl: as nb_launch_prepare
 // MD step loop (nb_md.cu / nb_host.cu): the integrator of one context, and the graph replay of
 // nsteps whole steps (no host wait)
-int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, const double *dpot,
-                        double dt, double doh, double dhh);
-int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double *dpot, double dt, double doh,
-               double dhh, int nsteps, bool host);
+int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, double dt, double doh,
+                        double dhh, int *ctl);
+int nb_md_loop(NbCtx *c, double *coor, double *vel, const double *mass, double dt, double doh, double dhh, int nsteps,
+               bool host);
 // per-replica energies and pair count of the last completed evaluation (e may be NULL)
 void read_energies_of(NbCtx *c, moil_energies *e);
 // parameter derivatives after an evaluation of c->d_coor (nb_adjoint.cu): dq, de, ds one after another;

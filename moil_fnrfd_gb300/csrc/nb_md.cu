@@ -16,7 +16,9 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
+#include "nb_grad.cuh"
 #include "nb_internal.h"
 
 namespace {
@@ -86,11 +88,39 @@ __device__ __forceinline__ void settle(const double p0[3][3], double p1[3][3], d
 // the multiprocessors: 28,800 waters in blocks of 128 left a third of them with half the work of the
 // others, 30.6 us; blocks of 32, and the constants and unit vectors with fewer square roots and
 // divisions, 19.7.
+// In a step graph the gradient comes from its parts (StepGrad), not from an array that a kernel before
+// has assembled.
 #define NB_LF 32
+struct ArrayGrad {
+    const double *dpot;
+    __device__ void operator()(size_t a, double g[3]) const
+    {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) g[d] = dpot[3 * a + d];
+    }
+};
+template <typename T> struct StepGrad {
+    const int *site_of, *atom_rep;
+    const RepDev *reps;
+    const long long *grad_site;
+    const double *grad_ex;
+    const T *part;
+    const double *q;
+    int nsw;
+    int *nan_h, *ctl;
+    __device__ void operator()(size_t a, double g[3]) const
+    {
+        if (!final_grad<T>((int)a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, g)) {
+            *nan_h = 1;
+            atomicOr(&ctl[2], NB_DEV_ERR_NAN);
+        }
+    }
+};
+template <typename G>
 __global__ void __launch_bounds__(NB_LF) k_leapfrog_water(int nW, const int *__restrict__ unit_atom,
                                                           const double *__restrict__ mass, double dt, double inv_dt,
                                                           double dhh, double h, double *__restrict__ coor,
-                                                          double *__restrict__ vel, const double *__restrict__ dpot)
+                                                          double *__restrict__ vel, G grad)
 {
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= nW) return;
@@ -100,13 +130,16 @@ __global__ void __launch_bounds__(NB_LF) k_leapfrog_water(int nW, const int *__r
 #pragma unroll
     for (int m = 0; m < 3; ++m) f[m] = m == 2 && ms[2] == ms[1] ? f[1] : dt * kAccel / ms[m];
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
+    for (int m = 0; m < 3; ++m) {
+        double g[3];
+        grad(a + m, g);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const size_t k = 3 * (a + m) + d;
             p0[m][d] = coor[k];
-            p1[m][d] = p0[m][d] + dt * (vel[k] - f[m] * dpot[k]);
+            p1[m][d] = p0[m][d] + dt * (vel[k] - f[m] * g[d]);
         }
+    }
     settle(p0, p1, dhh, h, ms[0], ms[1]);
 #pragma unroll
     for (int m = 0; m < 3; ++m)
@@ -119,16 +152,18 @@ __global__ void __launch_bounds__(NB_LF) k_leapfrog_water(int nW, const int *__r
 }
 
 // every atom outside a water, unconstrained
+template <typename G>
 __global__ void k_leapfrog_free(int natom, const unsigned *__restrict__ aflags, const double *__restrict__ mass,
-                                double dt, double *__restrict__ coor, double *__restrict__ vel,
-                                const double *__restrict__ dpot)
+                                double dt, double *__restrict__ coor, double *__restrict__ vel, G grad)
 {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= natom || (aflags[a] & SF_WATER)) return;
     const double f = dt * kAccel / mass[a];
+    double g[3];
+    grad(a, g);
     for (int d = 0; d < 3; ++d) {
         const size_t k = 3 * (size_t)a + d;
-        vel[k] -= f * dpot[k];
+        vel[k] -= f * g[d];
         coor[k] += dt * vel[k];
     }
 }
@@ -153,25 +188,34 @@ __global__ void __launch_bounds__(256) k_kinetic(int natom, const double *__rest
 }
 
 // the integrator kernels of one (ungrouped) context over its caller-atom range
-int integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, const double *dpot,
-              double dt, double doh, double dhh)
+template <typename G>
+int integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, G grad, double dt, double doh,
+              double dhh)
 {
     if (c->nW > 0)
         k_leapfrog_water<<<(int)((c->nW + NB_LF - 1) / NB_LF), NB_LF, 0, s>>>(
-            (int)c->nW, c->d_unit_atom, mass, dt, 1.0 / dt, dhh, sqrt(doh * doh - 0.25 * dhh * dhh), coor, vel, dpot);
+            (int)c->nW, c->d_unit_atom, mass, dt, 1.0 / dt, dhh, sqrt(doh * doh - 0.25 * dhh * dhh), coor, vel, grad);
     if (c->nA > 0)
-        k_leapfrog_free<<<(int)((c->natom + 255) / 256), 256, 0, s>>>((int)c->natom, c->d_aflags, mass, dt, coor,
-                                                                      vel, dpot);
+        k_leapfrog_free<<<(int)((c->natom + 255) / 256), 256, 0, s>>>((int)c->natom, c->d_aflags, mass, dt, coor, vel,
+                                                                      grad);
     NB_CUDA_OK(c, cudaGetLastError());
     return MOIL_NB_OK;
 }
 
 }  // namespace
 
-int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, const double *dpot,
-                        double dt, double doh, double dhh)
+int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, const double *mass, double dt, double doh,
+                        double dhh, int *ctl)
 {
-    return integrate(c, s, coor, vel, mass, dpot, dt, doh, dhh);
+    auto with = [&](auto part, int nsw) {
+        typedef std::remove_const_t<std::remove_pointer_t<decltype(part)>> T;
+        return integrate(c, s, coor, vel, mass,
+                         StepGrad<T>{c->d_site_of, c->d_atom_rep, c->d_reps, c->d_grad_site, c->d_grad_ex, part, c->d_q,
+                                     nsw, c->h_status + 23, ctl},
+                         dt, doh, dhh);
+    };
+    if (c->precision == MOIL_NB_FP64) return with((const double *)c->d_part, 0);
+    return with((const float *)c->d_part, c->water_excl_fast ? (int)(3 * c->nW) : 0);
 }
 
 namespace {
@@ -226,8 +270,7 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
                 NB_CUDA_OK(h, cudaEventRecord(h->ev[11], h->stream));            // the snapshot copies
                 NB_CUDA_OK(h, cudaStreamWaitEvent(c->stream, h->ev[11], 0));
             }
-            rc = nb_md_loop(c, d_coor + 3 * a0, d_vel + 3 * a0, d_mass + a0, h->d_md_dpot + 3 * a0, dt, doh, dhh, run,
-                            host);
+            rc = nb_md_loop(c, d_coor + 3 * a0, d_vel + 3 * a0, d_mass + a0, dt, doh, dhh, run, host);
         }
         int err = 0;
         for (NbCtx *c : ctxs) {
@@ -269,13 +312,13 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
         int rc = moil_nb_eval_device(h, d_coor, h->d_md_dpot, step + 1 == nsteps ? energies : nullptr);
         if (rc != MOIL_NB_OK) return rc;
         if (h->grp.empty()) {
-            rc = integrate(h, h->stream, d_coor, d_vel, d_mass, h->d_md_dpot, dt, doh, dhh);
+            rc = integrate(h, h->stream, d_coor, d_vel, d_mass, ArrayGrad{h->d_md_dpot}, dt, doh, dhh);
         } else {
             // each group integrates its own atoms on its stream; the handle's stream waits
             for (size_t g = 0; g < h->grp.size() && rc == MOIL_NB_OK; ++g) {
                 const int64_t a0 = h->grp_atom0[g];
                 rc = integrate(h->grp[g], h->grp[g]->stream, d_coor + 3 * a0, d_vel + 3 * a0, d_mass + a0,
-                               h->d_md_dpot + 3 * a0, dt, doh, dhh);
+                               ArrayGrad{h->d_md_dpot + 3 * a0}, dt, doh, dhh);
             }
             for (NbCtx *c : h->grp) {
                 NB_CUDA_OK(h, cudaEventRecord(c->ev[11], c->stream));

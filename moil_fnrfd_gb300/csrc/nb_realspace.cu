@@ -15,6 +15,7 @@
 // so nothing is written twice and no atomics are needed, except where a kernel evaluates each
 // water pair once (k_water_h, k_water_d).  Energies are halved at the end.
 #include "nb_internal.h"
+#include "nb_grad.cuh"
 #include "nb_pair.cuh"
 
 namespace {
@@ -1119,54 +1120,6 @@ __global__ void k_excl14(int n, const int *__restrict__ atoms, const int *__rest
 // energies, and the status words and energies written to the host's page-locked copies by the
 // blocks that have them.  Three launches and two copies took 22 us of a 216-water evaluation.
 
-// one atom's gradient: fixed-point real space + FP64 corrections + PME; false if not finite
-template <typename T>
-__device__ __forceinline__ bool final_grad(int a, const int *__restrict__ site_of, const int *__restrict__ atom_rep,
-                                           const RepDev *__restrict__ reps, const long long *__restrict__ grad_site,
-                                           const double *__restrict__ grad_ex, const T *__restrict__ part,
-                                           const double *__restrict__ q, int nsw, double *__restrict__ dpot)
-{
-    const RepDev &R = reps[atom_rep[a]];
-    int s = site_of[a];
-    bool bad = false;
-    if constexpr (sizeof(T) == 4) {
-        // FP32 path: the PME share (one float4 per site from k_pme_gather_f) is scaled in
-        // FP32 (its own precision) and joins the fixed-point real-space and correction terms
-        // as an integer; the double result is assembled with integer operations (no FP64
-        // instruction).  Sites below nsw (waters whose corrections the water kernel added)
-        // have no correction term.
-        const long long *gx = (const long long *)grad_ex + 3 * (size_t)a;
-        const bool ex = s >= nsw;
-        const float qs = (float)q[a];
-        const float4 p4 = ((const float4 *)part)[s];
-        const float pg[3] = {p4.x, p4.y, p4.z};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const long long v = grad_site[3 * (size_t)s + d] + (ex ? gx[d] : 0LL) + nb_f2fix(qs * R.pme_gs[d] * pg[d]);
-            bad |= (v > (1LL << 61)) | (v < -(1LL << 61));   // a saturated (non-finite) term
-            dpot[3 * (size_t)a + d] = nb_fix2d(v);
-        }
-    } else {
-        const T *p = part + 12 * (size_t)s;   // 4 plane slots per site (k_plane_inv)
-        double pg[3] = {0, 0, 0};
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            pg[0] += (double)p[3 * t];
-            pg[1] += (double)p[3 * t + 1];
-            pg[2] += (double)p[3 * t + 2];
-        }
-        double qf = q[a] * R.fcd;
-        double sc[3] = {qf * R.n1 * R.invLd[0], qf * R.n2 * R.invLd[1], qf * R.n3 * R.invLd[2]};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            double v = (double)grad_site[3 * (size_t)s + d] * NB_FIX_INV + grad_ex[3 * (size_t)a + d] + sc[d] * pg[d];
-            bad |= !(v == v);
-            dpot[3 * (size_t)a + d] = v;
-        }
-    }
-    return !bad;
-}
-
 // Per-replica energies in two passes with a fixed partition, so large replicas spread over
 // many blocks and the sums stay in a fixed order (deterministic):
 //  energy_chunk: one block per chunk (EChunk: up to NB_FE_SEG consecutive units, atoms or PME
@@ -1294,10 +1247,14 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
     const int t = threadIdx.x, b = blockIdx.x;
     if (b >= nchunk) {
         const int a = (b - nchunk) * NB_FE_THREADS + t;
-        if (a < natom && !final_grad<T>(a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, dpot)) {
+        if (a >= natom) return;
+        double g[3];
+        if (!final_grad<T>(a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, g)) {
             *nan_h = 1;
             if (ctl) atomicOr(&ctl[2], NB_DEV_ERR_NAN);
         }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) dpot[3 * (size_t)a + d] = g[d];
         return;
     }
     const EChunk ch = chunks[b];
@@ -1503,7 +1460,9 @@ void nb_launch_excl14(NbCtx *c, const double *d_coor)
 void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl, EvalMode mode)
 {
     const int period = mode == EVAL_DEVICE ? c->list_period : (mode == EVAL_KEEP ? -1 : 0);
-    const int nchunk = (int)c->echunks.size(), nb = nchunk + (int)((c->natom + NB_FE_THREADS - 1) / NB_FE_THREADS);
+    // (no gradient where the integrator forms it itself)
+    const int nchunk = (int)c->echunks.size(),
+              nb = nchunk + (d_dpot ? (int)((c->natom + NB_FE_THREADS - 1) / NB_FE_THREADS) : 0);
     auto launch = [&](auto kernel, auto part, int nsw) {
         kernel<<<nb, NB_FE_THREADS, 0, c->stream>>>(
             nchunk, c->d_echunks, c->d_echunk_begin, c->d_e_unit, c->d_e_ex, c->d_e_col, c->d_epart, c->d_edone,
