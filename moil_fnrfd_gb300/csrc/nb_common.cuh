@@ -172,7 +172,6 @@ __device__ __forceinline__ double4 pme_site(const RepDev &R, const double x[3], 
 struct EChunk { int rep, kind, begin, end; };
 #define NB_FE_SEG 1024
 
-// work descriptors for the PME plane / column kernels
 // Work items of the PME kernels.  They carry their replica's grid (sizes, first complex element) and
 // the place and length of the plans' tables (FP32 path, in 16-byte units of d_blob): a block's loads
 // then depend on one load, not on four in a row.

@@ -9,7 +9,7 @@
 #include "moil_nb.h"
 #include "nb_common.cuh"
 
-// FFT plan for one length: radices (4, 2, 3, 5 in that order), twiddles exp(-2 pi i k / n)
+// FFT plan for one length: radices (make_plan), twiddles exp(-2 pi i k / n)
 // at tw0, and per Stockham stage s: the span Ns, the butterfly count nb = n/R, the magic
 // multiplier for dividing by nb, and nb (twiddle step, destination index) entries at off[s]
 struct FftPlanDev {

@@ -15,11 +15,12 @@
 //                  exp(-pi^2 m^2 / alpha^2) / (pi V B(m) m^2) with the FP64 energy sum
 //                  (scalar_sum, :723-812), inverse C2C along z, written back in place
 //   plane_inv      one CTA per (replica, z plane): inverse C2C along y, C2R along x in shared
-//                  memory, then each atom's share of the gradient from this plane (grad_sum,
-//                  :815-970) into its own slot -- four planes, four slots, summed at the end
-// FFTs (FP32 path): Stockham autosort with radices 2..5 (plane kernels) or up to 10 (z
-// columns, two passes per line: the composite codelets of nb_fft.cuh); every pass transforms all lines
-// of a tile at once, the block's threads spread over (line, butterfly) pairs, with the
+//                  memory; FP32: the real plane back to HBM for pme_gather; FP64: each atom's
+//                  share of the gradient from this plane (grad_sum, :815-970) into its own slot --
+//                  four planes, four slots, summed at the end
+//   pme_gather     (FP32) each site's gradient from the real planes
+// FFTs (FP32 path): Stockham autosort with radices up to 10 (two passes per line for most lengths:
+// the composite codelets of nb_fft.cuh); every pass transforms all lines of a tile at once, the block's threads spread over (line, butterfly) pairs, with the
 // index arithmetic (twiddle step, destination) read from per-stage tables built on the host
 // and the line number obtained by a multiply-high by a precomputed magic constant.  The
 // last pass of a direction stores transposed, so the next direction reads contiguous lines.
@@ -1276,7 +1277,7 @@ int configure_t(NbCtx *c)
     std::vector<double> twr, twi;
     std::vector<int4> blob;
     std::vector<int> boff, blen;   // per plan (FP32 path)
-    std::vector<char> wide_of;     // per plan: wide radix set (the FP32 z columns)
+    std::vector<char> wide_of;     // per plan: wide radix set (FP32)
     for (int r = 0; r < c->nrep; ++r) {
         int ns[3] = {c->rd[r].n1, c->rd[r].n2, c->rd[r].n3};
         for (int d = 0; d < 3; ++d) {
@@ -1457,7 +1458,7 @@ void nb_pme_fp32_consts(RepDev *R)
 // ---------------------------------------------------------------------------------
 // Allocation-free PME reciprocal sum (moil_nb_pme_noalloc).
 //
-// For callers that cannot allocate device memory: the same bin / spread+FFT / convolution /
+// For callers that cannot allocate device memory: the same spread+FFT / convolution /
 // FFT+gather kernels as the handle path (FP32), with every scratch buffer carved out of one
 // file-scope device array.  The array is sized for at most NA_MAX_ATOMS atoms and PME
 // grids of at most NA_MAX_N points per side; every GPU that loads this library holds it
