@@ -48,8 +48,8 @@ SKIN = 1.0
 # lists, 256-water blocks, 48 replicas of 500-4,000 waters, 82,496 waters) 38.79 MB
 WATER_KERNEL_DRAM_BYTES_PER_WATER = {1: 504.9, 2: 470.2}
 WATER_KERNEL_NAME = {1: "k_water_s (full lists)", 2: "k_water_h (half lists)"}
-# DRAM bytes per atom of one evaluation's PME kernels (k_pme_sites, k_plane_fwd_f, k_zconv_f,
-# k_plane_inv_f, k_pme_gather_f: 5.96 + 4.42 + 12.05 + 12.02 + 16.59 MB, the same capture, 247,488
+# DRAM bytes per atom of one evaluation's PME kernels (k_pme_sites, k_plane_fwd, k_zconv_f,
+# k_plane_inv, k_pme_gather_f: 5.96 + 4.42 + 12.05 + 12.02 + 16.59 MB, the same capture, 247,488
 # atoms, caches flushed before each launch, so an upper bound)
 PME_DRAM_BYTES_PER_ATOM = 206.3
 

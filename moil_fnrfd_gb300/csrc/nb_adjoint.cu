@@ -638,7 +638,7 @@ __device__ __forceinline__ void two_fma(float2 &a, float2 w, float2 v)
     a.y += fmaf(w.x, v.y, fmaf(w.y, v.x, e));
 }
 
-// PME: fc * sum(theta * potential grid) at each site, from the real planes k_plane_inv_f
+// PME: fc * sum(theta * potential grid) at each site, from the real planes k_plane_inv
 // leaves in the grid storage (mixed path).  The weights are formed in FP64 and kept as hi + lo
 // pairs, as are the sums: 64 conversions and 84 FP64 multiply-adds per site took 70 us for 188,448
 // sites on the FP64 pipe, this 38.

@@ -173,7 +173,7 @@ struct EChunk { int rep, kind, begin, end; };
 #define NB_FE_SEG 1024
 
 // Work items of the PME kernels.  They carry their replica's grid (sizes, first complex element) and
-// the place and length of the plans' tables (FP32 path, in 16-byte units of d_blob): a block's loads
+// the place and length of the plans' tables (in 16-byte units of d_blob): a block's loads
 // then depend on one load, not on four in a row.
 struct alignas(16) PlaneWork {
     int rep, z, n1, n2;

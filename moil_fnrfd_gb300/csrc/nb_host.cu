@@ -97,7 +97,7 @@ void release_device(NbCtx *c)
     free_ptr(c->d_wl1_cnt); free_ptr(c->d_wl1); free_ptr(c->d_wl2_off); free_ptr(c->d_wl2); free_ptr(c->d_xl_off);
     free_ptr(c->d_xl); free_ptr(c->d_count_tmp); free_ptr(c->d_ex_off); free_ptr(c->d_ex_j); free_ptr(c->d_p14_off);
     free_ptr(c->d_p14_j); free_ptr(c->d_p14_par); free_ptr(c->d_grad_site); free_ptr(c->d_e_unit);
-    free_ptr(c->d_grad_ex); free_ptr(c->d_e_ex); free_ptr(c->d_plans); free_ptr(c->d_rep_plan); free_ptr(c->d_tw);
+    free_ptr(c->d_grad_ex); free_ptr(c->d_e_ex);
     free_ptr(c->d_blob); free_ptr(c->d_wtiles); free_ptr(c->d_scan_tmp);
     free_ptr(c->d_hblocks); free_ptr(c->d_hrow); free_ptr(c->d_hcnt); free_ptr(c->d_jset); free_ptr(c->d_jn);
     c->hblocks.clear();

@@ -9,11 +9,10 @@
 #include "moil_nb.h"
 #include "nb_common.cuh"
 
-// FFT plan for one length: radices (make_plan), twiddles exp(-2 pi i k / n)
-// at tw0, and per Stockham stage s: the span Ns, the butterfly count nb = n/R, the magic
+// FFT plan for one length: radices (make_plan) and per Stockham stage s: the span Ns, the butterfly count nb = n/R, the magic
 // multiplier for dividing by nb, and nb (twiddle step, destination index) entries at off[s]
 struct FftPlanDev {
-    int n, nst, tw0;
+    int n, nst;
     int rad[8];
     int ns[8];
     int nb[8];
@@ -129,12 +128,7 @@ struct NbCtx {
     double *d_e_ex = nullptr;          // natom*3
 
     // PME
-    std::vector<FftPlanDev> plans;
-    FftPlanDev *d_plans = nullptr;
-    std::vector<int> rep_plan;         // 3 plan indices per replica
-    int *d_rep_plan = nullptr;
-    void *d_tw = nullptr;              // float2 / double2 twiddles
-    int4 *d_blob = nullptr;            // FP32 path: per plan its constants, twiddles and stage table
+    int4 *d_blob = nullptr;            // per FFT plan its constants, twiddles (float2 / double2) and stage table
     std::vector<double> bsp_h;
     void *d_bsp = nullptr;             // float / double moduli
     float *d_etab = nullptr;           // FP32 path: exp(-pi^2 m^2 / (alpha L)^2) / B per dimension (bsp layout)

@@ -24,7 +24,7 @@
 // index arithmetic (twiddle step, destination) read from per-stage tables built on the host
 // and the line number obtained by a multiply-high by a precomputed magic constant.  The
 // last pass of a direction stores transposed, so the next direction reads contiguous lines.
-// The plain FP64 path uses a simpler one-warp-per-line FFT with the same layout.
+// The plain FP64 path runs the same passes in FP64.
 // Inverse transforms are conj(FFT(conj(x))), unnormalised like FFTPACK's cfftb.
 #include <mutex>
 
@@ -315,6 +315,7 @@ __device__ __forceinline__ T eterm_of(const RepDev &R, const T *bsp, int kx, int
 // FP32 path: block-cooperative table-driven Stockham passes
 
 #define NB_TKF 32     // z lines per zconv CTA (FP32 path)
+#define NB_TK 16      // (FP64 path)
 
 // Shared-memory layout of the intermediate results between Stockham stages: element e of a
 // buffer is stored at e + e/16 (one spare slot per 16 float2, i.e. per 128 bytes), so the
@@ -328,23 +329,24 @@ __host__ __device__ __forceinline__ int swz_elems(int m) { return m + (m >> 4) +
 // Where a transform's first stage reads and its last one writes, besides the shared-memory buffers
 enum FftIn { IN_LINES, IN_SPREAD, IN_CONJ, IN_PLANE };
 enum FftOut { OUT_LINES, OUT_SPREAD, OUT_TRANSPOSED, OUT_ROWS };
-struct FftEnds {
-    const float2 *in = nullptr;   // IN_CONJ: lines in global memory, conjugated
-    const int *acc = nullptr;     // IN_PLANE: the int32 charge plane, rows 2l and 2l + 1 as line l
-    float inv = 0.f;
+template <typename T> struct FftEnds {
+    typedef typename cplx<T>::type C;
+    const C *in = nullptr;   // IN_CONJ: lines in global memory, conjugated
+    const typename Acc<T>::type *acc = nullptr;     // IN_PLANE: the charge plane, rows 2l and 2l + 1 as line l
+    T inv = 0;
     int rows = 0;                 // rows of the plane (IN_PLANE, OUT_ROWS)
-    float2 *out = nullptr;        // OUT_LINES: to global memory
-    float *real = nullptr;        // OUT_ROWS: Re and -Im of line l as rows 2l and 2l + 1, in global memory
+    C *out = nullptr;        // OUT_LINES: to global memory
+    T *real = nullptr;        // OUT_ROWS: Re and -Im of line l as rows 2l and 2l + 1
 };
 
 // One Stockham stage over L lines of length n = RADIX * nb.  Source line l at src + l*ss (contiguous)
 // or in the spread layout (IN_SPREAD); destination dst + l*ds, in the spread layout (OUT_SPREAD) or
 // transposed (dst[k*ds + l]); or the ends above.  CONJ_OUT conjugates the stored values.  tab / tw
 // point into shared memory (fft_ctx_load).
-template <int RADIX, int IN, int OUT, bool CONJ_OUT>
-__device__ __forceinline__ void fft_pass_r(const float2 *__restrict__ src, float2 *__restrict__ dst, const FftEnds &E,
+template <int RADIX, int IN, int OUT, bool CONJ_OUT, typename T, typename C>
+__device__ __forceinline__ void fft_pass_r(const C *__restrict__ src, C *__restrict__ dst, const FftEnds<T> &E,
                                            int L, int ss, int ds, int Ns, int nb, unsigned magic,
-                                           const int2 *__restrict__ tab, const float2 *__restrict__ tw)
+                                           const int2 *__restrict__ tab, const C *__restrict__ tw)
 {
     const int total = L * nb;
     for (int b = threadIdx.x; b < total; b += blockDim.x) {
@@ -352,13 +354,16 @@ __device__ __forceinline__ void fft_pass_r(const float2 *__restrict__ src, float
         int j = b - line * nb;
         int2 e = tab[j];
         const int s0 = line * ss + j;
-        float2 v[RADIX];
+        C v[RADIX];
         if (IN == IN_PLANE) {
-            const int *a0 = E.acc + 2 * line * ss + j, *a1 = a0 + ss;
+            const typename Acc<T>::type *a0 = E.acc + 2 * line * ss + j, *a1 = a0 + ss;
             const bool two = 2 * line + 1 < E.rows;
 #pragma unroll
             for (int r = 0; r < RADIX; ++r)
-                v[r] = make_float2(Acc<float>::get(a0[r * nb], E.inv), two ? Acc<float>::get(a1[r * nb], E.inv) : 0.f);
+            {
+                v[r].x = Acc<T>::get(a0[r * nb], E.inv);
+                v[r].y = two ? Acc<T>::get(a1[r * nb], E.inv) : (T)0;
+            }
         } else {
 #pragma unroll
             for (int r = 0; r < RADIX; ++r)
@@ -371,7 +376,7 @@ __device__ __forceinline__ void fft_pass_r(const float2 *__restrict__ src, float
         bfly<RADIX>(v);
 #pragma unroll
         for (int r = 0; r < RADIX; ++r) {
-            float2 o = CONJ_OUT ? cconj(v[r]) : v[r];
+            C o = CONJ_OUT ? cconj(v[r]) : v[r];
             int k = e.y + r * Ns;
             if (OUT == OUT_TRANSPOSED) {
                 dst[k * ds + line] = o;
@@ -387,9 +392,9 @@ __device__ __forceinline__ void fft_pass_r(const float2 *__restrict__ src, float
     __syncthreads();
 }
 
-template <int IN, int OUT, bool CONJ_OUT>
-__device__ __forceinline__ void fft_pass(int R, const float2 *src, float2 *dst, const FftEnds &E, int L, int ss, int ds,
-                                         int Ns, int nb, unsigned magic, const int2 *tab, const float2 *tw)
+template <int IN, int OUT, bool CONJ_OUT, typename T, typename C>
+__device__ __forceinline__ void fft_pass(int R, const C *src, C *dst, const FftEnds<T> &E, int L, int ss, int ds,
+                                         int Ns, int nb, unsigned magic, const int2 *tab, const C *tw)
 {
     switch (R) {
     case 2: fft_pass_r<2, IN, OUT, CONJ_OUT>(src, dst, E, L, ss, ds, Ns, nb, magic, tab, tw); break;
@@ -405,14 +410,14 @@ __device__ __forceinline__ void fft_pass(int R, const float2 *src, float2 *dst, 
 
 // A plan with its twiddles and stage table, staged in shared memory by fft_ctx_load so the
 // butterflies read them without global-memory latency.
-struct FftCtx {
+template <typename C> struct FftCtx {
     const FftPlanDev *p;
     const int2 *tab;      // plan-local: stage s at tab + p->off[s]
-    const float2 *tw;     // plan-local twiddles, n entries
+    const C *tw;     // plan-local twiddles, n entries
 };
 
 // shared-memory bytes of one staged plan of length n
-size_t fft_ctx_bytes(int n, bool wide);
+size_t fft_ctx_bytes(int n, size_t elem);
 
 // copies from global to shared memory that no register and no thread waits for until async_wait
 __device__ __forceinline__ void async_copy16(void *dst, const void *src)
@@ -427,13 +432,14 @@ __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;"
 
 // the tables of a plan of length n: len 16-byte units (plan, twiddles, stage table); complete after
 // async_wait and a barrier
+template <typename C>
 __device__ __forceinline__ unsigned char *fft_ctx_load(unsigned char *dst, const int4 *__restrict__ src, int len, int n,
-                                                       FftCtx &ctx)
+                                                       FftCtx<C> &ctx)
 {
     for (int k = threadIdx.x; k < len; k += blockDim.x) async_copy16(dst + 16 * k, src + k);
     ctx.p = (const FftPlanDev *)dst;
-    ctx.tw = (const float2 *)(dst + align16(sizeof(FftPlanDev)));
-    ctx.tab = (const int2 *)((const unsigned char *)ctx.tw + align16(n * sizeof(float2)));
+    ctx.tw = (const C *)(dst + align16(sizeof(FftPlanDev)));
+    ctx.tab = (const int2 *)((const unsigned char *)ctx.tw + align16(n * sizeof(C)));
     return dst + 16 * (size_t)len;
 }
 
@@ -441,15 +447,15 @@ __device__ __forceinline__ unsigned char *fft_ctx_load(unsigned char *dst, const
 // scratch.  The last pass stores as OUT says with stride out_ds (OUT_TRANSPOSED: the transposed row
 // stride); the stages between keep the spread layout.  Returns the buffer holding the result;
 // CONJ_LAST conjugates the final output (second half of an inverse transform).
-template <int IN, int OUT, bool CONJ_LAST>
-__device__ float2 *fft_lines(const FftCtx &c, float2 *a, float2 *b, const FftEnds &E, int L, int in_ss, int out_ds)
+template <int IN, int OUT, bool CONJ_LAST, typename T, typename C>
+__device__ C *fft_lines(const FftCtx<C> &c, C *a, C *b, const FftEnds<T> &E, int L, int in_ss, int out_ds)
 {
     const FftPlanDev &p = *c.p;
-    float2 *src = a, *dst = b;
+    C *src = a, *dst = b;
     const int n = p.n, nst = p.nst;
     for (int s = 0; s < nst; ++s) {
         const int2 *t = c.tab + p.off[s];
-        float2 *o = s + 1 == nst && E.out ? E.out : dst;
+        C *o = s + 1 == nst && E.out ? E.out : dst;
         if (s + 1 < nst) {
             if (s == 0)
                 fft_pass<IN, OUT_SPREAD, false>(p.rad[s], src, o, E, L, in_ss, n, p.ns[s], p.nb[s], p.magic[s], t, c.tw);
@@ -460,12 +466,12 @@ __device__ float2 *fft_lines(const FftCtx &c, float2 *a, float2 *b, const FftEnd
         } else {
             fft_pass<IN_SPREAD, OUT, CONJ_LAST>(p.rad[s], src, o, E, L, n, out_ds, p.ns[s], p.nb[s], p.magic[s], t, c.tw);
         }
-        float2 *x = src; src = dst; dst = x;
+        C *x = src; src = dst; dst = x;
     }
     return src;
 }
 
-// float2 slots of each of the two plane buffers of the FP32 plane kernels: the packed rows
+// complex slots of each of the two plane buffers of the plane kernels: the packed rows
 // (ceil(n2/2) lines of n1), the half spectrum (n1/2+1 lines of n2, stored with the odd row
 // stride n2|1 after the forward x pass), the transposed inverse y output (n2 rows of stride
 // (n1/2+1)|1), and either kind in the spread layout of the stages between; even, so the
@@ -479,10 +485,11 @@ __host__ __device__ __forceinline__ int plane_buf_elems(int n1, int n2)
     return (m + 1) & ~1;
 }
 
-// float2 slots of each zconv buffer: NB_TKF lines of n3 at the odd stride n3|1 or spread
-__host__ __device__ __forceinline__ int zconv_buf_elems(int n3)
+// complex slots of each zconv buffer: the tile's lines of n3 at the odd stride n3|1 or spread
+template <typename T> __host__ __device__ constexpr int col_tile() { return sizeof(T) == 4 ? NB_TKF : NB_TK; }
+template <typename T> __host__ __device__ __forceinline__ int zconv_buf_elems(int n3)
 {
-    const int a = swz_elems(NB_TKF * n3), b = NB_TKF * (n3 | 1);
+    const int tk = col_tile<T>(), a = swz_elems(tk * n3), b = tk * (n3 | 1);
     return ((a > b ? a : b) + 1) & ~1;
 }
 
@@ -491,47 +498,55 @@ __host__ __device__ __forceinline__ int zconv_buf_elems(int n3)
 // transforms take 65, the selection of the sites 48, their stencils 42.  Two passes per axis (wide
 // radices), the first from the int32 plane and the last to the grid, without a staging copy at either
 // end: 512 replicas 1981 -> 1939 us per evaluation with the inverse's, 24 images 94.5 -> 90.6.
-__global__ void __launch_bounds__(256, 8) k_plane_fwd_f(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 2) k_plane_fwd(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
                                                      const int4 *__restrict__ blob,
                                                      int nW, const unsigned char *__restrict__ zidx,
-                                                     const float4 *__restrict__ fr, float2 *__restrict__ grid)
+                                                     const typename vec4<T>::type *__restrict__ fr,
+                                                     typename cplx<T>::type *__restrict__ grid)
 {
+    typedef typename cplx<T>::type C;
+    typedef typename Acc<T>::type A;
     extern __shared__ __align__(16) unsigned char smem[];
     const PlaneWork w = work[blockIdx.x];
     const RepDev &R = reps[w.rep];
     const int n1 = w.n1, n2 = w.n2, n1h = n1 / 2 + 1, n2p = (n2 + 1) >> 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    float2 *B0 = (float2 *)smem, *B1 = B0 + plane_buf_elems(n1, n2);
-    int *acc = (int *)B0;                        // the int32 plane lives in B0 until it is packed
-    FftCtx c1, c2;
+    C *B0 = (C *)smem, *B1 = B0 + plane_buf_elems(n1, n2);
+    A *acc = (A *)B0;                            // the charge plane lives in B0 until it is packed
+    FftCtx<C> c1, c2;
     unsigned char *ctx = (unsigned char *)(B1 + plane_buf_elems(n1, n2));
     ctx = fft_ctx_load(ctx, blob + w.bx, w.lx, n1, c1);
     fft_ctx_load(ctx, blob + w.by, w.ly, n2, c2);
     for (int k = threadIdx.x; k < n1 * n2; k += blockDim.x) acc[k] = 0;
-    plane_sites(R, nW, w.z, zidx, (int *)B1, 2 * plane_buf_elems(n1, n2),
-                [&](int n) { spread_sites<float>(R, (const int *)B1, n, fr, acc, R.spread216); });
+    plane_sites(R, nW, w.z, zidx, (int *)B1, (int)(sizeof(C) / 4) * plane_buf_elems(n1, n2),
+                [&](int n) { spread_sites<T>(R, (const int *)B1, n, fr, acc, sizeof(T) == 4 ? (T)R.spread216 : (T)1); });
     async_wait();
     __syncthreads();
     // x transform of real rows two at a time: line p carries row 2p as its real part and
     // row 2p+1 as its imaginary part, read from the int32 plane
-    FftEnds ex, ey;
-    ex.acc = acc; ex.inv = R.spread_inv; ex.rows = n2;
-    float2 *Z = fft_lines<IN_PLANE, OUT_LINES, false>(c1, B0, B1, ex, n2p, n1, n1);
-    float2 *T = Z == B1 ? B0 : B1;
+    FftEnds<T> ex, ey;
+    ex.acc = acc; ex.inv = sizeof(T) == 4 ? (T)R.spread_inv : (T)1; ex.rows = n2;
+    C *Z = fft_lines<IN_PLANE, OUT_LINES, false>(c1, B0, B1, ex, n2p, n1, n1);
+    C *X = Z == B1 ? B0 : B1;
     // separate the two real transforms (X_2p = (Z_k + conj Z_-k)/2, X_2p+1 = -i (Z_k - conj Z_-k)/2)
     // and keep kx < n1h, transposed to [kx][y] lines of n2 at the odd row stride sT (the lanes'
     // stores then fall in distinct banks)
     const int sT = n2 | 1;
     for (int p = warp; p < n2p; p += nwarp)
         for (int k = lane; k < n1h; k += 32) {
-            const float2 a = Z[p * n1 + k], b = Z[p * n1 + (k == 0 ? 0 : n1 - k)];
-            T[k * sT + 2 * p] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-            if (2 * p + 1 < n2) T[k * sT + 2 * p + 1] = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
+            const C a = Z[p * n1 + k], b = Z[p * n1 + (k == 0 ? 0 : n1 - k)];
+            const T h = (T)0.5;
+            C u, v;
+            u.x = h * (a.x + b.x); u.y = h * (a.y - b.y);
+            v.x = h * (a.y + b.y); v.y = h * (b.x - a.x);
+            X[k * sT + 2 * p] = u;
+            if (2 * p + 1 < n2) X[k * sT + 2 * p + 1] = v;
         }
     __syncthreads();
     // y: n1h lines of n2, to the grid
     ey.out = grid + w.g0 + (size_t)w.z * n1h * n2;
-    fft_lines<IN_LINES, OUT_LINES, false>(c2, T, Z, ey, n1h, sT, n2);
+    fft_lines<IN_LINES, OUT_LINES, false>(c2, X, Z, ey, n1h, sT, n2);
 }
 
 __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
@@ -546,9 +561,9 @@ __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ 
     const int n1 = w.n1, n2 = w.n2, n3 = w.n3, n1h = n1 / 2 + 1;
     const int tk = w.nky;
     const float *etab = etab_all + w.bsp0;
-    float2 *A = (float2 *)smem, *B = A + zconv_buf_elems(n3);
-    FftCtx c3;
-    fft_ctx_load((unsigned char *)(B + zconv_buf_elems(n3)), blob + w.bz, w.lz, n3, c3);
+    float2 *A = (float2 *)smem, *B = A + zconv_buf_elems<float>(n3);
+    FftCtx<float2> c3;
+    fft_ctx_load((unsigned char *)(B + zconv_buf_elems<float>(n3)), blob + w.bz, w.lz, n3, c3);
     const int sA = n3 | 1;    // odd line stride of the columns as loaded and stored
     float2 *g = grid + w.g0 + (size_t)w.kx * n2 + w.ky0;
     const size_t zs = (size_t)n1h * n2;
@@ -557,7 +572,7 @@ __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ 
         if (lane < tk) async_copy8(A + lane * sA + kz, g + kz * zs + lane);
     async_wait();
     __syncthreads();
-    float2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds(), tk, sA, n3);
+    float2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds<float>(), tk, sA, n3);
     float2 *Fo = F == A ? B : A;
     const float wgt = (w.kx == 0 || 2 * w.kx == n1) ? 1.f : 2.f;
     // influence function exp(-pi^2 m^2 / alpha^2) / (pi V B(m) m^2): the exponential and the
@@ -591,7 +606,7 @@ __global__ void __launch_bounds__(256, 6) k_zconv_f(const ColWork *__restrict__ 
         }
     }
     __syncthreads();
-    float2 *I = fft_lines<IN_LINES, OUT_LINES, true>(c3, F, Fo, FftEnds(), tk, n3, sA);
+    float2 *I = fft_lines<IN_LINES, OUT_LINES, true>(c3, F, Fo, FftEnds<float>(), tk, n3, sA);
     for (int kz = warp; kz < n3; kz += 8)
         if (lane < tk) g[kz * zs + lane] = I[lane * sA + kz];
     // fixed-order reduction: each thread's few terms in FP32, then FP64 across the warp and
@@ -624,9 +639,9 @@ __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict_
     const int n1 = w.n1, n2 = w.n2, n3 = w.n3, n1h = n1 / 2 + 1;
     const int tk = w.nky;
     const float *bsp = bsp_all + w.bsp0;
-    float2 *A = (float2 *)smem, *B = A + zconv_buf_elems(n3);
-    FftCtx c3;
-    fft_ctx_load((unsigned char *)(B + zconv_buf_elems(n3)), blob + w.bz, w.lz, n3, c3);
+    float2 *A = (float2 *)smem, *B = A + zconv_buf_elems<float>(n3);
+    FftCtx<float2> c3;
+    fft_ctx_load((unsigned char *)(B + zconv_buf_elems<float>(n3)), blob + w.bz, w.lz, n3, c3);
     const int sA = n3 | 1;
     const float2 *g = grid + w.g0 + (size_t)w.kx * n2 + w.ky0;
     const size_t zs = (size_t)n1h * n2;
@@ -635,7 +650,7 @@ __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict_
         if (lane < tk) async_copy8(A + lane * sA + kz, g + kz * zs + lane);
     async_wait();
     __syncthreads();
-    const float2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds(), tk, sA, n3);
+    const float2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds<float>(), tk, sA, n3);
     const float wgt = (w.kx == 0 || 2 * w.kx == n1) ? 1.f : 2.f;
     const float fac2 = R.pme_fac2f, pivol = R.pivolf, fac = (float)R.pme_fac;
     const int nf2 = (n2 + 1) / 2, nf3 = (n3 + 1) / 2;
@@ -677,49 +692,68 @@ __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict_
 // over the plane's own complex storage, which this block alone reads, for k_pme_gather_f
 // Inverse y and x transforms of plane z (the comment above): the first pass reads the grid and the last
 // one stores the real rows.
-__global__ void __launch_bounds__(256, 8) k_plane_inv_f(const PlaneWork *__restrict__ work,
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 2) k_plane_inv(const PlaneWork *__restrict__ work,
                                                      const int4 *__restrict__ blob,
-                                                     float2 *__restrict__ grid)
+                                                     typename cplx<T>::type *__restrict__ grid, const RepDev *__restrict__ reps, int nW,
+                                                     const unsigned char *__restrict__ zidx,
+                                                     const typename vec4<T>::type *__restrict__ fr,
+                                                     T *__restrict__ part, int pot)
 {
+    typedef typename cplx<T>::type C;
     extern __shared__ __align__(16) unsigned char smem[];
     const PlaneWork w = work[blockIdx.x];
     const int n1 = w.n1, n2 = w.n2, n1h = n1 / 2 + 1, n2p = (n2 + 1) >> 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    float2 *B0 = (float2 *)smem, *B1 = B0 + plane_buf_elems(n1, n2);
-    FftCtx c1, c2;
+    C *B0 = (C *)smem, *B1 = B0 + plane_buf_elems(n1, n2);
+    FftCtx<C> c1, c2;
     unsigned char *ctx = (unsigned char *)(B1 + plane_buf_elems(n1, n2));
     ctx = fft_ctx_load(ctx, blob + w.bx, w.lx, n1, c1);
     fft_ctx_load(ctx, blob + w.by, w.ly, n2, c2);
-    float2 *g = grid + w.g0 + (size_t)w.z * n1h * n2;
+    C *g = grid + w.g0 + (size_t)w.z * n1h * n2;
     async_wait();
     __syncthreads();
     // y: n1h lines [kx][ky] of n2 from the grid, conjugated (inverse through the forward transform); the
     // last pass conjugates back and stores transposed to H[ky][kx] at the odd row stride hs
     const int hs = n1h | 1;
-    FftEnds ey, ex;
+    FftEnds<T> ey, ex;
     ey.in = g;
-    float2 *H = fft_lines<IN_CONJ, OUT_TRANSPOSED, true>(c2, B1, B0, ey, n1h, n2, hs);
-    float2 *Zc = H == B0 ? B1 : B0;
+    C *H = fft_lines<IN_CONJ, OUT_TRANSPOSED, true>(c2, B1, B0, ey, n1h, n2, hs);
+    C *Zc = H == B0 ? B1 : B0;
     // x inverse of two real rows at a time: Z = H_2p + i H_2p+1 over the full Hermitian line of
     // n1, conjugated so the forward transform inverts it; row 2p = Re, row 2p+1 = -Im of the result
     for (int p = warp; p < n2p; p += nwarp)
         for (int k = lane; k < n1; k += 32) {
             const bool lo = k < n1h;
             const int kk = lo ? k : n1 - k;
-            float2 a = H[2 * p * hs + kk];
-            float2 b = 2 * p + 1 < n2 ? H[(2 * p + 1) * hs + kk] : make_float2(0.f, 0.f);
+            C a = H[2 * p * hs + kk], b;
+            b.x = b.y = (T)0;
+            if (2 * p + 1 < n2) b = H[(2 * p + 1) * hs + kk];
             if (!lo) { a = cconj(a); b = cconj(b); }
-            Zc[p * n1 + k] = make_float2(a.x - b.y, -(a.y + b.x));
+            C z;
+            z.x = a.x - b.y; z.y = -(a.y + b.x);
+            Zc[p * n1 + k] = z;
         }
     __syncthreads();
-    // the real potential plane over the plane's own complex storage (this block alone reads it)
-    ex.real = (float *)g; ex.rows = n2;
-    fft_lines<IN_LINES, OUT_ROWS, false>(c1, Zc, H, ex, n2p, n1, n1);
+    ex.rows = n2;
+    if constexpr (sizeof(T) == 4) {
+        // the real potential plane over the plane's own complex storage (this block alone reads it)
+        ex.real = (T *)g;
+        fft_lines<IN_LINES, OUT_ROWS, false>(c1, Zc, H, ex, n2p, n1, n1);
+    } else {
+        // the real plane in the buffer that the last pass does not read, the other one for the queue
+        C *rows = (c1.p->nst & 1) ? H : Zc, *queue = rows == H ? Zc : H;
+        ex.real = (T *)rows;
+        fft_lines<IN_LINES, OUT_ROWS, false>(c1, Zc, H, ex, n2p, n1, n1);
+        plane_sites(reps[w.rep], nW, w.z, zidx, (int *)queue, (int)(sizeof(C) / 4) * plane_buf_elems(n1, n2), [&](int n) {
+            gather_sites<T>(reps[w.rep], (const int *)queue, n, fr, (const T *)rows, part, pot != 0);
+        });
+    }
 }
 
 // PME gradient of each site from the real potential grid (grad_sum,
 // ewald_receip.f:815-970): order-4 weights and derivatives once per site, the 4x4x4 stencil
-// read from the grid planes k_plane_inv_f left in place; result (x, y, z) per site, to be
+// read from the grid planes k_plane_inv left in place; result (x, y, z) per site, to be
 // scaled by q * fc * n_d / L_d in the finalize.  LPS lanes per site, a share of the stencil's planes
 // each (their sums are added in plane order, so the result does not depend on LPS).  Bound: latency
 // of the 16 row loads while the sites do not fill the GPU, the issue of the stencil arithmetic
@@ -808,139 +842,48 @@ __global__ void __launch_bounds__(256, 4) k_pme_gather_f(int nsite, const int *_
 }
 
 // =================================================================================
-// FP64 (plain) path: one warp per line, same grid layout [z][kx][ky]
-
-template <typename C>
-__device__ C *warp_fft(C *x, C *y, const FftPlanDev &p, const C *__restrict__ tw, int lane)
+// FP64 (plain) path: the same planes and passes in FP64; the influence function with its exponential
+// and division per point, in FP64.  One warp per line with a butterfly per lane used 5 lanes in 32 of
+// the FP64 pipe for lines of 20: PME stages of 216 waters 131 us, 1,334 waters 211; shared by the block,
+// two real rows per x transform, 62 and 109.
+__global__ void __launch_bounds__(256) k_zconv_d(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
+                                                 const int4 *__restrict__ blob, const double *__restrict__ bsp_all,
+                                                 double2 *__restrict__ grid, double *__restrict__ e_col)
 {
-    int n = p.n, Ns = 1;
-    for (int st = 0; st < p.nst; ++st) {
-        int R = p.rad[st], nb = n / R, stride = n / (Ns * R);
-        for (int j = lane; j < nb; j += 32) {
-            C v[5];
-            int jm = j % Ns;
-            for (int r = 0; r < R; ++r) v[r] = x[j + r * nb];
-            int tstep = jm * stride;
-            for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw[r * tstep]);
-            if (R == 4) bfly4(v);
-            else if (R == 2) bfly2(v);
-            else if (R == 3) bfly3(v);
-            else bfly5(v);
-            int idxD = (j / Ns) * Ns * R + jm;
-            for (int r = 0; r < R; ++r) y[idxD + r * Ns] = v[r];
-        }
-        __syncwarp();
-        C *t = x; x = y; y = t;
-        Ns *= R;
-    }
-    return x;
-}
-
-#define NB_TK 16
-// ints in the line buffers of the one-warp-per-line kernels (two lines for each of 8 warps)
-template <typename C> constexpr int NB_SCR_INTS = (int)(sizeof(C) * 8 * 2 * NB_MAX_FFT / sizeof(int));
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_plane_fwd(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                                   const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                                   const void *tw_v, int nW, const unsigned char *__restrict__ zidx,
-                                                   const void *fr_v, void *grid_v)
-{
-    typedef typename cplx<T>::type C;
-    typedef typename Acc<T>::type A;
-    extern __shared__ __align__(16) unsigned char smem[];
-    PlaneWork w = work[blockIdx.x];
-    const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n1h = R.n1h, pitch = n1h | 1;
-    const FftPlanDev p1 = plans[rep_plan[3 * w.rep]], p2 = plans[rep_plan[3 * w.rep + 1]];
-    const C *tw = (const C *)tw_v;
-    A *acc = (A *)smem;
-    C *P = (C *)(smem + align16(sizeof(A) * n1 * n2));
-    C *scr = P + n2 * pitch;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int k = threadIdx.x; k < n1 * n2; k += blockDim.x) acc[k] = 0;
-    // the line buffers, free until the transforms, hold the queue
-    plane_sites(R, nW, w.z, zidx, (int *)scr, NB_SCR_INTS<C>, [&](int n) {
-        spread_sites<T>(R, (const int *)scr, n, (const typename vec4<T>::type *)fr_v, acc, (T)1);
-    });
-    __syncthreads();
-    C *x = scr + warp * 2 * NB_MAX_FFT, *y = x + NB_MAX_FFT;
-    for (int j = warp; j < n2; j += nwarp) {
-        for (int i = lane; i < n1; i += 32) { x[i].x = Acc<T>::get(acc[j * n1 + i], (T)1); x[i].y = 0; }
-        __syncwarp();
-        C *res = warp_fft<C>(x, y, p1, tw + p1.tw0, lane);
-        for (int k = lane; k < n1h; k += 32) P[j * pitch + k] = res[k];
-        __syncwarp();
-    }
-    __syncthreads();
-    for (int k = warp; k < n1h; k += nwarp) {
-        for (int j = lane; j < n2; j += 32) x[j] = P[j * pitch + k];
-        __syncwarp();
-        C *res = warp_fft<C>(x, y, p2, tw + p2.tw0, lane);
-        for (int j = lane; j < n2; j += 32) P[j * pitch + k] = res[j];
-        __syncwarp();
-    }
-    __syncthreads();
-    C *g = (C *)grid_v + R.g0 + (size_t)w.z * n2 * n1h;
-    for (int idx = threadIdx.x; idx < n2 * n1h; idx += blockDim.x) {
-        int kx = idx / n2, ky = idx - kx * n2;
-        g[idx] = P[ky * pitch + kx];
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_zconv(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                               const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                               const void *tw_v, const void *bsp_v, void *grid_v,
-                                               double *__restrict__ e_col)
-{
-    typedef typename cplx<T>::type C;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double red[256];
-    ColWork w = work[blockIdx.x];
+    const ColWork w = work[blockIdx.x];
     const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n3 = R.n3, n1h = R.n1h;
-    const int tk = w.nky;
-    const int n3p = n3 | 1;
-    const FftPlanDev p3 = plans[rep_plan[3 * w.rep + 2]];
-    const C *tw = (const C *)tw_v;
-    const T *bsp = (const T *)bsp_v + R.bsp0;
-    C *tile = (C *)smem;
-    C *scr = tile + NB_TK * n3p;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    C *g = (C *)grid_v + R.g0 + (size_t)w.kx * n2 + w.ky0;
+    const int n1 = w.n1, n2 = w.n2, n3 = w.n3, n1h = n1 / 2 + 1, tk = w.nky;
+    const double *bsp = bsp_all + w.bsp0;
+    double2 *A = (double2 *)smem, *B = A + zconv_buf_elems<double>(n3);
+    FftCtx<double2> c3;
+    fft_ctx_load((unsigned char *)(B + zconv_buf_elems<double>(n3)), blob + w.bz, w.lz, n3, c3);
+    const int sA = n3 | 1;
+    double2 *g = grid + w.g0 + (size_t)w.kx * n2 + w.ky0;
     const size_t zs = (size_t)n1h * n2;
     for (int idx = threadIdx.x; idx < tk * n3; idx += blockDim.x) {
-        int kz = idx / tk, c = idx - kz * tk;
-        tile[c * n3p + kz] = g[kz * zs + c];
+        const int kz = idx / tk, c = idx - kz * tk;
+        A[c * sA + kz] = g[kz * zs + c];
     }
+    async_wait();
     __syncthreads();
-    double en = 0;
-    C *x = scr + warp * 2 * NB_MAX_FFT, *y = x + NB_MAX_FFT;
-    const T wgt = (w.kx == 0 || (2 * w.kx == n1)) ? (T)1 : (T)2;
-    for (int c = warp; c < tk; c += nwarp) {
-        const int ky = w.ky0 + c;
-        for (int kz = lane; kz < n3; kz += 32) x[kz] = tile[c * n3p + kz];
-        __syncwarp();
-        C *res = warp_fft<C>(x, y, p3, tw + p3.tw0, lane);
-        for (int kz = lane; kz < n3; kz += 32) {
-            T et = eterm_of<T>(R, bsp, w.kx, ky, kz);
-            C v = res[kz];
-            en += (double)(wgt * et * (v.x * v.x + v.y * v.y));
-            v.x *= et;
-            v.y *= et;
-            res[kz] = cconj(v);
-        }
-        __syncwarp();
-        C *other = (res == x) ? y : x;
-        C *res2 = warp_fft<C>(res, other, p3, tw + p3.tw0, lane);
-        for (int kz = lane; kz < n3; kz += 32) tile[c * n3p + kz] = cconj(res2[kz]);
-        __syncwarp();
-    }
-    __syncthreads();
+    double2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds<double>(), tk, sA, n3);
+    double2 *Fo = F == A ? B : A;
+    const double wgt = (w.kx == 0 || 2 * w.kx == n1) ? 1.0 : 2.0;
+    double en = 0.0;
     for (int idx = threadIdx.x; idx < tk * n3; idx += blockDim.x) {
-        int kz = idx / tk, c = idx - kz * tk;
-        g[kz * zs + c] = tile[c * n3p + kz];
+        const int c = idx / n3, kz = idx - c * n3;
+        const double et = eterm_of<double>(R, bsp, w.kx, w.ky0 + c, kz);
+        const double2 v = F[idx];
+        en += wgt * et * (v.x * v.x + v.y * v.y);
+        F[idx] = make_double2(v.x * et, -v.y * et);      // conj: the inverse runs forward
+    }
+    __syncthreads();
+    double2 *I = fft_lines<IN_LINES, OUT_LINES, true>(c3, F, Fo, FftEnds<double>(), tk, n3, sA);
+    for (int idx = threadIdx.x; idx < tk * n3; idx += blockDim.x) {
+        const int kz = idx / tk, c = idx - kz * tk;
+        g[kz * zs + c] = I[c * sA + kz];
     }
     red[threadIdx.x] = en;
     __syncthreads();
@@ -951,58 +894,47 @@ __global__ void __launch_bounds__(256) k_zconv(const ColWork *__restrict__ work,
     if (threadIdx.x == 0) e_col[blockIdx.x] = red[0];
 }
 
-// reciprocal virial of the pressure analysis on the plain path: the z transform of k_zconv's
-// columns (one warp per line), then per m the diagonal terms
+// reciprocal virial of the pressure analysis on the plain path: the z transform of k_zconv_d's
+// columns, then per m the diagonal terms
 // E(m) (1 - 2 (1 + pi^2 m^2 / alpha^2) m_a^2 / m^2) (ewald_receip.f:799-807), E(m) as the
 // energy sum forms it; three FP64 sums per column work item
-template <typename T>
-__global__ void __launch_bounds__(256) k_press_zvir(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                                    const FftPlanDev *__restrict__ plans,
-                                                    const int *__restrict__ rep_plan, const void *tw_v,
-                                                    const void *bsp_v, const void *grid_v, double *__restrict__ v_col)
+__global__ void __launch_bounds__(256) k_press_zvir_d(const ColWork *__restrict__ work, const RepDev *__restrict__ reps,
+                                                      const int4 *__restrict__ blob, const double *__restrict__ bsp_all,
+                                                      const double2 *__restrict__ grid, double *__restrict__ v_col)
 {
-    typedef typename cplx<T>::type C;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double red[3][256];
     const ColWork w = work[blockIdx.x];
     const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n3 = R.n3, n1h = R.n1h;
-    const int tk = w.nky;
-    const int n3p = n3 | 1;
-    const FftPlanDev p3 = plans[rep_plan[3 * w.rep + 2]];
-    const C *tw = (const C *)tw_v;
-    const T *bsp = (const T *)bsp_v + R.bsp0;
-    C *tile = (C *)smem;
-    C *scr = tile + NB_TK * n3p;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    const C *g = (const C *)grid_v + R.g0 + (size_t)w.kx * n2 + w.ky0;
+    const int n1 = w.n1, n2 = w.n2, n3 = w.n3, n1h = n1 / 2 + 1, tk = w.nky;
+    const double *bsp = bsp_all + w.bsp0;
+    double2 *A = (double2 *)smem, *B = A + zconv_buf_elems<double>(n3);
+    FftCtx<double2> c3;
+    fft_ctx_load((unsigned char *)(B + zconv_buf_elems<double>(n3)), blob + w.bz, w.lz, n3, c3);
+    const int sA = n3 | 1;
+    const double2 *g = grid + w.g0 + (size_t)w.kx * n2 + w.ky0;
     const size_t zs = (size_t)n1h * n2;
     for (int idx = threadIdx.x; idx < tk * n3; idx += blockDim.x) {
         const int kz = idx / tk, c = idx - kz * tk;
-        tile[c * n3p + kz] = g[kz * zs + c];
+        A[c * sA + kz] = g[kz * zs + c];
     }
+    async_wait();
     __syncthreads();
+    const double2 *F = fft_lines<IN_LINES, OUT_LINES, false>(c3, A, B, FftEnds<double>(), tk, sA, n3);
     double v[3] = {0.0, 0.0, 0.0};
-    C *x = scr + warp * 2 * NB_MAX_FFT, *y = x + NB_MAX_FFT;
     const double wgt = (w.kx == 0 || (2 * w.kx == n1)) ? 1.0 : 2.0;
     const int nf2 = (n2 + 1) / 2, nf3 = (n3 + 1) / 2;
-    for (int c = warp; c < tk; c += nwarp) {
-        const int ky = w.ky0 + c;
-        for (int kz = lane; kz < n3; kz += 32) x[kz] = tile[c * n3p + kz];
-        __syncwarp();
-        const C *res = warp_fft<C>(x, y, p3, tw + p3.tw0, lane);
-        for (int kz = lane; kz < n3; kz += 32) {
-            if (w.kx == 0 && ky == 0 && kz == 0) continue;
-            const double mh[3] = {(double)w.kx * R.invLd[0], (double)(ky < nf2 ? ky : ky - n2) * R.invLd[1],
-                                  (double)(kz < nf3 ? kz : kz - n3) * R.invLd[2]};
-            const double msq = mh[0] * mh[0] + mh[1] * mh[1] + mh[2] * mh[2];
-            const double et = (double)eterm_of<T>(R, bsp, w.kx, ky, kz);
-            const C q = res[kz];
-            const double e = wgt * et * ((double)q.x * q.x + (double)q.y * q.y), b = 2.0 * (1.0 + R.pme_fac * msq) / msq;
+    for (int idx = threadIdx.x; idx < tk * n3; idx += blockDim.x) {
+        const int c = idx / n3, kz = idx - c * n3, ky = w.ky0 + c;
+        if (w.kx == 0 && ky == 0 && kz == 0) continue;
+        const double mh[3] = {(double)w.kx * R.invLd[0], (double)(ky < nf2 ? ky : ky - n2) * R.invLd[1],
+                              (double)(kz < nf3 ? kz : kz - n3) * R.invLd[2]};
+        const double msq = mh[0] * mh[0] + mh[1] * mh[1] + mh[2] * mh[2];
+        const double et = eterm_of<double>(R, bsp, w.kx, ky, kz);
+        const double2 q = F[idx];
+        const double e = wgt * et * (q.x * q.x + q.y * q.y), b = 2.0 * (1.0 + R.pme_fac * msq) / msq;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) v[d] += e * (1.0 - b * mh[d] * mh[d]);
-        }
-        __syncwarp();
+        for (int d = 0; d < 3; ++d) v[d] += e * (1.0 - b * mh[d] * mh[d]);
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) red[d][threadIdx.x] = v[d];
@@ -1017,57 +949,6 @@ __global__ void __launch_bounds__(256) k_press_zvir(const ColWork *__restrict__ 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_plane_inv(const PlaneWork *__restrict__ work, const RepDev *__restrict__ reps,
-                                                   const FftPlanDev *__restrict__ plans, const int *__restrict__ rep_plan,
-                                                   const void *tw_v, int nW, const unsigned char *__restrict__ zidx,
-                                                   const void *fr_v, const void *grid_v, T *__restrict__ part, int pot)
-{
-    typedef typename cplx<T>::type C;
-    extern __shared__ __align__(16) unsigned char smem[];
-    PlaneWork w = work[blockIdx.x];
-    const RepDev &R = reps[w.rep];
-    const int n1 = R.n1, n2 = R.n2, n1h = R.n1h, pitch = n1h | 1;
-    const FftPlanDev p1 = plans[rep_plan[3 * w.rep]], p2 = plans[rep_plan[3 * w.rep + 1]];
-    const C *tw = (const C *)tw_v;
-    T *Rp = (T *)smem;
-    C *P = (C *)(smem + align16(sizeof(T) * n1 * n2));
-    C *scr = P + n2 * pitch;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    const C *g = (const C *)grid_v + R.g0 + (size_t)w.z * n2 * n1h;
-    for (int idx = threadIdx.x; idx < n2 * n1h; idx += blockDim.x) {
-        int kx = idx / n2, ky = idx - kx * n2;
-        P[ky * pitch + kx] = g[idx];
-    }
-    __syncthreads();
-    C *x = scr + warp * 2 * NB_MAX_FFT, *y = x + NB_MAX_FFT;
-    for (int k = warp; k < n1h; k += nwarp) {
-        for (int j = lane; j < n2; j += 32) x[j] = cconj(P[j * pitch + k]);
-        __syncwarp();
-        C *res = warp_fft<C>(x, y, p2, tw + p2.tw0, lane);
-        for (int j = lane; j < n2; j += 32) P[j * pitch + k] = cconj(res[j]);
-        __syncwarp();
-    }
-    __syncthreads();
-    for (int j = warp; j < n2; j += nwarp) {
-        for (int i = lane; i < n1; i += 32) {
-            C v = i < n1h ? P[j * pitch + i] : cconj(P[j * pitch + (n1 - i)]);
-            x[i] = cconj(v);
-        }
-        __syncwarp();
-        C *res = warp_fft<C>(x, y, p1, tw + p1.tw0, lane);
-        for (int i = lane; i < n1; i += 32) Rp[j * n1 + i] = res[i].x;
-        __syncwarp();
-    }
-    __syncthreads();
-    plane_sites(R, nW, w.z, zidx, (int *)scr, NB_SCR_INTS<C>, [&](int n) {
-        gather_sites<T>(R, (const int *)scr, n, (const typename vec4<T>::type *)fr_v, Rp, part, pot != 0);
-    });
-}
-
-// ---------------------------------------------------------------------------------
-// launch sequence (both precisions)
-
-template <typename T>
 void pme_t(NbCtx *c)
 {
     cudaStream_t s = c->stream;
@@ -1077,15 +958,22 @@ void pme_t(NbCtx *c)
                                                                     c->d_site_q, c->d_fr, c->d_zidx);
         c->launches++;
     }
+    typedef typename cplx<T>::type C;
+    typedef typename vec4<T>::type T4;
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
-    if (sizeof(T) == 4) {
-        k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
-                                                           (const float4 *)c->d_fr, (float2 *)c->d_grid);
-        if (c->timing) cudaEventRecord(c->ev[7], s);
-        k_zconv_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, c->d_etab,
-                                                  (float2 *)c->d_grid, c->d_e_col);
-        if (c->timing) cudaEventRecord(c->ev[8], s);
-        k_plane_inv_f<<<np, 256, c->smem_plane_inv, s>>>(c->d_planes, c->d_blob, (float2 *)c->d_grid);
+    k_plane_fwd<T><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
+                                                      (const T4 *)c->d_fr, (C *)c->d_grid);
+    if (c->timing) cudaEventRecord(c->ev[7], s);
+    if constexpr (sizeof(T) == 4)
+        k_zconv_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, c->d_etab, (float2 *)c->d_grid,
+                                                 c->d_e_col);
+    else
+        k_zconv_d<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, (const double *)c->d_bsp,
+                                                 (double2 *)c->d_grid, c->d_e_col);
+    if (c->timing) cudaEventRecord(c->ev[8], s);
+    k_plane_inv<T><<<np, 256, c->smem_plane_inv, s>>>(c->d_planes, c->d_blob, (C *)c->d_grid, c->d_reps, (int)c->nW,
+                                                      c->d_zidx, (const T4 *)c->d_fr, (T *)c->d_part, 0);
+    if constexpr (sizeof(T) == 4) {
         // four lanes per site while they all fit the GPU at once (an evaluation of 216 waters 50.7 / 47.2 us
         // with 1 / 4, 460 waters and 203 atoms 65.0 / 61.1, 42,000 waters 148 / 148, 229,000 558 / 576)
         const int lps = c->nsite <= 40000 ? 4 : 1;
@@ -1093,26 +981,14 @@ void pme_t(NbCtx *c)
             (int)c->nsite, c->d_site_rep, c->d_reps, (const float4 *)c->d_fr, (const float2 *)c->d_grid,
             (float4 *)c->d_part);
         c->launches++;
-    } else {
-        k_plane_fwd<T><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
-                                                          (int)c->nW, c->d_zidx, c->d_fr, c->d_grid);
-        if (c->timing) cudaEventRecord(c->ev[7], s);
-        k_zconv<T><<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
-                                                   c->d_bsp, c->d_grid, c->d_e_col);
-        if (c->timing) cudaEventRecord(c->ev[8], s);
-        k_plane_inv<T><<<np, 256, c->smem_plane_inv, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
-                                                          (int)c->nW, c->d_zidx, c->d_fr, c->d_grid,
-                                                          (T *)c->d_part, 0);
     }
     if (c->timing) cudaEventRecord(c->ev[9], s);
     c->launches += 3;
 }
 
-// radix plan and Stockham tables; returns 0 if n is not 2/3/5-smooth or too long.  Narrow
-// plans (the FP64 one-warp-per-line transform) take 4s first, then 2, 3, 5.  Wide plans (FP32)
-// also have the composite codelets 6, 8, 9, 10 and take the fewest passes (a line of up to 100
-// points in two), the most even split on ties.  tab
-// receives (twiddle step, destination index) per butterfly.
+// radix plan and Stockham tables; returns 0 if n is not 2/3/5-smooth or too long.  Radices 2 to 10,
+// the fewest passes (a line of up to 100 points in two), the most even split on ties.  tab receives
+// (twiddle step, destination index) per butterfly.
 // fewest factors of m from the wide radix set, at most `left` of them, and of those the smallest sum
 // (the most even split: the longest butterfly sets the time of a pass); its count, -1 if none
 int wide_factors(int m, int left, int *out)
@@ -1136,23 +1012,13 @@ int wide_factors(int m, int left, int *out)
     return best;
 }
 
-int make_plan(int n, FftPlanDev *p, std::vector<int2> *tab, bool wide)
+int make_plan(int n, FftPlanDev *p, std::vector<int2> *tab)
 {
     memset(p, 0, sizeof(*p));
     p->n = n;
-    int m = n, k = 0;
     if (n < 2 || n > NB_MAX_FFT) return 0;
-    if (wide) {
-        k = wide_factors(n, 8, p->rad);
-        if (k < 0) return 0;
-        m = 1;
-    } else {
-        while (m % 4 == 0) { p->rad[k++] = 4; m /= 4; }
-        while (m % 2 == 0) { p->rad[k++] = 2; m /= 2; }
-        while (m % 3 == 0) { p->rad[k++] = 3; m /= 3; }
-        while (m % 5 == 0) { p->rad[k++] = 5; m /= 5; }
-    }
-    if (m != 1 || k > 8) return 0;
+    const int k = wide_factors(n, 8, p->rad);
+    if (k < 0) return 0;
     p->nst = k;
     int Ns = 1, off = 0;
     for (int s = 0; s < k; ++s) {
@@ -1173,39 +1039,26 @@ int make_plan(int n, FftPlanDev *p, std::vector<int2> *tab, bool wide)
     return 1;
 }
 
-size_t fft_ctx_bytes(int n, bool wide)
+size_t fft_ctx_bytes(int n, size_t elem)
 {
     FftPlanDev p;
-    if (!make_plan(n, &p, nullptr, wide)) return 0;
+    if (!make_plan(n, &p, nullptr)) return 0;
     size_t ntab = (size_t)p.off[p.nst - 1] + p.nb[p.nst - 1];
-    return align16(sizeof(FftPlanDev)) + align16(ntab * sizeof(int2)) + align16(n * sizeof(float2));
+    return align16(sizeof(FftPlanDev)) + align16(ntab * sizeof(int2)) + align16(n * elem);
 }
 
 template <typename T>
-size_t plane_fwd_smem(int n1, int n2)
+size_t plane_smem(int n1, int n2)
 {
-    if (sizeof(T) == 4) return (size_t)2 * plane_buf_elems(n1, n2) * sizeof(float2) + fft_ctx_bytes(n1, true) + fft_ctx_bytes(n2, true);
-    typedef typename cplx<T>::type C;
-    size_t acc = (sizeof(typename Acc<T>::type) * n1 * n2 + 15) & ~(size_t)15;
-    return acc + sizeof(C) * n2 * ((n1 / 2 + 1) | 1) + sizeof(C) * 8 * 2 * NB_MAX_FFT;
-}
-template <typename T>
-size_t plane_inv_smem(int n1, int n2)
-{
-    if (sizeof(T) == 4) return (size_t)2 * plane_buf_elems(n1, n2) * sizeof(float2) + fft_ctx_bytes(n1, true) + fft_ctx_bytes(n2, true);
-    typedef typename cplx<T>::type C;
-    size_t r = (sizeof(T) * n1 * n2 + 15) & ~(size_t)15;
-    return r + sizeof(C) * n2 * ((n1 / 2 + 1) | 1) + sizeof(C) * 8 * 2 * NB_MAX_FFT;
+    const size_t e = sizeof(typename cplx<T>::type);
+    return 2 * e * plane_buf_elems(n1, n2) + fft_ctx_bytes(n1, e) + fft_ctx_bytes(n2, e);
 }
 template <typename T>
 size_t zconv_smem(int n3)
 {
-    if (sizeof(T) == 4) return (size_t)2 * zconv_buf_elems(n3) * sizeof(float2) + fft_ctx_bytes(n3, true);
-    typedef typename cplx<T>::type C;
-    return sizeof(C) * NB_TK * (n3 | 1) + sizeof(C) * 8 * 2 * NB_MAX_FFT;
+    const size_t e = sizeof(typename cplx<T>::type);
+    return 2 * e * zconv_buf_elems<T>(n3) + fft_ctx_bytes(n3, e);
 }
-template <typename T> int col_tile() { return sizeof(T) == 4 ? NB_TKF : NB_TK; }
-
 // the z-column work items of one kx: the n2 columns in ceil(n2 / tile) runs of equal length
 // (within one), so no block of the column kernels works on a short remainder alone (n2 = 36
 // gives two runs of 18, not 32 and 4: every Stockham pass of a run then fits one sweep of the
@@ -1224,12 +1077,13 @@ void push_col_runs(std::vector<ColWork> &cols, ColWork w, int tile)
     }
 }
 
-// one plan's tables as the FP32 kernels stage them (fft_ctx_load), appended to blob; its offset and
+// one plan's tables as the kernels stage them (fft_ctx_load), appended to blob; its offset and
 // length in 16-byte units
-void push_blob(std::vector<int4> &blob, const FftPlanDev &p, const std::vector<int2> &tab, const std::vector<float2> &tw,
+template <typename C>
+void push_blob(std::vector<int4> &blob, const FftPlanDev &p, const std::vector<int2> &tab, const std::vector<C> &tw,
                int *off, int *len)
 {
-    const size_t b0 = align16(sizeof(FftPlanDev)), b1 = b0 + align16(p.n * sizeof(float2)),
+    const size_t b0 = align16(sizeof(FftPlanDev)), b1 = b0 + align16(p.n * sizeof(C)),
                  b2 = b1 + align16(tab.size() * sizeof(int2));
     *off = (int)blob.size();
     *len = (int)(b2 / 16);
@@ -1237,7 +1091,7 @@ void push_blob(std::vector<int4> &blob, const FftPlanDev &p, const std::vector<i
     unsigned char *d = (unsigned char *)(blob.data() + *off);
     memset(d, 0, b2);
     memcpy(d, &p, sizeof(p));
-    memcpy(d + b0, tw.data(), p.n * sizeof(float2));
+    memcpy(d + b0, tw.data(), p.n * sizeof(C));
     memcpy(d + b1, tab.data(), tab.size() * sizeof(int2));
 }
 
@@ -1256,69 +1110,51 @@ template <typename T>
 cudaError_t raise_pme_limits(size_t sf, size_t sz, size_t si)
 {
     cudaError_t e;
-    if (sizeof(T) == 4) {
-        if ((e = raise_smem_limit(k_plane_fwd_f, sf)) != cudaSuccess) return e;
-        if ((e = raise_smem_limit(k_zconv_f, sz)) != cudaSuccess) return e;
-        if ((e = raise_smem_limit(k_press_zvir_f, sz)) != cudaSuccess) return e;
-        return raise_smem_limit(k_plane_inv_f, si);
-    }
     if ((e = raise_smem_limit(k_plane_fwd<T>, sf)) != cudaSuccess) return e;
-    if ((e = raise_smem_limit(k_zconv<T>, sz)) != cudaSuccess) return e;
-    if ((e = raise_smem_limit(k_press_zvir<T>, sz)) != cudaSuccess) return e;
-    return raise_smem_limit(k_plane_inv<T>, si);
+    if ((e = raise_smem_limit(k_plane_inv<T>, si)) != cudaSuccess) return e;
+    if constexpr (sizeof(T) == 4) {
+        if ((e = raise_smem_limit(k_zconv_f, sz)) != cudaSuccess) return e;
+        return raise_smem_limit(k_press_zvir_f, sz);
+    } else {
+        if ((e = raise_smem_limit(k_zconv_d, sz)) != cudaSuccess) return e;
+        return raise_smem_limit(k_press_zvir_d, sz);
+    }
 }
 
 template <typename T>
 int configure_t(NbCtx *c)
 {
     typedef typename cplx<T>::type C;
-    c->plans.clear();
-    c->rep_plan.assign(3 * c->nrep, 0);
-    std::vector<double> twr, twi;
+    // plans by length: tables laid out as the kernels stage them
+    std::vector<int> plan_n, boff, blen, rep_plan(3 * c->nrep, 0);
     std::vector<int4> blob;
-    std::vector<int> boff, blen;   // per plan (FP32 path)
-    std::vector<char> wide_of;     // per plan: wide radix set (FP32)
     for (int r = 0; r < c->nrep; ++r) {
         int ns[3] = {c->rd[r].n1, c->rd[r].n2, c->rd[r].n3};
         for (int d = 0; d < 3; ++d) {
-            const bool wide = sizeof(T) == 4;
             int found = -1;
-            for (size_t k = 0; k < c->plans.size(); ++k)
-                if (c->plans[k].n == ns[d] && (bool)wide_of[k] == wide) found = (int)k;
+            for (size_t k = 0; k < plan_n.size(); ++k)
+                if (plan_n[k] == ns[d]) found = (int)k;
             if (found < 0) {
                 FftPlanDev p;
                 std::vector<int2> tab;
-                std::vector<float2> tw;
-                if (!make_plan(ns[d], &p, &tab, wide)) return MOIL_NB_ERR_GRID;
-                p.tw0 = (int)twr.size();
+                std::vector<C> tw(std::max(ns[d], 0));
+                if (!make_plan(ns[d], &p, &tab)) return MOIL_NB_ERR_GRID;
                 for (int t = 0; t < ns[d]; ++t) {
                     double ang = -2.0 * M_PI * (double)t / (double)ns[d];
-                    twr.push_back(cos(ang));
-                    twi.push_back(sin(ang));
-                    tw.push_back(make_float2((float)twr.back(), (float)twi.back()));
+                    tw[t].x = (T)cos(ang);
+                    tw[t].y = (T)sin(ang);
                 }
                 boff.push_back(0);
                 blen.push_back(0);
-                if (sizeof(T) == 4) push_blob(blob, p, tab, tw, &boff.back(), &blen.back());
-                c->plans.push_back(p);
-                wide_of.push_back(wide);
-                found = (int)c->plans.size() - 1;
+                push_blob(blob, p, tab, tw, &boff.back(), &blen.back());
+                plan_n.push_back(ns[d]);
+                found = (int)plan_n.size() - 1;
             }
-            c->rep_plan[3 * r + d] = found;
+            rep_plan[3 * r + d] = found;
         }
     }
-    std::vector<C> tw(twr.size());
-    for (size_t k = 0; k < twr.size(); ++k) { tw[k].x = (T)twr[k]; tw[k].y = (T)twi[k]; }
-    NB_CUDA_OK(c, cudaMalloc(&c->d_plans, sizeof(FftPlanDev) * c->plans.size()));
-    NB_CUDA_OK(c, cudaMemcpy(c->d_plans, c->plans.data(), sizeof(FftPlanDev) * c->plans.size(), cudaMemcpyHostToDevice));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_rep_plan, sizeof(int) * c->rep_plan.size()));
-    NB_CUDA_OK(c, cudaMemcpy(c->d_rep_plan, c->rep_plan.data(), sizeof(int) * c->rep_plan.size(), cudaMemcpyHostToDevice));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_tw, sizeof(C) * tw.size()));
-    NB_CUDA_OK(c, cudaMemcpy(c->d_tw, tw.data(), sizeof(C) * tw.size(), cudaMemcpyHostToDevice));
-    if (sizeof(T) == 4) {
-        NB_CUDA_OK(c, cudaMalloc(&c->d_blob, sizeof(int4) * blob.size()));
-        NB_CUDA_OK(c, cudaMemcpy(c->d_blob, blob.data(), sizeof(int4) * blob.size(), cudaMemcpyHostToDevice));
-    }
+    NB_CUDA_OK(c, cudaMalloc(&c->d_blob, sizeof(int4) * blob.size()));
+    NB_CUDA_OK(c, cudaMemcpy(c->d_blob, blob.data(), sizeof(int4) * blob.size(), cudaMemcpyHostToDevice));
     std::vector<T> bsp(c->bsp_h.size());
     for (size_t k = 0; k < bsp.size(); ++k) bsp[k] = (T)c->bsp_h[k];
     NB_CUDA_OK(c, cudaMalloc(&c->d_bsp, sizeof(T) * bsp.size()));
@@ -1340,14 +1176,14 @@ int configure_t(NbCtx *c)
     const int tk = col_tile<T>();
     for (int r = 0; r < c->nrep; ++r) {
         const RepDev &R = c->rd[r];
-        const int *pl = &c->rep_plan[3 * r];
+        const int *pl = &rep_plan[3 * r];
         for (int z = 0; z < R.n3; ++z)
             c->planes.push_back(PlaneWork{r, z, R.n1, R.n2, boff[pl[0]], blen[pl[0]], boff[pl[1]], blen[pl[1]], R.g0});
         c->col_begin[r] = (int)c->cols.size();
         for (int kx = 0; kx < R.n1h; ++kx)
             push_col_runs(c->cols, ColWork{r, kx, 0, 0, R.n1, R.n2, R.n3, R.bsp0, boff[pl[2]], blen[pl[2]], R.g0}, tk);
-        sf = std::max(sf, plane_fwd_smem<T>(R.n1, R.n2));
-        si = std::max(si, plane_inv_smem<T>(R.n1, R.n2));
+        sf = std::max(sf, plane_smem<T>(R.n1, R.n2));
+        si = std::max(si, plane_smem<T>(R.n1, R.n2));
         sz = std::max(sz, zconv_smem<T>(R.n3));
     }
     c->col_begin[c->nrep] = (int)c->cols.size();
@@ -1393,16 +1229,16 @@ void nb_launch_pme_virial(NbCtx *c, cudaStream_t s, void *grid, double *v_col)
 {
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
     if (c->precision == MOIL_NB_FP64) {
-        k_plane_fwd<double><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan,
-                                                               c->d_tw, (int)c->nW, c->d_zidx, c->d_fr, grid);
-        k_press_zvir<double><<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw,
-                                                            c->d_bsp, grid, v_col);
+        k_plane_fwd<double><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
+                                                               (const double4 *)c->d_fr, (double2 *)grid);
+        k_press_zvir_d<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, (const double *)c->d_bsp,
+                                                      (const double2 *)grid, v_col);
         return;
     }
-    k_plane_fwd_f<<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
-                                                       (const float4 *)c->d_fr, (float2 *)grid);
+    k_plane_fwd<float><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
+                                                          (const float4 *)c->d_fr, (float2 *)grid);
     k_press_zvir_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, (const float *)c->d_bsp,
-                                                   (const float2 *)grid, v_col);
+                                                  (const float2 *)grid, v_col);
 }
 
 // parameter derivatives on the plain path: the potential share of every plane at each site
@@ -1410,7 +1246,8 @@ void nb_launch_pme_virial(NbCtx *c, cudaStream_t s, void *grid, double *v_col)
 void nb_launch_pme_potential(NbCtx *c, double *phi4)
 {
     k_plane_inv<double><<<(int)c->planes.size(), 256, c->smem_plane_inv, c->stream>>>(
-        c->d_planes, c->d_reps, c->d_plans, c->d_rep_plan, c->d_tw, (int)c->nW, c->d_zidx, c->d_fr, c->d_grid, phi4, 1);
+        c->d_planes, c->d_blob, (double2 *)c->d_grid, c->d_reps, (int)c->nW, c->d_zidx, (const double4 *)c->d_fr, phi4,
+        1);
 }
 
 int nb_pme_configure(NbCtx *c)
@@ -1592,8 +1429,7 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     if (natom < 1 || natom > NA_MAX_ATOMS || !(alpha > 0) || !(eps > 0)) return MOIL_NB_ERR_ARG;
     for (int d = 0; d < 3; ++d) {
         FftPlanDev p;
-        if (!(box[d] > 0) || grid[d] < 4 || grid[d] > NA_MAX_N || !make_plan(grid[d], &p, nullptr, false) ||
-            !make_plan(grid[d], &p, nullptr, true))
+        if (!(box[d] > 0) || grid[d] < 4 || grid[d] > NA_MAX_N || !make_plan(grid[d], &p, nullptr))
             return MOIL_NB_ERR_GRID;
     }
     cudaStream_t stream = (cudaStream_t)stream_v;
@@ -1619,13 +1455,13 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
         int optin = 0;
         if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
             return MOIL_NB_ERR_CUDA;
-        if (plane_fwd_smem<float>(n1, n2) > (size_t)optin || plane_inv_smem<float>(n1, n2) > (size_t)optin ||
+        if (plane_smem<float>(n1, n2) > (size_t)optin || plane_smem<float>(n1, n2) > (size_t)optin ||
             zconv_smem<float>(n3) > (size_t)optin)
             return MOIL_NB_ERR_GRID;
     }
     // shared-memory limits for this grid (raise only; other handles may need more)
-    if (raise_pme_limits<float>(plane_fwd_smem<float>(n1, n2), zconv_smem<float>(n3),
-                                plane_inv_smem<float>(n1, n2)) != cudaSuccess)
+    if (raise_pme_limits<float>(plane_smem<float>(n1, n2), zconv_smem<float>(n3),
+                                plane_smem<float>(n1, n2)) != cudaSuccess)
         return MOIL_NB_ERR_CUDA;
     // one-replica constants, FFT plans and tables, work lists (host side)
     NaParams P;
@@ -1655,7 +1491,7 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
         FftPlanDev plan;
         std::vector<int2> tab;
         std::vector<float2> tw(grid[d]);
-        make_plan(grid[d], &plan, &tab, true);
+        make_plan(grid[d], &plan, &tab);
         for (int t = 0; t < grid[d]; ++t) {
             const double ang = -2.0 * M_PI * (double)t / (double)grid[d];
             tw[t] = make_float2((float)cos(ang), (float)sin(ang));
@@ -1670,8 +1506,8 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     for (int kx = 0; kx < R.n1h; ++kx)
         push_col_runs(tmp.cols, ColWork{0, kx, 0, 0, n1, n2, n3, 0, boff[2], blen[2], 0}, NB_TKF);
     if (NA_BLOB + sizeof(int4) * blob.size() > NA_HOST_BYTES) return MOIL_NB_ERR_GRID;
-    tmp.smem_plane_fwd = plane_fwd_smem<float>(n1, n2);
-    tmp.smem_plane_inv = plane_inv_smem<float>(n1, n2);
+    tmp.smem_plane_fwd = plane_smem<float>(n1, n2);
+    tmp.smem_plane_inv = plane_smem<float>(n1, n2);
     tmp.smem_zconv = zconv_smem<float>(n3);
     tmp.d_site_rep = (int *)(base + NA_REP);
     tmp.d_fr = base + NA_FR;

@@ -73,3 +73,16 @@ def test_sites_past_one_round(natom):
     else:
         assert np.abs(got - ref).max() <= 1e-5 * abs(eref)
     assert abs(e.value - eref) <= 1e-5 * abs(eref)
+
+
+@pytest.mark.parametrize("grid", [(10, 9, 8), (27, 50, 36), (96, 20, 6), (6, 75, 45), (5, 4, 125)])
+def test_transform_lengths_fp64(cfg0, grid):
+    """The plain path's passes: one, two and three along each axis, odd row counts."""
+    s = cfg0.copy()
+    s.nfft = grid
+    ref, eref = O.eforce(s, mode="parity")
+    nb = Nonbonded(s, precision=MOIL_NB_FP64)
+    dpot, e = nb.eforce(s.coor)
+    assert rel_rms(dpot, ref) <= 2.0 ** -25
+    assert abs(e["e_ew_receip"] - eref["e_ew_receip"]) <= 1e-10 * abs(eref["e_ew_receip"])
+    nb.close()
