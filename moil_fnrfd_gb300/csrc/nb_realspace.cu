@@ -558,6 +558,7 @@ __global__ void __launch_bounds__(WBLOCK, 4) k_water_s(int nW, const RepDev *__r
         const AtomK A(R, iL0, iL1, iL2, L0, L1, L2, m0, m1, m2, rmax2, rv2, K);
         water_vs_atoms(R, A, i, pos, lj_v, sflags, wl2_off, wl2, cap2, sub, LPW, cnt, g, e4, npair, flush_all);
     }
+    __syncwarp();     // the lanes' flushes into sG come before its reads (the shuffles below order no memory)
     float ecorr = 0.f;
     if (intra && sub == 0) {
         // the molecule's own exclusion corrections (every water excludes exactly its three pairs)
