@@ -1298,8 +1298,10 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
 // 114 / 80 / 77, 110,860 (64 replicas) 366 / 197 / 175, 433,195 1418 / 733 / 633 (one water per
 // thread: 78, 79, 82, 79, 120, 204, 657).  With atoms outside waters a water also has a list of
 // those (the solute system, 7,020 waters: 37 / 71 / 114; 34 at 32 lanes since its loop is packed).
+// 32-bit rows belong to replicas of 65,536 waters or more: four lanes.
 int water_lanes(const NbCtx *c)
 {
+    if (!c->row16) return 4;
     const bool atoms = c->na_handle > 0;
     return c->nw_handle <= (atoms ? 8192 : 4096) ? 32 : (c->nw_handle <= 32768 || atoms ? 8 : 4);
 }
@@ -1307,7 +1309,6 @@ int water_lanes(const NbCtx *c)
 using WaterSFn = decltype(&k_water_s<8, false, int>);
 WaterSFn water_s_fn(int lpw, bool vir, bool row16)
 {
-    // 32-bit rows belong to replicas of 65,536 waters or more
     if (!row16) return vir ? k_water_s<4, true, int> : k_water_s<4, false, int>;
     switch (lpw) {
     case 32: return vir ? k_water_s<32, true, unsigned short> : k_water_s<32, false, unsigned short>;
