@@ -313,7 +313,7 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     const moil_nb_params &p0 = *reps[0].params;
     c->precision = p0.precision == MOIL_NB_FP64 ? MOIL_NB_FP64 : MOIL_NB_MIXED;
     c->skin = (float)(p0.skin > 0 ? p0.skin : 0.0);
-    c->list_period = p0.list_period;
+    c->list_period = std::max(p0.list_period, 0);    // (no list period: any value up to 0)
     c->nrep = nrep;
     c->rh.assign(nrep, RepHost());
     c->rd.assign(nrep, RepDev());
