@@ -147,7 +147,9 @@ int moil_nb_get_alpha(const moil_nb_ctx *h, int r, double *alpha);
 /* Nonbonded energy + gradient of all replicas, host buffers (replica-major,
  * MOIL atom order within a replica).  dpot is overwritten with this block's
  * gradient; energies[r] per replica.  Lists rebuild as params->skin and
- * list_period require (replaces squeeze/nbondm/syminit + eforce nonbonded). */
+ * list_period require (replaces squeeze/nbondm/syminit + eforce nonbonded).
+ * When the status is not MOIL_NB_OK, a handle without replica groups leaves dpot as
+ * it was; with groups its contents are undefined. */
 int moil_nb_eval(moil_nb_ctx *h, const double *coor, double *dpot, moil_energies *energies);
 
 /* The same with coordinates and gradient already in device memory

@@ -1329,16 +1329,11 @@ int moil_nb_eval(moil_nb_ctx *h, const double *coor, double *dpot, moil_energies
     // the coordinates in and the gradient out took 0.7 ms together
     size_t bytes = sizeof(double) * 3 * h->natom;
     NB_CUDA_OK(h, cudaMemcpyAsync(h->d_coor, coor, bytes, cudaMemcpyHostToDevice, h->stream));
-    eval_launch(h, h->d_coor, h->d_dpot);
-    // queued behind the evaluation, as a group's copy is; copied again if that had to be redone
+    const int rc = eval_impl(h, h->d_coor, h->d_dpot, e);
+    if (rc != MOIL_NB_OK) return rc;       // the caller's gradient stays as it is
     NB_CUDA_OK(h, cudaMemcpyAsync(dpot, h->d_dpot, bytes, cudaMemcpyDeviceToHost, h->stream));
-    const int first = eval_complete(h);
-    int rc = eval_retry(h, h->d_coor, h->d_dpot, e, first, true);
-    if (rc == MOIL_NB_OK && first != MOIL_NB_OK) {
-        NB_CUDA_OK(h, cudaMemcpyAsync(dpot, h->d_dpot, bytes, cudaMemcpyDeviceToHost, h->stream));
-        NB_CUDA_OK(h, cudaStreamSynchronize(h->stream));
-    }
-    return rc;
+    NB_CUDA_OK(h, cudaStreamSynchronize(h->stream));
+    return MOIL_NB_OK;
 }
 
 int moil_nb_adjoint(moil_nb_ctx *h, const double *coor, double *dEdq, double *dEdeps, double *dEdsig,
