@@ -255,8 +255,11 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
     if (h->grp.empty()) ctxs.push_back(h);
     else for (NbCtx *c : h->grp) ctxs.push_back(c);
     if (loop && !h->d_md_save) NB_CUDA_OK(h, cudaMalloc(&h->d_md_save, sizeof(double) * 6 * std::max<size_t>(n, 1)));
+    // (a replica group's period is its own first replica's)
+    bool periods = true;
+    for (const NbCtx *c : ctxs) periods &= c->list_period > 0;
     while (loop && first < nsteps) {
-        const bool host = h->list_period > 0 && h->md_wary == 0;
+        const bool host = periods && h->md_wary == 0;
         const int run = host ? std::min(nsteps - first, 64) : nsteps - first;
         if (h->md_wary > 0) --h->md_wary;
         NB_CUDA_OK(h, cudaMemcpyAsync(h->d_md_save, d_coor, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, h->stream));

@@ -44,3 +44,36 @@ def test_negative_list_period_is_none():
         out.append(run(nb, state, 40))
         nb.close()
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]) and out[0][2:] == out[1][2:]
+
+
+def test_grouped_handle_does_not_keep_an_earlier_period():
+    """A handle that was ungrouped with a list period, made grouped without one, follows the schedule
+    of a handle made grouped in the first place (no rebuild while no site has moved half the skin)."""
+    ws = [waters(300, 31, 4.0), waters(216, 32, 4.0)]
+    state, systems = start(ws), [s for s, _ in ws]
+    fresh = Nonbonded(systems, skin=1.0, list_period=0, groups=2)
+    want = run(fresh, state, 40)
+    used = Nonbonded(systems, skin=1.0, list_period=7, groups=1)
+    run(used, state, 8)
+    for p in used._params:
+        p.list_period = 0
+    assert used.L.moil_nb_set_groups(used.h, 2) == 0
+    assert used.L.moil_nb_init_batch(used.h, len(systems), used._reps) == 0
+    assert used.groups() == fresh.groups() == 2
+    got = run(used, state, 40)
+    fresh.close()
+    used.close()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and got[2:] == want[2:]
+
+
+def test_grouped_steps_follow_the_ungrouped_schedule():
+    """With a list period, replica groups and the whole batch rebuild at the same steps and give the same bits."""
+    ws = [waters(216, 33, 4.0), waters(300, 34, 4.0), waters(260, 35, 4.0)]
+    state, systems = start(ws), [s for s, _ in ws]
+    out = []
+    for groups in (1, 3):
+        nb = Nonbonded(systems, skin=1.0, list_period=9, groups=groups)
+        assert (nb.groups() > 1) == (groups > 1)
+        out.append(run(nb, state, 40))
+        nb.close()
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]
