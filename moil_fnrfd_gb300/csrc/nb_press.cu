@@ -423,10 +423,10 @@ __global__ void __launch_bounds__(NB_PR_THREADS) k_press_reduce(int nW, const Re
                                                                double *__restrict__ out)
 {
     __shared__ double red[12][NB_PR_THREADS];
-    const int r = blockIdx.y, t = threadIdx.x;
+    const int r = blockIdx.x, t = threadIdx.x;     // (replicas along x: the other axes end at 65,535)
     const RepDev &R = reps[r];
-    if ((int)blockIdx.x >= press_blocks(R)) return;
-    const int first = blockIdx.x * NB_PR_THREADS + t, stride = press_blocks(R) * NB_PR_THREADS;
+    if ((int)blockIdx.y >= press_blocks(R)) return;
+    const int first = blockIdx.y * NB_PR_THREADS + t, stride = press_blocks(R) * NB_PR_THREADS;
     double acc[12];
 #pragma unroll
     for (int k = 0; k < 12; ++k) acc[k] = 0.0;
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(NB_PR_THREADS) k_press_reduce(int nW, const Re
             for (int k = 0; k < 12; ++k) red[k][t] += red[k][t + h];
         __syncthreads();
     }
-    if (t < 12) out[12 * ((size_t)r * gridDim.x + blockIdx.x) + t] = red[t][0];
+    if (t < 12) out[12 * ((size_t)r * gridDim.y + blockIdx.y) + t] = red[t][0];
 }
 
 __global__ void k_press_final(int n, int nsplit, const RepDev *__restrict__ reps, const double *__restrict__ part,
@@ -494,7 +494,7 @@ void pressure_t(NbCtx *c, const double *d_coor, double *d_out)
             (int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_site_lj, c->d_site_flags, c->d_xl_off,
             c->d_xl, cap_int(c->cap_xl), c->d_xsite, c->d_press_unit);
     cudaStreamWaitEvent(s, c->ev_join, 0);
-    k_press_reduce<T><<<dim3(c->press_split, c->nrep), NB_PR_THREADS, 0, s>>>(
+    k_press_reduce<T><<<dim3(c->nrep, c->press_split), NB_PR_THREADS, 0, s>>>(
         (int)c->nW, c->d_reps, c->d_site_orig, c->d_part, c->d_q, c->d_xsite, c->d_press_unit, c->d_press_col,
         c->d_col_begin, c->d_press_part);
     k_press_final<<<(12 * c->nrep + B - 1) / B, B, 0, s>>>(12 * c->nrep, c->press_split, c->d_reps, c->d_press_part, d_out);
