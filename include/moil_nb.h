@@ -258,7 +258,7 @@ int moil_nb_groups(const moil_nb_ctx *h);
  * (pot/nbondm.f:143-210, pot/nbond.f:54-157).  Every shape gives the same pair set and
  * results within the mixed path's tolerances; each is deterministic run to run. */
 enum {
-    MOIL_NB_WATER_AUTO = 0,       /* half lists for large water-only handles, else full lists */
+    MOIL_NB_WATER_AUTO = 0,       /* half lists for large handles, else full lists */
     MOIL_NB_WATER_FULL = 1,       /* every water over its full row (both directions) */
     MOIL_NB_WATER_HALF = 2        /* each water pair once; the partner's share summed per block in
                                      shared memory (mixed path, replicas below 65,536 waters) */

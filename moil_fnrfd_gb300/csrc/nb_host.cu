@@ -228,10 +228,26 @@ int alloc_half(NbCtx *c)
 // of 256 waters per multiprocessor leaves most of the GPU idle below it, while the full-list
 // kernel spreads each water over 8 or 32 lanes.  One evaluation in us (lists rebuilt every 10),
 // half / full lists: 216 waters 75 / 46, 1,334 94 / 52, 7,000 102 / 68, 12,000 105 / 79, 28,800 (16
-// replicas) 130 / 125, 32,000 149 / 154, 110,860 (64 replicas) 340 / 371.  Handles with atoms outside
-// waters take full lists at every size: the half-list kernel runs a water's list of them in one
-// thread (water stage of the solute system, 7,020 waters: 322 / 37 us).
+// replicas) 130 / 125, 32,000 149 / 154, 110,860 (64 replicas) 340 / 371.
+// The half-list kernel runs a water's list of atoms outside waters in one thread, the full-list one shares
+// it among the lanes.  A few ions change nothing (24 replicas, 40,800 waters, 1 entry per water 193 /
+// 211; 256 replicas 1296 / 1497, 13 entries 1523 / 1794).  A solute gathers its entries at the waters around
+// it, and the longest list sets the time until there are blocks enough to hide it: 24 replicas (39,400
+// waters) with 30 entries per water 298 / 278, 5 solute systems (35,100) with 59 353 / 290, 8 (56,160)
+// 442 / 452, 24 1097 / 1158.
 #define NB_FULL_MAX_WATERS 30000
+#define NB_FULL_MAX_WATERS_SOLUTE 50000
+bool auto_full(const NbCtx *c)
+{
+    return c->nw_handle <= (c->w2_handle < NB_W2_SOLUTE ? NB_FULL_MAX_WATERS : NB_FULL_MAX_WATERS_SOLUTE);
+}
+
+// List entries of atoms outside waters that a water of a replica has on average, times its waters
+double w2_entries(const moil_nb_params &p, double skin, double rwat, int64_t nwat, int64_t noth)
+{
+    const double r = std::max(p.rvmx, p.relx) + skin + rwat, vol = p.a * p.b * p.c;
+    return (double)nwat * (double)noth * std::min(4.0 / 3.0 * M_PI * r * r * r / vol, 1.0);
+}
 
 // Half-list set-up for the current shape: on for FP32 handles whose replicas all have fewer
 // than 65,536 waters (16-bit rows) unless full lists were asked for; blocks of hb waters
@@ -243,7 +259,7 @@ int setup_half(NbCtx *c)
     free_ptr(c->d_hrow); free_ptr(c->d_jset);
     c->hblocks.clear();
     c->whalf = c->precision != MOIL_NB_FP64 && c->row16 && c->nW > 0 && c->want_whalf != MOIL_NB_WATER_FULL;
-    if (c->want_whalf == MOIL_NB_WATER_AUTO && (c->nw_handle <= NB_FULL_MAX_WATERS || c->na_handle > 0)) c->whalf = 0;
+    if (c->want_whalf == MOIL_NB_WATER_AUTO && auto_full(c)) c->whalf = 0;
     if (!c->whalf) return MOIL_NB_OK;
     int maxw = 0;
     for (int r = 0; r < c->nrep; ++r) {
@@ -541,6 +557,11 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     c->nw_handle = std::max(c->nw_handle, c->nW);
     for (RepDev &R : c->rd) R.wtiled = tiled_choice(c, R);
     c->na_handle = std::max(c->na_handle, c->nA);
+    if (!c->pstream) {                     // (a replica group has the whole handle's)
+        double w2 = 0.0;
+        for (int r = 0; r < nrep; ++r) w2 += w2_entries(c->rh[r].p, c->skin, c->rwat, c->rd[r].nwat, c->rd[r].noth);
+        c->w2_handle = w2 / (double)std::max<int64_t>(c->nW, 1);
+    }
     c->row16 = 1;
     for (int r = 0; r < nrep; ++r) c->row16 &= c->rd[r].nwat < 65536;
     c->nsite = 3 * c->nW + c->nA;
@@ -1160,9 +1181,14 @@ int init_groups(moil_nb_ctx *h, int nrep, const moil_replica *reps, int P)
     h->grp_rep0.push_back(nrep);
     h->grp_atom0.push_back(total);
     int64_t nwat = 0;
+    double w2 = 0.0;
     for (int r = 0; r < nrep; ++r)
-        if (reps[r].topo && reps[r].topo->montype)
-            nwat += std::count(reps[r].topo->montype, reps[r].topo->montype + std::max(reps[r].topo->totmon, 0), (int)MOIL_MON_WATER);
+        if (reps[r].topo && reps[r].topo->montype) {
+            const moil_topology &t = *reps[r].topo;
+            const int64_t n = std::count(t.montype, t.montype + std::max(t.totmon, 0), (int)MOIL_MON_WATER);
+            nwat += n;
+            w2 += w2_entries(*reps[r].params, std::max(reps[0].params->skin, 0.0), h->rwat, n, t.npt - 3 * n);
+        }
     for (size_t g = 0; g + 1 < h->grp_rep0.size(); ++g) {
         moil_nb_ctx *c = nullptr;
         int rc = moil_nb_create(&c, h->device);
@@ -1175,6 +1201,7 @@ int init_groups(moil_nb_ctx *h, int nrep, const moil_replica *reps, int P)
         c->want_tiled = h->want_tiled;
         c->nw_handle = nwat;
         c->na_handle = total - 3 * nwat;
+        c->w2_handle = w2 / (double)std::max<int64_t>(nwat, 1);
         {
             // streams for host-buffer evaluations: earlier groups at higher priority finish
             // first, so their gradient copies overlap the later groups' kernels (device-

@@ -59,6 +59,7 @@ struct NbCtx {
     int64_t natom = 0, nW = 0, nA = 0, nsite = 0, nunit = 0;
     int64_t nw_handle = 0;        // waters of the whole handle: all replica groups together
     int64_t na_handle = 0;        // its atoms outside waters
+    double w2_handle = 0.0;       // of those, list entries expected per water
     float skin = 1.0f, rwat = 1.1f;
     int list_period = 0;
     int water_excl_fast = 0;      // every water's exclusions are exactly O-H1, O-H2, H1-H2
@@ -241,6 +242,10 @@ struct NbCtx {
     double *pend_dpot = nullptr;
     int on_prio = 0;                   // running on the prioritised group streams
 };
+
+// From this many list entries of atoms outside waters per water on, they set the time of the water
+// kernels (a solute; ions have a few)
+#define NB_W2_SOLUTE 16.0
 
 // the public handle is the context itself
 struct moil_nb_ctx : NbCtx {};

@@ -1296,14 +1296,14 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
 // partly filled rounds and to the sum over the lanes.  Water stage in us at 32 / 8 / 4 lanes:
 // 1,334 waters 14 / 19 / 27, 3,000 22 / 19 / 28, 7,000 32 / 21 / 30, 12,000 46 / 34 / 32, 32,000
 // 114 / 80 / 77, 110,860 (64 replicas) 366 / 197 / 175, 433,195 1418 / 733 / 633 (one water per
-// thread: 78, 79, 82, 79, 120, 204, 657).  With atoms outside waters a water also has a list of
-// those (the solute system, 7,020 waters: 37 / 71 / 114; 34 at 32 lanes since its loop is packed).
+// thread: 78, 79, 82, 79, 120, 204, 657).  In a solute a water also has a long list of atoms (the
+// solute system, 7,020 waters: 37 / 71 / 114; 34 at 32 lanes since its loop is packed; 5 of them, 35,100
+// waters, a whole evaluation 337 / 299 / 290).
 // 32-bit rows belong to replicas of 65,536 waters or more: four lanes.
 int water_lanes(const NbCtx *c)
 {
     if (!c->row16) return 4;
-    const bool atoms = c->na_handle > 0;
-    return c->nw_handle <= (atoms ? 8192 : 4096) ? 32 : (c->nw_handle <= 32768 || atoms ? 8 : 4);
+    return c->nw_handle <= (c->w2_handle < NB_W2_SOLUTE ? 4096 : 8192) ? 32 : (c->nw_handle <= 32768 ? 8 : 4);
 }
 
 using WaterSFn = decltype(&k_water_s<8, false, int>);
