@@ -96,6 +96,14 @@ __device__ __forceinline__ void two_add(float2 &a, float v)
     const float sm = a.x + v, bb = sm - a.x;
     a = make_float2(sm, a.y + ((a.x - (sm - bb)) + (v - bb)));
 }
+// the same for two sums at once, (hi.x, lo.x) and (hi.y, lo.y), on the packed pipe
+__device__ __forceinline__ void two_add2(float2 &hi, float2 &lo, float2 v)
+{
+    const float2 m1 = f2(-1.f), sm = __fadd2_rn(hi, v), bb = __ffma2_rn(hi, m1, sm);
+    const float2 eh = __ffma2_rn(__ffma2_rn(bb, m1, sm), m1, hi), ev = __ffma2_rn(bb, m1, v);
+    lo = __fadd2_rn(lo, __fadd2_rn(eh, ev));
+    hi = sm;
+}
 template <int W> __device__ __forceinline__ float2 sub_two_sum(float2 a)
 {
 #pragma unroll

@@ -853,16 +853,11 @@ __global__ void __launch_bounds__(128, 6) k_atom_f(int nA, int nW, const RepDev 
     const float2 lji = lj[si];
     const float qi = xi.w * A.ke;
     const unsigned fi = A.tiny ? sflags[si] & SF_HTINY : 0;
-    float g[3] = {0.f, 0.f, 0.f}, e6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float g[3] = {0.f, 0.f, 0.f};
     long long G[3] = {0, 0, 0};
-    float2 es[6];    // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
+    float2 eh[3], el[3];     // LJ, Coulomb and LJ virial, (primary box, images): hi and lo
 #pragma unroll
-    for (int m = 0; m < 6; ++m) es[m] = f2(0.f);
-    auto flush6 = [&]() {
-        flush(g, G, 3);
-#pragma unroll
-        for (int m = 0; m < 6; ++m) { two_add(es[m], e6[m]); e6[m] = 0.f; }
-    };
+    for (int m = 0; m < 3; ++m) { eh[m] = f2(0.f); el[m] = f2(0.f); }
     int cnt = 0, npair = 0;
     // an overflowed list is read within the buffer (the evaluation is redone)
     const int q0 = min(xl_off[k], capx), q1 = min(xl_off[k + 1], capx);
@@ -889,14 +884,14 @@ __global__ void __launch_bounds__(128, 6) k_atom_f(int nA, int nW, const RepDev 
             // LJ virial: a water partner's side of the pair (its W2 list) adds none, so it counts
             // twice here; pairs of two non-water atoms are seen from both sides
             if (sc < 3 * nW) vir += vir;
-            e6[0] += img ? 0.f : elj; e6[1] += img ? elj : 0.f;
-            e6[2] += img ? 0.f : eel; e6[3] += img ? eel : 0.f;
-            e6[4] += img ? 0.f : vir; e6[5] += img ? vir : 0.f;
-            if (++cnt == CHUNK_ATOM) { flush6(); cnt = 0; }
+            two_add2(eh[0], el[0], f2(img ? 0.f : elj, img ? elj : 0.f));
+            two_add2(eh[1], el[1], f2(img ? 0.f : eel, img ? eel : 0.f));
+            two_add2(eh[2], el[2], f2(img ? 0.f : vir, img ? vir : 0.f));
+            if (++cnt == CHUNK_ATOM) { flush(g, G, 3); cnt = 0; }
         }
     }
     __syncwarp();
-    flush6();
+    flush(g, G, 3);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const long long v = sub_sum<32>(G[d]);
@@ -905,7 +900,7 @@ __global__ void __launch_bounds__(128, 6) k_atom_f(int nA, int nW, const RepDev 
     double e[6];
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-        const float2 v = sub_two_sum<32>(es[m]);
+        const float2 v = sub_two_sum<32>(m & 1 ? f2(eh[m / 2].y, el[m / 2].y) : f2(eh[m / 2].x, el[m / 2].x));
         e[m] = (double)v.x + (double)v.y;
     }
     npair = sub_sum<32>(npair);
