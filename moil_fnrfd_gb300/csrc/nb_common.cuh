@@ -300,6 +300,15 @@ __device__ __forceinline__ double nb_fix2d(long long x)
 __device__ __forceinline__ long long nb_fix(float v) { return __float2ll_rn(v * NB_FIX_SCALE_F); }
 __device__ __forceinline__ long long nb_fix(double v) { return __double2ll_rn(v * NB_FIX_SCALE); }
 
+// FP64 path: the waters' gradient is summed in a second int64 array per site, at 2^42 units per kcal/mol/Å,
+// which holds 2^21: partner shares below 2^8 in magnitude (4,096 of them fit beside) and the 32 lanes'
+// parts of the own side below 2^14 each.  Every part is rounded to 2^-43; larger ones (rare) go to the site
+// gradient at NB_FIX_SCALE, whose range is 2^31.
+#define NB_FINE_SCALE 4398046511104.0   // 2^42
+// |x| < 2^e, by the exponent bits (a comparison would take the narrow FP64 pipe); false for NaN and inf
+__device__ __forceinline__ bool nb_below(double x, int e) { return (__double2hiint(x) & 0x7fffffff) < (1023 + e) << 20; }
+__device__ __forceinline__ unsigned long long nb_fine(double x) { return (unsigned long long)__double2ll_rn(x * NB_FINE_SCALE); }
+
 // Owner of the water pair (a, b) in the half lists (indices relative to the replica's first
 // water): the lower index when a + b is odd, the higher one when it is even.  Each water owns
 // about half of its partners whatever its position in the sorted order.

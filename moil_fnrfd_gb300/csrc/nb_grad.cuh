@@ -5,12 +5,14 @@
 
 namespace {
 
-// one atom's gradient: fixed-point real space + FP64 corrections + PME; false if not finite
+// one atom's gradient: fixed-point real space + FP64 corrections + PME; false if not finite.  fine (FP64
+// path): the water sites' part at NB_FINE_SCALE, sites below nfine
 template <typename T>
 __device__ __forceinline__ bool final_grad(int a, const int *__restrict__ site_of, const int *__restrict__ atom_rep,
                                            const RepDev *__restrict__ reps, const long long *__restrict__ grad_site,
                                            const double *__restrict__ grad_ex, const T *__restrict__ part,
-                                           const double *__restrict__ q, int nsw, double g[3])
+                                           const double *__restrict__ q, int nsw,
+                                           const long long *__restrict__ fine, int nfine, double g[3])
 {
     const RepDev &R = reps[atom_rep[a]];
     int s = site_of[a];
@@ -45,7 +47,9 @@ __device__ __forceinline__ bool final_grad(int a, const int *__restrict__ site_o
         double sc[3] = {qf * R.n1 * R.invLd[0], qf * R.n2 * R.invLd[1], qf * R.n3 * R.invLd[2]};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            double v = (double)grad_site[3 * (size_t)s + d] * NB_FIX_INV + grad_ex[3 * (size_t)a + d] + sc[d] * pg[d];
+            double v = (double)grad_site[3 * (size_t)s + d] * NB_FIX_INV;
+            if (s < nfine) v += (double)fine[3 * (size_t)s + d] * (1.0 / NB_FINE_SCALE);
+            v += grad_ex[3 * (size_t)a + d] + sc[d] * pg[d];
             bad |= !(v == v);
             g[d] = v;
         }

@@ -96,7 +96,9 @@ void release_device(NbCtx *c)
     free_ptr(c->d_pos); free_ptr(c->d_posb); free_ptr(c->d_opos); free_ptr(c->d_woff); free_ptr(c->d_site_lj); free_ptr(c->d_site_q);
     free_ptr(c->d_wl1_cnt); free_ptr(c->d_wl1); free_ptr(c->d_wl2_off); free_ptr(c->d_wl2); free_ptr(c->d_xl_off);
     free_ptr(c->d_xl); free_ptr(c->d_count_tmp); free_ptr(c->d_ex_off); free_ptr(c->d_ex_j); free_ptr(c->d_p14_off);
-    free_ptr(c->d_p14_j); free_ptr(c->d_p14_par); free_ptr(c->d_grad_site); free_ptr(c->d_e_unit);
+    free_ptr(c->d_p14_j); free_ptr(c->d_p14_par); free_ptr(c->d_e_unit);
+    if (c->d_grad_fine) c->d_grad_site = nullptr;
+    free_ptr(c->d_grad_fine); free_ptr(c->d_grad_site);
     free_ptr(c->d_grad_ex); free_ptr(c->d_e_ex);
     free_ptr(c->d_blob); free_ptr(c->d_wtiles); free_ptr(c->d_scan_tmp);
     free_ptr(c->d_hblocks); free_ptr(c->d_hrow); free_ptr(c->d_hcnt); free_ptr(c->d_jset); free_ptr(c->d_jn);
@@ -634,7 +636,13 @@ int init_impl(NbCtx *c, int nrep, const moil_replica *reps)
     NB_CUDA_OK(c, cudaMemset(c->d_wl2_off, 0, sizeof(int) * (c->nW + 1)));   // rebuilt where there are non-water atoms
     NB_CUDA_OK(c, cudaMalloc(&c->d_xl_off, sizeof(int) * (c->nA + 1)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_count_tmp, sizeof(int) * (3 * std::max(c->nW, c->nA) + 3)));
-    NB_CUDA_OK(c, cudaMalloc(&c->d_grad_site, sizeof(long long) * 3 * ns));
+    if (c->precision == MOIL_NB_FP64) {
+        // the waters' two arrays side by side: one launch clears them
+        NB_CUDA_OK(c, cudaMalloc(&c->d_grad_fine, sizeof(long long) * std::max<int64_t>(9 * c->nW + 3 * ns, 1)));
+        c->d_grad_site = c->d_grad_fine + 9 * c->nW;
+    } else {
+        NB_CUDA_OK(c, cudaMalloc(&c->d_grad_site, sizeof(long long) * 3 * ns));
+    }
     NB_CUDA_OK(c, cudaMalloc(&c->d_e_unit, sizeof(double) * NB_EU * std::max<int64_t>(nu, 1)));
     NB_CUDA_OK(c, cudaMalloc(&c->d_grad_ex, sizeof(double) * 3 * c->natom));
     NB_CUDA_OK(c, cudaMalloc(&c->d_e_ex, sizeof(double) * NB_EX * c->natom));

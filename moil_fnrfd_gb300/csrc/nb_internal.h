@@ -124,6 +124,8 @@ struct NbCtx {
 
     // outputs
     long long *d_grad_site = nullptr;  // nsite*3 fixed point
+    long long *d_grad_fine = nullptr;  // FP64 path: the waters' at NB_FINE_SCALE, 9 per water; the allocation
+                                       // that d_grad_site then follows in
     double *d_e_unit = nullptr;        // nunit*4
     double *d_grad_ex = nullptr;       // natom*3
     double *d_e_ex = nullptr;          // natom*3

@@ -107,10 +107,12 @@ template <typename T> struct StepGrad {
     const T *part;
     const double *q;
     int nsw;
+    const long long *fine;
+    int nfine;
     int *nan_h, *ctl;
     __device__ void operator()(size_t a, double g[3]) const
     {
-        if (!final_grad<T>((int)a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, g)) {
+        if (!final_grad<T>((int)a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, fine, nfine, g)) {
             *nan_h = 1;
             atomicOr(&ctl[2], NB_DEV_ERR_NAN);
         }
@@ -211,7 +213,7 @@ int nb_launch_integrate(NbCtx *c, cudaStream_t s, double *coor, double *vel, con
         typedef std::remove_const_t<std::remove_pointer_t<decltype(part)>> T;
         return integrate(c, s, coor, vel, mass,
                          StepGrad<T>{c->d_site_of, c->d_atom_rep, c->d_reps, c->d_grad_site, c->d_grad_ex, part, c->d_q,
-                                     nsw, c->h_status + 23, ctl},
+                                     nsw, c->d_grad_fine, c->d_grad_fine ? (int)(3 * c->nW) : 0, c->h_status + 23, ctl},
                          dt, doh, dhh);
     };
     if (c->precision == MOIL_NB_FP64) return with((const double *)c->d_part, 0);

@@ -84,14 +84,6 @@ __device__ __forceinline__ void flush(float g[], long long G[], int n)
         if (k < n) { G[k] += nb_fix(g[k]); g[k] = 0.f; }
     }
 }
-__device__ __forceinline__ void flush(double g[], long long G[], int n)
-{
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        if (k < n) { G[k] += nb_fix(g[k]); g[k] = 0.0; }
-    }
-}
-
 // water sites of molecule i against its W2 list of non-water atoms (entries first, first +
 // stride, ...): atom semantics per site pair; partial gradients and energies go to g / e4, which
 // already hold cnt entries, flushed every CHUNK entries and left to the caller after the last
@@ -219,9 +211,10 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, const AtomK &A, 
 // (nb_half_owner on the full rows), and a warp's 32 lanes share one water's pairs: the owned
 // in-cutoff entries are compacted into shared memory (their image-shifted O-O vectors with
 // them), and the lanes take (partner site, entry) items, three site pairs each, so about 50
-// entries fill five rounds of 32 items.  Gradients of both sides go to the int64 site gradient
-// (cleared before the launch) with atomics: integer sums, independent of their order.  erfc(x) is
-// exp(-x^2) erfcx(x), one exponential for the energy and the force.  A whole evaluation: 216
+// entries fill five rounds of 32 items.  Gradients of both sides go to int64 arrays (cleared before the
+// launch) with atomics: integer sums, independent of their order, of parts rounded to 2^-43 (nb_fine:
+// 32 lanes and about 65 partner shares per site; at 2^-33 each the sums were off by up to 2.5e-9).
+// erfc(x) is exp(-x^2) erfcx(x), one exponential for the energy and the force.  A whole evaluation: 216
 // waters 3258 -> 226 us, 1,334 waters 3867 -> 485 us (before: one water per thread, full lists).
 #define WARPS64 2
 #define WBUF64 96
@@ -236,6 +229,7 @@ __global__ void __launch_bounds__(32 * WARPS64) k_water_d(int nW, const RepDev *
                                                           const int *__restrict__ wl2_off,
                                                           const int *__restrict__ wl2, int cap2,
                                                           unsigned long long *__restrict__ grad,
+                                                          unsigned long long *__restrict__ fine,
                                                           double *__restrict__ e_unit)
 {
     __shared__ double sD[WARPS64][3][WBUF64];
@@ -292,9 +286,12 @@ __global__ void __launch_bounds__(32 * WARPS64) k_water_d(int nW, const RepDev *
                 H[0] -= df * dx; H[1] -= df * dy; H[2] -= df * dz;
             }
             e4[img ? 3 : 2] += e_el;
-            unsigned long long *gj = grad + 9 * (size_t)j + 3 * b;
+            const size_t gj = 9 * (size_t)j + 3 * b;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) atomicAdd(gj + d, (unsigned long long)nb_fix(H[d]));
+            for (int d = 0; d < 3; ++d) {
+                if (nb_below(H[d], 8)) atomicAdd(fine + gj + d, nb_fine(H[d]));
+                else atomicAdd(grad + gj + d, (unsigned long long)nb_fix(H[d]));
+            }
         }
         __syncwarp();
     };
@@ -330,10 +327,14 @@ __global__ void __launch_bounds__(32 * WARPS64) k_water_d(int nW, const RepDev *
     // water sites against non-water atoms (W2, full list): a lane's share of the entries
     auto none = []() {};
     water_vs_atoms(R, i, pos, lj_v, sflags, wl2_off, wl2, cap2, lane, 32, 0, g, e4, npair, none);
+    bool small = true;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) small &= nb_below(g[k], 14);
+    small = __all_sync(0xffffffffu, small);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-        const long long v = sub_sum<32>(nb_fix(g[k]));
-        if (lane == k) atomicAdd(grad + 9 * (size_t)i + k, (unsigned long long)v);
+        const long long v = small ? sub_sum<32>((long long)nb_fine(g[k])) : nb_fix(sub_sum<32>(g[k]));
+        if (lane == k) atomicAdd((small ? fine : grad) + 9 * (size_t)i + k, (unsigned long long)v);
     }
 #pragma unroll
     for (int k = 0; k < 6; ++k) e4[k] = sub_sum<32>(e4[k]);
@@ -938,9 +939,8 @@ __global__ void __launch_bounds__(128) k_atom_d(int nA, int nW, const RepDev *__
     T2 lji = lj[si];
     unsigned fi = sflags[si];
     T g[3] = {0, 0, 0};
-    long long G[3] = {0, 0, 0};
     T es[6] = {0, 0, 0, 0, 0, 0};    // LJ prim, LJ img, Coulomb prim, Coulomb img, LJ virial prim, img
-    int cnt = 0, npair = 0;
+    int npair = 0;
     // an overflowed list is read within the buffer (the evaluation is redone)
     const int q1 = min(xl_off[k + 1], capx);
     for (int q = min(xl_off[k], capx) + lane; q < q1; q += 32) {
@@ -960,13 +960,11 @@ __global__ void __launch_bounds__(128) k_atom_d(int nA, int nW, const RepDev *__
         es[0] += img ? (T)0 : elj; es[1] += img ? elj : (T)0;
         es[2] += img ? (T)0 : eel; es[3] += img ? eel : (T)0;
         es[4] += img ? (T)0 : vir; es[5] += img ? vir : (T)0;
-        if (++cnt == CHUNK) { flush(g, G, 3); cnt = 0; }
     }
-    flush(g, G, 3);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const long long v = sub_sum<32>(G[d]);
-        if (lane == d) grad[(size_t)3 * si + d] = v;
+        const double v = sub_sum<32>(g[d]);
+        if (lane == d) grad[(size_t)3 * si + d] = nb_fix(v);
     }
     double e[6];
 #pragma unroll
@@ -1247,7 +1245,8 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
     double *__restrict__ epart, int *__restrict__ done, double *__restrict__ e_rep_h, int natom,
     const int *__restrict__ site_of, const int *__restrict__ atom_rep, const RepDev *__restrict__ reps,
     const long long *__restrict__ grad_site, const double *__restrict__ grad_ex, const T *__restrict__ part,
-    const double *__restrict__ q, int nsw, double *__restrict__ dpot, int *__restrict__ st, int *__restrict__ st_h,
+    const double *__restrict__ q, int nsw, const long long *__restrict__ fine, int nfine, double *__restrict__ dpot,
+    int *__restrict__ st, int *__restrict__ st_h,
     int *__restrict__ nan_h, int *__restrict__ ctl, int list_period)
 {
     const int t = threadIdx.x, b = blockIdx.x;
@@ -1255,7 +1254,7 @@ __global__ void __launch_bounds__(NB_FE_THREADS) k_finalize(
         const int a = (b - nchunk) * NB_FE_THREADS + t;
         if (a >= natom) return;
         double g[3];
-        if (!final_grad<T>(a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, g)) {
+        if (!final_grad<T>(a, site_of, atom_rep, reps, grad_site, grad_ex, part, q, nsw, fine, nfine, g)) {
             *nan_h = 1;
             if (ctl) atomicOr(&ctl[2], NB_DEV_ERR_NAN);
         }
@@ -1343,7 +1342,8 @@ void water_t(NbCtx *c)
                                                                       32 * WARPS64, 0, s>>>(
                 (int)c->nW, c->d_reps, c->d_site_rep, (const double4 *)c->d_pos, (const double4 *)c->d_woff,
                 c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2,
-                cap_int(c->cap_wl2), (unsigned long long *)c->d_grad_site, c->d_e_unit);
+                cap_int(c->cap_wl2), (unsigned long long *)c->d_grad_site, (unsigned long long *)c->d_grad_fine,
+                c->d_e_unit);
         }
         c->launches++;
     }
@@ -1357,7 +1357,8 @@ void nb_launch_water(NbCtx *c)
     // the kernels that evaluate each water pair once add both sides with atomics: the water
     // sites' gradient starts at zero
     if (c->nW > 0 && (c->precision == MOIL_NB_FP64 || c->whalf))
-        cudaMemsetAsync(c->d_grad_site, 0, sizeof(long long) * 9 * (size_t)c->nW, c->stream);
+        cudaMemsetAsync(c->d_grad_fine ? c->d_grad_fine : c->d_grad_site, 0,
+                        sizeof(long long) * (c->d_grad_fine ? 18 : 9) * (size_t)c->nW, c->stream);
     if (c->precision == MOIL_NB_FP64) water_t<double>(c);
     else water_t<float>(c);
 }
@@ -1474,7 +1475,7 @@ void nb_launch_finalize(NbCtx *c, double *d_dpot, int *ctl, EvalMode mode)
         kernel<<<nb, NB_FE_THREADS, 0, c->stream>>>(
             nchunk, c->d_echunks, c->d_echunk_begin, c->d_e_unit, c->d_e_ex, c->d_e_col, c->d_epart, c->d_edone,
             c->h_e_rep, (int)c->natom, c->d_site_of, c->d_atom_rep, c->d_reps, c->d_grad_site, c->d_grad_ex, part,
-            c->d_q, nsw, d_dpot, c->d_status, c->h_status, c->h_status + 23, ctl, period);
+            c->d_q, nsw, c->d_grad_fine, c->d_grad_fine ? (int)(3 * c->nW) : 0, d_dpot, c->d_status, c->h_status, c->h_status + 23, ctl, period);
     };
     if (c->precision == MOIL_NB_FP64) launch(k_finalize<double>, (const double *)c->d_part, 0);
     else launch(k_finalize<float>, (const float *)c->d_part, c->water_excl_fast ? (int)(3 * c->nW) : 0);
