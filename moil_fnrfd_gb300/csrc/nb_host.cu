@@ -1319,6 +1319,8 @@ int moil_nb_init(moil_nb_ctx *h, const moil_nb_params *p, const moil_topology *t
     cudaSetDevice(h->device);
     destroy_groups(h);
     h->nw_handle = h->na_handle = 0;
+    h->wary = 0;                 // (what an earlier system taught the host about its lists)
+    h->md_lists.reset();
     return init_impl(h, 1, &r);
 }
 
@@ -1336,6 +1338,8 @@ int moil_nb_init_batch(moil_nb_ctx *h, int nrep, const moil_replica *reps)
     if (reps) nb_tune_cached_shape(h, nrep, reps);
     const int P = reps ? choose_groups(h, nrep, natom) : 1;
     h->nw_handle = h->na_handle = 0;
+    h->wary = 0;                 // (what an earlier system taught the host about its lists)
+    h->md_lists.reset();
     if (P <= 1) return init_impl(h, nrep, reps);
     if (h->inited) release_device(h);
     h->inited = 0;

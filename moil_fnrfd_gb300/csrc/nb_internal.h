@@ -8,6 +8,7 @@
 
 #include "moil_nb.h"
 #include "nb_common.cuh"
+#include "nb_foresight.h"
 
 // FFT plan for one length: radices (make_plan) and per Stockham stage s: the span Ns, the butterfly count nb = n/R, the magic
 // multiplier for dividing by nb, and nb (twiddle step, destination index) entries at off[s]
@@ -177,7 +178,7 @@ struct NbCtx {
                    gen == o.gen;
         }
     } gmd_key[3];
-    int md_wary = 0, md_backoff = 0;   // step loops left to the device's decision after a stale one
+    ListForesight md_lists;            // whether a run of MD steps follows the host's list schedule
     int *d_mdctl = nullptr;
     double *d_md_save = nullptr;       // the call's starting coordinates and velocities (the
                                        // per-step path redoes the call from them after an error)

@@ -247,8 +247,8 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
     // Device-side loop: every context replays graphs of whole steps with no host wait between them;
     // the error bits are read once at the end.  With a list period the host decides which steps
     // rebuild, in runs of at most 64 steps; a run whose lists were outrun before their time goes back
-    // to its saved state and leaves the decision to the device, as do some of the next runs (twice
-    // as many after each such run, 64 at most).  Any other error (a list overflow to regrow, a
+    // to its saved state and leaves the decision to the device, as do some of the next runs
+    // (ListForesight).  Any other error (a list overflow to regrow, a
     // non-finite coordinate) sends the run back to the saved state and the rest of the call through
     // the per-step path below, which handles it as a single evaluation does.
     int first = 0;
@@ -261,9 +261,9 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
     bool periods = true;
     for (const NbCtx *c : ctxs) periods &= c->list_period > 0;
     while (loop && first < nsteps) {
-        const bool host = periods && h->md_wary == 0;
+        const bool host = h->md_lists.host(periods);
         const int run = host ? std::min(nsteps - first, 64) : nsteps - first;
-        if (h->md_wary > 0) --h->md_wary;
+        h->md_lists.begin();
         NB_CUDA_OK(h, cudaMemcpyAsync(h->d_md_save, d_coor, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, h->stream));
         NB_CUDA_OK(h, cudaMemcpyAsync(h->d_md_save + 3 * n, d_vel, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice,
                                       h->stream));
@@ -292,6 +292,7 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
         }
         if (rc == MOIL_NB_OK && !err) {
             first += run;
+            if (host) h->md_lists.kept();
             continue;
         }
         NB_CUDA_OK(h, cudaMemcpyAsync(d_coor, h->d_md_save, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, h->stream));
@@ -301,7 +302,7 @@ int moil_nb_md_step(moil_nb_ctx *h, double *d_coor, double *d_vel, const double 
         for (NbCtx *c : ctxs) c->need_rebuild = 1;
         if (rc != MOIL_NB_OK) cudaGetLastError();
         if (rc != MOIL_NB_OK || err != NB_DEV_STALE) break;
-        h->md_wary = h->md_backoff = std::min(64, 2 * h->md_backoff + 2);
+        h->md_lists.outrun();
     }
     if (loop && first == nsteps) {
         if (!h->grp.empty()) {
