@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from moil_fnrfd_gb300 import systems as S
-from moil_fnrfd_gb300.nb import Nonbonded
+from moil_fnrfd_gb300.nb import MOIL_NB_FP64, MOIL_NB_MIXED, Nonbonded
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -77,3 +77,46 @@ def test_grouped_steps_follow_the_ungrouped_schedule():
         out.append(run(nb, state, 40))
         nb.close()
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]
+
+
+def loop_against_single_steps(make, state, steps, dt):
+    a = make()
+    got = run(a, state, steps, dt)
+    a.close()
+    b = make()
+    want = run(b, state, 1, dt, calls=steps)
+    b.close()
+    assert torch.isfinite(got[0]).all()
+    assert (got[0] - want[0]).abs().max() <= 1e-6 and (got[1] - want[1]).abs().max() <= 1e-3
+    assert all(abs(x - y) <= 1e-5 * abs(y) for x, y in zip(got[2], want[2])) and abs(got[3] - want[3]) <= 1e-5 * want[3]
+
+
+@pytest.mark.parametrize("precision", [MOIL_NB_MIXED, MOIL_NB_FP64], ids=["mixed", "fp64"])
+@pytest.mark.parametrize("name", ["waters", "solute"])
+def test_step_graphs_match_single_steps(name, precision):
+    """The gradient as the step graph's integrator forms it, in both precisions, with atoms outside waters (which
+    have correction terms and no rigid molecule) and without."""
+    if name == "waters":
+        state, s, dt = start([waters(216, 41, 4.0)]), waters(216, 41, 4.0)[0], 0.0005
+    else:
+        s, dt = S.config1(seed=7, n_solute=61, n_ions=7, n_waters=299, box=24.0), 0.00002    # (no bonded terms)
+        rng = np.random.Generator(np.random.PCG64(4))
+        v = rng.normal(0.0, 4.0, (s.npt, 3))
+        w = s.npt - 3 * s.nwaters
+        v[w:] = np.repeat(v[w::3], 3, axis=0)
+        state = (torch.tensor(s.coor, device="cuda"), torch.tensor(v, device="cuda"),
+                 torch.tensor(S.molecules(s)[1], device="cuda"))
+        torch.cuda.synchronize()
+    loop_against_single_steps(lambda: Nonbonded(s, precision=precision, skin=1.0, list_period=10), state, 25, dt)
+
+
+def test_one_group_outruns_its_lists():
+    """Fast waters in the first group only: the run goes back to its start in every group and is redone."""
+    ws = [waters(300, 51, 4.0), waters(216, 52, 0.05)]
+    systems = [s for s, _ in ws]
+
+    def make():
+        nb = Nonbonded(systems, skin=0.05, list_period=1000, groups=2)
+        assert nb.groups() == 2
+        return nb
+    loop_against_single_steps(make, start(ws), 40, 0.0005)
