@@ -102,10 +102,11 @@ __host__ __device__ inline int nb_spread_exp(double qfc_max)
 
 // PME fractional grid coordinates of a site.  FP64 path: fr in [0, n] as a double.  FP32 path:
 // fr as fixed point with 2^23 units per grid point (n <= 128, so below 2^30), kept in the bits
-// of a float -- a single FP32 value near n would hold the fraction to only 2^-24 n.
+// of a float -- a single FP32 value near n would hold the fraction to only 2^-24 n.  A fraction
+// outside [0, 1], from a coordinate of some 10^7 boxes or more, is cut off, so that no index leaves the grid.
 __device__ __forceinline__ float pme_fr_pack(int i, float w)
 {
-    return __int_as_float((i << 23) + min(__float2int_rn(w * 8388608.f), 8388607));
+    return __int_as_float((i << 23) + max(min(__float2int_rn(w * 8388608.f), 8388607), 0));
 }
 __device__ __forceinline__ void pme_fr_split(float v, int &i, float &w)
 {
