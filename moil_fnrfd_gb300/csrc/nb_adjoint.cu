@@ -71,16 +71,8 @@ __device__ __forceinline__ void lj_parts(int arith, double e12i, double e6i, dou
     }
 }
 
-template <typename T>
-__device__ __forceinline__ double2 lj_of(const void *lj_v, int s)
-{
-    typedef typename cplx<T>::type T2;
-    const T2 v = ((const T2 *)lj_v)[s];
-    return make_double2((double)v.x, (double)v.y);
-}
-
+// Plain FP64 path
 // one non-water-semantics site pair (atom_pair of the energy kernels) into site i's sums
-template <typename T>
 __device__ __forceinline__ void atom_pair_adj(const RepDev &R, double r2, double qi, double qj, double2 lji,
                                               double2 ljj, unsigned fi, unsigned fj, double &phi, double &de,
                                               double &ds)
@@ -103,26 +95,24 @@ __device__ __forceinline__ void atom_pair_adj(const RepDev &R, double r2, double
 
 // one warp per water: W1 (nine site pairs per molecule pair) and W2, the lanes taking the
 // entries of both lists in turn
-template <typename T, typename E>
+template <typename E>
 __global__ void __launch_bounds__(128) k_adj_water(int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
-                            const int *__restrict__ site_orig, const void *pos_v, const void *woff_v,
-                            const void *lj_v, const unsigned *__restrict__ sflags, const int2 *__restrict__ wl1_cnt,
+                            const int *__restrict__ site_orig, const double4 *__restrict__ pos,
+                            const double4 *__restrict__ woff, const double2 *__restrict__ lj,
+                            const unsigned *__restrict__ sflags, const int2 *__restrict__ wl1_cnt,
                             const void *__restrict__ wl1, int cap_row, const int *__restrict__ wl2_off,
                             const int *__restrict__ wl2, int cap2, double *__restrict__ dq, double *__restrict__ de,
                             double *__restrict__ ds)
 {
-    typedef typename vec4<T>::type T4;
     const int lane = threadIdx.x & 31, i = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (i >= nW) return;
-    const T4 *pos = (const T4 *)pos_v;
-    const T4 *woff = (const T4 *)woff_v;
     const RepDev &R = reps[site_rep[3 * i]];
-    const T4 oi = pos[3 * i];
-    const T4 h1 = woff[3 * i + 1], h2 = woff[3 * i + 2];
-    const T hi[3][3] = {{(T)0, (T)0, (T)0}, {h1.x, h1.y, h1.z}, {h2.x, h2.y, h2.z}};
+    const double4 oi = pos[3 * i];
+    const double4 h1 = woff[3 * i + 1], h2 = woff[3 * i + 2];
+    const double hi[3][3] = {{0.0, 0.0, 0.0}, {h1.x, h1.y, h1.z}, {h2.x, h2.y, h2.z}};
     double phi[3] = {0, 0, 0}, dE[3] = {0, 0, 0}, dS[3] = {0, 0, 0};
     double epsO, sigO;
-    const double2 ljO = lj_of<T>(lj_v, 3 * i);
+    const double2 ljO = lj[3 * i];
     lj_decode(R.arith, ljO.x, ljO.y, epsO, sigO);
     const int2 c = wl1_cnt[i];
     const int nn = min(c.x, cap_row), n = min(c.x + c.y, cap_row);
@@ -130,48 +120,47 @@ __global__ void __launch_bounds__(128) k_adj_water(int nW, const RepDev *__restr
     const int base = sizeof(E) == 2 ? R.wat0 : 0;   // uint16 entries: offsets from the replica's first water
     for (int v = lane; v < n; v += 32) {
         const int j = base + (int)row[v < nn ? v : cap_row - 1 - (v - nn)];
-        const T4 oj = pos[3 * j];
-        T dx = oi.x - oj.x, dy = oi.y - oj.y, dz = oi.z - oj.z;
-        const T nx = nb_rint(dx * rep_invL<T>(R, 0)), ny = nb_rint(dy * rep_invL<T>(R, 1)),
-                nz = nb_rint(dz * rep_invL<T>(R, 2));
+        const double4 oj = pos[3 * j];
+        double dx = oi.x - oj.x, dy = oi.y - oj.y, dz = oi.z - oj.z;
+        const double nx = nb_rint(dx * R.invLd[0]), ny = nb_rint(dy * R.invLd[1]), nz = nb_rint(dz * R.invLd[2]);
         dx = nb_shift(R, 0, dx, nx);
         dy = nb_shift(R, 1, dy, ny);
         dz = nb_shift(R, 2, dz, nz);
-        const T r2oo = dx * dx + dy * dy + dz * dz;
-        if (r2oo > (T)R.rmax2) continue;
-        const T4 j1 = woff[3 * j + 1], j2 = woff[3 * j + 2];
-        const T hj[3][3] = {{(T)0, (T)0, (T)0}, {j1.x, j1.y, j1.z}, {j2.x, j2.y, j2.z}};
-        const double qj[3] = {(double)oj.w, (double)pos[3 * j + 1].w, (double)pos[3 * j + 2].w};
+        const double r2oo = dx * dx + dy * dy + dz * dz;
+        if (r2oo > (double)R.rmax2) continue;
+        const double4 j1 = woff[3 * j + 1], j2 = woff[3 * j + 2];
+        const double hj[3][3] = {{0.0, 0.0, 0.0}, {j1.x, j1.y, j1.z}, {j2.x, j2.y, j2.z}};
+        const double qj[3] = {oj.w, pos[3 * j + 1].w, pos[3 * j + 2].w};
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
-                const double ex = (double)(hi[a][0] + dx - hj[b][0]), ey = (double)(hi[a][1] + dy - hj[b][1]),
-                             ez = (double)(hi[a][2] + dz - hj[b][2]);
+                const double ex = hi[a][0] + dx - hj[b][0], ey = hi[a][1] + dy - hj[b][1],
+                             ez = hi[a][2] + dz - hj[b][2];
                 const double r = sqrt(ex * ex + ey * ey + ez * ez);
                 phi[a] += R.epstmp * qj[b] * erfc(R.alphad * r) / r;
             }
-        if (r2oo <= (T)R.rv2) {
-            const double s2 = 1.0 / (double)r2oo, s6 = s2 * s2 * s2;
+        if (r2oo <= (double)R.rv2) {
+            const double s2 = 1.0 / r2oo, s6 = s2 * s2 * s2;
             double ej, sj;
-            const double2 ljj = lj_of<T>(lj_v, 3 * j);
+            const double2 ljj = lj[3 * j];
             lj_decode(R.arith, ljj.x, ljj.y, ej, sj);
             lj_adj(R.arith, R.w12d * s6 * s6, R.w6d * s6, epsO, sigO, sj, dE[0], dS[0]);
         }
     }
     for (int k = min(wl2_off[i], cap2) + lane; k < min(wl2_off[i + 1], cap2); k += 32) {
         const int s = wl2[k];
-        const T4 xj = pos[s];
-        const double2 ljj = lj_of<T>(lj_v, s);
+        const double4 xj = pos[s];
+        const double2 ljj = lj[s];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const T4 xi = pos[3 * i + a];
-            T dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-            dx = nb_shift(R, 0, dx, nb_rint(dx * rep_invL<T>(R, 0)));
-            dy = nb_shift(R, 1, dy, nb_rint(dy * rep_invL<T>(R, 1)));
-            dz = nb_shift(R, 2, dz, nb_rint(dz * rep_invL<T>(R, 2)));
-            atom_pair_adj<T>(R, (double)(dx * dx + dy * dy + dz * dz), (double)xi.w, (double)xj.w,
-                             lj_of<T>(lj_v, 3 * i + a), ljj, sflags[3 * i + a], sflags[s], phi[a], dE[a], dS[a]);
+            const double4 xi = pos[3 * i + a];
+            double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+            dx = nb_shift(R, 0, dx, nb_rint(dx * R.invLd[0]));
+            dy = nb_shift(R, 1, dy, nb_rint(dy * R.invLd[1]));
+            dz = nb_shift(R, 2, dz, nb_rint(dz * R.invLd[2]));
+            atom_pair_adj(R, dx * dx + dy * dy + dz * dz, xi.w, xj.w,
+                             lj[3 * i + a], ljj, sflags[3 * i + a], sflags[s], phi[a], dE[a], dS[a]);
         }
     }
 #pragma unroll
@@ -186,31 +175,28 @@ __global__ void __launch_bounds__(128) k_adj_water(int nW, const RepDev *__restr
 }
 
 // one warp per non-water atom over its X list
-template <typename T>
 __global__ void __launch_bounds__(128) k_adj_atom(int nA, int nW, const RepDev *__restrict__ reps, const int *__restrict__ site_rep,
-                           const int *__restrict__ site_orig, const void *pos_v, const void *lj_v,
+                           const int *__restrict__ site_orig, const double4 *__restrict__ pos, const double2 *__restrict__ lj,
                            const unsigned *__restrict__ sflags, const int *__restrict__ xl_off,
                            const int *__restrict__ xl, int capx, double *__restrict__ dq, double *__restrict__ de,
                            double *__restrict__ ds)
 {
-    typedef typename vec4<T>::type T4;
     const int lane = threadIdx.x & 31, k = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (k >= nA) return;
-    const T4 *pos = (const T4 *)pos_v;
     const int si = 3 * nW + k;
     const RepDev &R = reps[site_rep[si]];
-    const T4 xi = pos[si];
-    const double2 lji = lj_of<T>(lj_v, si);
+    const double4 xi = pos[si];
+    const double2 lji = lj[si];
     double phi = 0, dE = 0, dS = 0;
     for (int q = min(xl_off[k], capx) + lane; q < min(xl_off[k + 1], capx); q += 32) {
         const int s = xl[q];
-        const T4 xj = pos[s];
-        T dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        dx = nb_shift(R, 0, dx, nb_rint(dx * rep_invL<T>(R, 0)));
-        dy = nb_shift(R, 1, dy, nb_rint(dy * rep_invL<T>(R, 1)));
-        dz = nb_shift(R, 2, dz, nb_rint(dz * rep_invL<T>(R, 2)));
-        atom_pair_adj<T>(R, (double)(dx * dx + dy * dy + dz * dz), (double)xi.w, (double)xj.w, lji,
-                         lj_of<T>(lj_v, s), sflags[si], sflags[s], phi, dE, dS);
+        const double4 xj = pos[s];
+        double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+        dx = nb_shift(R, 0, dx, nb_rint(dx * R.invLd[0]));
+        dy = nb_shift(R, 1, dy, nb_rint(dy * R.invLd[1]));
+        dz = nb_shift(R, 2, dz, nb_rint(dz * R.invLd[2]));
+        atom_pair_adj(R, dx * dx + dy * dy + dz * dz, xi.w, xj.w, lji,
+                         lj[s], sflags[si], sflags[s], phi, dE, dS);
     }
     phi = sub_sum<32>(phi); dE = sub_sum<32>(dE); dS = sub_sum<32>(dS);
     if (lane != 0) return;
@@ -717,9 +703,9 @@ void adjoint_pairs(NbCtx *c, cudaStream_t sw, cudaStream_t sa, double *d_dq, dou
     const int B = 128, capx = cap_int(c->cap_xl), cap2 = cap_int(c->cap_wl2);
     const bool fp64 = c->precision == MOIL_NB_FP64;
     if (c->nW > 0 && fp64)
-        (c->row16 ? k_adj_water<double, unsigned short> : k_adj_water<double, int>)<<<(int)((c->nW + 3) / 4), B, 0, sw>>>(
-            (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_woff, c->d_site_lj, c->d_site_flags,
-            c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2, cap2, d_dq, d_de, d_ds);
+        (c->row16 ? k_adj_water<unsigned short> : k_adj_water<int>)<<<(int)((c->nW + 3) / 4), B, 0, sw>>>(
+            (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, (const double4 *)c->d_pos, (const double4 *)c->d_woff,
+            (const double2 *)c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2, cap2, d_dq, d_de, d_ds);
     else if (c->nW > 0) {
         // lanes per water as the energy kernel (32-bit rows belong to replicas of 65,536 waters or more)
         const int lpw = c->nw_handle <= 4096 ? 32 : 8;
@@ -731,9 +717,9 @@ void adjoint_pairs(NbCtx *c, cudaStream_t sw, cudaStream_t sa, double *d_dq, dou
             cap2, d_dq, d_de, d_ds);
     }
     if (c->nA > 0 && fp64)
-        k_adj_atom<double><<<(int)((c->nA + 3) / 4), B, 0, sa>>>(
-            (int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_site_lj, c->d_site_flags,
-            c->d_xl_off, c->d_xl, capx, d_dq, d_de, d_ds);
+        k_adj_atom<<<(int)((c->nA + 3) / 4), B, 0, sa>>>(
+            (int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, (const double4 *)c->d_pos,
+            (const double2 *)c->d_site_lj, c->d_site_flags, c->d_xl_off, c->d_xl, capx, d_dq, d_de, d_ds);
     else if (c->nA > 0)
         k_adj_atom_f<<<(int)((c->nA + 3) / 4), B, 0, sa>>>(
             (int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, (const float4 *)c->d_pos,

@@ -22,7 +22,6 @@
 #define NB_FIX_SCALE 4294967296.0     // 2^32
 #define NB_FIX_SCALE_F 4294967296.0f
 #define NB_FIX_INV (1.0 / 4294967296.0)
-#define NB_PLANE_SCALE 1099511627776.0  // 2^40: PME plane accumulation
 #define NB_MAX_FFT 128
 #define NB_TWO_OVER_SQRTPI 1.1283791670955126
 #define NB_EU 8                       // per-unit outputs: LJ prim, LJ img, Coul prim, Coul img, site pairs,

@@ -1259,7 +1259,8 @@ int moil_nb_create(moil_nb_ctx **out, int device)
     moil_nb_ctx *h = new moil_nb_ctx();
     h->device = device;
     int lo = 0, hi = 0;
-    if (cudaSetDevice(device) != cudaSuccess || cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess || cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
+    if (cudaSetDevice(device) != cudaSuccess || cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithPriority(&h->stream2, cudaStreamNonBlocking, hi) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->stream2n, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->stream3, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1272,6 +1273,7 @@ int moil_nb_create(moil_nb_ctx **out, int device)
         if (h->stream3) cudaStreamDestroy(h->stream3);
         if (h->ev_fork) cudaEventDestroy(h->ev_fork);
         if (h->ev_join) cudaEventDestroy(h->ev_join);
+        if (h->ev_join3) cudaEventDestroy(h->ev_join3);
         delete h;
         return MOIL_NB_ERR_CUDA;
     }

@@ -148,7 +148,7 @@ struct NbCtx {
     std::vector<int> col_begin;        // per replica, nrep+1
     int *d_col_begin = nullptr;
     double *d_e_col = nullptr;         // energy partial per column work item
-    size_t smem_plane_fwd = 0, smem_plane_inv = 0, smem_zconv = 0;
+    size_t smem_plane = 0, smem_zconv = 0;
     int max_n1 = 0, max_n2 = 0, max_n3 = 0;
 
     // energies

@@ -817,9 +817,9 @@ __device__ __forceinline__ long long block_excl_scan(long long s, long long *war
 #define NB_SCAN_PER 16
 #define NB_SCAN_TILE (NB_SCAN_PER * 256)
 __global__ void __launch_bounds__(256) k_scan_sums(const int *__restrict__ in, int n, long long *__restrict__ bsum,
-                                                   const int *st, int gate)
+                                                   const int *st)
 {
-    if (gate && rebuild_off(st)) return;
+    if (rebuild_off(st)) return;
     __shared__ long long ws[8];
     const int base = blockIdx.x * NB_SCAN_TILE;
     long long s = 0;
@@ -831,9 +831,9 @@ __global__ void __launch_bounds__(256) k_scan_sums(const int *__restrict__ in, i
 }
 
 __global__ void __launch_bounds__(1024) k_scan_top(long long *__restrict__ bsum, int nb, int *__restrict__ out, int n,
-                                                   int *total, const int *st, int gate)
+                                                   int *total, const int *st)
 {
-    if (gate && rebuild_off(st)) return;
+    if (rebuild_off(st)) return;
     __shared__ long long ws[32];
     long long carry = 0;
     for (int b0 = 0; b0 < nb; b0 += 1024) {
@@ -850,9 +850,9 @@ __global__ void __launch_bounds__(1024) k_scan_top(long long *__restrict__ bsum,
 }
 
 __global__ void __launch_bounds__(256) k_scan_tiles(const int *__restrict__ in, int *__restrict__ out, int n,
-                                                    const long long *__restrict__ bsum, const int *st, int gate)
+                                                    const long long *__restrict__ bsum, const int *st)
 {
-    if (gate && rebuild_off(st)) return;
+    if (rebuild_off(st)) return;
     __shared__ long long ws[8];
     const int i0 = blockIdx.x * NB_SCAN_TILE + threadIdx.x * NB_SCAN_PER;
     int v[NB_SCAN_PER];
@@ -875,9 +875,9 @@ __global__ void __launch_bounds__(256) k_scan_tiles(const int *__restrict__ in, 
 // to NB_SCAN_ONE entries (eight chunks, about 3 us) it is cheaper than three launches
 #define NB_SCAN_ONE 8192
 __global__ void __launch_bounds__(1024) k_scan_small(const int *__restrict__ in, int *__restrict__ out, int n,
-                                                     int *total, const int *st, int gate)
+                                                     int *total, const int *st)
 {
-    if (gate && rebuild_off(st)) return;
+    if (rebuild_off(st)) return;
     __shared__ long long ws[32];
     long long carry = 0;
     for (int i0 = 0; i0 < n; i0 += 1024) {
@@ -894,20 +894,19 @@ __global__ void __launch_bounds__(1024) k_scan_small(const int *__restrict__ in,
 }
 
 // out[0..n] = exclusive prefix sums of in[0..n), out[n] = total (also to *total when given);
-// gate: skip unless the rebuild flag is set
-void nb_scan(NbCtx *c, const int *in, int *out, int n, int *total, int gate)
+// (skipped unless the rebuild flag is set)
+void nb_scan(NbCtx *c, const int *in, int *out, int n, int *total)
 {
     const int nb = std::max(1, (n + NB_SCAN_TILE - 1) / NB_SCAN_TILE);
     cudaStream_t s = c->stream;
-    if (n <= NB_SCAN_ONE || !c->d_scan_tmp) {
-        // (the allocation-free entry point has no tile-sum scratch)
-        k_scan_small<<<1, 1024, 0, s>>>(in, out, n, total, c->d_status, gate);
+    if (n <= NB_SCAN_ONE) {
+        k_scan_small<<<1, 1024, 0, s>>>(in, out, n, total, c->d_status);
         c->launches++;
         return;
     }
-    k_scan_sums<<<nb, 256, 0, s>>>(in, n, c->d_scan_tmp, c->d_status, gate);
-    k_scan_top<<<1, 1024, 0, s>>>(c->d_scan_tmp, nb, out, n, total, c->d_status, gate);
-    k_scan_tiles<<<nb, 256, 0, s>>>(in, out, n, c->d_scan_tmp, c->d_status, gate);
+    k_scan_sums<<<nb, 256, 0, s>>>(in, n, c->d_scan_tmp, c->d_status);
+    k_scan_top<<<1, 1024, 0, s>>>(c->d_scan_tmp, nb, out, n, total, c->d_status);
+    k_scan_tiles<<<nb, 256, 0, s>>>(in, out, n, c->d_scan_tmp, c->d_status);
     c->launches += 3;
 }
 
@@ -977,7 +976,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
     k_unit_keys<<<grid(c->nunit, B), B, 0, s>>>((int)c->nunit, (int)c->nW, c->ncell, c->d_unit_atom, c->d_unit_rep,
                                                 c->d_reps, d_coor, c->d_unit_key, c->d_unit_slot, c->d_bin_count,
                                                 c->d_status);
-    nb_scan(c, c->d_bin_count, c->d_bin_start, nbin, nullptr, 1);
+    nb_scan(c, c->d_bin_count, c->d_bin_start, nbin, nullptr);
     k_unit_scatter<<<grid(c->nunit, B), B, 0, s>>>((int)c->nunit, c->d_unit_key, c->d_unit_slot, c->d_bin_start,
                                                    c->d_sorted_unit, c->d_status);
     k_bin_sort<<<grid(nbin, 4), 128, 0, s>>>(nbin, c->d_bin_start, c->d_sorted_unit, c->d_status);
@@ -1009,7 +1008,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
                                                         c->d_wl1, c->cap_row1, c->d_status);
         c->launches += (search ? 1 : 0) + (nt > 0 ? 1 : 0);
         if (c->nA == 0) return;
-        nb_scan(c, cnt2, c->d_wl2_off, (int)c->nW, c->d_status + 3, 1);
+        nb_scan(c, cnt2, c->d_wl2_off, (int)c->nW, c->d_status + 3);
         k_wlist<T, 1, E><<<gw, 32 * NB_LW, 0, s>>>((int)c->nW, c->d_reps, c->d_site_rep, c->d_pos, c->d_opos, c->d_bin_start,
                                             c->ncell, nullptr, nullptr, c->d_wl2_off, nullptr, 0, c->d_wl2, c->cap_wl2,
                                             c->d_status);
@@ -1033,7 +1032,7 @@ void build_lists_t(NbCtx *c, const double *d_coor)
         k_xlist<T, 0><<<ga, 32 * NB_LW, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_opos,
                                          c->d_bin_start, c->ncell, c->d_ex_off, c->d_ex_j, c->d_count_tmp, nullptr,
                                          nullptr, 0, c->d_status);
-        nb_scan(c, c->d_count_tmp, c->d_xl_off, (int)c->nA, c->d_status + 4, 1);
+        nb_scan(c, c->d_count_tmp, c->d_xl_off, (int)c->nA, c->d_status + 4);
         k_xlist<T, 1><<<ga, 32 * NB_LW, 0, s>>>((int)c->nA, (int)c->nW, c->d_reps, c->d_site_rep, c->d_site_orig, c->d_pos, c->d_opos,
                                          c->d_bin_start, c->ncell, c->d_ex_off, c->d_ex_j, nullptr, c->d_xl_off,
                                          c->d_xl, c->cap_xl, c->d_status);

@@ -688,10 +688,9 @@ __global__ void __launch_bounds__(256) k_press_zvir_f(const ColWork *__restrict_
     }
 }
 
-// inverse y and x transforms of plane z; the real potential plane (n1 x n2 floats) is stored
-// over the plane's own complex storage, which this block alone reads, for k_pme_gather_f
-// Inverse y and x transforms of plane z (the comment above): the first pass reads the grid and the last
-// one stores the real rows.
+// Inverse y and x transforms of plane z: the first pass reads the grid and the last one stores the real
+// rows (k_plane_fwd).  FP32: the real potential plane (n1 x n2 floats) goes over the plane's own complex storage,
+// which this block alone reads, for k_pme_gather_f; FP64: the block gathers its sites' shares itself.
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 2) k_plane_inv(const PlaneWork *__restrict__ work,
                                                      const int4 *__restrict__ blob,
@@ -961,7 +960,7 @@ void pme_t(NbCtx *c)
     typedef typename cplx<T>::type C;
     typedef typename vec4<T>::type T4;
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
-    k_plane_fwd<T><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
+    k_plane_fwd<T><<<np, 256, c->smem_plane, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
                                                       (const T4 *)c->d_fr, (C *)c->d_grid);
     if (c->timing) cudaEventRecord(c->ev[7], s);
     if constexpr (sizeof(T) == 4)
@@ -971,7 +970,7 @@ void pme_t(NbCtx *c)
         k_zconv_d<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, (const double *)c->d_bsp,
                                                  (double2 *)c->d_grid, c->d_e_col);
     if (c->timing) cudaEventRecord(c->ev[8], s);
-    k_plane_inv<T><<<np, 256, c->smem_plane_inv, s>>>(c->d_planes, c->d_blob, (C *)c->d_grid, c->d_reps, (int)c->nW,
+    k_plane_inv<T><<<np, 256, c->smem_plane, s>>>(c->d_planes, c->d_blob, (C *)c->d_grid, c->d_reps, (int)c->nW,
                                                       c->d_zidx, (const T4 *)c->d_fr, (T *)c->d_part, 0);
     if constexpr (sizeof(T) == 4) {
         // four lanes per site while they all fit the GPU at once (an evaluation of 216 waters 50.7 / 47.2 us
@@ -1107,11 +1106,11 @@ cudaError_t raise_smem_limit(K *kernel, size_t bytes)
 }
 
 template <typename T>
-cudaError_t raise_pme_limits(size_t sf, size_t sz, size_t si)
+cudaError_t raise_pme_limits(size_t sp, size_t sz)
 {
     cudaError_t e;
-    if ((e = raise_smem_limit(k_plane_fwd<T>, sf)) != cudaSuccess) return e;
-    if ((e = raise_smem_limit(k_plane_inv<T>, si)) != cudaSuccess) return e;
+    if ((e = raise_smem_limit(k_plane_fwd<T>, sp)) != cudaSuccess) return e;
+    if ((e = raise_smem_limit(k_plane_inv<T>, sp)) != cudaSuccess) return e;
     if constexpr (sizeof(T) == 4) {
         if ((e = raise_smem_limit(k_zconv_f, sz)) != cudaSuccess) return e;
         return raise_smem_limit(k_press_zvir_f, sz);
@@ -1172,7 +1171,7 @@ int configure_t(NbCtx *c)
     c->planes.clear();
     c->cols.clear();
     c->col_begin.assign(c->nrep + 1, 0);
-    size_t sf = 0, si = 0, sz = 0;
+    size_t sp = 0, sz = 0;
     const int tk = col_tile<T>();
     for (int r = 0; r < c->nrep; ++r) {
         const RepDev &R = c->rd[r];
@@ -1182,22 +1181,20 @@ int configure_t(NbCtx *c)
         c->col_begin[r] = (int)c->cols.size();
         for (int kx = 0; kx < R.n1h; ++kx)
             push_col_runs(c->cols, ColWork{r, kx, 0, 0, R.n1, R.n2, R.n3, R.bsp0, boff[pl[2]], blen[pl[2]], R.g0}, tk);
-        sf = std::max(sf, plane_smem<T>(R.n1, R.n2));
-        si = std::max(si, plane_smem<T>(R.n1, R.n2));
+        sp = std::max(sp, plane_smem<T>(R.n1, R.n2));
         sz = std::max(sz, zconv_smem<T>(R.n3));
     }
     c->col_begin[c->nrep] = (int)c->cols.size();
     int dev_smem = 0;
     cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-    if ((int)sf > dev_smem || (int)si > dev_smem || (int)sz > dev_smem) {
+    if ((int)sp > dev_smem || (int)sz > dev_smem) {
         c->err = "PME grid plane does not fit in shared memory";
         return MOIL_NB_ERR_GRID;
     }
-    c->smem_plane_fwd = sf;
-    c->smem_plane_inv = si;
+    c->smem_plane = sp;
     c->smem_zconv = sz;
     // the limit is per kernel, shared by every handle in the process: only ever raise it
-    NB_CUDA_OK(c, raise_pme_limits<T>(sf, sz, si));
+    NB_CUDA_OK(c, raise_pme_limits<T>(sp, sz));
     NB_CUDA_OK(c, cudaMalloc(&c->d_planes, sizeof(PlaneWork) * c->planes.size()));
     NB_CUDA_OK(c, cudaMemcpy(c->d_planes, c->planes.data(), sizeof(PlaneWork) * c->planes.size(), cudaMemcpyHostToDevice));
     NB_CUDA_OK(c, cudaMalloc(&c->d_cols, sizeof(ColWork) * c->cols.size()));
@@ -1229,13 +1226,13 @@ void nb_launch_pme_virial(NbCtx *c, cudaStream_t s, void *grid, double *v_col)
 {
     const int np = (int)c->planes.size(), nc = (int)c->cols.size();
     if (c->precision == MOIL_NB_FP64) {
-        k_plane_fwd<double><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
+        k_plane_fwd<double><<<np, 256, c->smem_plane, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
                                                                (const double4 *)c->d_fr, (double2 *)grid);
         k_press_zvir_d<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, (const double *)c->d_bsp,
                                                       (const double2 *)grid, v_col);
         return;
     }
-    k_plane_fwd<float><<<np, 256, c->smem_plane_fwd, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
+    k_plane_fwd<float><<<np, 256, c->smem_plane, s>>>(c->d_planes, c->d_reps, c->d_blob, (int)c->nW, c->d_zidx,
                                                           (const float4 *)c->d_fr, (float2 *)grid);
     k_press_zvir_f<<<nc, 256, c->smem_zconv, s>>>(c->d_cols, c->d_reps, c->d_blob, (const float *)c->d_bsp,
                                                   (const float2 *)grid, v_col);
@@ -1245,7 +1242,7 @@ void nb_launch_pme_virial(NbCtx *c, cudaStream_t s, void *grid, double *v_col)
 // (4 slots per site) from the convolved grid the evaluation left in place
 void nb_launch_pme_potential(NbCtx *c, double *phi4)
 {
-    k_plane_inv<double><<<(int)c->planes.size(), 256, c->smem_plane_inv, c->stream>>>(
+    k_plane_inv<double><<<(int)c->planes.size(), 256, c->smem_plane, c->stream>>>(
         c->d_planes, c->d_blob, (double2 *)c->d_grid, c->d_reps, (int)c->nW, c->d_zidx, (const double4 *)c->d_fr, phi4,
         1);
 }
@@ -1455,13 +1452,11 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
         int optin = 0;
         if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
             return MOIL_NB_ERR_CUDA;
-        if (plane_smem<float>(n1, n2) > (size_t)optin || plane_smem<float>(n1, n2) > (size_t)optin ||
-            zconv_smem<float>(n3) > (size_t)optin)
+        if (plane_smem<float>(n1, n2) > (size_t)optin || zconv_smem<float>(n3) > (size_t)optin)
             return MOIL_NB_ERR_GRID;
     }
     // shared-memory limits for this grid (raise only; other handles may need more)
-    if (raise_pme_limits<float>(plane_smem<float>(n1, n2), zconv_smem<float>(n3),
-                                plane_smem<float>(n1, n2)) != cudaSuccess)
+    if (raise_pme_limits<float>(plane_smem<float>(n1, n2), zconv_smem<float>(n3)) != cudaSuccess)
         return MOIL_NB_ERR_CUDA;
     // one-replica constants, FFT plans and tables, work lists (host side)
     NaParams P;
@@ -1506,8 +1501,7 @@ extern "C" int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int 
     for (int kx = 0; kx < R.n1h; ++kx)
         push_col_runs(tmp.cols, ColWork{0, kx, 0, 0, n1, n2, n3, 0, boff[2], blen[2], 0}, NB_TKF);
     if (NA_BLOB + sizeof(int4) * blob.size() > NA_HOST_BYTES) return MOIL_NB_ERR_GRID;
-    tmp.smem_plane_fwd = plane_smem<float>(n1, n2);
-    tmp.smem_plane_inv = plane_smem<float>(n1, n2);
+    tmp.smem_plane = plane_smem<float>(n1, n2);
     tmp.smem_zconv = zconv_smem<float>(n3);
     tmp.d_site_rep = (int *)(base + NA_REP);
     tmp.d_fr = base + NA_FR;

@@ -4,7 +4,7 @@
 //                555-566, image pairs symm/symwat_ewald.f:161-173, symm/symcdie_ewald.f:151-161)
 //   V_PIdirXX..  real-space Ewald Coulomb pairs (watwat_ewald.f:196-204,
 //                cdie_ewald.f:412-429, symwat_ewald.f:193-203)
-//   V_PIrecXX..  reciprocal sum (pot/ewald_receip.f:799-807; k_press_zvir_f / k_press_zvir in
+//   V_PIrecXX..  reciprocal sum (pot/ewald_receip.f:799-807; k_press_zvir_f / _d in
 //                nb_pme.cu)
 //   V_PIrelXX..  PME force times the atom's position relative to its molecule's centre of
 //                mass (ewald_receip.f:928-933)

@@ -114,7 +114,7 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const dou
             bool img;
             min_image(R, dx, dy, dz, img);
             double r2 = dx * dx + dy * dy + dz * dz;
-            double eel = 0, elj = 0, vir = 0;   // the virial of these pairs is counted by k_atom
+            double eel = 0, elj = 0, vir = 0;   // the virial of these pairs is counted by k_atom_d
             double df = atom_pair(R, r2, si[a].w, xj.w, lji[a].x, lji[a].y, ljj.x, ljj.y, fi[a], fj, eel, elj, vir,
                                 npair);
             g[3 * a] += df * dx;
@@ -160,7 +160,7 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, const AtomK &A, 
         xb = pos[sb]; lb = lj[sb];
         sn = entry(k + 2 * stride);
         const unsigned fj = A.tiny ? sflags[s] & SF_HTINY : 0;
-        float eel, elj, vir;      // the virial of these pairs is counted by k_atom
+        float eel, elj, vir;      // the virial of these pairs is counted by k_atom_f
         bool img;
         {
             float dx = o.x - xj.x, dy = o.y - xj.y, dz = o.z - xj.z;
@@ -200,10 +200,9 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, const AtomK &A, 
 }
 
 // ---------------------------------------------------------------------------------
-// water molecule per thread: W1 (water-water, 9 site pairs) then W2 (water-site x other).
-// Per-lane FP32 partial gradients and energies are flushed every CHUNK list entries into
-// int64 / FP64 accumulators kept in shared memory (one column per thread), which keeps
-// them out of the register file.
+// Water kernels: W1 (water-water, 9 site pairs) then W2 (water sites x other atoms).  FP32 partial gradients
+// and energies are flushed every CHUNK list entries of a lane, gradients as int64 fixed point, energies
+// as hi + lo pairs.
 #define WBLOCK 128
 
 // Plain FP64 path: one warp per water.  Bound: the FP64 pipe (two lanes per clock and SM), about
