@@ -133,7 +133,7 @@ __device__ __forceinline__ void water_vs_atoms(const RepDev &R, int i, const dou
 template <typename Flush>
 __device__ __forceinline__ void water_vs_atoms(const RepDev &R, const AtomK &A, int i, const float4 *pos, const void *lj_v,
                                                const unsigned *__restrict__ sflags, const int *__restrict__ wl2_off,
-                                               const int *__restrict__ wl2, int cap2, int first, int stride, int cnt,
+                                               const int *__restrict__ wl2, int cap2, int first, int stride, int &cnt,
                                                float g[9], float e4[4], int &npair, Flush &flush_all)
 {
     const int q0 = min(wl2_off[i], cap2), q1 = min(wl2_off[i + 1], cap2);
@@ -409,8 +409,11 @@ __device__ __forceinline__ float water_intra_f(const RepDev &R, float4 h1, float
 // partner site) -- and the O-O pair with its LJ part runs scalar, so one partner record is
 // live at a time.  Bound: for small handles the latency of a row's rounds, beyond the L1 wavefronts of
 // the record gathers.  Water stage against one water per thread: 216 waters 62 -> 13 us, 7,000 79 -> 21
-// (the lane counts at water_lanes).  VIR: also the water-water LJ virial terms.
-template <int LPW, bool VIR, typename E>
+// (the lane counts at water_lanes).  VIR: also the water-water LJ virial terms.  ATOMS: the handle has atoms
+// outside waters, whose lists (W2) come first, so that one barrier stands between the last flush of either
+// list and the sums; with W2 after the rows and a barrier behind it the water stage of 28,900 waters without
+// an atom took 62 us, 55 without that part, and that of 5 solute systems 129, 122 in this order.
+template <int LPW, bool VIR, bool ATOMS, typename E>
 __global__ void __launch_bounds__(WBLOCK, 4) k_water_s(int nW, const RepDev *__restrict__ reps,
                                                        const int *__restrict__ site_rep, const float4 *__restrict__ pos,
                                                        const float4 *__restrict__ woff, const void *lj_v,
@@ -531,9 +534,16 @@ __global__ void __launch_bounds__(WBLOCK, 4) k_water_s(int nW, const RepDev *__r
             npair += 9;
         }
     };
+    int cnt = 0;
+    if constexpr (ATOMS) {
+        if (act) {
+            const AtomK A(R, iL0, iL1, iL2, L0, L1, L2, m0, m1, m2, rmax2, rv2, K);
+            water_vs_atoms(R, A, i, pos, lj_v, sflags, wl2_off, wl2, cap2, sub, LPW, cnt, g, e4, npair, flush_all);
+        }
+        __syncwarp();
+    }
     // two record buffers in turn, as in k_water_h: the next entry's record is on its way while one is
     // worked on, row entries two ahead of their records
-    int cnt = 0;
     if (sub < n) {
         auto entry = [&](int k) { return row.at(min(k, n - 1)); };
         int ja = entry(sub), jb = entry(sub + LPW);
@@ -549,27 +559,21 @@ __global__ void __launch_bounds__(WBLOCK, 4) k_water_s(int nW, const RepDev *__r
             if (k + LPW < n) pair(ob, hb, ib);
             jb = jd;
             cnt += 2;
-            if (cnt >= CHUNK) { flush_all(); cnt = 0; }
+            if (cnt >= CHUNK - 1) { flush_all(); cnt = 0; }     // (64 entries; 63 or 64 behind a list of atoms)
         }
     }
-    __syncwarp();     // rows differ in length: the lanes that end early wait here
-    fold();
-    if (act) {
-        const AtomK A(R, iL0, iL1, iL2, L0, L1, L2, m0, m1, m2, rmax2, rv2, K);
-        water_vs_atoms(R, A, i, pos, lj_v, sflags, wl2_off, wl2, cap2, sub, LPW, cnt, g, e4, npair, flush_all);
-    }
-    __syncwarp();     // the lanes' flushes into sG come before its reads (the shuffles below order no memory)
-    float ecorr = 0.f;
-    if (intra && sub == 0) {
-        // the molecule's own exclusion corrections (every water excludes exactly its three pairs); as large
-        // as all its other forces together, they are rounded to fixed point by themselves
-        const float qs[3] = {oi0.w, oi1.w, oi2.w};
-        float gi[9] = {};
-        ecorr = water_intra_f(R, oi1, oi2, qs, gi);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) sG[w][k] += (unsigned long long)nb_fix(gi[k]);
-    }
+    // rows differ in length: the lanes that end early wait here, and the last flushes into sG come before
+    // its reads (the shuffles below order no memory)
     __syncwarp();
+    fold();
+    // the molecule's own exclusion corrections (every water excludes exactly its three pairs), in every lane; as
+    // large as all its other forces together, they join them after the sum over the lanes (a fixed-point
+    // number of their own cost 5 us of 28,900 waters' evaluation: conversions to 64 bits take the FP64 pipe)
+    float ecorr = 0.f, gi[9] = {};
+    if (intra) {
+        const float qs[3] = {oi0.w, oi1.w, oi2.w};
+        ecorr = water_intra_f(R, oi1, oi2, qs, gi);
+    }
     flush_e();
 #pragma unroll
     for (int k = 0; k < 9; ++k)
@@ -582,7 +586,7 @@ __global__ void __launch_bounds__(WBLOCK, 4) k_water_s(int nW, const RepDev *__r
     if (!act) return;
 #pragma unroll
     for (int k = 0; k < 9; ++k)
-        if (sub == k % LPW) grad[(size_t)9 * i + k] = nb_fix(g[k]) + (long long)sG[w][k];
+        if (sub == k % LPW) grad[(size_t)9 * i + k] = nb_fix(g[k] + gi[k]) + (long long)sG[w][k];
     if (sub == 0) {
         double *eu = e_unit + NB_EU * (size_t)i;
 #pragma unroll
@@ -811,7 +815,8 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
         flush(2.f, gx);
         if (wl2_off[i] < wl2_off[i + 1]) {
             const AtomK A(R, iL0, iL1, iL2, L0, L1, L2, m0, m1, m2, rmax2, rv2, K);
-            water_vs_atoms(R, A, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, 0, g, e4, npair, flush1);
+            cnt = 0;
+            water_vs_atoms(R, A, i, pos, lj_v, sflags, wl2_off, wl2, cap2, 0, 1, cnt, g, e4, npair, flush1);
             flush1();
         }
 #pragma unroll
@@ -1307,15 +1312,22 @@ int water_lanes(const NbCtx *c)
     return c->nw_handle <= (c->w2_handle < NB_W2_SOLUTE ? 4096 : 8192) ? 32 : (c->nw_handle <= 32768 ? 8 : 4);
 }
 
-using WaterSFn = decltype(&k_water_s<8, false, int>);
-WaterSFn water_s_fn(int lpw, bool vir, bool row16)
+using WaterSFn = decltype(&k_water_s<8, false, false, int>);
+template <bool VIR, bool ATOMS>
+WaterSFn water_s_fn(int lpw, bool row16)
 {
-    if (!row16) return vir ? k_water_s<4, true, int> : k_water_s<4, false, int>;
+    if (!row16) return k_water_s<4, VIR, ATOMS, int>;
     switch (lpw) {
-    case 32: return vir ? k_water_s<32, true, unsigned short> : k_water_s<32, false, unsigned short>;
-    case 8: return vir ? k_water_s<8, true, unsigned short> : k_water_s<8, false, unsigned short>;
-    default: return vir ? k_water_s<4, true, unsigned short> : k_water_s<4, false, unsigned short>;
+    case 32: return k_water_s<32, VIR, ATOMS, unsigned short>;
+    case 8: return k_water_s<8, VIR, ATOMS, unsigned short>;
+    default: return k_water_s<4, VIR, ATOMS, unsigned short>;
     }
+}
+// (atoms: of the whole handle, so every replica group runs the same kernel)
+WaterSFn water_s_fn(int lpw, bool vir, bool atoms, bool row16)
+{
+    if (atoms) return vir ? water_s_fn<true, true>(lpw, row16) : water_s_fn<false, true>(lpw, row16);
+    return vir ? water_s_fn<true, false>(lpw, row16) : water_s_fn<false, false>(lpw, row16);
 }
 
 template <typename T>
@@ -1332,7 +1344,7 @@ void water_t(NbCtx *c)
     } else if (c->nW > 0) {
         if constexpr (sizeof(T) == 4) {
             const int lpw = water_lanes(c);
-            water_s_fn(lpw, c->virial, c->row16)<<<(int)((c->nW * lpw + WBLOCK - 1) / WBLOCK), WBLOCK, 0, s>>>(
+            water_s_fn(lpw, c->virial, c->na_handle > 0, c->row16)<<<(int)((c->nW * lpw + WBLOCK - 1) / WBLOCK), WBLOCK, 0, s>>>(
                 (int)c->nW, c->d_reps, c->d_site_rep, (const float4 *)c->d_pos, (const float4 *)c->d_woff,
                 c->d_site_lj, c->d_site_flags, c->d_wl1_cnt, c->d_wl1, c->cap_row1, c->d_wl2_off, c->d_wl2,
                 cap_int(c->cap_wl2), c->d_grad_site, c->d_e_unit, c->water_excl_fast);
@@ -1391,11 +1403,11 @@ static int carveout_pct(NbCtx *c, size_t bytes)
 
 int nb_realspace_configure(NbCtx *c)
 {
-    // full-list FP32 water kernel: four resident blocks of static shared memory; the smallest
+    // full-list FP32 water kernels: four resident blocks of static shared memory; the smallest
     // carveout that holds them leaves the most L1 for the partner-record gathers
     for (int lpw : {32, 8, 4})
-        for (int k = 0; k < 4; ++k) {
-            const void *fn = (const void *)water_s_fn(lpw, k & 1, k & 2);
+        for (int k = 0; k < 8; ++k) {
+            const void *fn = (const void *)water_s_fn(lpw, k & 1, k & 2, k & 4);
             cudaFuncAttributes fa;
             NB_CUDA_OK(c, cudaFuncGetAttributes(&fa, fn));
             NB_CUDA_OK(c, cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
