@@ -185,8 +185,9 @@ int moil_nb_get_virial(moil_nb_ctx *h, int replica, double *virvdw);
  * dE/dsigma of the atom's LJ parameters decoded from the epsgm encoding
  * (connect/fillpt.f:136-184).  Any output may be NULL; energies as moil_nb_eval.  No
  * counterpart in the reference, which computes no parameter derivatives; both precisions
- * (pair terms in the handle's arithmetic, sums in FP64).  The LJ switch extension is not
- * differentiated. */
+ * (FP64 throughout; mixed: FP32 pair terms, summed in FP32 over at most 64 list entries and
+ * then as unevaluated pairs of FP32 numbers, the corrections in FP64).  The LJ switch extension
+ * is not differentiated. */
 int moil_nb_adjoint(moil_nb_ctx *h, const double *coor, double *dEdq, double *dEdeps, double *dEdsig,
                     moil_energies *energies);
 
@@ -319,7 +320,7 @@ int moil_nb_autotune(moil_nb_ctx *h, int nrep, const moil_replica *reps, const d
  * synchronisation that cudaMalloc/cudaFree may impose in the middle of its own
  * stream work.  It computes the PME reciprocal energy and its gradient for one
  * system with the same kernels as the handle path, taking every scratch buffer
- * from one file-scope device array of about 7.5 MB that each GPU loading this
+ * from one file-scope device array of about 5.6 MB that each GPU loading this
  * library holds until the process exits.
  *   limits   natom <= 65536; each grid side 4..64 and 2/3/5-smooth; order 4;
  *            mixed precision (FP32 spline and FFT math, FP64 energy)
@@ -336,9 +337,8 @@ int moil_nb_autotune(moil_nb_ctx *h, int nrep, const moil_replica *reps, const d
  * starts, or raised by its launches, is returned as MOIL_NB_ERR_CUDA and left pending;
  * a grid whose planes do not fit in shared memory is refused with MOIL_NB_ERR_GRID.
  * Every call reuses the same array
- * and leaves the last call's contents in it (the bin counters are cleared each call,
- * all other regions are rewritten before they are read), so calls that overlap on
- * the GPU -- from two streams or two host threads -- race: serialise them. */
+ * and leaves the last call's contents in it (every region is rewritten before it is
+ * read), so calls that overlap on the GPU -- from two streams or two host threads -- race: serialise them. */
 int moil_nb_pme_noalloc(const double *d_coor, const double *d_q, int natom, const double *box,
                         const int *grid, double alpha, double eps, double *d_dpot, double *e_recip,
                         void *stream);

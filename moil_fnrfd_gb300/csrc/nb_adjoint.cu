@@ -5,7 +5,8 @@
 // One evaluation (moil_nb_eval semantics) leaves the lists, the site-ordered positions and
 // the PME grid on the device (the real potential planes on the mixed path, the convolved
 // spectrum on the plain path, whose inverse plane kernel then gives each site's potential
-// shares); these kernels then accumulate, in FP64:
+// shares); these kernels then accumulate (FP64; mixed path: pair sums and the grid's part as hi + lo FP32
+// pairs):
 //   dE/dq_i     = sum over i's real-space partners of k q_j erfc(alpha r)/r
 //               - sum over i's excluded partners of k q_j erf(alpha r)/r
 //               + 1-4 Coulomb p14(3)/(q_i r) + fc * sum(theta * potential grid)

@@ -1296,7 +1296,7 @@ void nb_pme_fp32_consts(RepDev *R)
 // FFT+gather kernels as the handle path (FP32), with every scratch buffer carved out of one
 // file-scope device array.  The array is sized for at most NA_MAX_ATOMS atoms and PME
 // grids of at most NA_MAX_N points per side; every GPU that loads this library holds it
-// (about 7.5 MB) until the process exits.
+// (about 5.6 MB) until the process exits.
 
 namespace {
 

@@ -845,11 +845,11 @@ __global__ void __launch_bounds__(HB, 512 / HB) k_water_h(const int2 *__restrict
 
 // One warp per non-water atom over its full site list: the lanes take the list's entries in turn
 // (consecutive entries are mostly the sites of one water, so the position loads coalesce) and
-// their partial gradients and energies are summed over the warp at the end, energies as hi + lo
-// pairs.  One atom per thread ran its ~600 entries in series: 486 us for 2,496 atoms, 363 us for
+// their partial gradients and energies are summed over the warp at the end; every pair's energies and LJ
+// virial go into hi + lo pairs (two_add2).  One atom per thread ran its ~600 entries in series: 486 us for 2,496 atoms, 363 us for
 // 203.  Bound: instruction issue; with the constants loaded again for every pair and six hi + lo
-// sums per pair 19,968 atoms took 90 us, with held constants, records one entry ahead and six blocks
-// per multiprocessor 68.
+// sums per pair 19,968 atoms took 90 us, with held constants, records one entry ahead, six blocks per
+// multiprocessor and the sums two at once 71 (68 with FP32 sums of 16 pairs between).
 #define CHUNK_ATOM 16
 __global__ void __launch_bounds__(128, 6) k_atom_f(int nA, int nW, const RepDev *__restrict__ reps,
                                                 const int *__restrict__ site_rep, const float4 *__restrict__ pos,
