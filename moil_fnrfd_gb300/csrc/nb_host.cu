@@ -232,11 +232,11 @@ int alloc_half(NbCtx *c)
 // half / full lists: 216 waters 75 / 46, 1,334 94 / 52, 7,000 102 / 68, 12,000 105 / 79, 28,800 (16
 // replicas) 130 / 125, 32,000 149 / 154, 110,860 (64 replicas) 340 / 371.
 // The half-list kernel runs a water's list of atoms outside waters in one thread, the full-list one shares
-// it among the lanes.  A few ions change nothing (24 replicas, 40,800 waters, 1 entry per water 193 /
-// 211; 256 replicas 1296 / 1497, 13 entries 1523 / 1794).  A solute gathers its entries at the waters around
+// it among the lanes.  A few ions change nothing (24 replicas, 40,800 waters, 4 entries per water 205 /
+// 222; 256 replicas 1399 / 1632, 13 entries 1531 / 1798).  A solute gathers its entries at the waters around
 // it, and the longest list sets the time until there are blocks enough to hide it: 24 replicas (39,400
-// waters) with 30 entries per water 298 / 278, 5 solute systems (35,100) with 59 353 / 290, 8 (56,160)
-// 442 / 452, 24 1097 / 1158.
+// waters) with 30 entries per water 291 / 273, 5 solute systems (35,100) with 59 357 / 290, 8 (56,160)
+// 417 / 430, 24 1108 / 1158.
 #define NB_FULL_MAX_WATERS 30000
 #define NB_FULL_MAX_WATERS_SOLUTE 50000
 bool auto_full(const NbCtx *c)
