@@ -55,3 +55,18 @@ def test_long_atom_lists_match_oracle(filler):
         assert rel_rms(dps[0][-w - 9:-w], ref[-w - 9:-w]) <= 1e-5          # the waters in the holes
         assert all(abs(es[0][k] - eref[k]) <= 1e-6 * scale for k in ENERGY_TERMS + ("e_total",))
     nb.close()
+
+
+def test_group_without_atoms_gives_the_same_bits():
+    """Water boxes in a replica group of their own beside a group with the solute: the kernels are chosen by what
+    the whole handle holds."""
+    s = waters_in_a_dense_solute()[0]
+    box = S.water_box(800, (800 / S.WATER_DENSITY) ** (1 / 3), 10)
+    out = []
+    for groups in (1, 2):
+        nb = Nonbonded([s, box], groups=groups)
+        assert nb.groups() == groups
+        dps, es = nb.eforce()
+        out.append((np.concatenate(dps), [e["e_total"] for e in es]))
+        nb.close()
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
